@@ -18,6 +18,7 @@
 #include "homs_internal.cuh"
 #include "homs_kspace.cuh"
 #include "homs_phantom.cuh"
+#include "homs_precess64.cuh"
 #include "homs_split.cuh"
 
 using namespace homs;
@@ -134,6 +135,9 @@ struct homs_context {
     std::mutex mu;
     // reusable scratch
     DevBuf scratch_csm, scratch_partial, scratch_acc, scratch_bnd, scratch_sig, scratch_conv;
+    // FP64 precession blocks: sample index per node, column sources, spin table,
+    // prefix table, aligned copy of the state
+    DevBuf block_rank, block_src, block_table, block_prefix, block_xy;
     // encoding export (homs_kspace): staged inputs, metadata, work and outputs,
     // and the events around its kernels
     DevBuf kspace_in, kspace_meta, kspace_work, kspace_out;
@@ -400,8 +404,11 @@ struct Resident : ResidentBase {
     double gamma = 0;
     SplitResident split;  // split-precision operands (built on demand)
     bool split_ready = false;
-    // Split-path tables of the sequence: the global ADC sample index of every
-    // node, and the 17 prefix-table column sources of `src_method`.
+    // Plain FP64 precession: the phantom's spin table and the prefix table of a segment.
+    DevBuf spin_table, prefix;
+    bool spin_table_ready = false;
+    // Prefix-table inputs of the sequence: the global ADC sample index of every
+    // node, and the 17 column sources of `src_method`.
     DevBuf grank, src_table;
     bool grank_ready = false;
     uint32_t src_method = ~0u;
@@ -430,7 +437,8 @@ struct Resident : ResidentBase {
     size_t device_bytes() const override {
         size_t b = x.bytes + y.bytes + z.bytes + rho.bytes + T1.bytes + T2.bytes + dw.bytes + csm_rows.bytes + t.bytes +
                    dt.bytes + gx.bytes + gy.bytes + gz.bytes + b1.bytes + df.bytes + psi.bytes + adc.bytes + bnd.bytes +
-                   xy.bytes + mz.bytes + acc.bytes + rho_init.bytes + partial.bytes + sig.bytes + split.device_bytes();
+                   xy.bytes + mz.bytes + acc.bytes + rho_init.bytes + partial.bytes + sig.bytes + spin_table.bytes +
+                   prefix.bytes + split.device_bytes();
         for (int k = 0; k < 16; ++k) b += h[k].bytes;
         return b;
     }
@@ -476,6 +484,7 @@ namespace {
 template <typename T>
 void fill_phantom(homs_context *ctx, Resident<T> *r, const homs_phantom *p) {
     r->split_ready = false;
+    r->spin_table_ready = false;
     r->dtype = sizeof(T) == 8 ? HOMS_F64 : HOMS_F32;
     r->ns = p->nspins;
     r->nc = p->ncoils;
@@ -510,6 +519,8 @@ void attach_phantom(Resident<T> *r, const Resident<T> &src) {
         HOMS_CUDA(split_attach(r->split, src.split));
         r->split_ready = true;
     }
+    r->spin_table_ready = src.spin_table_ready;
+    if (src.spin_table_ready) r->spin_table.view(src.spin_table);
 }
 
 // Upload a sampled sequence and size the run's state and signal buffers for
@@ -630,6 +641,78 @@ std::vector<std::pair<Launch, T>> plan_plain(const Resident<T> &r, int64_t max_s
     return out;
 }
 
+// The prefix table's inputs: the global ADC sample index of every
+// owned node (blocks share boundary nodes; a node belongs to the block that
+// ends on it) and the prefix-table column sources of `method`.  Uploaded
+// from the host only when the sequence or the method changed.
+template <typename T>
+void ensure_prefix_tables(homs_context *ctx, Resident<T> &r, uint32_t method) {
+    if (!r.grank_ready) {
+        std::vector<int32_t> g((size_t)r.nt, 0);
+        int64_t c = 0;
+        for (size_t k = 0; k < r.first.size(); ++k)
+            for (int64_t n = r.first[k] + 1; n <= r.last[k]; ++n) {
+                g[(size_t)n] = (int32_t)c;
+                if (r.adc_host[(size_t)n]) ++c;
+            }
+        HOMS_REQUIRE(c <= INT32_MAX, "too many ADC samples for one run");
+        HOMS_CUDA(r.grank.ensure(sizeof(int32_t) * (size_t)r.nt));
+        HOMS_CUDA(cudaMemcpyAsync(r.grank.p, g.data(), sizeof(int32_t) * (size_t)r.nt, cudaMemcpyHostToDevice,
+                                  ctx->stream));
+        r.grank_ready = true;
+    }
+    if (r.src_method != method) {
+        const void *h[16];
+        for (int k = 0; k < 16; ++k) h[k] = r.h[k].p;
+        const void *src[17];
+        split_column_sources(method, h, r.gx.p, r.gy.p, r.gz.p, src);
+        HOMS_CUDA(r.src_table.ensure(sizeof(src)));
+        HOMS_CUDA(cudaMemcpyAsync(r.src_table.p, src, sizeof(src), cudaMemcpyHostToDevice, ctx->stream));
+        r.src_method = method;
+    }
+}
+
+// The plain FP64 path's spin table, unless `r` has it, its own or a resident phantom's.
+inline void ensure_spin_table(homs_context *ctx, Resident<double> &r) {
+    if (r.spin_table_ready) return;
+    HOMS_CUDA(r.spin_table.ensure(precess64_table_bytes(r.ns)));
+    HOMS_CUDA(precess64_table(r.x.as<double>(), r.y.as<double>(), r.z.as<double>(), r.dw.as<double>(),
+                              r.T2.as<double>(), r.ns, r.spin_table.p, ctx->stream));
+    r.spin_table_ready = true;
+}
+
+// One plain FP64 precession segment (intervals [n_lo, n_hi), `nsamples` samples from sample0 on).
+inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t method, bool capture, int64_t n_lo,
+                            int64_t n_hi, int64_t sample0, int64_t nsamples) {
+    HOMS_CUDA(r.prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nsamples)));
+    HOMS_CUDA(split_prefix_launch(r.dt.as<double>(), r.src_table.as<const void *>(), r.adc.as<uint8_t>(),
+                                  r.grank.as<int32_t>(), n_lo, n_hi, sample0, nsamples, r.gamma,
+                                  r.prefix.as<double>(), ctx->stream));
+    r.launches += 2;
+    const Precess64Plan pp = precess64_plan(r.ns, r.nc, nsamples);
+    HOMS_CUDA(r.partial.ensure(pp.partial_bytes));
+    Precess64Args a;
+    a.ns = r.ns;
+    a.nsamples = nsamples;
+    a.nc = r.nc;
+    a.method = method;
+    a.table = r.spin_table.p;
+    a.prefix = r.prefix.as<double>();
+    a.csm_rows = r.csm_rows.as<cplx<double>>();
+    a.T1 = r.T1.as<double>();
+    a.T2 = r.T2.as<double>();
+    a.rho = r.rho.as<double>();
+    a.xy = r.xy.as<cplx<double>>();
+    a.mz = r.mz.as<double>();
+    a.partial = r.partial.as<cplx<double>>();
+    a.sig = r.sig.as<cplx<double>>() + sample0;
+    a.ldsig = r.nadc;
+    std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
+    if (nsamples > 0) ev = r.next_events();
+    HOMS_CUDA(precess64_run(a, pp, ev.first, ev.second, capture ? cudaEventRecordExternal : cudaEventRecordDefault,
+                            &r.launches, ctx->stream));
+}
+
 template <typename T>
 void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture) {
     const unsigned ev_flags = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -640,13 +723,37 @@ void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture)
     max_samples = std::min<int64_t>(max_samples, std::max<int64_t>(r.nadc, 1));
     auto plan = plan_plain<T>(r, max_samples);
     int64_t need = 0;
-    for (auto &pl : plan) need = std::max(need, pl.first.nsamples);
+    for (auto &pl : plan)
+        if (sizeof(T) == 4 || pl.first.rf) need = std::max(need, pl.first.nsamples);
+    if constexpr (sizeof(T) == 8) {
+        if (capture) {
+            HOMS_REQUIRE(r.spin_table_ready && r.grank_ready && r.src_method == method,
+                         "internal: precession tables missing under capture");
+        } else {
+            ensure_spin_table(ctx, r);
+            ensure_prefix_tables<T>(ctx, r, method);
+        }
+    }
     HOMS_CUDA(r.partial.ensure(row_bytes * (size_t)std::max<int64_t>(need, 1)));
     PhantomDev<T> p = r.phantom();
     SeqDev<T> q = r.seq();
     StateDev<T> st{reinterpret_cast<cplx<T> *>(r.xy.p), reinterpret_cast<T *>(r.mz.p), reinterpret_cast<T *>(r.acc.p)};
-    for (auto &pl : plan) {
+    for (size_t i = 0; i < plan.size(); ++i) {
+        const auto &pl = plan[i];
         const Launch &L = pl.first;
+        if constexpr (sizeof(T) == 8) {
+            if (!L.rf) {
+                // a run's precession launches are one segment
+                int64_t n_hi = L.n_hi, nsamples = L.nsamples;
+                while (i + 1 < plan.size() && plan[i + 1].first.run == L.run) {
+                    ++i;
+                    n_hi = plan[i].first.n_hi;
+                    nsamples += plan[i].first.nsamples;
+                }
+                plain_segment64(ctx, r, method, capture, L.n_lo, n_hi, L.sample0, nsamples);
+                continue;
+            }
+        }
         SegmentArgs<T> a;
         a.n_lo = L.n_lo;
         a.n_hi = L.n_hi;
@@ -704,37 +811,6 @@ void check_split(homs_context *ctx, Resident<T> &r) {
     HOMS_CUDA(split_check(r.split, ctx->stream, &err));
     if (!err.empty())
         throw Failure{err.find("timed out") != std::string::npos ? HOMS_ETIMEDOUT : HOMS_EUNSUPPORTED, err};
-}
-
-// The split path's sequence tables: the global ADC sample index of every
-// owned node (blocks share boundary nodes; a node belongs to the block that
-// ends on it) and the prefix-table column sources of `method`.  Uploaded
-// from the host only when the sequence or the method changed.
-template <typename T>
-void ensure_split_tables(homs_context *ctx, Resident<T> &r, uint32_t method) {
-    if (!r.grank_ready) {
-        std::vector<int32_t> g((size_t)r.nt, 0);
-        int64_t c = 0;
-        for (size_t k = 0; k < r.first.size(); ++k)
-            for (int64_t n = r.first[k] + 1; n <= r.last[k]; ++n) {
-                g[(size_t)n] = (int32_t)c;
-                if (r.adc_host[(size_t)n]) ++c;
-            }
-        HOMS_REQUIRE(c <= INT32_MAX, "too many ADC samples for the split path");
-        HOMS_CUDA(r.grank.ensure(sizeof(int32_t) * (size_t)r.nt));
-        HOMS_CUDA(cudaMemcpyAsync(r.grank.p, g.data(), sizeof(int32_t) * (size_t)r.nt, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-        r.grank_ready = true;
-    }
-    if (r.src_method != method) {
-        const void *h[16];
-        for (int k = 0; k < 16; ++k) h[k] = r.h[k].p;
-        const void *src[17];
-        split_column_sources(method, h, r.gx.p, r.gy.p, r.gz.p, src);
-        HOMS_CUDA(r.src_table.ensure(sizeof(src)));
-        HOMS_CUDA(cudaMemcpyAsync(r.src_table.p, src, sizeof(src), cudaMemcpyHostToDevice, ctx->stream));
-        r.src_method = method;
-    }
 }
 
 // One split-mode run of the block plan, issued in steps so that several
@@ -914,7 +990,7 @@ void run_resident(homs_context *ctx, Resident<T> &r, const homs_run_options *opt
                          "internal: split tables missing under capture");
         } else {
             ensure_split<T>(ctx, r);
-            ensure_split_tables<T>(ctx, r, method);
+            ensure_prefix_tables<T>(ctx, r, method);
         }
         HOMS_CUDA(split_reset_error(r.split, ctx->stream));
         SplitRunner<T> run;
@@ -1177,6 +1253,11 @@ homs_status homs_context_destroy(homs_context *ctx) {
         ctx->scratch_bnd.release();
         ctx->scratch_sig.release();
         ctx->scratch_conv.release();
+        ctx->block_rank.release();
+        ctx->block_src.release();
+        ctx->block_table.release();
+        ctx->block_prefix.release();
+        ctx->block_xy.release();
         ctx->kspace_in.release();
         ctx->kspace_meta.release();
         ctx->kspace_work.release();
@@ -1339,6 +1420,66 @@ homs_status homs_plan_destroy(homs_plan *plan) {
 
 namespace {
 
+// A precession block of caller device arrays in FP64: its tables are built in
+// the context's scratch, then it runs as a segment of its own.  `adc`: the
+// flags of nodes first + 1 .. last.
+void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDev<double> &q, const homs_state &state,
+                     int64_t first, int64_t last, uint32_t method, double gamma, const std::vector<uint8_t> &adc,
+                     int64_t nadc, void *sig, int64_t ldsig) {
+    // Sample index of the block's nodes (indexed by node) and the column sources.
+    std::vector<int32_t> rank((size_t)(last - first));
+    int32_t c = 0;
+    for (size_t i = 0; i < adc.size(); ++i) {
+        rank[i] = c;
+        if (adc[i]) ++c;
+    }
+    const void *h[16], *src[17];
+    for (int k = 0; k < 16; ++k) h[k] = q.h[k];
+    split_column_sources(method, h, q.gx, q.gy, q.gz, src);
+    HOMS_CUDA(ctx->block_rank.ensure(sizeof(int32_t) * rank.size()));
+    HOMS_CUDA(ctx->block_src.ensure(sizeof(src)));
+    HOMS_CUDA(ctx->block_table.ensure(precess64_table_bytes(p.ns)));
+    HOMS_CUDA(ctx->block_prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nadc)));
+    HOMS_CUDA(cudaMemcpyAsync(ctx->block_rank.p, rank.data(), sizeof(int32_t) * rank.size(), cudaMemcpyHostToDevice,
+                              ctx->stream));
+    HOMS_CUDA(cudaMemcpyAsync(ctx->block_src.p, src, sizeof(src), cudaMemcpyHostToDevice, ctx->stream));
+    HOMS_CUDA(precess64_table(p.x, p.y, p.z, p.dw, p.T2, p.ns, ctx->block_table.p, ctx->stream));
+    // the prefix kernel looks ranks up by node
+    HOMS_CUDA(split_prefix_launch(q.dt, ctx->block_src.as<const void *>(), q.adc,
+                                  ctx->block_rank.as<int32_t>() - (first + 1), first, last, 0, nadc, gamma,
+                                  ctx->block_prefix.as<double>(), ctx->stream));
+    const Precess64Plan pp = precess64_plan(p.ns, p.nc, nadc);
+    HOMS_CUDA(ctx->scratch_partial.ensure(pp.partial_bytes));
+    // The kernels read and write the state as 16-byte pairs: a caller's array off
+    // that boundary goes through a copy.
+    cplx<double> *xy = static_cast<cplx<double> *>(state.xy);
+    const size_t xy_bytes = sizeof(cplx<double>) * (size_t)p.ns;
+    const bool aligned = (reinterpret_cast<uintptr_t>(state.xy) & 15) == 0;
+    if (!aligned) {
+        HOMS_CUDA(ctx->block_xy.ensure(xy_bytes));
+        xy = ctx->block_xy.as<cplx<double>>();
+        HOMS_CUDA(cudaMemcpyAsync(xy, state.xy, xy_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+    Precess64Args a;
+    a.ns = p.ns;
+    a.nsamples = nadc;
+    a.nc = p.nc;
+    a.method = method;
+    a.table = ctx->block_table.p;
+    a.prefix = ctx->block_prefix.as<double>();
+    a.csm_rows = p.csm;
+    a.T1 = p.T1;
+    a.T2 = p.T2;
+    a.rho = p.rho;
+    a.xy = xy;
+    a.mz = static_cast<double *>(state.z);
+    a.partial = ctx->scratch_partial.as<cplx<double>>();
+    a.sig = static_cast<cplx<double> *>(sig);
+    a.ldsig = ldsig;
+    HOMS_CUDA(precess64_run(a, pp, nullptr, nullptr, cudaEventRecordDefault, nullptr, ctx->stream));
+    if (!aligned) HOMS_CUDA(cudaMemcpyAsync(state.xy, xy, xy_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+}
+
 template <typename T>
 homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const homs_sequence *q, int64_t first,
                        int64_t last, uint32_t method, homs_state *state, void *sig, int64_t ldsig) {
@@ -1364,10 +1505,6 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     const uint8_t one = 1;
     HOMS_CUDA(cudaMemcpyAsync(reinterpret_cast<uint8_t *>(ctx->scratch_bnd.p) + last, &one, 1, cudaMemcpyHostToDevice, ctx->stream));
     upload_csm_rows<T>(ctx, ctx->scratch_csm, p->csm, p->dtype, HOMS_DEVICE, ns, nc, ns);
-    HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
-    const int grid = (int)((ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-    HOMS_CUDA(ctx->scratch_partial.ensure(sizeof(cplx<T>) * (size_t)grid * (size_t)std::max<int64_t>(nadc, 1) * nc));
-    HOMS_CUDA(ctx->scratch_sig.ensure(sizeof(cplx<T>) * (size_t)std::max<int64_t>(nadc, 1) * nc));
     PhantomDev<T> pd{ns, nc, (const T *)p->x, (const T *)p->y, (const T *)p->z, (const T *)p->rho, (const T *)p->T1,
                      (const T *)p->T2, (const T *)p->dw, reinterpret_cast<cplx<T> *>(ctx->scratch_csm.p), nc};
     SeqDev<T> qd;
@@ -1383,6 +1520,16 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     qd.adc = q->adc;
     qd.boundary = reinterpret_cast<uint8_t *>(ctx->scratch_bnd.p);
     for (int k = 0; k < 16; ++k) qd.h[k] = (const T *)q->h[k];
+    if constexpr (sizeof(T) == 8) {
+        if (!rf) {
+            block_precess64(ctx, pd, qd, *state, first, last, method, q->gamma, adc, nadc, sig, ldsig);
+            return HOMS_OK;
+        }
+    }
+    HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
+    const int grid = (int)((ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
+    HOMS_CUDA(ctx->scratch_partial.ensure(sizeof(cplx<T>) * (size_t)grid * (size_t)std::max<int64_t>(nadc, 1) * nc));
+    HOMS_CUDA(ctx->scratch_sig.ensure(sizeof(cplx<T>) * (size_t)std::max<int64_t>(nadc, 1) * nc));
     StateDev<T> st{(cplx<T> *)state->xy, (T *)state->z, reinterpret_cast<T *>(ctx->scratch_acc.p)};
     SegmentArgs<T> a;
     a.n_lo = first;
@@ -1499,6 +1646,7 @@ homs_status homs_resident_create(homs_context *ctx, const homs_phantom *phantom,
             auto r = std::make_unique<Resident<double>>();
             fill_phantom<double>(ctx, r.get(), phantom);
             if (mode == HOMS_SPLIT) ensure_split<double>(ctx, *r);
+            else ensure_spin_table(ctx, *r);
             h->res = std::move(r);
         } else {
             auto r = std::make_unique<Resident<float>>();
@@ -1922,7 +2070,7 @@ homs_status server_run_prepare(homs_context *ctx, const homs_phantom *phantom, c
         }
         init_state<double>(ctx, *r, state, run->out_dt);
         ensure_split<double>(ctx, *r);
-        ensure_split_tables<double>(ctx, *r, opts->method);
+        ensure_prefix_tables<double>(ctx, *r, opts->method);
         HOMS_CUDA(split_reset_error(r->split, ctx->stream));
         r->events_used = 0;
         r->launches = 0;

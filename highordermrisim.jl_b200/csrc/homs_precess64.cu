@@ -1,0 +1,458 @@
+// Free precession in FP64, in parallel over time and spins.
+//
+// Within a segment (a run of precession blocks) the field is a sum of 16 terms
+// per spin times one coefficient waveform each, so the phase at sample j is
+//   theta(s, j) = kappa_0(j) + sum_k b_k(s) kappa_k(j)   (turns)
+// with kappa_k the running trapezoid integral of waveform k from the segment
+// start (the prefix table of homs_split.cu; trapezoid and decay as
+// src/simulation/Bloch/BlochHighOrderSimulatitonMethod.jl:76-92), and
+//   M(s, j) = m0(s) exp(-t_j / T2(s)) cis(2 pi theta),   S(j, c) = sum_s M csm.
+// No sample depends on another one, so samples spread over CTAs; a walk node by
+// node leaves a small phantom's few CTAs waiting on one dependent chain.  The
+// blocks of a run only restart the same exponentials, so a run is one segment.
+//
+// What bounds it: the FP64 pipe (64 multiply-adds per SM and clock, the same
+// for DFMA and for the FP64 matrix instruction; the pipe is about 72% busy).
+// Per spin and sample 16 multiply-adds of phase, 41 FP64 operations of sine,
+// cosine, decay and the complex product, 3 per coil of contraction.
+//
+// Organisation: CTA = 8 warps, a tile of samples x a range of 32-spin chunks
+// (cp.async, NSTAGE stages).  A warp owns 16 samples (8 for more than 16
+// coils, whose sums would not fit beside them: 5.60 against 5.74 ms at 32
+// coils) and keeps their kappa rows and coil sums in registers.  Both
+// contractions are m8n8k4 FP64 matrix instructions: the phase as (samples x
+// terms) (terms x spins), whose result fragment (sample lane / 4, spins
+// 2 (lane % 4) + {0, 1}) is, taken one spin parity at a time, exactly the A
+// fragment of the coil product (samples x spins) (spins x coils), so M never
+// leaves its registers.  The complex product takes three real ones: k1 = (Re M + Im M) Re c, k2 = Re M (Im c - Re c),
+// k3 = Im M (Re c + Im c); Re = k1 - k3, Im = k1 + k2 (10.87 -> 10.31 ms at 8
+// coils, 6.15 -> 5.86 ms at 32).  wj < 8 (segments of few samples): the other
+// warps take other spin groups of the chunk and write partial sums of their own.
+//
+// Measured (B200, prepared runs, against the sequential per-spin kernel that it
+// replaces): 40,000 spins x 4 segments of 10,000 samples x 8 coils 44.6 ->
+// 10.3 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.9 ms.  Three
+// CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
+#include <algorithm>
+
+#include "homs_precess64.cuh"
+#include "homs_split.cuh"
+
+namespace homs {
+
+namespace precess64 {
+
+constexpr int THREADS = 256;
+__host__ __device__ constexpr int mtiles(int nt) { return nt == 4 ? 1 : 2; }  // 8-sample tiles per warp
+constexpr int CHUNK = 32;    // spins per stage
+constexpr int NSTAGE = 3;
+constexpr int TERMS = 16;    // phase slots: basis terms 1..15, dw/(2 pi)
+constexpr int GROUP = 32;    // coils per launch slice
+constexpr int BROW = 144;    // bytes of a staged basis row (128 + 16: conflict-free fragment loads)
+constexpr double TWO_PI = 2.0 * 3.141592653589793;
+
+__host__ __device__ constexpr int csm_row(int nt) { return nt * 128 + 16; }  // bytes of a staged sensitivity row
+__host__ __device__ constexpr int stage_bytes(int nt) { return CHUNK * (BROW + 16 + 8 + csm_row(nt)); }
+
+__host__ __device__ inline int64_t pad_spins(int64_t ns) { return (ns + CHUNK - 1) / CHUNK * CHUNK; }
+
+// Phase slots switched on by a method (slot k: basis term k + 1, slot 15: dw).
+__host__ __device__ inline uint32_t slot_mask(uint32_t method) {
+    uint32_t m = 0x7u;  // first order: the field coefficients or the nominal gradients
+    if (method & HOMS_HO2) m |= 0xF8u;
+    if (method & HOMS_HO3) m |= 0x7F00u;
+    if (method & HOMS_DW_PRECESSION) m |= 0x8000u;
+    return m;
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+// cos and sin of 2 pi theta.  theta is reduced to its nearest quarter turn (an
+// exact subtraction); on [-1/8, 1/8] turn sin(2 pi r) / r is a polynomial of
+// degree 6 and (cos(2 pi r) - 1) / r^2 one of degree 6 in r^2, the interpolants
+// at the Chebyshev nodes of the interval (relative error 4e-18 before the
+// coefficients' rounding); 18 FP64 operations.  Beyond 2^48 turns (infinities
+// and NaN included) theta is first reduced to the nearest turn.
+__device__ __forceinline__ void cis_turns(double th, double &cs, double &sn) {
+    if ((__double2hiint(th) & 0x7FFFFFFF) >= 0x42F00000) th -= rint(th);
+    constexpr double MAGIC = 6755399441055744.0;  // 1.5 * 2^52: adds round to an integer
+    const double t = fma(th, 4.0, MAGIC);
+    const int quad = __double2loint(t);
+    const double r = fma(t - MAGIC, -0.25, th), z = r * r;
+    double s = 3.7808689593022957, c = -1.6990343940660637;
+    s = fma(s, z, -15.093804209987114);
+    c = fma(c, z, 7.903206911569678);
+    s = fma(s, z, 42.058685020160894);
+    c = fma(c, z, -26.426253275854723);
+    s = fma(s, z, -76.70585970427454);
+    c = fma(c, z, 60.24464135270201);
+    s = fma(s, z, 81.60524927594804);
+    c = fma(c, z, -85.4568172066438);
+    s = fma(s, z, -41.341702240399634);
+    c = fma(c, z, 64.93939402266824);
+    s = fma(s, z, 6.283185307179586);
+    c = fma(c, z, -19.739208802178716);
+    s = s * r;
+    c = fma(c, z, 1.0);
+    // a quarter turn swaps the two and a half turn flips both signs
+    const double a = (quad & 1) ? s : c, b = (quad & 1) ? c : s;
+    cs = __hiloint2double(__double2hiint(a) ^ (((quad + 1) & 2) << 30), __double2loint(a));
+    sn = __hiloint2double(__double2hiint(b) ^ ((quad & 2) << 30), __double2loint(b));
+}
+
+// 2^y: nearest integer k, then 1 + f q(f) on |f| <= 1/2 with q the degree-10
+// interpolant of (2^f - 1) / f at the Chebyshev nodes (relative error 1e-17 before
+// the coefficients' rounding), and k added to the exponent; 15 FP64 operations.
+// |y| >= 1008 (infinities and NaN included) goes to exp2.
+__device__ __forceinline__ double pow2(double y) {
+    if ((__double2hiint(y) & 0x7FFFFFFF) >= 0x408F8000) return exp2(y);
+    constexpr double MAGIC = 6755399441055744.0;
+    const double t = y + MAGIC;
+    const int k = __double2loint(t);
+    const double f = y - (t - MAGIC);
+    double p = 4.4549605981865186e-10;
+    p = fma(p, f, 7.072585949269223e-09);
+    p = fma(p, f, 1.0178062445845774e-07);
+    p = fma(p, f, 1.321544258792169e-06);
+    p = fma(p, f, 1.525273382983612e-05);
+    p = fma(p, f, 0.0001540353044173605);
+    p = fma(p, f, 0.0013333558146416936);
+    p = fma(p, f, 0.009618129107606888);
+    p = fma(p, f, 0.0555041086648216);
+    p = fma(p, f, 0.24022650695910097);
+    p = fma(p, f, 0.6931471805599453);
+    p = fma(p, f, 1.0);
+    return __hiloint2double(__double2hiint(p) + (k << 20), __double2loint(p));
+}
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+__global__ void table_kernel(const double *x, const double *y, const double *z, const double *dw, const double *T2,
+                             int64_t ns, int64_t ns_pad, double *basis, double *r2) {
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < ns_pad; s += (int64_t)gridDim.x * blockDim.x) {
+        double b[TERMS] = {};
+        double r = 0.0;
+        if (s < ns) {
+            const double X = x[s], Y = y[s], Z = z[s];
+            const double x2 = X * X, y2 = Y * Y, z2 = Z * Z;
+            const double q = (x2 + y2) + z2;
+            b[0] = X;
+            b[1] = Y;
+            b[2] = Z;
+            b[3] = X * Y;
+            b[4] = Z * Y;
+            b[5] = 3.0 * z2 - q;
+            b[6] = X * Z;
+            b[7] = x2 - y2;
+            b[8] = (3.0 * Y) * x2 - (y2 * Y);
+            b[9] = (X * Z) * Y;
+            b[10] = (5.0 * z2 - q) * Y;
+            b[11] = 5.0 * (z2 * Z) - (3.0 * Z) * q;
+            b[12] = (5.0 * z2 - q) * X;
+            b[13] = x2 * Z - y2 * Z;
+            b[14] = (x2 * X) - (3.0 * X) * y2;
+            b[15] = dw[s] / TWO_PI;
+            r = -1.4426950408889634 / T2[s];
+        }
+        double2 *out = reinterpret_cast<double2 *>(basis + s * TERMS);
+#pragma unroll
+        for (int k = 0; k < TERMS / 2; ++k) out[k] = make_double2(b[2 * k], b[2 * k + 1]);
+        r2[s] = r;
+    }
+}
+
+struct KernelArgs {
+    int64_t ns, nsamples, sample0, nchunks;  // samples sample0 + [0, tiles of the round)
+    int64_t round_samples;                   // samples of the round (rows of a partial block)
+    int32_t nc, parts;
+    uint32_t slots;
+    const double *basis, *r2, *prefix;
+    const cplx<double> *xy, *csm_rows;
+    cplx<double> *partial;
+};
+
+// NT: 8-coil tiles (at most GROUP coils per z slice); WJ: warps along the samples.
+template <int NT, int WJ>
+__global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
+    constexpr int CS = csm_row(NT), STAGE = stage_bytes(NT), KSPLIT = 8 / WJ, MT = mtiles(NT);
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, r = lane >> 2;
+    const int wj = warp % WJ, kw = warp / WJ;
+    const int c0 = (int)blockIdx.z * GROUP;
+    const int ncg = min(GROUP, a.nc - c0);
+    const int64_t ch0 = a.nchunks * blockIdx.y / a.parts, ch1 = a.nchunks * (blockIdx.y + 1) / a.parts;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+
+    // Sensitivity columns past the last coil are zero in every stage.
+    if (ncg < NT * 8) {
+        const int extra = NT * 8 - ncg;
+        for (int i = tid; i < NSTAGE * CHUNK * extra; i += THREADS) {
+            const int row = i / extra, col = ncg + i % extra;
+            *reinterpret_cast<double2 *>(smem + (row / CHUNK) * STAGE + CHUNK * (BROW + 24) + (row % CHUNK) * CS +
+                                         col * 16) = make_double2(0.0, 0.0);
+        }
+    }
+    auto issue = [&](int64_t ch, int stage) {
+        const uint32_t st = sbase + (uint32_t)(stage * STAGE);
+        const int64_t s0 = ch * CHUNK;
+        {
+            const int spin = tid >> 3, piece = tid & 7;
+            cp16(st + spin * BROW + piece * 16, a.basis + (s0 + spin) * TERMS + piece * 2, true);
+        }
+        if (tid < CHUNK) {
+            const bool ok = s0 + tid < a.ns;
+            cp16(st + CHUNK * BROW + tid * 16, a.xy + (ok ? s0 + tid : 0), ok);
+        } else if (tid < CHUNK + CHUNK / 2) {
+            const int p = tid - CHUNK;
+            cp16(st + CHUNK * (BROW + 16) + p * 16, a.r2 + s0 + 2 * p, true);
+        }
+#pragma unroll
+        for (int i = 0; i < CHUNK * NT * 8 / THREADS; ++i) {
+            const int p = tid + i * THREADS, spin = p / (NT * 8), coil = p % (NT * 8);
+            if (coil < ncg) {
+                const bool ok = s0 + spin < a.ns;
+                cp16(st + CHUNK * (BROW + 24) + spin * CS + coil * 16,
+                     a.csm_rows + (ok ? (s0 + spin) * a.nc + c0 + coil : 0), ok);
+            }
+        }
+    };
+
+    // This warp's samples: rows 8 mt + r of its 16.  Phase slot of lane q in
+    // step i: 4 q + i (the term order of a sum is free, and this one makes a
+    // spin's fragment contiguous).
+    double kap[MT][4], k0[MT], tj[MT];
+    const int64_t jw = (int64_t)blockIdx.x * (8 * MT * WJ) + wj * (8 * MT);
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        const int64_t j = jw + mt * 8 + r;
+        const bool ok = j < a.round_samples;
+        const double *row = a.prefix + (a.sample0 + (ok ? j : 0)) * SPLIT_PREFIX_STRIDE;
+        k0[mt] = ok ? row[0] : 0.0;
+        tj[mt] = ok ? row[SPLIT_PREFIX_T] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kap[mt][i] = ok ? row[1 + 4 * q + i] : 0.0;
+    }
+    const uint32_t on = (a.slots >> (4 * q)) & 15u;
+    double k1[MT][NT][2], k2[MT][NT][2], k3[MT][NT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) k1[mt][nt][e] = k2[mt][nt][e] = k3[mt][nt][e] = 0.0;
+
+#pragma unroll
+    for (int s = 0; s < NSTAGE - 1; ++s) {
+        if (ch0 + s < ch1) issue(ch0 + s, s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int stage = 0;
+    for (int64_t ch = ch0; ch < ch1; ++ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(NSTAGE - 2) : "memory");
+        __syncthreads();
+        const int fill = stage == 0 ? NSTAGE - 1 : stage - 1;  // the stage consumed last
+        if (ch + NSTAGE - 1 < ch1) issue(ch + NSTAGE - 1, fill);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const uint8_t *st = smem + stage * STAGE;
+        if (++stage == NSTAGE) stage = 0;
+#pragma unroll 1
+        for (int g = kw; g < CHUNK / 8; g += KSPLIT) {
+            const double2 *brow = reinterpret_cast<const double2 *>(st + (g * 8 + r) * BROW + q * 32);
+            const double2 b01 = brow[0], b23 = brow[1];
+            const double b[4] = {(on & 1u) ? b01.x : 0.0, (on & 2u) ? b01.y : 0.0, (on & 4u) ? b23.x : 0.0,
+                                 (on & 8u) ? b23.y : 0.0};
+            const double2 *m0p = reinterpret_cast<const double2 *>(st + CHUNK * BROW + (g * 8 + 2 * q) * 16);
+            const double2 m0[2] = {m0p[0], m0p[1]};
+            const double2 rr = *reinterpret_cast<const double2 *>(st + CHUNK * (BROW + 16) + (g * 8 + 2 * q) * 8);
+            double th[MT][2];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) th[mt][0] = th[mt][1] = k0[mt];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) dmma(th[mt], kap[mt][i], b[i]);
+            double mr[MT][2], mi[MT][2], ms[MT][2];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    double sn, cs;
+                    cis_turns(th[mt][e], cs, sn);
+                    const double ex = pow2(tj[mt] * (e ? rr.y : rr.x));
+                    const double ec = ex * cs, es = ex * sn;
+                    mr[mt][e] = m0[e].x * ec - m0[e].y * es;
+                    mi[mt][e] = m0[e].x * es + m0[e].y * ec;
+                    ms[mt][e] = mr[mt][e] + mi[mt][e];
+                }
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    const double2 w = *reinterpret_cast<const double2 *>(st + CHUNK * (BROW + 24) +
+                                                                         (g * 8 + 2 * q + e) * CS + (nt * 8 + r) * 16);
+                    const double wd = w.y - w.x, ws = w.x + w.y;
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        dmma(k1[mt][nt], ms[mt][e], w.x);
+                        dmma(k2[mt][nt], mr[mt][e], wd);
+                        dmma(k3[mt][nt], mi[mt][e], ws);
+                    }
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    cplx<double> *out = a.partial + (size_t)(blockIdx.y * KSPLIT + kw) * a.round_samples * a.nc + c0;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        const int64_t j = jw + mt * 8 + r;
+        if (j >= a.round_samples) continue;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = nt * 8 + 2 * q + e;
+                if (c < ncg) out[j * a.nc + c] = cplx<double>{k1[mt][nt][e] - k3[mt][nt][e], k1[mt][nt][e] + k2[mt][nt][e]};
+            }
+    }
+}
+
+// State at the segment's end: the same formula at the end row of the prefix
+// table, and Mz = Mz e^{-T/T1} + rho (1 - e^{-T/T1}).
+__global__ void __launch_bounds__(256) state_kernel(const double *basis, const double *endrow, uint32_t slots,
+                                                    const double *T1, const double *T2, const double *rho, int64_t ns,
+                                                    cplx<double> *xy, double *mz) {
+    double kap[TERMS];
+#pragma unroll
+    for (int k = 0; k < TERMS; ++k) kap[k] = endrow[1 + k];
+    const double k0 = endrow[0], T = endrow[SPLIT_PREFIX_T];
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < ns; s += (int64_t)gridDim.x * blockDim.x) {
+        double th = k0;
+#pragma unroll
+        for (int k = 0; k < TERMS; ++k)
+            if ((slots >> k) & 1u) th = fma(basis[s * TERMS + k], kap[k], th);
+        double sn, cs;
+        sincospi(2.0 * (th - rint(th)), &sn, &cs);
+        const double e2 = exp(0.0 - T / T2[s]);
+        const cplx<double> m0 = xy[s];
+        const double ec = e2 * cs, es = e2 * sn;
+        xy[s] = cplx<double>{m0.re * ec - m0.im * es, m0.re * es + m0.im * ec};
+        const double e1 = exp(0.0 - T / T1[s]);
+        mz[s] = mz[s] * e1 + rho[s] * (1.0 - e1);
+    }
+}
+
+inline int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)); }
+
+// 8-coil tiles of a launch, and samples per warp, for nc coils.
+inline int coil_tiles(int32_t nc) { return nc <= 8 ? 1 : nc <= 16 ? 2 : 4; }
+inline int warp_samples(int32_t nc) { return 8 * mtiles(coil_tiles(nc)); }
+
+template <int NT, int WJ>
+cudaError_t launch(const KernelArgs &ka, int64_t tiles, int groups, cudaStream_t stream) {
+    cudaError_t e = allow_max_dynamic_smem((const void *)main_kernel<NT, WJ>);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned)tiles, (unsigned)ka.parts, (unsigned)groups);
+    main_kernel<NT, WJ><<<grid, THREADS, NSTAGE * stage_bytes(NT), stream>>>(ka);
+    return cudaGetLastError();
+}
+template <int NT>
+cudaError_t launch(int wj, const KernelArgs &ka, int64_t tiles, int groups, cudaStream_t stream) {
+    return wj == 8 ? launch<NT, 8>(ka, tiles, groups, stream)
+                   : wj == 4 ? launch<NT, 4>(ka, tiles, groups, stream) : launch<NT, 2>(ka, tiles, groups, stream);
+}
+
+}  // namespace precess64
+
+using namespace precess64;
+
+size_t precess64_table_bytes(int64_t ns) { return sizeof(double) * (TERMS + 1) * (size_t)pad_spins(ns); }
+
+cudaError_t precess64_table(const double *x, const double *y, const double *z, const double *dw, const double *T2,
+                            int64_t ns, void *table, cudaStream_t stream) {
+    const int64_t np = pad_spins(ns);
+    double *basis = static_cast<double *>(table);
+    table_kernel<<<grid_for(np), 256, 0, stream>>>(x, y, z, dw, T2, ns, np, basis, basis + TERMS * np);
+    return cudaGetLastError();
+}
+
+Precess64Plan precess64_plan(int64_t ns, int32_t nc, int64_t nsamples) {
+    Precess64Plan p;
+    if (nsamples <= 0) return p;
+    // Sample tile: 8 warps along the samples, or fewer where that would be mostly padding.
+    const int per_warp = warp_samples(nc);
+    auto padded = [&](int wj) { return (nsamples + per_warp * wj - 1) / (per_warp * wj) * (per_warp * wj); };
+    for (int wj : {4, 2})
+        if (padded(wj) * 10 <= padded(p.wj) * 8) p.wj = wj;
+    const int tile = per_warp * p.wj, ksplit = 8 / p.wj;
+    const int64_t tiles = (nsamples + tile - 1) / tile, chunks = pad_spins(ns) / CHUNK;
+    const int64_t groups = (nc + GROUP - 1) / GROUP;
+    // Rounds: one part of a round's samples takes at most 256 MB of partial sums.
+    const size_t tile_bytes = sizeof(cplx<double>) * (size_t)ksplit * tile * nc, budget = size_t(256) << 20;
+    p.round_tiles = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)(budget / tile_bytes)));
+    // Spin parts: the waves of 2 CTAs per SM x (chunks of a CTA + 2 for its start and its sums) least.
+    const int64_t slots = 148 * 2, per_wave = p.round_tiles * groups;
+    const int64_t most = std::max<int64_t>(
+        1, std::min<int64_t>(std::min<int64_t>(chunks, 1024), (int64_t)(budget / (tile_bytes * p.round_tiles))));
+    int64_t best = INT64_MAX;
+    for (int64_t waves = 1; waves <= 8; ++waves) {
+        const int64_t n = std::max<int64_t>(1, std::min<int64_t>(most, waves * slots / per_wave));
+        const int64_t cost = ((per_wave * n + slots - 1) / slots) * ((chunks + n - 1) / n + 2);
+        if (cost < best) {
+            best = cost;
+            p.parts = (int)n;
+        }
+    }
+    p.partial_bytes = tile_bytes * p.round_tiles * p.parts;
+    return p;
+}
+
+cudaError_t precess64_run(const Precess64Args &a, const Precess64Plan &plan, cudaEvent_t ev_start,
+                          cudaEvent_t ev_stop, unsigned ev_flags, int64_t *launches, cudaStream_t stream) {
+    const int64_t np = pad_spins(a.ns);
+    const double *basis = static_cast<const double *>(a.table);
+    const uint32_t slots = slot_mask(a.method);
+    cudaError_t e;
+    if (a.nsamples > 0) {
+        const int tile = warp_samples(a.nc) * plan.wj, groups = (a.nc + GROUP - 1) / GROUP, ksplit = 8 / plan.wj;
+        const int64_t tiles = (a.nsamples + tile - 1) / tile;
+        if (ev_start) cudaEventRecordWithFlags(ev_start, stream, ev_flags);
+        for (int64_t t0 = 0; t0 < tiles; t0 += plan.round_tiles) {
+            const int64_t nt = std::min(plan.round_tiles, tiles - t0);
+            KernelArgs ka;
+            ka.ns = a.ns;
+            ka.nsamples = a.nsamples;
+            ka.sample0 = t0 * tile;
+            ka.round_samples = std::min<int64_t>(nt * tile, a.nsamples - ka.sample0);
+            ka.nchunks = np / CHUNK;
+            ka.nc = a.nc;
+            ka.parts = plan.parts;
+            ka.slots = slots;
+            ka.basis = basis;
+            ka.r2 = basis + TERMS * np;
+            ka.prefix = a.prefix;
+            ka.xy = a.xy;
+            ka.csm_rows = a.csm_rows;
+            ka.partial = a.partial;
+            e = a.nc <= 8 ? launch<1>(plan.wj, ka, nt, groups, stream)
+                          : a.nc <= 16 ? launch<2>(plan.wj, ka, nt, groups, stream)
+                                       : launch<4>(plan.wj, ka, nt, groups, stream);
+            if (e != cudaSuccess) return e;
+            if (ev_stop && t0 + plan.round_tiles >= tiles) cudaEventRecordWithFlags(ev_stop, stream, ev_flags);
+            e = launch_partial_finalize<double>(a.partial, (int64_t)plan.parts * ksplit, ka.round_samples, a.nc,
+                                                a.sig + ka.sample0, a.ldsig, stream);
+            if (e != cudaSuccess) return e;
+            if (launches) *launches += 2;
+        }
+    }
+    state_kernel<<<grid_for(a.ns), 256, 0, stream>>>(basis, a.prefix + (size_t)a.nsamples * SPLIT_PREFIX_STRIDE, slots,
+                                                     a.T1, a.T2, a.rho, a.ns, a.xy, a.mz);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+}
+
+}  // namespace homs

@@ -90,8 +90,8 @@ constexpr int TM = 128;          // samples per tile (UMMA M)
 constexpr int KC = 32;           // spins per chunk
 constexpr int NSLOT = 16;        // phase terms per spin: basis 1..15 and dw/(2 pi)
 constexpr int PHASE_DIGITS = 5;  // base-256 digits of the phase integers
-constexpr int PREFIX_STRIDE = 24;  // doubles per prefix row: kappa_0..kappa_16, t at PREFIX_T
-constexpr int PREFIX_T = 20;
+constexpr int PREFIX_STRIDE = SPLIT_PREFIX_STRIDE;  // doubles per prefix row: kappa_0..kappa_16, t at PREFIX_T
+constexpr int PREFIX_T = SPLIT_PREFIX_T;
 constexpr int GROUP_COILS = 32;  // coils per kernel pass (N <= 64 output columns)
 constexpr int NMAG_WARPS = 16;
 constexpr int MMA_WARP = 16;    // coil MMA issuer (allocates TMEM)
@@ -1584,6 +1584,18 @@ cudaError_t split_launch(const SplitJobDesc *jobs, int n_jobs, cudaStream_t stre
     return launch_precession(n_mma, ka, (unsigned)G, kernel_smem(n_mma), stream);
 }
 
+size_t split_prefix_rows(int64_t nsamples) { return (size_t)nsamples + 2 + PREFIX_PARTS; }
+
+cudaError_t split_prefix_launch(const double *dt, const void *const *src_dev, const uint8_t *adc, const int32_t *grank,
+                                int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
+                                double *prefix, cudaStream_t stream) {
+    const dim3 pgrid(PREFIX_COLS, PREFIX_PARTS);
+    const double *const *src = reinterpret_cast<const double *const *>(src_dev);
+    prefix_part_kernel<<<pgrid, 256, 0, stream>>>(dt, src, n_lo, n_hi, nsamples, gamma, prefix);
+    prefix_kernel<<<pgrid, 256, 0, stream>>>(dt, src, adc, grank, sample0, n_lo, n_hi, nsamples, gamma, prefix);
+    return cudaGetLastError();
+}
+
 // Prologue of one precession segment: the prefix table, the spin parameters
 // and amplitude scale, the phase A tiles and the work-item split.
 cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t n_lo, int64_t n_hi, int64_t sample0,
@@ -1599,16 +1611,13 @@ cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t
     seg->tiles = tiles;
     seg->nchunks = nchunks;
     seg->slabs = 0;
-    const size_t prefix_rows = (size_t)std::max<int64_t>(tiles * TM, nsamples + 2 + PREFIX_PARTS);
+    const size_t prefix_rows = std::max<size_t>((size_t)(tiles * TM), split_prefix_rows(nsamples));
     if ((e = grow(r.prefix, r.prefix_bytes, prefix_rows * PREFIX_STRIDE * sizeof(double))) != cudaSuccess) return e;
     if ((e = grow(r.params, r.params_bytes, (size_t)nchunks * PARAM_BYTES)) != cudaSuccess) return e;
     // The segment's samples are the global ADC indices sample0 .. sample0 + nsamples - 1.
-    const dim3 pgrid(PREFIX_COLS, PREFIX_PARTS);
-    prefix_part_kernel<<<pgrid, 256, 0, stream>>>((const double *)a.dt, reinterpret_cast<const double *const *>(a.src_dev),
-                                                  n_lo, n_hi, nsamples, a.gamma, (double *)r.prefix);
-    prefix_kernel<<<pgrid, 256, 0, stream>>>((const double *)a.dt, reinterpret_cast<const double *const *>(a.src_dev),
-                                             (const uint8_t *)a.adc, a.grank, sample0, n_lo, n_hi, nsamples, a.gamma,
-                                             (double *)r.prefix);
+    if ((e = split_prefix_launch((const double *)a.dt, a.src_dev, (const uint8_t *)a.adc, a.grank, n_lo, n_hi, sample0,
+                                 nsamples, a.gamma, (double *)r.prefix, stream)) != cudaSuccess)
+        return e;
     if ((e = cudaMemsetAsync(r.amp, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
     spin_params_kernel<<<grid_for(r.ns_pad), 256, 0, stream>>>((const double *)a.T2, (const cplx<double> *)a.xy,
                                                                r.ns, nchunks, (unsigned long long *)r.amp,

@@ -97,6 +97,16 @@ cudaError_t split_prepare(SplitResident &r, int64_t ns, int32_t nc, const void *
 // share one `src` may overlap on the device.
 cudaError_t split_attach(SplitResident &r, const SplitResident &src);
 
+// Prefix table of a segment (nodes n_lo .. n_hi, `nsamples` ADC samples of
+// global index sample0 ..): FP64 rows of kappa_0 .. kappa_16 and, at
+// SPLIT_PREFIX_T, the elapsed time, one row per sample, then the row of the end
+// node.  `prefix` holds split_prefix_rows(nsamples) rows.
+constexpr int SPLIT_PREFIX_STRIDE = 24, SPLIT_PREFIX_T = 20;
+size_t split_prefix_rows(int64_t nsamples);
+cudaError_t split_prefix_launch(const double *dt, const void *const *src_dev, const uint8_t *adc, const int32_t *grank,
+                                int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
+                                double *prefix, cudaStream_t stream);
+
 // Clear the device error word before a run.
 cudaError_t split_reset_error(SplitResident &r, cudaStream_t stream);
 
