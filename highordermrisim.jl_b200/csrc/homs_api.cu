@@ -18,6 +18,7 @@
 #include "homs_internal.cuh"
 #include "homs_kspace.cuh"
 #include "homs_phantom.cuh"
+#include "homs_precess32.cuh"
 #include "homs_precess64.cuh"
 #include "homs_split.cuh"
 
@@ -135,8 +136,8 @@ struct homs_context {
     std::mutex mu;
     // reusable scratch
     DevBuf scratch_csm, scratch_partial, scratch_acc, scratch_bnd, scratch_sig, scratch_conv;
-    // FP64 precession blocks: sample index per node, column sources, spin table,
-    // prefix table, aligned copy of the state
+    // Precession blocks: per-node values (sample index or block time), column
+    // sources, spin or node table, prefix table or phases, aligned copy of the state
     DevBuf block_rank, block_src, block_table, block_prefix, block_xy;
     // encoding export (homs_kspace): staged inputs, metadata, work and outputs,
     // and the events around its kernels
@@ -407,6 +408,11 @@ struct Resident : ResidentBase {
     // Plain FP64 precession: the phantom's spin table and the prefix table of a segment.
     DevBuf spin_table, prefix;
     bool spin_table_ready = false;
+    // Plain FP32 precession: the block time of every node, the node table of
+    // `nodes_method`, a launch round's phases and initial states.
+    DevBuf block_time, nodes, walk;
+    bool block_time_ready = false;
+    uint32_t nodes_method = ~0u;
     // Prefix-table inputs of the sequence: the global ADC sample index of every
     // node, and the 17 column sources of `src_method`.
     DevBuf grank, src_table;
@@ -438,7 +444,7 @@ struct Resident : ResidentBase {
         size_t b = x.bytes + y.bytes + z.bytes + rho.bytes + T1.bytes + T2.bytes + dw.bytes + csm_rows.bytes + t.bytes +
                    dt.bytes + gx.bytes + gy.bytes + gz.bytes + b1.bytes + df.bytes + psi.bytes + adc.bytes + bnd.bytes +
                    xy.bytes + mz.bytes + acc.bytes + rho_init.bytes + partial.bytes + sig.bytes + spin_table.bytes +
-                   prefix.bytes + split.device_bytes();
+                   prefix.bytes + block_time.bytes + nodes.bytes + walk.bytes + split.device_bytes();
         for (int k = 0; k < 16; ++k) b += h[k].bytes;
         return b;
     }
@@ -531,6 +537,8 @@ void fill_sequence(homs_context *ctx, Resident<T> *r, const homs_sequence *q) {
     r->gamma = q->gamma;
     r->grank_ready = false;
     r->src_method = ~0u;
+    r->block_time_ready = false;
+    r->nodes_method = ~0u;
     const int64_t ns = r->ns, nt = q->nnodes;
     upload<T>(ctx, r->t, q->t, q->dtype, q->memory, nt);
     upload<T>(ctx, r->dt, q->dt, q->dtype, q->memory, nt - 1);
@@ -586,20 +594,22 @@ Resident<T> *cached_resident(homs_context *ctx, const homs_phantom *p, const hom
     return r;
 }
 
-// Launch plan of the plain path: runs of same-kind blocks cut into launches
-// of at most `max_samples` ADC samples.
+// Launch plan: the runs of same-kind blocks, cut into launches of at most the
+// given numbers of ADC samples and (precession) blocks.
+struct LaunchLimits {
+    int64_t rf_samples, precession_samples, precession_blocks;
+};
 struct Launch {
-    int64_t run;
     bool rf;
     int64_t n_lo, n_hi;
-    int block_start;
-    double tp0;  // informational; the typed value is recomputed below
+    int block_start;  // n_lo is the first node of a block
     int64_t sample0, nsamples;
+    int32_t nblocks;  // blocks with intervals in the launch
 };
 
 template <typename T>
-std::vector<std::pair<Launch, T>> plan_plain(const Resident<T> &r, int64_t max_samples) {
-    std::vector<std::pair<Launch, T>> out;
+std::vector<Launch> plan_launches(const Resident<T> &r, const LaunchLimits &lim) {
+    std::vector<Launch> out;
     const auto &adc = r.adc_host;
     int64_t sample = 0;
     size_t k = 0;
@@ -609,31 +619,28 @@ std::vector<std::pair<Launch, T>> plan_plain(const Resident<T> &r, int64_t max_s
         size_t k2 = k;
         while (k2 < nb && (r.exc[k2] != 0) == rf) ++k2;
         // run: blocks k .. k2-1, nodes first[k] .. last[k2-1]
+        const int64_t max_samples = rf ? lim.rf_samples : lim.precession_samples;
+        const int64_t max_blocks = rf ? INT64_MAX : lim.precession_blocks;
         size_t blk = k;
-        T tp = T(0);
         int64_t n = r.first[k];
         const int64_t n_end = r.last[k2 - 1];
         while (n < n_end) {
-            Launch L{(int64_t)k, rf, n, n, n == r.first[blk] ? 1 : 0, 0.0, sample, 0};
-            const T tp0 = tp;
-            int64_t cnt = 0;
+            Launch L{rf, n, n, n == r.first[blk] ? 1 : 0, sample, 0, 1};
             int64_t m = n;
             while (m < n_end) {
                 // interval m -> node m+1
-                tp = tp + r.dt_host[(size_t)m];
-                const bool a = adc[(size_t)(m + 1)] != 0;
-                if (a) ++cnt;
+                if (adc[(size_t)(m + 1)]) ++L.nsamples;
                 ++m;
-                if (m == r.last[blk]) {
-                    tp = T(0);
-                    if (blk + 1 < k2) ++blk;
+                if (m == r.last[blk] && m < n_end) {
+                    ++blk;
+                    if (L.nblocks >= max_blocks) break;
+                    if (L.nsamples < max_samples) ++L.nblocks;
                 }
-                if (cnt >= max_samples) break;
+                if (L.nsamples >= max_samples) break;
             }
             L.n_hi = m;
-            L.nsamples = cnt;
-            sample += cnt;
-            out.emplace_back(L, tp0);
+            sample += L.nsamples;
+            out.push_back(L);
             n = m;
         }
         k = k2;
@@ -689,7 +696,7 @@ inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t met
                                   r.grank.as<int32_t>(), n_lo, n_hi, sample0, nsamples, r.gamma,
                                   r.prefix.as<double>(), ctx->stream));
     r.launches += 2;
-    const Precess64Plan pp = precess64_plan(r.ns, r.nc, nsamples);
+    const CoilCut pp = precess64_cut(r.ns, r.nc, nsamples);
     HOMS_CUDA(r.partial.ensure(pp.partial_bytes));
     Precess64Args a;
     a.ns = r.ns;
@@ -713,18 +720,92 @@ inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t met
                             &r.launches, ctx->stream));
 }
 
+// The plain FP32 path's node table of the sequence and method: the block times
+// are summed here, node by node in FP32 from each block's start.
+inline void ensure_nodes32(homs_context *ctx, Resident<float> &r, uint32_t method) {
+    if (!r.block_time_ready) {
+        std::vector<float> tp((size_t)r.nt, 0.0f);
+        for (size_t k = 0; k < r.first.size(); ++k) {
+            float t = 0.0f;
+            for (int64_t n = r.first[k] + 1; n <= r.last[k]; ++n) tp[(size_t)n] = t = t + r.dt_host[(size_t)(n - 1)];
+        }
+        HOMS_CUDA(r.block_time.ensure(sizeof(float) * (size_t)r.nt));
+        HOMS_CUDA(cudaMemcpyAsync(r.block_time.p, tp.data(), sizeof(float) * (size_t)r.nt, cudaMemcpyHostToDevice,
+                                  ctx->stream));
+        r.block_time_ready = true;
+        r.nodes_method = ~0u;
+    }
+    if (r.nodes_method != method) {
+        HOMS_CUDA(r.nodes.ensure(precess32_node_bytes(r.nt)));
+        HOMS_CUDA(precess32_nodes(r.seq(), method, r.block_time.as<float>(), r.nodes.p, ctx->stream));
+        r.nodes_method = method;
+    }
+}
+
+// One launch round of a plain FP32 precession run.
+inline void plain_round32(homs_context *ctx, Resident<float> &r, uint32_t method, bool capture, const Launch &L) {
+    const CoilCut cut = precess32_cut(r.ns, r.nc, L.nsamples);
+    HOMS_CUDA(r.walk.ensure(precess32_work_bytes(r.ns, L.nsamples, L.nblocks)));
+    HOMS_CUDA(r.partial.ensure(cut.partial_bytes));
+    Precess32Args a;
+    a.phantom = r.phantom();
+    a.state = StateDev<float>{r.xy.as<cplx<float>>(), r.mz.as<float>(), r.acc.as<float>()};
+    a.nodes = r.nodes.p;
+    a.nnodes = r.nt;
+    a.n_lo = L.n_lo;
+    a.n_hi = L.n_hi;
+    a.block_start = L.block_start;
+    a.nsamples = L.nsamples;
+    a.nblocks = L.nblocks;
+    a.method = method;
+    a.gamma = r.gamma;
+    a.work = r.walk.p;
+    a.partial = r.partial.as<cplx<double>>();
+    a.sig = r.sig.as<cplx<float>>() + L.sample0;
+    a.ldsig = r.nadc;
+    const auto ev = r.next_events();
+    HOMS_CUDA(precess32_run(a, cut, ev.first, ev.second, capture ? cudaEventRecordExternal : cudaEventRecordDefault,
+                            &r.launches, ctx->stream));
+}
+
+// One launch of an excitation run (at most excitation_samples samples).
+template <typename T>
+void excitation_launch(Resident<T> &r, uint32_t method, const Launch &L, cudaStream_t stream) {
+    const int grid = (int)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
+    HOMS_CUDA(r.partial.ensure(sizeof(cplx<T>) * (size_t)r.nc * (size_t)grid *
+                               (size_t)std::max<int64_t>(L.nsamples, 1)));
+    SegmentArgs<T> a;
+    a.n_lo = L.n_lo;
+    a.n_hi = L.n_hi;
+    a.block_start = L.block_start;
+    a.nsamples = L.nsamples;
+    a.method = method;
+    a.gamma = T(r.gamma);
+    a.gamma_d = r.gamma;
+    a.partial = r.partial.template as<cplx<T>>();
+    PhantomDev<T> p = r.phantom();
+    SeqDev<T> q = r.seq();
+    StateDev<T> st{r.xy.template as<cplx<T>>(), r.mz.template as<T>(), r.acc.template as<T>()};
+    HOMS_CUDA(launch_excitation<T>(p, q, st, a, grid, stream));
+    r.launches += 1;
+    if (L.nsamples > 0) {
+        HOMS_CUDA(launch_partial_finalize(a.partial, grid, L.nsamples, r.nc,
+                                          r.sig.template as<cplx<T>>() + L.sample0, r.nadc, stream));
+        r.launches += 1;
+    }
+}
+
+// Samples of an excitation launch whose partial sums take at most 512 MB.
+template <typename T>
+int64_t excitation_samples(const Resident<T> &r) {
+    const size_t grid = (size_t)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
+    return std::max<int64_t>(PLAIN_STAGE, (int64_t)((size_t(512) << 20) / (sizeof(cplx<T>) * (size_t)r.nc * grid)));
+}
+
 template <typename T>
 void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture) {
     const unsigned ev_flags = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
-    const int grid = (int)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-    const size_t row_bytes = sizeof(cplx<T>) * (size_t)r.nc * (size_t)grid;
-    const size_t budget = size_t(768) << 20;
-    int64_t max_samples = std::max<int64_t>(PLAIN_STAGE, (int64_t)(budget / row_bytes));
-    max_samples = std::min<int64_t>(max_samples, std::max<int64_t>(r.nadc, 1));
-    auto plan = plan_plain<T>(r, max_samples);
-    int64_t need = 0;
-    for (auto &pl : plan)
-        if (sizeof(T) == 4 || pl.first.rf) need = std::max(need, pl.first.nsamples);
+    LaunchLimits lim{excitation_samples(r), INT64_MAX, INT64_MAX};
     if constexpr (sizeof(T) == 8) {
         if (capture) {
             HOMS_REQUIRE(r.spin_table_ready && r.grank_ready && r.src_method == method,
@@ -733,47 +814,27 @@ void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture)
             ensure_spin_table(ctx, r);
             ensure_prefix_tables<T>(ctx, r, method);
         }
+    } else {
+        lim.precession_samples = precess32_max_samples(r.ns);
+        lim.precession_blocks = precess32_max_blocks(r.ns);
+        if (capture) {
+            HOMS_REQUIRE(r.nodes_method == method, "internal: precession tables missing under capture");
+        } else {
+            ensure_nodes32(ctx, r, method);
+        }
     }
-    HOMS_CUDA(r.partial.ensure(row_bytes * (size_t)std::max<int64_t>(need, 1)));
-    PhantomDev<T> p = r.phantom();
-    SeqDev<T> q = r.seq();
-    StateDev<T> st{reinterpret_cast<cplx<T> *>(r.xy.p), reinterpret_cast<T *>(r.mz.p), reinterpret_cast<T *>(r.acc.p)};
-    for (size_t i = 0; i < plan.size(); ++i) {
-        const auto &pl = plan[i];
-        const Launch &L = pl.first;
-        if constexpr (sizeof(T) == 8) {
-            if (!L.rf) {
-                // a run's precession launches are one segment
-                int64_t n_hi = L.n_hi, nsamples = L.nsamples;
-                while (i + 1 < plan.size() && plan[i + 1].first.run == L.run) {
-                    ++i;
-                    n_hi = plan[i].first.n_hi;
-                    nsamples += plan[i].first.nsamples;
-                }
-                plain_segment64(ctx, r, method, capture, L.n_lo, n_hi, L.sample0, nsamples);
-                continue;
-            }
+    for (const Launch &L : plan_launches<T>(r, lim)) {
+        if (L.rf) {
+            const auto ev = r.next_events();
+            HOMS_CUDA(cudaEventRecordWithFlags(ev.first, ctx->stream, ev_flags));
+            excitation_launch<T>(r, method, L, ctx->stream);
+            HOMS_CUDA(cudaEventRecordWithFlags(ev.second, ctx->stream, ev_flags));
+            continue;
         }
-        SegmentArgs<T> a;
-        a.n_lo = L.n_lo;
-        a.n_hi = L.n_hi;
-        a.block_start = L.block_start;
-        a.tp0 = pl.second;
-        a.nsamples = L.nsamples;
-        a.method = method;
-        a.gamma = T(r.gamma);
-        a.gamma_d = r.gamma;
-        a.partial = reinterpret_cast<cplx<T> *>(r.partial.p);
-        auto ev = r.next_events();
-        HOMS_CUDA(cudaEventRecordWithFlags(ev.first, ctx->stream, ev_flags));
-        HOMS_CUDA(launch_segment<T>(L.rf, p, q, st, a, grid, ctx->stream));
-        HOMS_CUDA(cudaEventRecordWithFlags(ev.second, ctx->stream, ev_flags));
-        r.launches += 1;
-        if (L.nsamples > 0) {
-            HOMS_CUDA(launch_partial_finalize<T>(a.partial, grid, L.nsamples, r.nc,
-                                                 reinterpret_cast<cplx<T> *>(r.sig.p) + L.sample0, r.nadc, ctx->stream));
-            r.launches += 1;
-        }
+        if constexpr (sizeof(T) == 8)
+            plain_segment64(ctx, r, method, capture, L.n_lo, L.n_hi, L.sample0, L.nsamples);
+        else
+            plain_round32(ctx, r, method, capture, L);
     }
 }
 
@@ -826,13 +887,10 @@ struct SplitRunner {
     homs_context *ctx = nullptr;
     Resident<T> *r = nullptr;
     SplitRunArgs sa{};
-    std::vector<std::pair<Launch, T>> plan;
+    std::vector<Launch> plan;
     size_t i = 0;  // next plan entry
-    int grid = 0;
-    size_t row_bytes = 0;
     // the segment in progress
     bool in_segment = false;
-    size_t seg_next = 0;  // plan entry after the segment
     int64_t seg_sample0 = 0;
     int grp = 0;
     SplitSegment seg;
@@ -881,37 +939,9 @@ struct SplitRunner {
         sa.launches = &res.launches;
         // RF runs use the plain FP64 excitation kernel; precession runs are
         // whole segments on the split kernel.
-        grid = (int)((res.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-        row_bytes = sizeof(cplx<T>) * (size_t)res.nc * (size_t)grid;
-        const int64_t max_samples = std::max<int64_t>(PLAIN_STAGE, (int64_t)((size_t(512) << 20) / row_bytes));
-        plan = plan_plain<T>(res, max_samples);
+        plan = plan_launches<T>(res, LaunchLimits{excitation_samples(res), INT64_MAX, INT64_MAX});
         i = 0;
         in_segment = false;
-    }
-
-    void rf_launch(const Launch &L, T tp0, cudaStream_t stream) {
-        HOMS_CUDA(r->partial.ensure(row_bytes * (size_t)std::max<int64_t>(L.nsamples, 1)));
-        SegmentArgs<T> a;
-        a.n_lo = L.n_lo;
-        a.n_hi = L.n_hi;
-        a.block_start = L.block_start;
-        a.tp0 = tp0;
-        a.nsamples = L.nsamples;
-        a.method = sa.method;
-        a.gamma = T(r->gamma);
-        a.gamma_d = r->gamma;
-        a.partial = reinterpret_cast<cplx<T> *>(r->partial.p);
-        PhantomDev<T> p = r->phantom();
-        SeqDev<T> q = r->seq();
-        StateDev<T> st{reinterpret_cast<cplx<T> *>(r->xy.p), reinterpret_cast<T *>(r->mz.p),
-                       reinterpret_cast<T *>(r->acc.p)};
-        HOMS_CUDA(launch_segment<T>(true, p, q, st, a, grid, stream));
-        r->launches += 1;
-        if (L.nsamples > 0) {
-            HOMS_CUDA(launch_partial_finalize<T>(a.partial, grid, L.nsamples, r->nc,
-                                                 reinterpret_cast<cplx<T> *>(r->sig.p) + L.sample0, r->nadc, stream));
-            r->launches += 1;
-        }
     }
 
     bool next(cudaStream_t stream, SplitJobDesc *job) {
@@ -920,33 +950,24 @@ struct SplitRunner {
             return true;
         }
         while (i < plan.size()) {
-            const Launch &L = plan[i].first;
+            const Launch &L = plan[i];
             if (L.rf) {
-                rf_launch(L, plan[i].second, stream);
+                excitation_launch<T>(*r, sa.method, L, stream);
                 ++i;
                 continue;
             }
-            // merge consecutive precession launches of one run into a segment
-            size_t j = i;
-            int64_t ns_total = 0;
-            while (j < plan.size() && !plan[j].first.rf && plan[j].first.run == L.run) {
-                ns_total += plan[j].first.nsamples;
-                ++j;
-            }
             std::string err;
-            const cudaError_t e =
-                split_segment_begin(r->split, sa, L.n_lo, plan[j - 1].first.n_hi, L.sample0, ns_total, stream, &err,
-                                    &seg);
+            const cudaError_t e = split_segment_begin(r->split, sa, L.n_lo, L.n_hi, L.sample0, L.nsamples, stream,
+                                                      &err, &seg);
             if (e != cudaSuccess) throw Failure{e == cudaErrorMemoryAllocation ? HOMS_ENOMEM : HOMS_ECUDA,
                                                 std::string("split segment: ") + cudaGetErrorString(e)};
             if (!err.empty()) throw Failure{HOMS_EUNSUPPORTED, err};
-            if (ns_total == 0) {
+            if (L.nsamples == 0) {
                 HOMS_CUDA(split_segment_end(r->split, sa, seg, stream));
-                i = j;
+                ++i;
                 continue;
             }
             in_segment = true;
-            seg_next = j;
             seg_sample0 = L.sample0;
             grp = 0;
             *job = split_segment_job(r->split, seg, grp);
@@ -960,7 +981,7 @@ struct SplitRunner {
         if (++grp < r->split.ngroups) return;
         HOMS_CUDA(split_segment_end(r->split, sa, seg, stream));
         in_segment = false;
-        i = seg_next;
+        ++i;
     }
 
     bool first_group() const { return grp == 0; }
@@ -1448,7 +1469,7 @@ void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDe
     HOMS_CUDA(split_prefix_launch(q.dt, ctx->block_src.as<const void *>(), q.adc,
                                   ctx->block_rank.as<int32_t>() - (first + 1), first, last, 0, nadc, gamma,
                                   ctx->block_prefix.as<double>(), ctx->stream));
-    const Precess64Plan pp = precess64_plan(p.ns, p.nc, nadc);
+    const CoilCut pp = precess64_cut(p.ns, p.nc, nadc);
     HOMS_CUDA(ctx->scratch_partial.ensure(pp.partial_bytes));
     // The kernels read and write the state as 16-byte pairs: a caller's array off
     // that boundary goes through a copy.
@@ -1478,6 +1499,64 @@ void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDe
     a.ldsig = ldsig;
     HOMS_CUDA(precess64_run(a, pp, nullptr, nullptr, cudaEventRecordDefault, nullptr, ctx->stream));
     if (!aligned) HOMS_CUDA(cudaMemcpyAsync(state.xy, xy, xy_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+}
+
+// The same in FP32: the block's nodes get a table of their own, then the block
+// runs in launch rounds.
+void block_precess32(homs_context *ctx, const PhantomDev<float> &p, const SeqDev<float> &q, const homs_state &state,
+                     int64_t first, int64_t last, uint32_t method, double gamma, int64_t nadc, void *sig,
+                     int64_t ldsig) {
+    Resident<float> r;  // the block as a sequence of its own (host side only)
+    r.ns = p.ns;
+    r.nc = p.nc;
+    r.nt = last - first + 1;
+    r.nadc = nadc;
+    r.first = {0};
+    r.last = {r.nt - 1};
+    r.exc = {0};
+    r.adc_host.resize((size_t)r.nt);
+    HOMS_CUDA(cudaMemcpyAsync(r.adc_host.data(), q.adc + first, (size_t)r.nt, cudaMemcpyDeviceToHost, ctx->stream));
+    r.dt_host = host_array<float>(ctx, q.dt + first, HOMS_F32, HOMS_DEVICE, r.nt - 1);  // waits for both copies
+    std::vector<float> tp((size_t)r.nt, 0.0f);
+    for (int64_t n = 1; n < r.nt; ++n) tp[(size_t)n] = tp[(size_t)(n - 1)] + r.dt_host[(size_t)(n - 1)];
+    HOMS_CUDA(ctx->block_rank.ensure(sizeof(float) * (size_t)r.nt));
+    HOMS_CUDA(cudaMemcpyAsync(ctx->block_rank.p, tp.data(), sizeof(float) * (size_t)r.nt, cudaMemcpyHostToDevice,
+                              ctx->stream));
+    SeqDev<float> b = q;
+    b.nnodes = r.nt;
+    b.dt += first;
+    b.gx += first;
+    b.gy += first;
+    b.gz += first;
+    b.adc += first;
+    b.boundary += first;
+    for (int k = 0; k < 16; ++k) b.h[k] += first;
+    HOMS_CUDA(ctx->block_table.ensure(precess32_node_bytes(r.nt)));
+    HOMS_CUDA(precess32_nodes(b, method, ctx->block_rank.as<float>(), ctx->block_table.p, ctx->stream));
+    HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(float) * (size_t)p.ns));
+    for (const Launch &L : plan_launches<float>(r, LaunchLimits{INT64_MAX, precess32_max_samples(p.ns), INT64_MAX})) {
+        const CoilCut cut = precess32_cut(p.ns, p.nc, L.nsamples);
+        HOMS_CUDA(ctx->block_prefix.ensure(precess32_work_bytes(p.ns, L.nsamples, L.nblocks)));
+        HOMS_CUDA(ctx->scratch_partial.ensure(cut.partial_bytes));
+        Precess32Args a;
+        a.phantom = p;
+        a.state = StateDev<float>{static_cast<cplx<float> *>(state.xy), static_cast<float *>(state.z),
+                                  ctx->scratch_acc.as<float>()};
+        a.nodes = ctx->block_table.p;
+        a.nnodes = r.nt;
+        a.n_lo = L.n_lo;
+        a.n_hi = L.n_hi;
+        a.block_start = L.block_start;
+        a.nsamples = L.nsamples;
+        a.nblocks = L.nblocks;
+        a.method = method;
+        a.gamma = gamma;
+        a.work = ctx->block_prefix.p;
+        a.partial = ctx->scratch_partial.as<cplx<double>>();
+        a.sig = static_cast<cplx<float> *>(sig) + L.sample0;
+        a.ldsig = ldsig;
+        HOMS_CUDA(precess32_run(a, cut, nullptr, nullptr, cudaEventRecordDefault, nullptr, ctx->stream));
+    }
 }
 
 template <typename T>
@@ -1520,11 +1599,12 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     qd.adc = q->adc;
     qd.boundary = reinterpret_cast<uint8_t *>(ctx->scratch_bnd.p);
     for (int k = 0; k < 16; ++k) qd.h[k] = (const T *)q->h[k];
-    if constexpr (sizeof(T) == 8) {
-        if (!rf) {
+    if (!rf) {
+        if constexpr (sizeof(T) == 8)
             block_precess64(ctx, pd, qd, *state, first, last, method, q->gamma, adc, nadc, sig, ldsig);
-            return HOMS_OK;
-        }
+        else
+            block_precess32(ctx, pd, qd, *state, first, last, method, q->gamma, nadc, sig, ldsig);
+        return HOMS_OK;
     }
     HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
     const int grid = (int)((ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
@@ -1535,15 +1615,14 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     a.n_lo = first;
     a.n_hi = last;
     a.block_start = 1;
-    a.tp0 = T(0);
     a.nsamples = nadc;
     a.method = method;
     a.gamma = T(q->gamma);
     a.gamma_d = q->gamma;
     a.partial = reinterpret_cast<cplx<T> *>(ctx->scratch_partial.p);
-    HOMS_CUDA(launch_segment<T>(rf, pd, qd, st, a, grid, ctx->stream));
+    HOMS_CUDA(launch_excitation<T>(pd, qd, st, a, grid, ctx->stream));
     if (nadc > 0) {
-        HOMS_CUDA(launch_partial_finalize<T>(a.partial, grid, nadc, nc, reinterpret_cast<cplx<T> *>(ctx->scratch_sig.p), nadc, ctx->stream));
+        HOMS_CUDA(launch_partial_finalize(a.partial, grid, nadc, nc, reinterpret_cast<cplx<T> *>(ctx->scratch_sig.p), nadc, ctx->stream));
         HOMS_CUDA(cudaMemcpy2DAsync(sig, sizeof(cplx<T>) * (size_t)ldsig, ctx->scratch_sig.p, sizeof(cplx<T>) * (size_t)nadc,
                                     sizeof(cplx<T>) * (size_t)nadc, (size_t)nc, cudaMemcpyDeviceToDevice, ctx->stream));
     }
@@ -1612,13 +1691,13 @@ homs_status homs_coil_reduce(homs_context *ctx, homs_dtype dtype, int64_t nspins
             HOMS_CUDA(launch_coil_reduce<double>(nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
                                                  (const cplx<double> *)csm, ldcsm, reinterpret_cast<cplx<double> *>(ctx->scratch_partial.p),
                                                  ctx->stream));
-            HOMS_CUDA(launch_partial_finalize<double>(reinterpret_cast<cplx<double> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
+            HOMS_CUDA(launch_partial_finalize(reinterpret_cast<cplx<double> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
                                                       (cplx<double> *)sig, ldsig, ctx->stream));
         } else {
             HOMS_CUDA(launch_coil_reduce<float>(nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
                                                 (const cplx<float> *)csm, ldcsm, reinterpret_cast<cplx<float> *>(ctx->scratch_partial.p),
                                                 ctx->stream));
-            HOMS_CUDA(launch_partial_finalize<float>(reinterpret_cast<cplx<float> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
+            HOMS_CUDA(launch_partial_finalize(reinterpret_cast<cplx<float> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
                                                      (cplx<float> *)sig, ldsig, ctx->stream));
         }
         return HOMS_OK;

@@ -48,13 +48,12 @@ struct StateDev {
     T *acc;  // running trapezoid sum of the current precession block
 };
 
-// One launch of the plain segment kernel: intervals [n_lo, n_hi) of a run of
-// blocks of one kind (precession or excitation).
+// One launch of the excitation kernel: intervals [n_lo, n_hi) of a run of
+// excitation blocks.
 template <typename T>
 struct SegmentArgs {
     int64_t n_lo, n_hi;
     int block_start;      // n_lo is the first node of a block
-    T tp0;                // precession: elapsed block time at n_lo
     int64_t nsamples;     // ADC samples in (n_lo, n_hi]
     uint32_t method;
     T gamma;              // T(γ)
@@ -71,12 +70,14 @@ constexpr int PLAIN_STAGE = 8;  // ADC samples staged per reduction
 namespace homs {
 
 template <typename T>
-cudaError_t launch_segment(bool rf, const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st,
+cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st,
                            const SegmentArgs<T> &a, int grid, cudaStream_t stream);
 
-template <typename T>
-cudaError_t launch_partial_finalize(const cplx<T> *partial, int64_t nparts, int64_t nsamples, int32_t nc,
-                                    cplx<T> *sig, int64_t ldsig, cudaStream_t stream);
+// Sum of nparts partial (nsamples x nc) blocks into sig, added in type P, in an
+// order that depends on nparts only.
+template <typename P, typename S>
+cudaError_t launch_partial_finalize(const cplx<P> *partial, int64_t nparts, int64_t nsamples, int32_t nc,
+                                    cplx<S> *sig, int64_t ldsig, cudaStream_t stream);
 
 // Standalone coil reduction, split-K over spin ranges: coil_reduce_parts()
 // partial (nadc x nc) blocks, at most ceil(ns / PLAIN_THREADS) of them, which

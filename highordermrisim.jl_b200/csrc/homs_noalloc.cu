@@ -83,13 +83,13 @@ extern "C" homs_status homs_coil_reduce_noalloc(void *stream, homs_dtype dtype, 
         e = homs::launch_coil_reduce<double>(nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
                                              (const cplx<double> *)csm, ldcsm, (cplx<double> *)scratch, st);
         if (e == cudaSuccess)
-            e = homs::launch_partial_finalize<double>((const cplx<double> *)scratch, parts, nadc, ncoils,
+            e = homs::launch_partial_finalize((const cplx<double> *)scratch, parts, nadc, ncoils,
                                                       (cplx<double> *)sig, ldsig, st);
     } else {
         e = homs::launch_coil_reduce<float>(nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
                                             (const cplx<float> *)csm, ldcsm, (cplx<float> *)scratch, st);
         if (e == cudaSuccess)
-            e = homs::launch_partial_finalize<float>((const cplx<float> *)scratch, parts, nadc, ncoils,
+            e = homs::launch_partial_finalize((const cplx<float> *)scratch, parts, nadc, ncoils,
                                                      (cplx<float> *)sig, ldsig, st);
     }
     return e == cudaSuccess ? HOMS_OK : HOMS_ECUDA;

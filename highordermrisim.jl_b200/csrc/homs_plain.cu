@@ -1,8 +1,8 @@
-// Plain fused kernels of libhoms: free precession and RF excitation in the
-// phantom's own precision (FP64 or FP32) on CUDA cores, fused with a
-// deterministic multi-coil reduction.  No per-spin ADC history is written to
-// HBM: ADC states are staged in shared memory and contracted with the
-// receive sensitivities on chip, one CTA partial per (CTA, sample, coil),
+// RF excitation in the phantom's own precision (FP64 or FP32) on CUDA cores,
+// fused with a deterministic multi-coil reduction of the samples acquired during
+// the pulse, and the standalone coil reduction.  No per-spin ADC history is
+// written to HBM: ADC states are staged in shared memory and contracted with
+// the receive sensitivities on chip, one CTA partial per (CTA, sample, coil),
 // then summed over CTAs in a fixed order.
 //
 // This translation unit is compiled with -fmad=false so that every product
@@ -43,30 +43,6 @@ __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
     return cplx<T>{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 }
 
-// Sixteen unnormalised solid harmonics in the CPU expression order
-// (BlochHighOrderSimulatitonMethod.jl:54-68).
-template <typename T>
-__device__ __forceinline__ void basis16(T x, T y, T z, T *b) {
-    T x2 = x * x, y2 = y * y, z2 = z * z;
-    T r2 = (x2 + y2) + z2;
-    b[0] = T(1);
-    b[1] = x;
-    b[2] = y;
-    b[3] = z;
-    b[4] = x * y;
-    b[5] = z * y;
-    b[6] = T(3) * z2 - r2;
-    b[7] = x * z;
-    b[8] = x2 - y2;
-    b[9] = (T(3) * y) * x2 - (y2 * y);
-    b[10] = (x * z) * y;
-    b[11] = (T(5) * z2 - r2) * y;
-    b[12] = T(5) * (z2 * z) - (T(3) * z) * r2;
-    b[13] = (T(5) * z2 - r2) * x;
-    b[14] = x2 * z - y2 * z;
-    b[15] = (x2 * x) - (T(3) * x) * y2;
-}
-
 constexpr int NODE_CHUNK = 32;
 
 // Shared-memory node cache for one chunk of nodes [c0, c0 + NODE_CHUNK].
@@ -74,41 +50,16 @@ template <typename T>
 struct NodeCache {
     T dt[NODE_CHUNK + 1];
     T g[3][NODE_CHUNK + 1];
-    T h[16][NODE_CHUNK + 1];
-    T df[NODE_CHUNK + 1];
     T psi[NODE_CHUNK + 1];
     cplx<T> b1[NODE_CHUNK + 1];
-    T ab1[NODE_CHUNK + 1];  // |B1| of the node (RF segments)
-    T dfg[NODE_CHUNK + 1];  // df / gamma of the node (RF segments)
+    T ab1[NODE_CHUNK + 1];  // |B1| of the node
+    T dfg[NODE_CHUNK + 1];  // df / gamma of the node
     uint8_t adc[NODE_CHUNK + 1];
     uint8_t bnd[NODE_CHUNK + 1];
 };
 
-// Bz at a cached node (BlochHighOrderSimulatitonMethod.jl:70-75).
 template <typename T>
-__device__ __forceinline__ T field_cached(const NodeCache<T> &nc, int i, const T *b, T dwterm, uint32_t m) {
-    T bz0 = (m & HOMS_HO0) ? nc.h[0][i] : T(0);
-    T bz1;
-    if (m & HOMS_HO1)
-        bz1 = (b[1] * nc.h[1][i] + b[2] * nc.h[2][i]) + b[3] * nc.h[3][i];
-    else
-        bz1 = (b[1] * nc.g[0][i] + b[2] * nc.g[1][i]) + b[3] * nc.g[2][i];
-    T bz2 = T(0), bz3 = T(0);
-    if (m & HOMS_HO2)
-        bz2 = (((b[4] * nc.h[4][i] + b[5] * nc.h[5][i]) + b[6] * nc.h[6][i]) + b[7] * nc.h[7][i]) +
-              b[8] * nc.h[8][i];
-    if (m & HOMS_HO3)
-        bz3 = (((((b[9] * nc.h[9][i] + b[10] * nc.h[10][i]) + b[11] * nc.h[11][i]) + b[12] * nc.h[12][i]) +
-                b[13] * nc.h[13][i]) +
-               b[14] * nc.h[14][i]) +
-              b[15] * nc.h[15][i];
-    T bz = ((bz0 + bz1) + bz2) + bz3;
-    if (m & HOMS_DW_PRECESSION) bz = bz + dwterm;
-    return bz;
-}
-
-template <typename T, bool RF>
-__device__ void load_nodes(NodeCache<T> &nc, const SeqDev<T> &q, int64_t c0, int64_t c_end, uint32_t m, T gamma) {
+__device__ void load_nodes(NodeCache<T> &nc, const SeqDev<T> &q, int64_t c0, int64_t c_end, T gamma) {
     // nodes c0 .. min(c0 + NODE_CHUNK, c_end) inclusive
     const int n = (int)imin64(NODE_CHUNK, c_end - c0) + 1;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -116,27 +67,16 @@ __device__ void load_nodes(NodeCache<T> &nc, const SeqDev<T> &q, int64_t c0, int
         nc.dt[i] = (g < q.nnodes - 1) ? q.dt[g] : T(0);
         nc.adc[i] = q.adc[g];
         nc.bnd[i] = q.boundary[g];
-        if (RF) {
-            nc.g[0][i] = q.gx[g];
-            nc.g[1][i] = q.gy[g];
-            nc.g[2][i] = q.gz[g];
-            const cplx<T> b1 = q.b1[g];
-            nc.b1[i] = b1;
-            nc.df[i] = q.df[g];
-            nc.psi[i] = q.psi[g];
-            // Spin-independent parts of the RF step, computed once per node
-            // with the same operations as the per-spin code used.
-            nc.ab1[i] = Math<T>::hyp(b1.re, b1.im);
-            nc.dfg[i] = nc.df[i] / gamma;
-        } else {
-            if (!(m & HOMS_HO1)) {
-                nc.g[0][i] = q.gx[g];
-                nc.g[1][i] = q.gy[g];
-                nc.g[2][i] = q.gz[g];
-            }
-#pragma unroll
-            for (int k = 0; k < 16; ++k) nc.h[k][i] = q.h[k][g];
-        }
+        nc.g[0][i] = q.gx[g];
+        nc.g[1][i] = q.gy[g];
+        nc.g[2][i] = q.gz[g];
+        const cplx<T> b1 = q.b1[g];
+        nc.b1[i] = b1;
+        nc.psi[i] = q.psi[g];
+        // Spin-independent parts of the RF step, computed once per node
+        // with the same operations as the per-spin code used.
+        nc.ab1[i] = Math<T>::hyp(b1.re, b1.im);
+        nc.dfg[i] = q.df[g] / gamma;
     }
 }
 
@@ -208,18 +148,15 @@ size_t segment_smem_bytes(int32_t nc) {
     return (bytes + 127) & ~size_t(127);
 }
 
-// Plain segment kernel.  One thread per spin; all threads of a CTA walk the
-// same node range in lockstep, so ADC staging and the coil reduction are
-// CTA-uniform.  RF=false: free precession (per-spin sequential trapezoid in
-// the CPU order, BlochHighOrderSimulatitonMethod.jl:76-92).  RF=true:
-// excitation (per-node hard-pulse spinor, :100-134; spinor of
-// kernels/HighOrderGPU.jl:181-192).  The excitation variant asks for three
-// CTAs per SM (80 registers: its launches without ADC samples use the node
-// cache alone); the precession variant leaves the count to the compiler
-// (0: none asked), which keeps it at 64 (FP32) and 128 (FP64) registers.
-template <typename T, bool RF>
-__global__ void __launch_bounds__(PLAIN_THREADS, RF ? 3 : 0)
-    segment_kernel(PhantomDev<T> p, SeqDev<T> q, StateDev<T> st, SegmentArgs<T> a) {
+// Excitation kernel.  One thread per spin; all threads of a CTA walk the same
+// node range in lockstep, so ADC staging and the coil reduction are
+// CTA-uniform.  Per node a hard-pulse spinor
+// (BlochHighOrderSimulatitonMethod.jl:100-134; kernels/HighOrderGPU.jl:181-192).
+// Three CTAs per SM (80 registers: launches without ADC samples use the node
+// cache alone).
+template <typename T>
+__global__ void __launch_bounds__(PLAIN_THREADS, 3)
+    excitation_kernel(PhantomDev<T> p, SeqDev<T> q, StateDev<T> st, SegmentArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     NodeCache<T> &nc = *reinterpret_cast<NodeCache<T> *>(smem_raw);
     cplx<T> *X = reinterpret_cast<cplx<T> *>(smem_raw + ((sizeof(NodeCache<T>) + 15) & ~size_t(15)));
@@ -260,19 +197,7 @@ __global__ void __launch_bounds__(PLAIN_THREADS, RF ? 3 : 0)
     cplx<T> xy = active ? st.xy[si] : cplx<T>{T(0), T(0)};
     T mz = active ? st.z[si] : T(0);
 
-    T b[16];
-    T dwterm = T(0);
-    T off = T(0);
-    T acc = T(0);
-    T tp = a.tp0;
-    T prev = T(0);
-    if (!RF) {
-        basis16(px, py, pz, b);
-        dwterm = p.dw[si] / c_twopig;
-        acc = a.block_start ? T(0) : (active ? st.acc[si] : T(0));
-    } else {
-        off = (m & HOMS_DW_EXCITATION) ? p.dw[si] / c_twopig : T(0);
-    }
+    const T off = (m & HOMS_DW_EXCITATION) ? p.dw[si] / c_twopig : T(0);
 
     T dt_rel = T(-1), e1_rel = T(0), e2_rel = T(0);  // RF relaxation factors of the last dt
     int staged = 0;
@@ -281,79 +206,54 @@ __global__ void __launch_bounds__(PLAIN_THREADS, RF ? 3 : 0)
 
     for (int64_t c0 = a.n_lo; c0 < a.n_hi; c0 += NODE_CHUNK) {
         __syncthreads();
-        load_nodes<T, RF>(nc, q, c0, a.n_hi, m, gamma);
+        load_nodes<T>(nc, q, c0, a.n_hi, gamma);
         __syncthreads();
         const int nint = (int)imin64(NODE_CHUNK, a.n_hi - c0);
-        if (c0 == a.n_lo) {
-            if (!RF) {
-                prev = field_cached(nc, 0, b, dwterm, m);
-            } else if (a.block_start) {
-                T sn, cs;
-                Math<T>::sc(-nc.psi[0], &sn, &cs);
-                xy = cmul(xy, cplx<T>{cs, sn});
-            }
+        if (c0 == a.n_lo && a.block_start) {
+            T sn, cs;
+            Math<T>::sc(-nc.psi[0], &sn, &cs);
+            xy = cmul(xy, cplx<T>{cs, sn});
         }
         for (int i = 0; i < nint; ++i) {
             const T dt = nc.dt[i];
-            cplx<T> xs;
-            bool have = false;
-            if (!RF) {
-                const T next = field_cached(nc, i + 1, b, dwterm, m);
-                const T y = (next + prev) * dt;
-                acc = acc + y;
-                tp = tp + dt;
-                prev = next;
-                if (nc.adc[i + 1] || nc.bnd[i + 1]) {
-                    const T phi = c_neg * (T(0.5) * acc);
-                    const T e = Math<T>::ex(T(0) - tp / T2);
-                    T sn, cs;
-                    Math<T>::sc(phi, &sn, &cs);
-                    xs = cmul(xy, cplx<T>{e * cs, e * sn});
-                    have = true;
-                }
-            } else {
-                const T dbz = off - nc.dfg[i];
-                const T bz = ((nc.g[0][i] * px + nc.g[1][i] * py) + nc.g[2][i] * pz) + dbz;
-                const cplx<T> b1 = nc.b1[i];
-                const T ab1 = nc.ab1[i];
-                T B = Math<T>::sq(ab1 * ab1 + bz * bz);
-                if (B == T(0)) B = Math<T>::eps();
-                const T phi = c_neg * (B * dt);
-                T sh, ch;
-                Math<T>::sc(phi / T(2), &sh, &ch);
-                // Unit field direction (one reciprocal; within an ulp of three divisions).
-                const T rB = T(1) / B;
-                const T nz = bz * rB, nxr = b1.re * rB, nxi = b1.im * rB;
-                const cplx<T> al{ch, -(nz * sh)};
-                const cplx<T> be{nxi * sh, -(nxr * sh)};
-                cplx<T> t1 = cmul(cplx<T>{T(2) * al.re, -(T(2) * al.im)}, be);
-                t1.re = t1.re * mz;
-                t1.im = t1.im * mz;
-                const cplx<T> ca{al.re, -al.im};
-                const cplx<T> t2 = cmul(cmul(ca, ca), xy);
-                const cplx<T> t3 = cmul(cmul(be, be), cplx<T>{xy.re, -xy.im});
-                const cplx<T> nxy{(t1.re + t2.re) - t3.re, (t1.im + t2.im) - t3.im};
-                // |alpha|^2 - |beta|^2 as sums of squares (the reference's abs2;
-                // within an ulp of hypot()^2).
-                const T aa2 = al.re * al.re + al.im * al.im, bb2 = be.re * be.re + be.im * be.im;
-                const cplx<T> pr = cmul(cmul(al, be), cplx<T>{xy.re, -xy.im});
-                const T nz2 = (aa2 - bb2) * mz - T(2) * pr.re;
-                // Relaxation factors depend on dt only: reuse them while dt repeats.
-                if (!(dt == dt_rel)) {
-                    e2_rel = Math<T>::ex(-dt / T2);
-                    e1_rel = Math<T>::ex(-dt / T1);
-                    dt_rel = dt;
-                }
-                xy = cplx<T>{nxy.re * e2_rel, nxy.im * e2_rel};
-                mz = nz2 * e1_rel + rho * (T(1) - e1_rel);
-                if (nc.adc[i + 1]) {
-                    T sn, cs;
-                    Math<T>::sc(nc.psi[i + 1], &sn, &cs);
-                    xs = cmul(xy, cplx<T>{cs, sn});
-                    have = true;
-                }
+            const T dbz = off - nc.dfg[i];
+            const T bz = ((nc.g[0][i] * px + nc.g[1][i] * py) + nc.g[2][i] * pz) + dbz;
+            const cplx<T> b1 = nc.b1[i];
+            const T ab1 = nc.ab1[i];
+            T B = Math<T>::sq(ab1 * ab1 + bz * bz);
+            if (B == T(0)) B = Math<T>::eps();
+            const T phi = c_neg * (B * dt);
+            T sh, ch;
+            Math<T>::sc(phi / T(2), &sh, &ch);
+            // Unit field direction (one reciprocal; within an ulp of three divisions).
+            const T rB = T(1) / B;
+            const T nz = bz * rB, nxr = b1.re * rB, nxi = b1.im * rB;
+            const cplx<T> al{ch, -(nz * sh)};
+            const cplx<T> be{nxi * sh, -(nxr * sh)};
+            cplx<T> t1 = cmul(cplx<T>{T(2) * al.re, -(T(2) * al.im)}, be);
+            t1.re = t1.re * mz;
+            t1.im = t1.im * mz;
+            const cplx<T> ca{al.re, -al.im};
+            const cplx<T> t2 = cmul(cmul(ca, ca), xy);
+            const cplx<T> t3 = cmul(cmul(be, be), cplx<T>{xy.re, -xy.im});
+            const cplx<T> nxy{(t1.re + t2.re) - t3.re, (t1.im + t2.im) - t3.im};
+            // |alpha|^2 - |beta|^2 as sums of squares (the reference's abs2;
+            // within an ulp of hypot()^2).
+            const T aa2 = al.re * al.re + al.im * al.im, bb2 = be.re * be.re + be.im * be.im;
+            const cplx<T> pr = cmul(cmul(al, be), cplx<T>{xy.re, -xy.im});
+            const T nz2 = (aa2 - bb2) * mz - T(2) * pr.re;
+            // Relaxation factors depend on dt only: reuse them while dt repeats.
+            if (!(dt == dt_rel)) {
+                e2_rel = Math<T>::ex(-dt / T2);
+                e1_rel = Math<T>::ex(-dt / T1);
+                dt_rel = dt;
             }
+            xy = cplx<T>{nxy.re * e2_rel, nxy.im * e2_rel};
+            mz = nz2 * e1_rel + rho * (T(1) - e1_rel);
             if (stage_adc && nc.adc[i + 1]) {
+                T sn, cs;
+                Math<T>::sc(nc.psi[i + 1], &sn, &cs);
+                const cplx<T> xs = cmul(xy, cplx<T>{cs, sn});
                 X[staged * PLAIN_THREADS + threadIdx.x] = active ? xs : cplx<T>{T(0), T(0)};
                 staged++;
                 if (staged == PLAIN_STAGE) {
@@ -364,22 +264,12 @@ __global__ void __launch_bounds__(PLAIN_THREADS, RF ? 3 : 0)
                 }
             }
             if (nc.bnd[i + 1]) {
-                if (!RF) {
-                    // Block end: Mxy = last column, Mz relaxes over the block, phase restarts.
-                    (void)have;
-                    xy = xs;
-                    const T e1 = Math<T>::ex(-tp / T1);
-                    mz = mz * e1 + rho * (T(1) - e1);
-                    acc = T(0);
-                    tp = T(0);
-                } else {
-                    T sn, cs;
-                    Math<T>::sc(nc.psi[i + 1], &sn, &cs);
+                T sn, cs;
+                Math<T>::sc(nc.psi[i + 1], &sn, &cs);
+                xy = cmul(xy, cplx<T>{cs, sn});
+                if (c0 + i + 1 < a.n_hi) {
+                    Math<T>::sc(-nc.psi[i + 1], &sn, &cs);
                     xy = cmul(xy, cplx<T>{cs, sn});
-                    if (c0 + i + 1 < a.n_hi) {
-                        Math<T>::sc(-nc.psi[i + 1], &sn, &cs);
-                        xy = cmul(xy, cplx<T>{cs, sn});
-                    }
                 }
             }
         }
@@ -391,19 +281,21 @@ __global__ void __launch_bounds__(PLAIN_THREADS, RF ? 3 : 0)
     if (active) {
         st.xy[s] = xy;
         st.z[s] = mz;
-        if (!RF) st.acc[s] = acc;
     }
 }
 
 // sig[(j) + c*ldsig] = sum over parts k of partial[(k*nsamples + j)*nc + c].
-// A block takes 32 consecutive outputs; warp q of its 8 sums the parts
-// k = q, q + 8, ... in increasing order (coalesced: 32 outputs of one part per
-// load), then warp 0 adds the 8 sums in warp order.  The order depends only on
-// nparts, so repeated runs are bit-identical.
-constexpr int FIN_OUT = 32, FIN_SLICES = 8;
-template <typename T>
+// A block takes 32 consecutive outputs; warp q of its FIN_SLICES sums the parts
+// k = q, q + FIN_SLICES, ... in increasing order (coalesced: 32 outputs of one
+// part per load), then warp 0 adds those sums in warp order.  The order depends
+// only on nparts, so repeated runs are bit-identical.  Bound by the latency of
+// a warp's chain of loads: 32 slices from 64 parts on (1,024 outputs of 296
+// parts: 12.5 us with 8 slices, 6.8 us with 32), 8 below, where most of 32
+// warps would have nothing to add.
+constexpr int FIN_OUT = 32;
+template <typename T, typename S, int FIN_SLICES>
 __global__ void __launch_bounds__(FIN_OUT *FIN_SLICES)
-    partial_finalize_kernel(const cplx<T> *partial, int64_t nparts, int64_t nsamples, int32_t nc, cplx<T> *sig,
+    partial_finalize_kernel(const cplx<T> *partial, int64_t nparts, int64_t nsamples, int32_t nc, cplx<S> *sig,
                             int64_t ldsig) {
     __shared__ cplx<T> red[FIN_SLICES][FIN_OUT];
     const int64_t total = nsamples * nc;
@@ -427,7 +319,7 @@ __global__ void __launch_bounds__(FIN_OUT *FIN_SLICES)
             }
             const int64_t jj = o / nc;
             const int32_t c = (int32_t)(o % nc);
-            sig[jj + (int64_t)c * ldsig] = s;
+            sig[jj + (int64_t)c * ldsig] = cplx<S>{S(s.re), S(s.im)};
         }
         __syncthreads();
     }
@@ -509,29 +401,26 @@ __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
 }
 
 template <typename T>
-cudaError_t launch_segment(bool rf, const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st,
-                           const SegmentArgs<T> &a, int grid, cudaStream_t stream) {
+cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st, const SegmentArgs<T> &a,
+                              int grid, cudaStream_t stream) {
     const size_t smem = a.nsamples > 0 ? segment_smem_bytes<T>(p.nc) : segment_smem_bytes_no_adc<T>();
-    cudaError_t e;
-    if (rf) {
-        e = allow_max_dynamic_smem((const void *)segment_kernel<T, true>);
-        if (e != cudaSuccess) return e;
-        segment_kernel<T, true><<<grid, PLAIN_THREADS, smem, stream>>>(p, q, st, a);
-    } else {
-        e = allow_max_dynamic_smem((const void *)segment_kernel<T, false>);
-        if (e != cudaSuccess) return e;
-        segment_kernel<T, false><<<grid, PLAIN_THREADS, smem, stream>>>(p, q, st, a);
-    }
+    cudaError_t e = allow_max_dynamic_smem((const void *)excitation_kernel<T>);
+    if (e != cudaSuccess) return e;
+    excitation_kernel<T><<<grid, PLAIN_THREADS, smem, stream>>>(p, q, st, a);
     return cudaGetLastError();
 }
 
-template <typename T>
+template <typename T, typename S>
 cudaError_t launch_partial_finalize(const cplx<T> *partial, int64_t nparts, int64_t nsamples, int32_t nc,
-                                    cplx<T> *sig, int64_t ldsig, cudaStream_t stream) {
+                                    cplx<S> *sig, int64_t ldsig, cudaStream_t stream) {
     const int64_t total = nsamples * nc;
     if (total == 0) return cudaSuccess;
     const int64_t blocks = std::min<int64_t>((total + FIN_OUT - 1) / FIN_OUT, 148 * 16);
-    partial_finalize_kernel<T><<<(int)blocks, FIN_OUT * FIN_SLICES, 0, stream>>>(partial, nparts, nsamples, nc, sig,
+    if (nparts >= 64)
+        partial_finalize_kernel<T, S, 32><<<(int)blocks, FIN_OUT * 32, 0, stream>>>(partial, nparts, nsamples, nc, sig,
+                                                                                    ldsig);
+    else
+        partial_finalize_kernel<T, S, 8><<<(int)blocks, FIN_OUT * 8, 0, stream>>>(partial, nparts, nsamples, nc, sig,
                                                                                   ldsig);
     return cudaGetLastError();
 }
@@ -558,14 +447,16 @@ cudaError_t launch_coil_reduce(int64_t ns, int64_t nadc, int32_t nc, const cplx<
     return cudaGetLastError();
 }
 
-template cudaError_t launch_segment<double>(bool, const PhantomDev<double> &, const SeqDev<double> &,
-                                            StateDev<double> &, const SegmentArgs<double> &, int, cudaStream_t);
-template cudaError_t launch_segment<float>(bool, const PhantomDev<float> &, const SeqDev<float> &,
-                                           StateDev<float> &, const SegmentArgs<float> &, int, cudaStream_t);
-template cudaError_t launch_partial_finalize<double>(const cplx<double> *, int64_t, int64_t, int32_t,
-                                                     cplx<double> *, int64_t, cudaStream_t);
-template cudaError_t launch_partial_finalize<float>(const cplx<float> *, int64_t, int64_t, int32_t, cplx<float> *,
-                                                    int64_t, cudaStream_t);
+template cudaError_t launch_excitation<double>(const PhantomDev<double> &, const SeqDev<double> &, StateDev<double> &,
+                                               const SegmentArgs<double> &, int, cudaStream_t);
+template cudaError_t launch_excitation<float>(const PhantomDev<float> &, const SeqDev<float> &, StateDev<float> &,
+                                              const SegmentArgs<float> &, int, cudaStream_t);
+template cudaError_t launch_partial_finalize<double, double>(const cplx<double> *, int64_t, int64_t, int32_t,
+                                                             cplx<double> *, int64_t, cudaStream_t);
+template cudaError_t launch_partial_finalize<float, float>(const cplx<float> *, int64_t, int64_t, int32_t,
+                                                           cplx<float> *, int64_t, cudaStream_t);
+template cudaError_t launch_partial_finalize<double, float>(const cplx<double> *, int64_t, int64_t, int32_t,
+                                                            cplx<float> *, int64_t, cudaStream_t);
 template cudaError_t launch_coil_reduce<double>(int64_t, int64_t, int32_t, const cplx<double> *, int64_t,
                                                 const cplx<double> *, int64_t, cplx<double> *, cudaStream_t);
 template cudaError_t launch_coil_reduce<float>(int64_t, int64_t, int32_t, const cplx<float> *, int64_t,

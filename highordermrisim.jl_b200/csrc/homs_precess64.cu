@@ -35,6 +35,7 @@
 // CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
 #include <algorithm>
 
+#include "homs_fp64mma.cuh"
 #include "homs_precess64.cuh"
 #include "homs_split.cuh"
 
@@ -43,11 +44,9 @@ namespace homs {
 namespace precess64 {
 
 constexpr int THREADS = 256;
-__host__ __device__ constexpr int mtiles(int nt) { return nt == 4 ? 1 : 2; }  // 8-sample tiles per warp
 constexpr int CHUNK = 32;    // spins per stage
 constexpr int NSTAGE = 3;
 constexpr int TERMS = 16;    // phase slots: basis terms 1..15, dw/(2 pi)
-constexpr int GROUP = 32;    // coils per launch slice
 constexpr int BROW = 144;    // bytes of a staged basis row (128 + 16: conflict-free fragment loads)
 constexpr double TWO_PI = 2.0 * 3.141592653589793;
 
@@ -65,11 +64,6 @@ __host__ __device__ inline uint32_t slot_mask(uint32_t method) {
     return m;
 }
 
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
 // cos and sin of 2 pi theta.  theta is reduced to its nearest quarter turn (an
 // exact subtraction); on [-1/8, 1/8] turn sin(2 pi r) / r is a polynomial of
 // degree 6 and (cos(2 pi r) - 1) / r^2 one of degree 6 in r^2, the interpolants
@@ -128,10 +122,6 @@ __device__ __forceinline__ double pow2(double y) {
     return __hiloint2double(__double2hiint(p) + (k << 20), __double2loint(p));
 }
 
-__device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-
 __global__ void table_kernel(const double *x, const double *y, const double *z, const double *dw, const double *T2,
                              int64_t ns, int64_t ns_pad, double *basis, double *r2) {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < ns_pad; s += (int64_t)gridDim.x * blockDim.x) {
@@ -176,15 +166,15 @@ struct KernelArgs {
     cplx<double> *partial;
 };
 
-// NT: 8-coil tiles (at most GROUP coils per z slice); WJ: warps along the samples.
+// NT: 8-coil tiles (at most COIL_GROUP coils per z slice); WJ: warps along the samples.
 template <int NT, int WJ>
 __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
-    constexpr int CS = csm_row(NT), STAGE = stage_bytes(NT), KSPLIT = 8 / WJ, MT = mtiles(NT);
+    constexpr int CS = csm_row(NT), STAGE = stage_bytes(NT), KSPLIT = 8 / WJ, MT = sample_tiles(NT);
     extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, r = lane >> 2;
     const int wj = warp % WJ, kw = warp / WJ;
-    const int c0 = (int)blockIdx.z * GROUP;
-    const int ncg = min(GROUP, a.nc - c0);
+    const int c0 = (int)blockIdx.z * COIL_GROUP;
+    const int ncg = min(COIL_GROUP, a.nc - c0);
     const int64_t ch0 = a.nchunks * blockIdx.y / a.parts, ch1 = a.nchunks * (blockIdx.y + 1) / a.parts;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
 
@@ -249,15 +239,15 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
 #pragma unroll
     for (int s = 0; s < NSTAGE - 1; ++s) {
         if (ch0 + s < ch1) issue(ch0 + s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        cp_commit();
     }
     int stage = 0;
     for (int64_t ch = ch0; ch < ch1; ++ch) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(NSTAGE - 2) : "memory");
+        cp_wait<NSTAGE - 2>();
         __syncthreads();
         const int fill = stage == 0 ? NSTAGE - 1 : stage - 1;  // the stage consumed last
         if (ch + NSTAGE - 1 < ch1) issue(ch + NSTAGE - 1, fill);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        cp_commit();
         const uint8_t *st = smem + stage * STAGE;
         if (++stage == NSTAGE) stage = 0;
 #pragma unroll 1
@@ -305,7 +295,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
                 }
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    cp_wait<0>();
     cplx<double> *out = a.partial + (size_t)(blockIdx.y * KSPLIT + kw) * a.round_samples * a.nc + c0;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -348,10 +338,6 @@ __global__ void __launch_bounds__(256) state_kernel(const double *basis, const d
 
 inline int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)); }
 
-// 8-coil tiles of a launch, and samples per warp, for nc coils.
-inline int coil_tiles(int32_t nc) { return nc <= 8 ? 1 : nc <= 16 ? 2 : 4; }
-inline int warp_samples(int32_t nc) { return 8 * mtiles(coil_tiles(nc)); }
-
 template <int NT, int WJ>
 cudaError_t launch(const KernelArgs &ka, int64_t tiles, int groups, cudaStream_t stream) {
     cudaError_t e = allow_max_dynamic_smem((const void *)main_kernel<NT, WJ>);
@@ -380,49 +366,22 @@ cudaError_t precess64_table(const double *x, const double *y, const double *z, c
     return cudaGetLastError();
 }
 
-Precess64Plan precess64_plan(int64_t ns, int32_t nc, int64_t nsamples) {
-    Precess64Plan p;
-    if (nsamples <= 0) return p;
-    // Sample tile: 8 warps along the samples, or fewer where that would be mostly padding.
-    const int per_warp = warp_samples(nc);
-    auto padded = [&](int wj) { return (nsamples + per_warp * wj - 1) / (per_warp * wj) * (per_warp * wj); };
-    for (int wj : {4, 2})
-        if (padded(wj) * 10 <= padded(p.wj) * 8) p.wj = wj;
-    const int tile = per_warp * p.wj, ksplit = 8 / p.wj;
-    const int64_t tiles = (nsamples + tile - 1) / tile, chunks = pad_spins(ns) / CHUNK;
-    const int64_t groups = (nc + GROUP - 1) / GROUP;
-    // Rounds: one part of a round's samples takes at most 256 MB of partial sums.
-    const size_t tile_bytes = sizeof(cplx<double>) * (size_t)ksplit * tile * nc, budget = size_t(256) << 20;
-    p.round_tiles = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)(budget / tile_bytes)));
-    // Spin parts: the waves of 2 CTAs per SM x (chunks of a CTA + 2 for its start and its sums) least.
-    const int64_t slots = 148 * 2, per_wave = p.round_tiles * groups;
-    const int64_t most = std::max<int64_t>(
-        1, std::min<int64_t>(std::min<int64_t>(chunks, 1024), (int64_t)(budget / (tile_bytes * p.round_tiles))));
-    int64_t best = INT64_MAX;
-    for (int64_t waves = 1; waves <= 8; ++waves) {
-        const int64_t n = std::max<int64_t>(1, std::min<int64_t>(most, waves * slots / per_wave));
-        const int64_t cost = ((per_wave * n + slots - 1) / slots) * ((chunks + n - 1) / n + 2);
-        if (cost < best) {
-            best = cost;
-            p.parts = (int)n;
-        }
-    }
-    p.partial_bytes = tile_bytes * p.round_tiles * p.parts;
-    return p;
+CoilCut precess64_cut(int64_t ns, int32_t nc, int64_t nsamples) {
+    return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, size_t(256) << 20);
 }
 
-cudaError_t precess64_run(const Precess64Args &a, const Precess64Plan &plan, cudaEvent_t ev_start,
+cudaError_t precess64_run(const Precess64Args &a, const CoilCut &cut, cudaEvent_t ev_start,
                           cudaEvent_t ev_stop, unsigned ev_flags, int64_t *launches, cudaStream_t stream) {
     const int64_t np = pad_spins(a.ns);
     const double *basis = static_cast<const double *>(a.table);
     const uint32_t slots = slot_mask(a.method);
     cudaError_t e;
     if (a.nsamples > 0) {
-        const int tile = warp_samples(a.nc) * plan.wj, groups = (a.nc + GROUP - 1) / GROUP, ksplit = 8 / plan.wj;
+        const int tile = cut.tile(a.nc), groups = (a.nc + COIL_GROUP - 1) / COIL_GROUP, ksplit = 8 / cut.wj;
         const int64_t tiles = (a.nsamples + tile - 1) / tile;
         if (ev_start) cudaEventRecordWithFlags(ev_start, stream, ev_flags);
-        for (int64_t t0 = 0; t0 < tiles; t0 += plan.round_tiles) {
-            const int64_t nt = std::min(plan.round_tiles, tiles - t0);
+        for (int64_t t0 = 0; t0 < tiles; t0 += cut.round_tiles) {
+            const int64_t nt = std::min(cut.round_tiles, tiles - t0);
             KernelArgs ka;
             ka.ns = a.ns;
             ka.nsamples = a.nsamples;
@@ -430,7 +389,7 @@ cudaError_t precess64_run(const Precess64Args &a, const Precess64Plan &plan, cud
             ka.round_samples = std::min<int64_t>(nt * tile, a.nsamples - ka.sample0);
             ka.nchunks = np / CHUNK;
             ka.nc = a.nc;
-            ka.parts = plan.parts;
+            ka.parts = cut.parts;
             ka.slots = slots;
             ka.basis = basis;
             ka.r2 = basis + TERMS * np;
@@ -438,12 +397,14 @@ cudaError_t precess64_run(const Precess64Args &a, const Precess64Plan &plan, cud
             ka.xy = a.xy;
             ka.csm_rows = a.csm_rows;
             ka.partial = a.partial;
-            e = a.nc <= 8 ? launch<1>(plan.wj, ka, nt, groups, stream)
-                          : a.nc <= 16 ? launch<2>(plan.wj, ka, nt, groups, stream)
-                                       : launch<4>(plan.wj, ka, nt, groups, stream);
+            switch (coil_tiles(a.nc)) {
+                case 1: e = launch<1>(cut.wj, ka, nt, groups, stream); break;
+                case 2: e = launch<2>(cut.wj, ka, nt, groups, stream); break;
+                default: e = launch<4>(cut.wj, ka, nt, groups, stream); break;
+            }
             if (e != cudaSuccess) return e;
-            if (ev_stop && t0 + plan.round_tiles >= tiles) cudaEventRecordWithFlags(ev_stop, stream, ev_flags);
-            e = launch_partial_finalize<double>(a.partial, (int64_t)plan.parts * ksplit, ka.round_samples, a.nc,
+            if (ev_stop && t0 + cut.round_tiles >= tiles) cudaEventRecordWithFlags(ev_stop, stream, ev_flags);
+            e = launch_partial_finalize(a.partial, (int64_t)cut.parts * ksplit, ka.round_samples, a.nc,
                                                 a.sig + ka.sample0, a.ldsig, stream);
             if (e != cudaSuccess) return e;
             if (launches) *launches += 2;

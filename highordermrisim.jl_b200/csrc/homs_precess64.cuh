@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "homs_common.cuh"
+#include "homs_fp64mma.cuh"
 
 namespace homs {
 
@@ -15,16 +16,8 @@ size_t precess64_table_bytes(int64_t ns);
 cudaError_t precess64_table(const double *x, const double *y, const double *z, const double *dw, const double *T2,
                             int64_t ns, void *table, cudaStream_t stream);
 
-// How a segment of `nsamples` samples is cut: sample tiles of 16 * wj, `parts`
-// ranges of spin chunks, and rounds of at most `round_tiles` tiles whose
-// partial sums fit the workspace.
-struct Precess64Plan {
-    int wj = 8;
-    int parts = 1;
-    int64_t round_tiles = 0;
-    size_t partial_bytes = 0;
-};
-Precess64Plan precess64_plan(int64_t ns, int32_t nc, int64_t nsamples);
+// How a segment is cut (homs_fp64mma.cuh); its partial sums take at most 256 MB.
+CoilCut precess64_cut(int64_t ns, int32_t nc, int64_t nsamples);
 
 struct Precess64Args {
     int64_t ns, nsamples;
@@ -36,13 +29,13 @@ struct Precess64Args {
     const double *T1, *T2, *rho;
     cplx<double> *xy;  // state at the segment's start, replaced by the state at its end
     double *mz;
-    cplx<double> *partial;  // plan.partial_bytes
+    cplx<double> *partial;  // cut.partial_bytes
     cplx<double> *sig;      // sample 0 of coil 0; coil stride ldsig
     int64_t ldsig;
 };
 // The segment's signal and its final state.  ev_start / ev_stop (may be NULL)
 // bracket the main kernel's launches; *launches counts kernels.
-cudaError_t precess64_run(const Precess64Args &a, const Precess64Plan &plan, cudaEvent_t ev_start,
+cudaError_t precess64_run(const Precess64Args &a, const CoilCut &cut, cudaEvent_t ev_start,
                           cudaEvent_t ev_stop, unsigned ev_flags, int64_t *launches, cudaStream_t stream);
 
 }  // namespace homs

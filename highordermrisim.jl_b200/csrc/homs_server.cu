@@ -85,7 +85,12 @@ size_t estimate_bytes(int64_t nspins, int32_t ncoils, homs_dtype dtype, const ho
         b += tiles * slots * 128 * 64 * 8 + (double)nadc * (192.0 + 96.0 + 8.0);
     } else {
         const double grid = std::ceil(ns / 256.0);
-        b += std::min(768.0 * (1 << 20), grid * nc * 2 * es * (double)nadc);  // split-K partials
+        b += std::min(512.0 * (1 << 20), grid * nc * 2 * es * (double)nadc);  // partial sums
+        if (es == 8.0)
+            b += (resident ? 0.0 : ns * 136.0) + (double)nadc * 192.0;  // spin table, prefix table
+        else  // phases and initial states of a round, node table
+            b += std::min(384.0 * (1 << 20), ns * 4.0 * (double)nadc) + std::min(64.0 * (1 << 20), ns * 8.0 * q.nblocks) +
+                 nt * 80.0;
     }
     return (size_t)(b + (64 << 20));
 }

@@ -3,9 +3,9 @@
     python -m homs.build            # from highordermrisim.jl_b200/
     python highordermrisim.jl_b200/homs/build.py
 
-homs_plain.cu is compiled with -fmad=false (no multiply-add contraction, so
-its results follow the reference's rounding order); everything else uses
-default contraction.
+homs_plain.cu and homs_precess32.cu are compiled with -fmad=false (no
+multiply-add contraction, so their results follow the reference's rounding
+order); everything else uses default contraction.
 """
 from __future__ import annotations
 
@@ -25,6 +25,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-Xptxas", "-v"]
 UNITS = {
     "homs_plain.cu": ["-fmad=false"],
+    "homs_precess32.cu": ["-fmad=false"],
     "homs_precess64.cu": [],
     "homs_split.cu": [],
     "homs_api.cu": [],
