@@ -73,6 +73,10 @@ template <typename T>
 cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st,
                            const SegmentArgs<T> &a, int grid, cudaStream_t stream);
 
+// An FP64 excitation launch without ADC samples (homs_excite64.cu).
+cudaError_t launch_excite64(const PhantomDev<double> &p, const SeqDev<double> &q, StateDev<double> &st,
+                            const SegmentArgs<double> &a, cudaStream_t stream);
+
 // Sum of nparts partial (nsamples x nc) blocks into sig, added in type P, in an
 // order that depends on nparts only.
 template <typename P, typename S>

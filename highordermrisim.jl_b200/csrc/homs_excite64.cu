@@ -1,0 +1,151 @@
+// RF excitation in FP64 without acquisition during the pulse: one thread per
+// spin walks the pulse's nodes.
+//
+// Per node the magnetisation turns about B = (Re B1, Im B1, Bz) by the angle
+// -2 pi gamma |B| dt and relaxes (hard-pulse spinor of
+// src/simulation/kernels/HighOrderGPU.jl:181-192 and
+// src/simulation/Bloch/BlochHighOrderSimulatitonMethod.jl:100-134).  As a
+// rotation of (Mx, My, Mz): with half-angle cosine w and sine v about the unit
+// field n, t = q x M and M' = M + w' t + q x t for q = sqrt(2) v n, w' = sqrt(2) w:
+// 15 operations where the spinor's complex products take about 60.
+//
+// What bounds it: the FP64 pipe and its latency, about 45 operations per spin and
+// node (field 4, |B| and 1/|B| 7, half-angle cosine and sine 17, rotation 21,
+// relaxation 3).  The rotations of UNROLL nodes are formed before they are
+// applied, so that only rotation and relaxation are in the spin's dependent
+// chain.  CTAs of 64 threads spread an uneven number of warps over the SMs.
+//
+// Measured (B200, against the spinor kernel of homs_plain.cu): 80,000 spins x 400
+// nodes 449 -> 168 us; a TR loop of 35 such pulses with its split-mode readouts
+// 28.2 -> 18.7 ms.
+#include <algorithm>
+
+#include "homs_common.cuh"
+#include "homs_fp64math.cuh"
+
+namespace homs {
+
+namespace excite64 {
+
+constexpr int THREADS = 64;
+constexpr int NODES = 64;  // nodes per stage
+constexpr int UNROLL = 4;  // rotations formed together (2: 18.89, 3: 18.79, 4: 18.70 ms for the TR loop below)
+
+// 1/sqrt(x) from the hardware's approximation (2^-20 or better) by one step of
+// third order; 0 for x below 1e-300 (no field), NaN for NaN.
+__device__ __forceinline__ double rsq(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    y = fma(y * e, fma(0.375, e, 0.5), y);
+    return x < 1e-300 ? 0.0 : y;
+}
+
+// Spin-independent part of a node's step (the interval that starts there).
+// Its relaxation relative to the stage's first interval dt0: SAME for an equal
+// dt; NEAR for one within 1e-9 dt0 (the differences of rounded node times), dt -
+// dt0 to first order; OTHER anew.
+enum : int { SAME, NEAR, OTHER };
+struct alignas(16) Node {
+    double gx, gy, gz, dfg;  // gradient, df / gamma
+    double b1r, b1i, b2, c;  // B1, |B1|^2, -gamma dt / 2 (half-angle in turns per tesla)
+    double dt;               // dt, or dt - dt0 (NEAR)
+    int relax;
+};
+struct Rotation {
+    double w, x, y, z;
+};
+
+__global__ void __launch_bounds__(THREADS, 9)
+    excite_kernel(PhantomDev<double> p, SeqDev<double> q, StateDev<double> st, SegmentArgs<double> a) {
+    __shared__ Node nodes[NODES];
+    const int64_t s = (int64_t)blockIdx.x * THREADS + threadIdx.x;
+    const bool active = s < p.ns;
+    const int64_t si = active ? s : 0;
+    const double px = p.x[si], py = p.y[si], pz = p.z[si], rho = p.rho[si], T1 = p.T1[si], T2 = p.T2[si];
+    const double off = (a.method & HOMS_DW_EXCITATION) ? p.dw[si] / (2.0 * 3.141592653589793 * a.gamma_d) : 0.0;
+    double mx = active ? st.xy[si].re : 0.0, my = active ? st.xy[si].im : 0.0, mz = active ? st.z[si] : 0.0;
+    auto turn = [&](double psi) {  // Mxy cis(psi)
+        double sn, cs;
+        sincos(psi, &sn, &cs);
+        const double x = mx * cs - my * sn;
+        my = mx * sn + my * cs;
+        mx = x;
+    };
+    // The frame of psi: entered at the first block's start and left at the last
+    // one's end; the blocks between leave and enter it at the same node.
+    if (a.block_start) turn(-q.psi[a.n_lo]);
+
+    // Relaxation over the stage's first interval: factors, rho (1 - e1).
+    double e1 = 0.0, e2 = 0.0, c1 = 0.0;
+    auto rotation = [&](const Node &n) {
+        const double bz = fma(n.gx, px, fma(n.gy, py, fma(n.gz, pz, off - n.dfg)));
+        const double B2 = fma(bz, bz, n.b2);
+        const double rB = rsq(B2);
+        const double th = n.c * (B2 * rB);
+        double ch, sh;
+        if (__all_sync(0xffffffffu, (__double2hiint(th) & 0x7FFFFFFF) < 0x3FC00000)) cis_eighth(th, ch, sh);
+        else cis_turns(th, ch, sh);
+        constexpr double SQRT2 = 1.4142135623730951;
+        const double f = (SQRT2 * sh) * rB;
+        return Rotation{SQRT2 * ch, n.b1r * f, n.b1i * f, bz * f};
+    };
+    auto step = [&](const Rotation &r, const Node &n) {
+        const double tx = fma(r.y, mz, -(r.z * my)), ty = fma(r.z, mx, -(r.x * mz)), tz = fma(r.x, my, -(r.y * mx));
+        const double nx = fma(r.w, tx, mx), ny = fma(r.w, ty, my), nz = fma(r.w, tz, mz);
+        double f2 = e2, f1 = e1, g1 = c1;
+        if (n.relax != SAME) {
+            f2 = n.relax == NEAR ? fma(e2, -n.dt / T2, e2) : exp(-n.dt / T2);
+            f1 = n.relax == NEAR ? fma(e1, -n.dt / T1, e1) : exp(-n.dt / T1);
+            g1 = rho * (1.0 - f1);
+        }
+        mx = fma(r.y, tz, fma(-r.z, ty, nx)) * f2;
+        my = fma(r.z, tx, fma(-r.x, tz, ny)) * f2;
+        mz = fma(fma(r.x, ty, fma(-r.y, tx, nz)), f1, g1);
+    };
+    for (int64_t n0 = a.n_lo; n0 < a.n_hi; n0 += NODES) {
+        const int cnt = (int)imin64(NODES, a.n_hi - n0);
+        __syncthreads();
+        const double dt0 = q.dt[n0];
+        for (int i = threadIdx.x; i < cnt; i += THREADS) {
+            const int64_t g = n0 + i;
+            const cplx<double> b1 = q.b1[g];
+            const double dt = q.dt[g], d = dt - dt0;
+            const int relax = d == 0.0 ? SAME : fabs(d) <= 1e-9 * dt0 ? NEAR : OTHER;
+            nodes[i] = Node{q.gx[g], q.gy[g], q.gz[g], q.df[g] / a.gamma_d, b1.re, b1.im,
+                            b1.re * b1.re + b1.im * b1.im, -0.5 * a.gamma_d * dt, relax == NEAR ? d : dt, relax};
+        }
+        if (n0 == a.n_lo || dt0 != q.dt[n0 - NODES]) {
+            e2 = exp(-dt0 / T2);
+            e1 = exp(-dt0 / T1);
+            c1 = rho * (1.0 - e1);
+        }
+        __syncthreads();
+        constexpr int U = UNROLL;
+        int i = 0;
+        for (; i + U <= cnt; i += U) {
+            Rotation r[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) r[u] = rotation(nodes[i + u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) step(r[u], nodes[i + u]);
+        }
+        for (; i < cnt; ++i) step(rotation(nodes[i]), nodes[i]);
+    }
+    if (q.boundary[a.n_hi]) turn(q.psi[a.n_hi]);
+    if (active) {
+        st.xy[s] = cplx<double>{mx, my};
+        st.z[s] = mz;
+    }
+}
+
+}  // namespace excite64
+
+cudaError_t launch_excite64(const PhantomDev<double> &p, const SeqDev<double> &q, StateDev<double> &st,
+                            const SegmentArgs<double> &a, cudaStream_t stream) {
+    const int64_t grid = (p.ns + excite64::THREADS - 1) / excite64::THREADS;
+    excite64::excite_kernel<<<(unsigned)grid, excite64::THREADS, 0, stream>>>(p, q, st, a);
+    return cudaGetLastError();
+}
+
+}  // namespace homs

@@ -1,0 +1,75 @@
+// FP64 functions of the precession and excitation kernels, written for their
+// arguments; each stays within 1.4e-16 of the exact value (absolute for the
+// cosine and sine, relative for the power).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace homs {
+
+// cos and sin of 2 pi r for |r| <= 1/8: sin(2 pi r) / r is a polynomial of degree 6
+// and (cos(2 pi r) - 1) / r^2 one of degree 6 in r^2, the interpolants at the
+// Chebyshev nodes of the interval (relative error 4e-18 before the coefficients'
+// rounding); 16 FP64 operations.
+__device__ __forceinline__ void cis_eighth(double r, double &cs, double &sn) {
+    const double z = r * r;
+    double s = 3.7808689593022957, c = -1.6990343940660637;
+    s = fma(s, z, -15.093804209987114);
+    c = fma(c, z, 7.903206911569678);
+    s = fma(s, z, 42.058685020160894);
+    c = fma(c, z, -26.426253275854723);
+    s = fma(s, z, -76.70585970427454);
+    c = fma(c, z, 60.24464135270201);
+    s = fma(s, z, 81.60524927594804);
+    c = fma(c, z, -85.4568172066438);
+    s = fma(s, z, -41.341702240399634);
+    c = fma(c, z, 64.93939402266824);
+    s = fma(s, z, 6.283185307179586);
+    c = fma(c, z, -19.739208802178716);
+    sn = s * r;
+    cs = fma(c, z, 1.0);
+}
+
+// cos and sin of 2 pi theta: theta is reduced to its nearest quarter turn (an
+// exact subtraction).  Beyond 2^48 turns (infinities and NaN included) it is first
+// reduced to the nearest turn.
+__device__ __forceinline__ void cis_turns(double th, double &cs, double &sn) {
+    if ((__double2hiint(th) & 0x7FFFFFFF) >= 0x42F00000) th -= rint(th);
+    constexpr double MAGIC = 6755399441055744.0;  // 1.5 * 2^52: adds round to an integer
+    const double t = fma(th, 4.0, MAGIC);
+    const int quad = __double2loint(t);
+    const double r = fma(t - MAGIC, -0.25, th);
+    double s, c;
+    cis_eighth(r, c, s);
+    // a quarter turn swaps the two and a half turn flips both signs
+    const double a = (quad & 1) ? s : c, b = (quad & 1) ? c : s;
+    cs = __hiloint2double(__double2hiint(a) ^ (((quad + 1) & 2) << 30), __double2loint(a));
+    sn = __hiloint2double(__double2hiint(b) ^ ((quad & 2) << 30), __double2loint(b));
+}
+
+// 2^y: nearest integer k, then 1 + f q(f) on |f| <= 1/2 with q the degree-10
+// interpolant of (2^f - 1) / f at the Chebyshev nodes (relative error 1e-17 before
+// the coefficients' rounding), and k added to the exponent; 15 FP64 operations.
+// |y| >= 1008 (infinities and NaN included) goes to exp2.
+__device__ __forceinline__ double pow2(double y) {
+    if ((__double2hiint(y) & 0x7FFFFFFF) >= 0x408F8000) return exp2(y);
+    constexpr double MAGIC = 6755399441055744.0;
+    const double t = y + MAGIC;
+    const int k = __double2loint(t);
+    const double f = y - (t - MAGIC);
+    double p = 4.4549605981865186e-10;
+    p = fma(p, f, 7.072585949269223e-09);
+    p = fma(p, f, 1.0178062445845774e-07);
+    p = fma(p, f, 1.321544258792169e-06);
+    p = fma(p, f, 1.525273382983612e-05);
+    p = fma(p, f, 0.0001540353044173605);
+    p = fma(p, f, 0.0013333558146416936);
+    p = fma(p, f, 0.009618129107606888);
+    p = fma(p, f, 0.0555041086648216);
+    p = fma(p, f, 0.24022650695910097);
+    p = fma(p, f, 0.6931471805599453);
+    p = fma(p, f, 1.0);
+    return __hiloint2double(__double2hiint(p) + (k << 20), __double2loint(p));
+}
+
+}  // namespace homs

@@ -133,13 +133,6 @@ __device__ void reduce_stage(const cplx<T> *X, cplx<T> *P, int na, const cplx<T>
     }
 }
 
-// Shared memory of a segment without ADC samples: the node cache alone (the
-// kernel stages no samples and no sensitivities then).
-template <typename T>
-size_t segment_smem_bytes_no_adc() {
-    return (sizeof(NodeCache<T>) + 127) & ~size_t(127);
-}
-
 template <typename T>
 size_t segment_smem_bytes(int32_t nc) {
     size_t bytes = sizeof(NodeCache<T>) + 2 * sizeof(cplx<T>) * PLAIN_STAGE * PLAIN_THREADS;
@@ -152,10 +145,18 @@ size_t segment_smem_bytes(int32_t nc) {
 // node range in lockstep, so ADC staging and the coil reduction are
 // CTA-uniform.  Per node a hard-pulse spinor
 // (BlochHighOrderSimulatitonMethod.jl:100-134; kernels/HighOrderGPU.jl:181-192).
-// Three CTAs per SM (80 registers: launches without ADC samples use the node
-// cache alone).
-template <typename T>
-__global__ void __launch_bounds__(PLAIN_THREADS, 3)
+// ADC: the launch acquires samples (256 threads, the coil reduction's shape).
+// Else (FP32 only; FP64 pulses without samples run in homs_excite64.cu) the node
+// cache is all it holds, CTAs of 64 threads spread the warps evenly over the
+// SMs, and the spinors of UNROLL nodes, which do not depend on the state, are
+// formed together before they are applied.  Bound by latency and issue (about
+// 150 unfused instructions per node in a chain of square root, sine, reciprocal
+// and complex products): 29,929 spins x 64 nodes 27.3 -> 24.8 us.  The
+// operations and their order stay the reference's: FP32 roundings of a pulse's
+// nodes add up in one direction, and the rotation form of homs_excite64.cu, though
+// more exact, ends 4e-5 away from them after 48 pulses.
+template <typename T, bool ADC>
+__global__ void __launch_bounds__(ADC ? PLAIN_THREADS : 64, ADC ? 3 : 8)
     excitation_kernel(PhantomDev<T> p, SeqDev<T> q, StateDev<T> st, SegmentArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     NodeCache<T> &nc = *reinterpret_cast<NodeCache<T> *>(smem_raw);
@@ -163,15 +164,12 @@ __global__ void __launch_bounds__(PLAIN_THREADS, 3)
     cplx<T> *P = X + PLAIN_STAGE * PLAIN_THREADS;
     cplx<T> *csm_s = P + PLAIN_STAGE * PLAIN_THREADS;
 
-    const int64_t spin0 = (int64_t)blockIdx.x * PLAIN_THREADS;
+    const int64_t spin0 = (int64_t)blockIdx.x * blockDim.x;
     const int64_t s = spin0 + threadIdx.x;
     const bool active = s < p.ns;
     const int nvalid = (int)imin64(PLAIN_THREADS, p.ns - spin0);
     const int32_t ncoil = p.nc;
-    // A segment without ADC samples stages nothing (and is launched with the
-    // node cache alone).
-    const bool stage_adc = a.nsamples > 0;
-    const bool csm_in_smem = stage_adc && sizeof(cplx<T>) * (size_t)ncoil * PLAIN_THREADS <= 128 * 1024;
+    const bool csm_in_smem = ADC && sizeof(cplx<T>) * (size_t)ncoil * PLAIN_THREADS <= 128 * 1024;
 
     // Stage this CTA's sensitivities (rows s, coil-fastest).
     const cplx<T> *csm_rows;
@@ -214,22 +212,26 @@ __global__ void __launch_bounds__(PLAIN_THREADS, 3)
             Math<T>::sc(-nc.psi[0], &sn, &cs);
             xy = cmul(xy, cplx<T>{cs, sn});
         }
-        for (int i = 0; i < nint; ++i) {
-            const T dt = nc.dt[i];
+        // Spinor of the interval that starts at cached node i.
+        auto spinor = [&](int i, cplx<T> &al, cplx<T> &be) {
             const T dbz = off - nc.dfg[i];
             const T bz = ((nc.g[0][i] * px + nc.g[1][i] * py) + nc.g[2][i] * pz) + dbz;
             const cplx<T> b1 = nc.b1[i];
             const T ab1 = nc.ab1[i];
             T B = Math<T>::sq(ab1 * ab1 + bz * bz);
             if (B == T(0)) B = Math<T>::eps();
-            const T phi = c_neg * (B * dt);
+            const T phi = c_neg * (B * nc.dt[i]);
             T sh, ch;
             Math<T>::sc(phi / T(2), &sh, &ch);
             // Unit field direction (one reciprocal; within an ulp of three divisions).
             const T rB = T(1) / B;
             const T nz = bz * rB, nxr = b1.re * rB, nxi = b1.im * rB;
-            const cplx<T> al{ch, -(nz * sh)};
-            const cplx<T> be{nxi * sh, -(nxr * sh)};
+            al = cplx<T>{ch, -(nz * sh)};
+            be = cplx<T>{nxi * sh, -(nxr * sh)};
+        };
+        // Rotation by the spinor, then relaxation over the interval.
+        auto apply = [&](int i, const cplx<T> &al, const cplx<T> &be) {
+            const T dt = nc.dt[i];
             cplx<T> t1 = cmul(cplx<T>{T(2) * al.re, -(T(2) * al.im)}, be);
             t1.re = t1.re * mz;
             t1.im = t1.im * mz;
@@ -250,19 +252,9 @@ __global__ void __launch_bounds__(PLAIN_THREADS, 3)
             }
             xy = cplx<T>{nxy.re * e2_rel, nxy.im * e2_rel};
             mz = nz2 * e1_rel + rho * (T(1) - e1_rel);
-            if (stage_adc && nc.adc[i + 1]) {
-                T sn, cs;
-                Math<T>::sc(nc.psi[i + 1], &sn, &cs);
-                const cplx<T> xs = cmul(xy, cplx<T>{cs, sn});
-                X[staged * PLAIN_THREADS + threadIdx.x] = active ? xs : cplx<T>{T(0), T(0)};
-                staged++;
-                if (staged == PLAIN_STAGE) {
-                    __syncthreads();
-                    reduce_stage(X, P, staged, csm_rows, csm_ld, nvalid, ncoil, out_base + sample * ncoil);
-                    sample += staged;
-                    staged = 0;
-                }
-            }
+        };
+        // Block end: leave the frame of psi, and enter it again for the next block.
+        auto frame = [&](int i) {
             if (nc.bnd[i + 1]) {
                 T sn, cs;
                 Math<T>::sc(nc.psi[i + 1], &sn, &cs);
@@ -272,9 +264,49 @@ __global__ void __launch_bounds__(PLAIN_THREADS, 3)
                     xy = cmul(xy, cplx<T>{cs, sn});
                 }
             }
+        };
+        if (ADC) {
+            for (int i = 0; i < nint; ++i) {
+                cplx<T> al, be;
+                spinor(i, al, be);
+                apply(i, al, be);
+                if (nc.adc[i + 1]) {
+                    T sn, cs;
+                    Math<T>::sc(nc.psi[i + 1], &sn, &cs);
+                    const cplx<T> xs = cmul(xy, cplx<T>{cs, sn});
+                    X[staged * PLAIN_THREADS + threadIdx.x] = active ? xs : cplx<T>{T(0), T(0)};
+                    staged++;
+                    if (staged == PLAIN_STAGE) {
+                        __syncthreads();
+                        reduce_stage(X, P, staged, csm_rows, csm_ld, nvalid, ncoil, out_base + sample * ncoil);
+                        sample += staged;
+                        staged = 0;
+                    }
+                }
+                frame(i);
+            }
+        } else {
+            constexpr int UNROLL = 4;
+            int i = 0;
+            for (; i + UNROLL <= nint; i += UNROLL) {
+                cplx<T> al[UNROLL], be[UNROLL];
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) spinor(i + u, al[u], be[u]);
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) {
+                    apply(i + u, al[u], be[u]);
+                    frame(i + u);
+                }
+            }
+            for (; i < nint; ++i) {
+                cplx<T> al, be;
+                spinor(i, al, be);
+                apply(i, al, be);
+                frame(i);
+            }
         }
     }
-    if (staged > 0) {
+    if (ADC && staged > 0) {
         __syncthreads();
         reduce_stage(X, P, staged, csm_rows, csm_ld, nvalid, ncoil, out_base + sample * ncoil);
     }
@@ -403,10 +435,17 @@ __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
 template <typename T>
 cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st, const SegmentArgs<T> &a,
                               int grid, cudaStream_t stream) {
-    const size_t smem = a.nsamples > 0 ? segment_smem_bytes<T>(p.nc) : segment_smem_bytes_no_adc<T>();
-    cudaError_t e = allow_max_dynamic_smem((const void *)excitation_kernel<T>);
+    if (a.nsamples == 0) {
+        if constexpr (sizeof(T) == 8) {
+            return launch_excite64(p, q, st, a, stream);
+        } else {
+            excitation_kernel<T, false><<<(unsigned)((p.ns + 63) / 64), 64, sizeof(NodeCache<T>), stream>>>(p, q, st, a);
+            return cudaGetLastError();
+        }
+    }
+    cudaError_t e = allow_max_dynamic_smem((const void *)excitation_kernel<T, true>);
     if (e != cudaSuccess) return e;
-    excitation_kernel<T><<<grid, PLAIN_THREADS, smem, stream>>>(p, q, st, a);
+    excitation_kernel<T, true><<<grid, PLAIN_THREADS, segment_smem_bytes<T>(p.nc), stream>>>(p, q, st, a);
     return cudaGetLastError();
 }
 

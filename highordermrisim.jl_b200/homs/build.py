@@ -25,6 +25,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-Xptxas", "-v"]
 UNITS = {
     "homs_plain.cu": ["-fmad=false"],
+    "homs_excite64.cu": [],
     "homs_precess32.cu": ["-fmad=false"],
     "homs_precess64.cu": [],
     "homs_split.cu": [],
