@@ -11,8 +11,10 @@
 // not contract multiply-adds; the FP64 kernel therefore agrees with the FP64
 // CPU restatement to ~1e-15.
 #include <cfloat>
+#include <type_traits>
 
 #include "homs_common.cuh"
+#include "homs_fp64mma.cuh"
 
 namespace homs {
 
@@ -358,77 +360,169 @@ __global__ void __launch_bounds__(FIN_OUT *FIN_SLICES)
 }
 
 // Standalone coil reduction (states^T csm, no conjugation), split-K over spin
-// ranges.  CTA (p, jt, ct) sums spins [ns p / P, ns (p + 1) / P) for samples
-// 64 jt .. +63 and coils 32 ct .. +31 into its partial block: chunks of 16
-// spins of both operands are staged in shared memory with coalesced loads
-// along the spins (both arrays are column-major), then thread t accumulates
-// sample t % 64 against coils 8 (t / 64) .. +7 in registers (a warp reads 32
-// consecutive samples of one spin; the 8 sensitivities are broadcasts).
-constexpr int CR_JB = 64, CR_CB = 32, CR_SK = 16, CR_THREADS = 256, CR_CTAS_PER_SM = 2;
-constexpr int CR_XL = CR_SK * CR_JB / CR_THREADS, CR_CL = CR_SK * CR_CB / CR_THREADS;  // loads per thread and chunk
+// ranges.  CTA (p, jt, ct) sums the p-th range of 32-spin chunks for samples
+// 8 WJ jt .. and coils 8 NT ct .. into its partial block.  Both operands are
+// column-major, so a chunk is a set of short rows (32 consecutive spins of a
+// sample or of a coil), staged by asynchronous copies a chunk ahead, and the
+// product is taken by FP64 matrix instructions (m8n8k4, samples x spins times
+// spins x coils; FP32 operands are widened, their products and sums kept in
+// FP64).  Warp w takes the tile's samples 8 (w % WJ) .. +7; the 8 / WJ warps that
+// share them split a chunk's spins and are added at the end in warp order.
+//
+// What bounds it: for many coils the FP64 pipe, 4 multiply-adds per spin, sample
+// and coil (FP32: 3, by three products, whose extra rounding is lost in FP64; in
+// FP64 they would raise the error from 2.65e-15 to 2.78e-15), 91 us at its peak for
+// 200,000 x 64 x 32 in FP64; for few, memory.  Measured (B200, with the finalize;
+// against register-blocked multiply-adds from shared memory, which spent their
+// issue slots on loads): 200,000 x 64 x 32 FP64 200 -> 138 us, FP32 121 -> 111;
+// 200,000 x 64 x 8 FP64 188 -> 59; 200,000 x 96 x 1 FP32 205 -> 80; 30,011 x 33 x 31
+// FP64 47 -> 35; 5,000 x 17 x 3 FP64 41 -> 13.  Chunks of 16 spins in 3 stages: 142 us
+// for the first; 32 in 3, which leaves one CTA per SM: 171.
+constexpr int CR_SK = 32, CR_THREADS = 256, CR_CTAS_PER_SM = 2, CR_STAGES = 2;
+// Bytes of a staged row (CR_SK spins and a pad that keeps fragment loads conflict-free).
 template <typename T>
+constexpr int cr_row() {
+    return (int)sizeof(cplx<T>) * CR_SK + (sizeof(T) == 8 ? 64 : 32);
+}
+template <typename T>
+constexpr int cr_stage(int nt, int wj) {
+    return 8 * (nt + wj) * cr_row<T>();
+}
+template <typename T, int NT, int WJ>
 __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
     coil_reduce_kernel(int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
-                       const cplx<T> *csm, int64_t ldcsm, int64_t parts, cplx<T> *partial) {
-    __shared__ cplx<T> Xs[CR_SK][CR_JB + 1];
-    __shared__ cplx<T> Cs[CR_SK][CR_CB + 1];
-    const int64_t p = blockIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.y * CR_JB;
-    const int c0 = (int)blockIdx.z * CR_CB;
-    const int jn = (int)imin64(CR_JB, nadc - j0), cn = (int)imin64(CR_CB, nc - c0);
-    const int64_t s_begin = ns * p / parts, s_end = ns * (p + 1) / parts;
-    const int t = threadIdx.x;
-    const int jl = t % CR_JB, cb = (t / CR_JB) * 8;
-    // The next chunk's operands are fetched into registers while the current
-    // chunk is contracted from shared memory.
-    cplx<T> xr[CR_XL], cr[CR_CL];
-    auto fetch = [&](int64_t s0) {
-        const int sn = (int)imin64(CR_SK, s_end - s0);
-#pragma unroll
-        for (int r = 0; r < CR_XL; ++r) {
-            const int i = t + r * CR_THREADS, sl = i % CR_SK, jj = i / CR_SK;
-            xr[r] = (sl < sn && jj < jn) ? states[(s0 + sl) + (j0 + jj) * ldstates] : cplx<T>{T(0), T(0)};
-        }
-#pragma unroll
-        for (int r = 0; r < CR_CL; ++r) {
-            const int i = t + r * CR_THREADS, sl = i % CR_SK, c = i / CR_SK;
-            cr[r] = (sl < sn && c < cn) ? csm[(s0 + sl) + (int64_t)(c0 + c) * ldcsm] : cplx<T>{T(0), T(0)};
+                       const cplx<T> *csm, int64_t ldcsm, int64_t parts, int width, cplx<T> *partial) {
+    using Pair = std::conditional_t<sizeof(T) == 8, double2, float2>;
+    constexpr int ROW = cr_row<T>(), STAGE = cr_stage<T>(NT, WJ), KS = 8 / WJ, JB = 8 * WJ, CB = 8 * NT;
+    extern __shared__ __align__(16) uint8_t cr_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, r = lane >> 2;
+    const int wj = warp % WJ, kw = warp / WJ;
+    const int64_t p = blockIdx.x, j0 = (int64_t)blockIdx.y * JB;
+    const int c0 = (int)blockIdx.z * CB;
+    const int jn = (int)imin64(JB, nadc - j0), cn = (int)imin64(CB, nc - c0);
+    const int64_t nch = (ns + CR_SK - 1) / CR_SK, ch0 = nch * p / parts, ch1 = nch * (p + 1) / parts;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(cr_smem);
+    // Rows past the last sample or coil are zero in every stage.
+    for (int i = tid; i < CR_STAGES * STAGE / 16; i += CR_THREADS) {
+        const int row = i % (STAGE / 16) / (ROW / 16);
+        if (row < JB ? row >= jn : row - JB >= cn)
+            *reinterpret_cast<float4 *>(cr_smem + (size_t)i * 16) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    // One chunk into a stage, in pieces of `width` bytes (the alignment that the
+    // operands have); spins past the last one are zero.
+    const int pieces = CR_SK * (int)sizeof(cplx<T>) / width;  // per row: a power of two
+    const int shift = 31 - __clz(pieces);
+    auto issue = [&](int64_t ch, int stage) {
+        const int64_t s0 = ch * CR_SK;
+        const int64_t left = (ns - s0) * (int64_t)sizeof(cplx<T>);  // bytes of the rows from here on
+        for (int i = tid; i < (jn + cn) << shift; i += CR_THREADS) {
+            const int k = i >> shift, at = (i & (pieces - 1)) * width;
+            const char *src = reinterpret_cast<const char *>(k < jn ? states + (j0 + k) * ldstates + s0
+                                                                    : csm + (int64_t)(c0 + k - jn) * ldcsm + s0);
+            const uint32_t dst = sbase + (uint32_t)(stage * STAGE + (k < jn ? k : JB + k - jn) * ROW + at);
+            const int n = (int)imax64(0, imin64(width, left - at));
+            if (n > 0) src += at;
+            if (width == 16)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+            else if (width == 8)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
         }
     };
-    cplx<T> acc[8];
+    double re[NT][2], im[NT][2], k3[NT][2];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) acc[m] = cplx<T>{T(0), T(0)};
-    if (s_begin < s_end) fetch(s_begin);
-    for (int64_t s0 = s_begin; s0 < s_end; s0 += CR_SK) {
-        const int sn = (int)imin64(CR_SK, s_end - s0);
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) re[nt][e] = im[nt][e] = k3[nt][e] = 0.0;
+#pragma unroll
+    for (int s = 0; s < CR_STAGES - 1; ++s) {
+        if (ch0 + s < ch1) issue(ch0 + s, s);
+        cp_commit();
+    }
+    int stage = 0;
+    for (int64_t ch = ch0; ch < ch1; ++ch) {
+        cp_wait<CR_STAGES - 2>();
         __syncthreads();
+        if (ch + CR_STAGES - 1 < ch1) issue(ch + CR_STAGES - 1, stage == 0 ? CR_STAGES - 1 : stage - 1);
+        cp_commit();
+        const uint8_t *st = cr_smem + stage * STAGE;
+        if (++stage == CR_STAGES) stage = 0;
 #pragma unroll
-        for (int r = 0; r < CR_XL; ++r) {
-            const int i = t + r * CR_THREADS;
-            Xs[i % CR_SK][i / CR_SK] = xr[r];
-        }
+        for (int k = 0; k < CR_SK / 4; k += KS) {
+            const int at = (4 * (k + kw) + q) * (int)sizeof(cplx<T>);
+            const auto x = *reinterpret_cast<const Pair *>(st + (8 * wj + r) * ROW + at);
+            const double xr = x.x, xi = x.y;
+            double wr[NT], wi[NT];
 #pragma unroll
-        for (int r = 0; r < CR_CL; ++r) {
-            const int i = t + r * CR_THREADS;
-            Cs[i % CR_SK][i / CR_SK] = cr[r];
-        }
-        __syncthreads();
-        if (s0 + CR_SK < s_end) fetch(s0 + CR_SK);
-        for (int sl = 0; sl < sn; ++sl) {
-            const cplx<T> x = Xs[sl][jl];
+            for (int nt = 0; nt < NT; ++nt) {
+                const auto w = *reinterpret_cast<const Pair *>(st + (JB + 8 * nt + r) * ROW + at);
+                wr[nt] = w.x;
+                wi[nt] = w.y;
+            }
+            if (sizeof(T) == 8) {
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const cplx<T> w = Cs[sl][cb + m];
-                acc[m].re = fma(x.re, w.re, fma(-x.im, w.im, acc[m].re));
-                acc[m].im = fma(x.re, w.im, fma(x.im, w.re, acc[m].im));
+                for (int nt = 0; nt < NT; ++nt) dmma(re[nt], xr, wr[nt]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) dmma(im[nt], xr, wi[nt]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) dmma(re[nt], -xi, wi[nt]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) dmma(im[nt], xi, wr[nt]);
+            } else {
+                // three products: Re = k1 - k3, Im = k1 + k2
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    dmma(re[nt], xr + xi, wr[nt]);
+                    dmma(im[nt], xr, wi[nt] - wr[nt]);
+                    dmma(k3[nt], xi, wr[nt] + wi[nt]);
+                }
             }
         }
     }
-    if (jl < jn) {
-        cplx<T> *out = partial + (p * nadc + j0 + jl) * nc + c0;
+    cp_wait<0>();
+    if (sizeof(T) == 4)
 #pragma unroll
-        for (int m = 0; m < 8; ++m)
-            if (cb + m < cn) out[cb + m] = acc[m];
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                im[nt][e] += re[nt][e];
+                re[nt][e] -= k3[nt][e];
+            }
+    if (KS > 1) {  // add the warps that share the samples, in warp order
+        double *sums = reinterpret_cast<double *>(cr_smem);
+        __syncthreads();
+        if (kw > 0)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    double *d = sums + ((((kw - 1) * WJ + wj) * NT + nt) * 2 + e) * 64 + lane;
+                    d[0] = re[nt][e];
+                    d[32] = im[nt][e];
+                }
+        __syncthreads();
+        if (kw > 0) return;
+        for (int k = 0; k < KS - 1; ++k)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const double *d = sums + (((k * WJ + wj) * NT + nt) * 2 + e) * 64 + lane;
+                    re[nt][e] += d[0];
+                    im[nt][e] += d[32];
+                }
+    }
+    const int j = 8 * wj + r;
+    if (j < jn) {
+        cplx<T> *out = partial + (p * nadc + j0 + j) * nc + c0;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = 8 * nt + 2 * q + e;
+                if (c < cn) out[c] = cplx<T>{(T)re[nt][e], (T)im[nt][e]};
+            }
     }
 }
 
@@ -464,26 +558,53 @@ cudaError_t launch_partial_finalize(const cplx<T> *partial, int64_t nparts, int6
     return cudaGetLastError();
 }
 
+// Tile of the reduction: 8-coil tiles (1, 2 or 4) and warps along the samples (2,
+// 4 or 8), the smallest that take all coils (samples) or the largest.
+static int cr_coil_tiles(int32_t nc) { return nc <= 8 ? 1 : nc <= 16 ? 2 : 4; }
+static int cr_sample_warps(int64_t nadc) { return nadc <= 16 ? 2 : nadc <= 32 ? 4 : 8; }
+
 // Parts of the split-K: one wave of CR_CTAS_PER_SM CTAs per SM over all
 // (sample, coil) tiles, at least 256 spins per part (so at most
 // ceil(ns / PLAIN_THREADS) parts).
 int64_t coil_reduce_parts(int64_t ns, int64_t nadc, int32_t nc) {
-    const int64_t tiles = ((nadc + CR_JB - 1) / CR_JB) * ((nc + CR_CB - 1) / CR_CB);
+    const int jb = 8 * cr_sample_warps(nadc), cb = 8 * cr_coil_tiles(nc);
+    const int64_t tiles = ((nadc + jb - 1) / jb) * ((nc + cb - 1) / cb);
     const int64_t want = std::max<int64_t>(1, (148 * CR_CTAS_PER_SM) / tiles);
     return std::max<int64_t>(1, std::min<int64_t>(want, (ns + PLAIN_THREADS - 1) / PLAIN_THREADS));
+}
+
+template <typename T, int NT, int WJ>
+static cudaError_t cr_launch(dim3 grid, int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
+                             const cplx<T> *csm, int64_t ldcsm, int width, cplx<T> *partial, cudaStream_t stream) {
+    const size_t smem = std::max<size_t>(CR_STAGES * cr_stage<T>(NT, WJ), sizeof(double) * 128 * NT * (8 - WJ));
+    cudaError_t e = allow_max_dynamic_smem((const void *)coil_reduce_kernel<T, NT, WJ>);
+    if (e != cudaSuccess) return e;
+    coil_reduce_kernel<T, NT, WJ><<<grid, CR_THREADS, smem, stream>>>(ns, nadc, nc, states, ldstates, csm, ldcsm,
+                                                                      (int64_t)grid.x, width, partial);
+    return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_coil_reduce(int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
                                const cplx<T> *csm, int64_t ldcsm, cplx<T> *partial, cudaStream_t stream) {
     if (ns == 0 || nadc == 0 || nc == 0) return cudaSuccess;
+    const int nt = cr_coil_tiles(nc), wj = cr_sample_warps(nadc);
     const int64_t parts = coil_reduce_parts(ns, nadc, nc);
-    const int64_t jt = (nadc + CR_JB - 1) / CR_JB, ct = (nc + CR_CB - 1) / CR_CB;
+    const int64_t jt = (nadc + 8 * wj - 1) / (8 * wj), ct = (nc + 8 * nt - 1) / (8 * nt);
     if (jt > 65535 || ct > 65535) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)parts, (unsigned)jt, (unsigned)ct);
-    coil_reduce_kernel<T><<<grid, CR_THREADS, 0, stream>>>(ns, nadc, nc, states, ldstates, csm, ldcsm, parts,
-                                                          partial);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)parts, (unsigned)jt, (unsigned)ct);
+    // Widest copy that every row of both operands is aligned to.
+    const uint64_t bits = reinterpret_cast<uintptr_t>(states) | reinterpret_cast<uintptr_t>(csm) |
+                          (uint64_t)ldstates * sizeof(cplx<T>) | (uint64_t)ldcsm * sizeof(cplx<T>);
+    const int width = (bits & 15) == 0 ? 16 : (bits & 7) == 0 ? 8 : 4;
+#define CR_CASE(NT_, WJ_) \
+    if (nt == NT_ && wj == WJ_) \
+        return cr_launch<T, NT_, WJ_>(grid, ns, nadc, nc, states, ldstates, csm, ldcsm, width, partial, stream);
+    CR_CASE(1, 2) CR_CASE(1, 4) CR_CASE(1, 8)
+    CR_CASE(2, 2) CR_CASE(2, 4) CR_CASE(2, 8)
+    CR_CASE(4, 2) CR_CASE(4, 4) CR_CASE(4, 8)
+#undef CR_CASE
+    return cudaErrorInvalidValue;
 }
 
 template cudaError_t launch_excitation<double>(const PhantomDev<double> &, const SeqDev<double> &, StateDev<double> &,
