@@ -7,11 +7,15 @@
 // src/simulation/SimulatorCore.jl:96-152 is planned on the host into launches
 // of the fused segment kernels.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "homs_common.cuh"
@@ -66,6 +70,13 @@ struct DevBuf {
         bytes = src.bytes;
         owned = false;
     }
+    void view(void *at, size_t n) {
+        release();
+        p = at;
+        bytes = n;
+        owned = false;
+    }
+    size_t owned_bytes() const { return owned ? bytes : 0; }
     cudaError_t ensure(size_t n) {
         if (n <= bytes && p && owned) return cudaSuccess;
         release();
@@ -122,6 +133,92 @@ __global__ void transpose_csm_kernel(cplx<D> *dst, const S *src, int64_t ns, int
 
 inline int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 32)); }
 
+// Host copies between a caller's pageable arrays and a context's page-locked
+// chunks, shared by the calling thread and up to three helper threads (started
+// on the first large copy, joined with the context).  One thread copies about
+// 10 GB/s here and, into fresh pages, waits for the kernel to clear them.
+class CopyPool {
+public:
+    struct Piece {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    };
+    ~CopyPool() {
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            stop_ = true;
+        }
+        cv_.notify_all();
+        for (auto &t : threads_) t.join();
+    }
+    // Returns when every piece is copied.
+    void run(const std::vector<Piece> &pieces) {
+        size_t total = 0;
+        for (const Piece &p : pieces) total += p.bytes;
+        if (total < PARALLEL_MIN || !start()) {
+            for (const Piece &p : pieces) std::memcpy(p.dst, p.src, p.bytes);
+            return;
+        }
+        std::vector<Piece> work;
+        for (const Piece &p : pieces)
+            for (size_t off = 0; off < p.bytes; off += SLICE)
+                work.push_back({static_cast<char *>(p.dst) + off, static_cast<const char *>(p.src) + off,
+                                std::min(SLICE, p.bytes - off)});
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            work_ = &work;
+            next_.store(0);
+            busy_ = threads_.size();
+            ++round_;
+        }
+        cv_.notify_all();
+        drain(work);
+        std::unique_lock<std::mutex> l(mu_);
+        done_.wait(l, [&] { return busy_ == 0; });
+        work_ = nullptr;
+    }
+
+private:
+    static constexpr size_t PARALLEL_MIN = size_t(2) << 20, SLICE = size_t(1) << 20;
+    bool start() {
+        if (!threads_.empty()) return true;
+        const unsigned n = std::min(3u, std::thread::hardware_concurrency() / 4);
+        try {
+            for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { loop(); });
+        } catch (const std::system_error &) {  // no more threads: copy with those there are
+        }
+        return !threads_.empty();
+    }
+    void drain(const std::vector<Piece> &work) {
+        for (size_t i; (i = next_.fetch_add(1)) < work.size();) std::memcpy(work[i].dst, work[i].src, work[i].bytes);
+    }
+    void loop() {
+        uint64_t seen = 0;
+        for (;;) {
+            const std::vector<Piece> *work;
+            {
+                std::unique_lock<std::mutex> l(mu_);
+                cv_.wait(l, [&] { return stop_ || (work_ && round_ != seen); });
+                if (stop_) return;
+                seen = round_;
+                work = work_;
+            }
+            drain(*work);
+            std::lock_guard<std::mutex> l(mu_);
+            if (--busy_ == 0) done_.notify_one();
+        }
+    }
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable cv_, done_;
+    const std::vector<Piece> *work_ = nullptr;
+    std::atomic<size_t> next_{0};
+    size_t busy_ = 0;
+    uint64_t round_ = 0;
+    bool stop_ = false;
+};
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -136,9 +233,9 @@ struct homs_context {
     std::mutex mu;
     // reusable scratch
     DevBuf scratch_csm, scratch_partial, scratch_acc, scratch_bnd, scratch_sig, scratch_conv;
-    // Precession blocks: per-node values (sample index or block time), column
-    // sources, spin or node table, prefix table or phases, aligned copy of the state
-    DevBuf block_rank, block_src, block_table, block_prefix, block_xy;
+    // Precession blocks: per-node values (sample index or block time), spin or node
+    // table, prefix table or phases, aligned copy of the state
+    DevBuf block_rank, block_table, block_prefix, block_xy;
     // encoding export (homs_kspace): staged inputs, metadata, work and outputs,
     // and the events around its kernels
     DevBuf kspace_in, kspace_meta, kspace_work, kspace_out;
@@ -152,6 +249,7 @@ struct homs_context {
     void *stage[2] = {nullptr, nullptr};
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     int stage_next = 0;  // the chunk the next staged copy fills
+    CopyPool copies;     // moves bytes between the chunks and pageable arrays
     // Device workspace of homs_simulate, kept between calls (per dtype) so that
     // repeated simulations reuse their buffers instead of reallocating them.
     std::unique_ptr<struct ResidentBase> cache[2];
@@ -224,7 +322,7 @@ void h2d(homs_context *ctx, void *dst, const void *src, size_t bytes) {
         const int b = ctx->stage_next;
         ctx->stage_next ^= 1;
         HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));  // the copy that last read this chunk is done
-        std::memcpy(ctx->stage[b], s + off, n);
+        ctx->copies.run({{ctx->stage[b], s + off, n}});
         HOMS_CUDA(cudaMemcpyAsync(d + off, ctx->stage[b], n, cudaMemcpyHostToDevice, ctx->stream));
         HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
     }
@@ -255,14 +353,14 @@ void d2h(homs_context *ctx, void *dst, const void *src, size_t bytes) {
         HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
         if (prev >= 0) {
             HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[prev]));
-            std::memcpy(d + prev_off, ctx->stage[prev], prev_n);
+            ctx->copies.run({{d + prev_off, ctx->stage[prev], prev_n}});
         }
         prev = b;
         prev_off = off;
         prev_n = n;
     }
     HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[prev]));
-    std::memcpy(d + prev_off, ctx->stage[prev], prev_n);
+    ctx->copies.run({{d + prev_off, ctx->stage[prev], prev_n}});
 }
 
 // Copy `n` elements of dtype `src_dt` at `src` (host or device) into a device
@@ -294,6 +392,70 @@ void upload(homs_context *ctx, DevBuf &dst, const void *src, homs_dtype src_dt, 
     else
         convert_kernel<T, float><<<grid_for(n), 256, 0, ctx->stream>>>(reinterpret_cast<T *>(dst.p), static_cast<const float *>(src), n);
     HOMS_CUDA(cudaGetLastError());
+}
+
+// Several small host arrays of one upload: gathered in a page-locked chunk,
+// copied to one device block and, when their type differs from T, widened or
+// narrowed there by one kernel; each destination becomes a view of the block.
+// (Copied one by one, each array costs a driver call and, from pageable
+// memory, its own staging.)  `reals` hold n values of `src_dt`, `raw` n bytes.
+// False, and nothing done, when an array is not ordinary pageable memory, they
+// exceed a chunk or there is none: the caller then uploads them one by one.
+struct UploadItem {
+    DevBuf *dst;
+    const void *src;
+    size_t n;
+};
+template <typename T>
+bool upload_packed(homs_context *ctx, DevBuf &block, homs_dtype src_dt, const std::vector<UploadItem> &reals,
+                   const std::vector<UploadItem> &raw) {
+    constexpr size_t ALIGN = 64;  // elements of a real, and below 256 bytes of a raw array
+    const size_t es = dsize(src_dt);
+    size_t count = 0, raw_bytes = 0;
+    for (const UploadItem &u : reals) count += (u.n + ALIGN - 1) / ALIGN * ALIGN;
+    for (const UploadItem &u : raw) raw_bytes += (u.n + 255) / 256 * 256;
+    if (count * es + raw_bytes > STAGE_CHUNK) return false;
+    for (const UploadItem &u : reals)
+        if (!pageable(u.src)) return false;
+    if (!stage_ready(ctx)) return false;
+    HOMS_CUDA(block.ensure(count * sizeof(T) + raw_bytes));
+    const int b = ctx->stage_next;
+    ctx->stage_next ^= 1;
+    HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));
+    char *host = static_cast<char *>(ctx->stage[b]), *dev = block.as<char>();
+    std::vector<CopyPool::Piece> pieces;
+    size_t at = 0;
+    for (const UploadItem &u : reals) {
+        pieces.push_back({host + at * es, u.src, u.n * es});
+        u.dst->view(dev + at * sizeof(T), u.n * sizeof(T));
+        at += (u.n + ALIGN - 1) / ALIGN * ALIGN;
+    }
+    size_t off = 0;
+    for (const UploadItem &u : raw) {
+        pieces.push_back({host + count * es + off, u.src, u.n});
+        u.dst->view(dev + count * sizeof(T) + off, u.n);
+        off += (u.n + 255) / 256 * 256;
+    }
+    ctx->copies.run(pieces);
+    if (es == sizeof(T)) {
+        HOMS_CUDA(cudaMemcpyAsync(dev, host, count * es + raw_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+        HOMS_CUDA(ctx->scratch_conv.ensure(count * es));
+        HOMS_CUDA(cudaMemcpyAsync(ctx->scratch_conv.p, host, count * es, cudaMemcpyHostToDevice, ctx->stream));
+        if (raw_bytes)
+            HOMS_CUDA(cudaMemcpyAsync(dev + count * sizeof(T), host + count * es, raw_bytes, cudaMemcpyHostToDevice,
+                                      ctx->stream));
+        const int64_t n = (int64_t)count;
+        if (src_dt == HOMS_F64)
+            convert_kernel<T, double><<<grid_for(n), 256, 0, ctx->stream>>>(block.as<T>(),
+                                                                            ctx->scratch_conv.as<double>(), n);
+        else
+            convert_kernel<T, float><<<grid_for(n), 256, 0, ctx->stream>>>(block.as<T>(),
+                                                                           ctx->scratch_conv.as<float>(), n);
+        HOMS_CUDA(cudaGetLastError());
+    }
+    HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
+    return true;
 }
 
 template <typename T>
@@ -395,13 +557,13 @@ struct ResidentBase {
 
 template <typename T>
 struct Resident : ResidentBase {
+    DevBuf phantom_block, sequence_block;  // small uploads: the arrays below are views of them
     DevBuf x, y, z, rho, T1, T2, dw, csm_rows;
     DevBuf t, dt, gx, gy, gz, b1, df, psi, adc, bnd, h[16];
     DevBuf xy, mz, acc, rho_init;
     DevBuf partial, sig;
     std::vector<int64_t> first, last;
     std::vector<uint8_t> exc, adc_host;
-    std::vector<T> dt_host;
     double gamma = 0;
     SplitResident split;  // split-precision operands (built on demand)
     bool split_ready = false;
@@ -411,13 +573,9 @@ struct Resident : ResidentBase {
     // Plain FP32 precession: the block time of every node, the node table of
     // `nodes_method`, a launch round's phases and initial states.
     DevBuf block_time, nodes, walk;
-    bool block_time_ready = false;
     uint32_t nodes_method = ~0u;
-    // Prefix-table inputs of the sequence: the global ADC sample index of every
-    // node, and the 17 column sources of `src_method`.
-    DevBuf grank, src_table;
-    bool grank_ready = false;
-    uint32_t src_method = ~0u;
+    // Prefix-table input of the sequence: the global ADC sample index of every node.
+    DevBuf grank;
     // Instrumentation of the last run: events around every launch of the
     // dominant fused kernel, and a count of all kernels launched.
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
@@ -441,11 +599,12 @@ struct Resident : ResidentBase {
     }
 
     size_t device_bytes() const override {
-        size_t b = x.bytes + y.bytes + z.bytes + rho.bytes + T1.bytes + T2.bytes + dw.bytes + csm_rows.bytes + t.bytes +
-                   dt.bytes + gx.bytes + gy.bytes + gz.bytes + b1.bytes + df.bytes + psi.bytes + adc.bytes + bnd.bytes +
-                   xy.bytes + mz.bytes + acc.bytes + rho_init.bytes + partial.bytes + sig.bytes + spin_table.bytes +
-                   prefix.bytes + block_time.bytes + nodes.bytes + walk.bytes + split.device_bytes();
-        for (int k = 0; k < 16; ++k) b += h[k].bytes;
+        size_t b = split.device_bytes();
+        for (const DevBuf *d : {&phantom_block, &sequence_block, &x, &y, &z, &rho, &T1, &T2, &dw, &csm_rows, &t, &dt, &gx,
+                                &gy, &gz, &b1, &df, &psi, &adc, &bnd, &xy, &mz, &acc, &rho_init, &partial, &sig,
+                                &spin_table, &prefix, &block_time, &nodes, &walk, &grank})
+            b += d->owned_bytes();
+        for (int k = 0; k < 16; ++k) b += h[k].owned_bytes();
         return b;
     }
 
@@ -495,13 +654,12 @@ void fill_phantom(homs_context *ctx, Resident<T> *r, const homs_phantom *p) {
     r->ns = p->nspins;
     r->nc = p->ncoils;
     const int64_t ns = p->nspins;
-    upload<T>(ctx, r->x, p->x, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->y, p->y, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->z, p->z, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->rho, p->rho, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->T1, p->T1, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->T2, p->T2, p->dtype, p->memory, ns);
-    upload<T>(ctx, r->dw, p->dw, p->dtype, p->memory, ns);
+    const std::vector<UploadItem> arrays = {{&r->x, p->x, (size_t)ns},   {&r->y, p->y, (size_t)ns},
+                                            {&r->z, p->z, (size_t)ns},   {&r->rho, p->rho, (size_t)ns},
+                                            {&r->T1, p->T1, (size_t)ns}, {&r->T2, p->T2, (size_t)ns},
+                                            {&r->dw, p->dw, (size_t)ns}};
+    if (p->memory != HOMS_HOST || !upload_packed<T>(ctx, r->phantom_block, p->dtype, arrays, {}))
+        for (const UploadItem &u : arrays) upload<T>(ctx, *u.dst, u.src, p->dtype, p->memory, (int64_t)u.n);
     upload_csm_rows<T>(ctx, r->csm_rows, p->csm, p->dtype, p->memory, ns, p->ncoils, ns);
 }
 
@@ -535,35 +693,47 @@ template <typename T>
 void fill_sequence(homs_context *ctx, Resident<T> *r, const homs_sequence *q) {
     r->nt = q->nnodes;
     r->gamma = q->gamma;
-    r->grank_ready = false;
-    r->src_method = ~0u;
-    r->block_time_ready = false;
     r->nodes_method = ~0u;
     const int64_t ns = r->ns, nt = q->nnodes;
-    upload<T>(ctx, r->t, q->t, q->dtype, q->memory, nt);
-    upload<T>(ctx, r->dt, q->dt, q->dtype, q->memory, nt - 1);
-    upload<T>(ctx, r->gx, q->gx, q->dtype, q->memory, nt);
-    upload<T>(ctx, r->gy, q->gy, q->dtype, q->memory, nt);
-    upload<T>(ctx, r->gz, q->gz, q->dtype, q->memory, nt);
-    upload<T>(ctx, r->b1, q->b1, q->dtype, q->memory, 2 * nt);
-    upload<T>(ctx, r->df, q->df, q->dtype, q->memory, nt);
-    upload<T>(ctx, r->psi, q->psi, q->dtype, q->memory, nt);
-    for (int k = 0; k < 16; ++k) upload<T>(ctx, r->h[k], q->h[k], q->dtype, q->memory, nt);
     r->adc_host = host_adc(ctx, q);
-    HOMS_CUDA(r->adc.ensure((size_t)nt));
-    HOMS_CUDA(cudaMemcpyAsync(r->adc.p, r->adc_host.data(), (size_t)nt, cudaMemcpyHostToDevice, ctx->stream));
     r->first.assign(q->block_first, q->block_first + q->nblocks);
     r->last.assign(q->block_last, q->block_last + q->nblocks);
     r->exc.assign(q->block_excitation, q->block_excitation + q->nblocks);
     std::vector<uint8_t> bnd((size_t)nt, 0);
     for (int64_t l : r->last) bnd[(size_t)l] = 1;
-    HOMS_CUDA(r->bnd.ensure((size_t)nt));
-    HOMS_CUDA(cudaMemcpyAsync(r->bnd.p, bnd.data(), (size_t)nt, cudaMemcpyHostToDevice, ctx->stream));
-    r->dt_host = host_array<T>(ctx, q->dt, q->dtype, q->memory, nt - 1);
+    // Per node: the global ADC sample index (blocks share boundary nodes; a node
+    // belongs to the block that ends on it) for the FP64 paths' prefix table, or
+    // the block time, summed node by node in FP32 from each block's start.
+    std::vector<int32_t> rank(sizeof(T) == 8 ? (size_t)nt : 0, 0);
+    std::vector<float> tp(sizeof(T) == 4 ? (size_t)nt : 0, 0.0f);
+    std::vector<T> dt_host;
+    if (sizeof(T) == 4) dt_host = host_array<T>(ctx, q->dt, q->dtype, q->memory, nt - 1);
     int64_t nadc = 0;
-    for (size_t k = 0; k < r->first.size(); ++k)
-        for (int64_t n = r->first[k] + 1; n <= r->last[k]; ++n) nadc += r->adc_host[(size_t)n] ? 1 : 0;
+    for (size_t k = 0; k < r->first.size(); ++k) {
+        float t = 0.0f;
+        for (int64_t n = r->first[k] + 1; n <= r->last[k]; ++n) {
+            if (sizeof(T) == 8) rank[(size_t)n] = (int32_t)nadc;
+            else tp[(size_t)n] = t = t + (float)dt_host[(size_t)(n - 1)];
+            nadc += r->adc_host[(size_t)n] ? 1 : 0;
+        }
+    }
+    HOMS_REQUIRE(sizeof(T) == 4 || nadc <= INT32_MAX, "too many ADC samples for one run");
     r->nadc = nadc;
+    const size_t n = (size_t)nt;
+    std::vector<UploadItem> reals = {{&r->dt, q->dt, n - 1}, {&r->t, q->t, n},   {&r->gx, q->gx, n}, {&r->gy, q->gy, n},
+                                     {&r->gz, q->gz, n},     {&r->b1, q->b1, 2 * n}, {&r->df, q->df, n},
+                                     {&r->psi, q->psi, n}};
+    for (int k = 0; k < 16; ++k) reals.push_back({&r->h[k], q->h[k], n});
+    std::vector<UploadItem> raw = {{&r->adc, r->adc_host.data(), n}, {&r->bnd, bnd.data(), n}};
+    if (sizeof(T) == 8) raw.push_back({&r->grank, rank.data(), sizeof(int32_t) * n});
+    else raw.push_back({&r->block_time, tp.data(), sizeof(float) * n});
+    if (q->memory != HOMS_HOST || !upload_packed<T>(ctx, r->sequence_block, q->dtype, reals, raw)) {
+        for (const UploadItem &u : reals) upload<T>(ctx, *u.dst, u.src, q->dtype, q->memory, (int64_t)u.n);
+        for (const UploadItem &u : raw) {
+            HOMS_CUDA(u.dst->ensure(u.n));
+            HOMS_CUDA(cudaMemcpyAsync(u.dst->p, u.src, u.n, cudaMemcpyHostToDevice, ctx->stream));
+        }
+    }
     HOMS_CUDA(r->xy.ensure(sizeof(cplx<T>) * (size_t)ns));
     HOMS_CUDA(r->mz.ensure(sizeof(T) * (size_t)ns));
     HOMS_CUDA(r->acc.ensure(sizeof(T) * (size_t)ns));
@@ -648,35 +818,12 @@ std::vector<Launch> plan_launches(const Resident<T> &r, const LaunchLimits &lim)
     return out;
 }
 
-// The prefix table's inputs: the global ADC sample index of every
-// owned node (blocks share boundary nodes; a node belongs to the block that
-// ends on it) and the prefix-table column sources of `method`.  Uploaded
-// from the host only when the sequence or the method changed.
+// The field columns of `method` for the prefix table.
 template <typename T>
-void ensure_prefix_tables(homs_context *ctx, Resident<T> &r, uint32_t method) {
-    if (!r.grank_ready) {
-        std::vector<int32_t> g((size_t)r.nt, 0);
-        int64_t c = 0;
-        for (size_t k = 0; k < r.first.size(); ++k)
-            for (int64_t n = r.first[k] + 1; n <= r.last[k]; ++n) {
-                g[(size_t)n] = (int32_t)c;
-                if (r.adc_host[(size_t)n]) ++c;
-            }
-        HOMS_REQUIRE(c <= INT32_MAX, "too many ADC samples for one run");
-        HOMS_CUDA(r.grank.ensure(sizeof(int32_t) * (size_t)r.nt));
-        HOMS_CUDA(cudaMemcpyAsync(r.grank.p, g.data(), sizeof(int32_t) * (size_t)r.nt, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-        r.grank_ready = true;
-    }
-    if (r.src_method != method) {
-        const void *h[16];
-        for (int k = 0; k < 16; ++k) h[k] = r.h[k].p;
-        const void *src[17];
-        split_column_sources(method, h, r.gx.p, r.gy.p, r.gz.p, src);
-        HOMS_CUDA(r.src_table.ensure(sizeof(src)));
-        HOMS_CUDA(cudaMemcpyAsync(r.src_table.p, src, sizeof(src), cudaMemcpyHostToDevice, ctx->stream));
-        r.src_method = method;
-    }
+SplitColumns prefix_columns(const Resident<T> &r, uint32_t method) {
+    const void *h[16];
+    for (int k = 0; k < 16; ++k) h[k] = r.h[k].p;
+    return split_column_sources(method, h, r.gx.p, r.gy.p, r.gz.p);
 }
 
 // The plain FP64 path's spin table, unless `r` has it, its own or a resident phantom's.
@@ -692,7 +839,7 @@ inline void ensure_spin_table(homs_context *ctx, Resident<double> &r) {
 inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t method, bool capture, int64_t n_lo,
                             int64_t n_hi, int64_t sample0, int64_t nsamples) {
     HOMS_CUDA(r.prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nsamples)));
-    HOMS_CUDA(split_prefix_launch(r.dt.as<double>(), r.src_table.as<const void *>(), r.adc.as<uint8_t>(),
+    HOMS_CUDA(split_prefix_launch(r.dt.as<double>(), prefix_columns(r, method), r.adc.as<uint8_t>(),
                                   r.grank.as<int32_t>(), n_lo, n_hi, sample0, nsamples, r.gamma,
                                   r.prefix.as<double>(), ctx->stream));
     r.launches += 2;
@@ -720,21 +867,8 @@ inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t met
                             &r.launches, ctx->stream));
 }
 
-// The plain FP32 path's node table of the sequence and method: the block times
-// are summed here, node by node in FP32 from each block's start.
+// The plain FP32 path's node table of the sequence and method.
 inline void ensure_nodes32(homs_context *ctx, Resident<float> &r, uint32_t method) {
-    if (!r.block_time_ready) {
-        std::vector<float> tp((size_t)r.nt, 0.0f);
-        for (size_t k = 0; k < r.first.size(); ++k) {
-            float t = 0.0f;
-            for (int64_t n = r.first[k] + 1; n <= r.last[k]; ++n) tp[(size_t)n] = t = t + r.dt_host[(size_t)(n - 1)];
-        }
-        HOMS_CUDA(r.block_time.ensure(sizeof(float) * (size_t)r.nt));
-        HOMS_CUDA(cudaMemcpyAsync(r.block_time.p, tp.data(), sizeof(float) * (size_t)r.nt, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-        r.block_time_ready = true;
-        r.nodes_method = ~0u;
-    }
     if (r.nodes_method != method) {
         HOMS_CUDA(r.nodes.ensure(precess32_node_bytes(r.nt)));
         HOMS_CUDA(precess32_nodes(r.seq(), method, r.block_time.as<float>(), r.nodes.p, ctx->stream));
@@ -808,11 +942,9 @@ void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture)
     LaunchLimits lim{excitation_samples(r), INT64_MAX, INT64_MAX};
     if constexpr (sizeof(T) == 8) {
         if (capture) {
-            HOMS_REQUIRE(r.spin_table_ready && r.grank_ready && r.src_method == method,
-                         "internal: precession tables missing under capture");
+            HOMS_REQUIRE(r.spin_table_ready, "internal: spin table missing under capture");
         } else {
             ensure_spin_table(ctx, r);
-            ensure_prefix_tables<T>(ctx, r, method);
         }
     } else {
         lim.precession_samples = precess32_max_samples(r.ns);
@@ -865,13 +997,19 @@ void ensure_split(homs_context *ctx, Resident<T> &r) {
     r.split_ready = true;
 }
 
+void throw_split_error(unsigned int word) {
+    const std::string err = split_error_text(word);
+    if (!err.empty())
+        throw Failure{err.find("timed out") != std::string::npos ? HOMS_ETIMEDOUT : HOMS_EUNSUPPORTED, err};
+}
+
 // Read the split kernel's device error word (synchronises the stream).
 template <typename T>
 void check_split(homs_context *ctx, Resident<T> &r) {
-    std::string err;
-    HOMS_CUDA(split_check(r.split, ctx->stream, &err));
-    if (!err.empty())
-        throw Failure{err.find("timed out") != std::string::npos ? HOMS_ETIMEDOUT : HOMS_EUNSUPPORTED, err};
+    unsigned int word = 0;
+    HOMS_CUDA(split_read_error(r.split, &word, ctx->stream));
+    HOMS_CUDA(cudaStreamSynchronize(ctx->stream));
+    throw_split_error(word);
 }
 
 // One split-mode run of the block plan, issued in steps so that several
@@ -911,7 +1049,7 @@ struct SplitRunner {
         sa.nblocks = (int32_t)res.first.size();
         sa.adc_host = res.adc_host.data();
         sa.grank = reinterpret_cast<const int32_t *>(res.grank.p);
-        sa.src_dev = reinterpret_cast<const void *const *>(res.src_table.p);
+        sa.cols = prefix_columns(res, method);
         sa.capture = capture;
         sa.t = res.t.p;
         sa.dt = res.dt.p;
@@ -992,11 +1130,9 @@ struct SplitRunner {
 // stream is being captured into a CUDA graph: every host-side table and
 // buffer must already be in place (an earlier run of the same plan built
 // them), and only kernels, memsets, device copies and graph-external event
-// records are issued.  `check` reads the split kernel's error word
-// afterwards (a synchronisation; not possible under capture).
+// records are issued.  copy_out reads the split kernel's error word.
 template <typename T>
-void run_resident(homs_context *ctx, Resident<T> &r, const homs_run_options *opts, bool capture = false,
-                  bool check = true) {
+void run_resident(homs_context *ctx, Resident<T> &r, const homs_run_options *opts, bool capture = false) {
     r.events_used = 0;
     r.launches = 0;
     const uint32_t method = opts ? opts->method : 0x3Fu;
@@ -1007,11 +1143,9 @@ void run_resident(homs_context *ctx, Resident<T> &r, const homs_run_options *opt
     } else if (mode == HOMS_SPLIT) {
         if (sizeof(T) != 8) throw Failure{HOMS_EUNSUPPORTED, "internal: split mode runs on FP64 resident arrays"};
         if (capture) {
-            HOMS_REQUIRE(r.split_ready && r.grank_ready && r.src_method == method,
-                         "internal: split tables missing under capture");
+            HOMS_REQUIRE(r.split_ready, "internal: split tables missing under capture");
         } else {
             ensure_split<T>(ctx, r);
-            ensure_prefix_tables<T>(ctx, r, method);
         }
         HOMS_CUDA(split_reset_error(r.split, ctx->stream));
         SplitRunner<T> run;
@@ -1031,7 +1165,6 @@ void run_resident(homs_context *ctx, Resident<T> &r, const homs_run_options *opt
             if (e != cudaSuccess) throw Failure{HOMS_ECUDA, std::string("split segment: ") + cudaGetErrorString(e)};
             run.after(ctx->stream);
         }
-        if (check) check_split<T>(ctx, r);
     } else {
         throw Failure{HOMS_EINVAL, "unknown run mode"};
     }
@@ -1061,19 +1194,72 @@ void download(homs_context *ctx, void *dst, homs_memory mem, const void *src, in
     if (mem == HOMS_HOST) d2h(ctx, dst, narrow, sizeof(float) * (size_t)n);
 }
 
-// Signal and final state out, in the caller's dtype `out_dt`.
+// Signal and final state out, in the caller's dtype `out_dt`; waits for the run.
+// `split`: the run's device error word is read first, and a failed run writes
+// nothing.  Small pageable results share one page-locked chunk, and with the
+// error word one wait; others are copied one by one.
 template <typename T>
 void copy_out(homs_context *ctx, Resident<T> &r, void *sig, homs_memory sig_memory, homs_state *state,
-              homs_dtype out_dt) {
+              homs_dtype out_dt, bool split) {
+    struct Out {
+        void *dst;
+        homs_memory mem;
+        const void *src;
+        int64_t n;
+    };
+    std::vector<Out> outs;
     if (r.nadc * r.nc > 0) {
         HOMS_REQUIRE(sig != nullptr, "sig is NULL");
-        download<T>(ctx, sig, sig_memory, r.sig.p, 2 * r.nadc * r.nc, out_dt);
+        outs.push_back({sig, sig_memory, r.sig.p, 2 * r.nadc * r.nc});
     }
     if (state && state->xy && state->z) {
-        download<T>(ctx, state->xy, state->memory, r.xy.p, 2 * r.ns, out_dt);
-        download<T>(ctx, state->z, state->memory, r.mz.p, r.ns, out_dt);
+        outs.push_back({state->xy, state->memory, r.xy.p, 2 * r.ns});
+        outs.push_back({state->z, state->memory, r.mz.p, r.ns});
     }
+    const size_t es = dsize(out_dt);
+    size_t total = 256;  // the error word
+    bool pack = true;
+    for (const Out &o : outs) {
+        total += (es * (size_t)o.n + 255) / 256 * 256;
+        pack = pack && o.mem == HOMS_HOST;
+    }
+    pack = pack && total <= STAGE_CHUNK;
+    for (const Out &o : outs) pack = pack && pageable(o.dst);
+    if (!pack || !stage_ready(ctx)) {
+        if (split) check_split<T>(ctx, r);
+        for (const Out &o : outs) download<T>(ctx, o.dst, o.mem, o.src, o.n, out_dt);
+        HOMS_CUDA(cudaStreamSynchronize(ctx->stream));
+        return;
+    }
+    const int b = ctx->stage_next;
+    ctx->stage_next ^= 1;
+    HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));  // no upload still reads this chunk
+    char *host = static_cast<char *>(ctx->stage[b]);
+    const bool narrow = es != sizeof(T);
+    HOMS_REQUIRE(!narrow || (sizeof(T) == 8 && out_dt == HOMS_F32), "internal: unsupported output conversion");
+    if (narrow) HOMS_CUDA(ctx->scratch_conv.ensure(total));
+    std::vector<CopyPool::Piece> pieces;
+    size_t off = 256;
+    for (const Out &o : outs) {
+        const size_t bytes = es * (size_t)o.n;
+        const void *src = o.src;
+        if (narrow) {
+            float *dst = reinterpret_cast<float *>(ctx->scratch_conv.as<char>() + off);
+            convert_kernel<float, double><<<grid_for(o.n), 256, 0, ctx->stream>>>(
+                dst, static_cast<const double *>(o.src), o.n);
+            HOMS_CUDA(cudaGetLastError());
+            src = dst;
+        }
+        HOMS_CUDA(cudaMemcpyAsync(host + off, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        pieces.push_back({o.dst, host + off, bytes});
+        off += (bytes + 255) / 256 * 256;
+    }
+    unsigned int *word = reinterpret_cast<unsigned int *>(host);
+    *word = 0;
+    if (split) HOMS_CUDA(split_read_error(r.split, word, ctx->stream));
     HOMS_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (split) throw_split_error(*word);
+    ctx->copies.run(pieces);
 }
 
 // Split mode computes in FP64 whatever the caller's dtype: FP32 phantom and
@@ -1149,7 +1335,7 @@ void simulate_on_resident(homs_context *ctx, const homs_resident *res, const hom
     fill_sequence<T>(ctx, r, seq);
     init_state<T>(ctx, *r, state, res->in_dtype);
     run_resident<T>(ctx, *r, opts);
-    copy_out<T>(ctx, *r, sig, sig_memory, state, res->in_dtype);
+    copy_out<T>(ctx, *r, sig, sig_memory, state, res->in_dtype, opts->mode == HOMS_SPLIT);
 }
 
 }  // namespace
@@ -1170,7 +1356,7 @@ void plan_run_typed(homs_plan *plan, void *sig, homs_memory sig_memory, homs_sta
             std::string why;
             try {
                 init_state<T>(ctx, r, nullptr, rdt);
-                run_resident<T>(ctx, r, &plan->opts, /*capture=*/true, /*check=*/false);
+                run_resident<T>(ctx, r, &plan->opts, /*capture=*/true);
             } catch (const Failure &f) {
                 why = f.msg;
             }
@@ -1203,10 +1389,9 @@ void plan_run_typed(homs_plan *plan, void *sig, homs_memory sig_memory, homs_sta
     }
     if (!issued) {
         init_state<T>(ctx, r, nullptr, rdt);
-        run_resident<T>(ctx, r, &plan->opts, /*capture=*/false, /*check=*/false);
+        run_resident<T>(ctx, r, &plan->opts);
     }
-    if (plan->opts.mode == HOMS_SPLIT) check_split<T>(ctx, r);
-    copy_out<T>(ctx, r, sig, sig_memory, state_out, plan->out_dtype);
+    copy_out<T>(ctx, r, sig, sig_memory, state_out, plan->out_dtype, plan->opts.mode == HOMS_SPLIT);
     ++plan->runs;
 }
 
@@ -1275,7 +1460,6 @@ homs_status homs_context_destroy(homs_context *ctx) {
         ctx->scratch_sig.release();
         ctx->scratch_conv.release();
         ctx->block_rank.release();
-        ctx->block_src.release();
         ctx->block_table.release();
         ctx->block_prefix.release();
         ctx->block_xy.release();
@@ -1336,12 +1520,12 @@ homs_status homs_simulate(homs_context *ctx, const homs_phantom *phantom, const 
             Resident<double> *r = cached_resident<double>(ctx, phantom, seq);
             init_state<double>(ctx, *r, state, phantom->dtype);
             run_resident<double>(ctx, *r, opts);
-            copy_out<double>(ctx, *r, sig, sig_memory, state, phantom->dtype);
+            copy_out<double>(ctx, *r, sig, sig_memory, state, phantom->dtype, opts && opts->mode == HOMS_SPLIT);
         } else {
             Resident<float> *r = cached_resident<float>(ctx, phantom, seq);
             init_state<float>(ctx, *r, state, phantom->dtype);
             run_resident<float>(ctx, *r, opts);
-            copy_out<float>(ctx, *r, sig, sig_memory, state, phantom->dtype);
+            copy_out<float>(ctx, *r, sig, sig_memory, state, phantom->dtype, false);
         }
         return HOMS_OK;
     } catch (const Failure &f) {
@@ -1396,6 +1580,9 @@ homs_status homs_plan_run(homs_plan *plan, void *sig, homs_memory sig_memory, ho
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1454,19 +1641,16 @@ void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDe
         rank[i] = c;
         if (adc[i]) ++c;
     }
-    const void *h[16], *src[17];
+    const void *h[16];
     for (int k = 0; k < 16; ++k) h[k] = q.h[k];
-    split_column_sources(method, h, q.gx, q.gy, q.gz, src);
     HOMS_CUDA(ctx->block_rank.ensure(sizeof(int32_t) * rank.size()));
-    HOMS_CUDA(ctx->block_src.ensure(sizeof(src)));
     HOMS_CUDA(ctx->block_table.ensure(precess64_table_bytes(p.ns)));
     HOMS_CUDA(ctx->block_prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nadc)));
     HOMS_CUDA(cudaMemcpyAsync(ctx->block_rank.p, rank.data(), sizeof(int32_t) * rank.size(), cudaMemcpyHostToDevice,
                               ctx->stream));
-    HOMS_CUDA(cudaMemcpyAsync(ctx->block_src.p, src, sizeof(src), cudaMemcpyHostToDevice, ctx->stream));
     HOMS_CUDA(precess64_table(p.x, p.y, p.z, p.dw, p.T2, p.ns, ctx->block_table.p, ctx->stream));
     // the prefix kernel looks ranks up by node
-    HOMS_CUDA(split_prefix_launch(q.dt, ctx->block_src.as<const void *>(), q.adc,
+    HOMS_CUDA(split_prefix_launch(q.dt, split_column_sources(method, h, q.gx, q.gy, q.gz), q.adc,
                                   ctx->block_rank.as<int32_t>() - (first + 1), first, last, 0, nadc, gamma,
                                   ctx->block_prefix.as<double>(), ctx->stream));
     const CoilCut pp = precess64_cut(p.ns, p.nc, nadc);
@@ -1516,9 +1700,9 @@ void block_precess32(homs_context *ctx, const PhantomDev<float> &p, const SeqDev
     r.exc = {0};
     r.adc_host.resize((size_t)r.nt);
     HOMS_CUDA(cudaMemcpyAsync(r.adc_host.data(), q.adc + first, (size_t)r.nt, cudaMemcpyDeviceToHost, ctx->stream));
-    r.dt_host = host_array<float>(ctx, q.dt + first, HOMS_F32, HOMS_DEVICE, r.nt - 1);  // waits for both copies
+    const std::vector<float> dt = host_array<float>(ctx, q.dt + first, HOMS_F32, HOMS_DEVICE, r.nt - 1);  // waits for both
     std::vector<float> tp((size_t)r.nt, 0.0f);
-    for (int64_t n = 1; n < r.nt; ++n) tp[(size_t)n] = tp[(size_t)(n - 1)] + r.dt_host[(size_t)(n - 1)];
+    for (int64_t n = 1; n < r.nt; ++n) tp[(size_t)n] = tp[(size_t)(n - 1)] + dt[(size_t)(n - 1)];
     HOMS_CUDA(ctx->block_rank.ensure(sizeof(float) * (size_t)r.nt));
     HOMS_CUDA(cudaMemcpyAsync(ctx->block_rank.p, tp.data(), sizeof(float) * (size_t)r.nt, cudaMemcpyHostToDevice,
                               ctx->stream));
@@ -1646,6 +1830,8 @@ homs_status homs_precession_block(homs_context *ctx, const homs_phantom *phantom
                    : block_impl<float>(ctx, false, phantom, seq, first, last, method, state, sig, ldsig);
     } catch (const Failure &f) {
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1662,6 +1848,8 @@ homs_status homs_excitation_block(homs_context *ctx, const homs_phantom *phantom
                    : block_impl<float>(ctx, true, phantom, seq, first, last, method, state, sig, ldsig);
     } catch (const Failure &f) {
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1703,6 +1891,8 @@ homs_status homs_coil_reduce(homs_context *ctx, homs_dtype dtype, int64_t nspins
         return HOMS_OK;
     } catch (const Failure &f) {
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1869,6 +2059,9 @@ homs_status homs_brain_phantom_count(homs_context *ctx, const homs_brain_spec *s
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1924,6 +2117,9 @@ homs_status homs_brain_phantom_fill(homs_context *ctx, const homs_brain_spec *sp
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -1950,6 +2146,9 @@ homs_status homs_csm_birdcage(homs_context *ctx, int64_t nx, int64_t ny, int32_t
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -2018,7 +2217,7 @@ homs_status homs_kspace(homs_context *ctx, const homs_sequence *seq, int32_t nrf
         if (nq > 0) std::memcpy(meta.data() + off_q, q_times, sizeof(double) * (size_t)nq);
         HOMS_CUDA(ctx->kspace_meta.ensure(meta.size()));
         uint8_t *dmeta = ctx->kspace_meta.as<uint8_t>();
-        HOMS_CUDA(cudaMemcpyAsync(dmeta, meta.data(), meta.size(), cudaMemcpyHostToDevice, ctx->stream));
+        h2d(ctx, dmeta, meta.data(), meta.size());
         // Outputs: the caller's device arrays or a staging buffer.
         double *dk = k, *dkq = k_q;
         const size_t k_bytes = sizeof(double) * (size_t)m * NCOLS, kq_bytes = sizeof(double) * (size_t)nq * NCOLS;
@@ -2060,6 +2259,9 @@ homs_status homs_kspace(homs_context *ctx, const homs_sequence *seq, int32_t nrf
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -2080,6 +2282,9 @@ homs_status homs_selftest_wait_timeout(homs_context *ctx, int64_t budget_cycles)
     } catch (const Failure &f) {
         cudaStreamSynchronize(ctx->stream);
         return fail(ctx, f);
+    } catch (const std::bad_alloc &) {
+        cudaStreamSynchronize(ctx->stream);
+        return fail(ctx, Failure{HOMS_ENOMEM, "host allocation failed"});
     }
 }
 
@@ -2149,7 +2354,6 @@ homs_status server_run_prepare(homs_context *ctx, const homs_phantom *phantom, c
         }
         init_state<double>(ctx, *r, state, run->out_dt);
         ensure_split<double>(ctx, *r);
-        ensure_prefix_tables<double>(ctx, *r, opts->method);
         HOMS_CUDA(split_reset_error(r->split, ctx->stream));
         r->events_used = 0;
         r->launches = 0;
@@ -2218,8 +2422,7 @@ homs_status server_run_finish(ServerRun *run, void *sig, homs_memory sig_memory,
         HOMS_REQUIRE(run->done_recorded, "internal: the run's work was not issued");
         HOMS_CUDA(cudaStreamWaitEvent(ctx->stream, run->done, 0));
         HOMS_REQUIRE(sig_memory == HOMS_HOST || sig_memory == HOMS_DEVICE, "invalid signal memory kind");
-        check_split<double>(ctx, *run->r);
-        copy_out<double>(ctx, *run->r, sig, sig_memory, state, run->out_dt);
+        copy_out<double>(ctx, *run->r, sig, sig_memory, state, run->out_dt, true);
         return HOMS_OK;
     } catch (const Failure &f) {
         run->failed = true;

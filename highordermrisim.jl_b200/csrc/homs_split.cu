@@ -1191,9 +1191,9 @@ struct PrefixColumn {
     double scale;
     int out_col;
 };
-__device__ __forceinline__ PrefixColumn prefix_column(const double *const *src, int col, double gamma) {
+__device__ __forceinline__ PrefixColumn prefix_column(const SplitColumns &src, int col, double gamma) {
     PrefixColumn c;
-    c.f = col < 17 ? src[col] : reinterpret_cast<const double *>(1);  // nullptr: zero; 1: constant one
+    c.f = col < 17 ? static_cast<const double *>(src.p[col]) : reinterpret_cast<const double *>(1);  // nullptr: zero; 1: constant one
     c.one = c.f == reinterpret_cast<const double *>(1);
     c.zero = c.f == nullptr;
     c.scale = col < 16 ? -gamma * 0.5 : (col == 16 ? -0.5 : 0.5);
@@ -1229,7 +1229,7 @@ __device__ double block_exclusive(double *part, double local) {
     return total;
 }
 
-__global__ void prefix_part_kernel(const double *dt, const double *const *src, int64_t n_lo, int64_t n_hi,
+__global__ void prefix_part_kernel(const double *dt, const __grid_constant__ SplitColumns src, int64_t n_lo, int64_t n_hi,
                                    int64_t nsamples, double gamma, double *prefix) {
     __shared__ double part[256];
     const int col = blockIdx.x, pt = blockIdx.y;
@@ -1245,7 +1245,7 @@ __global__ void prefix_part_kernel(const double *dt, const double *const *src, i
     }
 }
 
-__global__ void prefix_kernel(const double *dt, const double *const *src, const uint8_t *adc, const int32_t *rank,
+__global__ void prefix_kernel(const double *dt, const __grid_constant__ SplitColumns src, const uint8_t *adc, const int32_t *rank,
                               int64_t rank_base, int64_t n_lo, int64_t n_hi, int64_t nsamples, double gamma,
                               double *prefix) {
     __shared__ double part[256];
@@ -1611,13 +1611,12 @@ cudaError_t split_launch(const SplitJobDesc *jobs, int n_jobs, cudaStream_t stre
 
 size_t split_prefix_rows(int64_t nsamples) { return (size_t)nsamples + 2 + PREFIX_PARTS; }
 
-cudaError_t split_prefix_launch(const double *dt, const void *const *src_dev, const uint8_t *adc, const int32_t *grank,
+cudaError_t split_prefix_launch(const double *dt, const SplitColumns &cols, const uint8_t *adc, const int32_t *grank,
                                 int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
                                 double *prefix, cudaStream_t stream) {
     const dim3 pgrid(PREFIX_COLS, PREFIX_PARTS);
-    const double *const *src = reinterpret_cast<const double *const *>(src_dev);
-    prefix_part_kernel<<<pgrid, 256, 0, stream>>>(dt, src, n_lo, n_hi, nsamples, gamma, prefix);
-    prefix_kernel<<<pgrid, 256, 0, stream>>>(dt, src, adc, grank, sample0, n_lo, n_hi, nsamples, gamma, prefix);
+    prefix_part_kernel<<<pgrid, 256, 0, stream>>>(dt, cols, n_lo, n_hi, nsamples, gamma, prefix);
+    prefix_kernel<<<pgrid, 256, 0, stream>>>(dt, cols, adc, grank, sample0, n_lo, n_hi, nsamples, gamma, prefix);
     return cudaGetLastError();
 }
 
@@ -1628,8 +1627,8 @@ cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t
     cudaError_t e;
     const int64_t nchunks = r.ns_pad / KC;
     const int64_t tiles = (nsamples + TM - 1) / TM;
-    if (!a.grank || !a.src_dev) {
-        *err = "internal: split segment without its ADC rank and column tables";
+    if (!a.grank) {
+        *err = "internal: split segment without its ADC rank table";
         return cudaSuccess;
     }
     seg->nsamples = nsamples;
@@ -1640,7 +1639,7 @@ cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t
     if ((e = grow(r.prefix, r.prefix_bytes, prefix_rows * PREFIX_STRIDE * sizeof(double))) != cudaSuccess) return e;
     if ((e = grow(r.params, r.params_bytes, (size_t)nchunks * PARAM_BYTES)) != cudaSuccess) return e;
     // The segment's samples are the global ADC indices sample0 .. sample0 + nsamples - 1.
-    if ((e = split_prefix_launch((const double *)a.dt, a.src_dev, (const uint8_t *)a.adc, a.grank, n_lo, n_hi, sample0,
+    if ((e = split_prefix_launch((const double *)a.dt, a.cols, (const uint8_t *)a.adc, a.grank, n_lo, n_hi, sample0,
                                  nsamples, a.gamma, (double *)r.prefix, stream)) != cudaSuccess)
         return e;
     if ((e = cudaMemsetAsync(r.amp, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
@@ -1744,13 +1743,16 @@ cudaError_t split_attach(SplitResident &r, const SplitResident &src) {
     return cudaSuccess;
 }
 
-void split_column_sources(uint32_t m, const void *const h[16], const void *gx, const void *gy, const void *gz,
-                          const void *out[17]) {
+SplitColumns split_column_sources(uint32_t m, const void *const h[16], const void *gx, const void *gy,
+                                  const void *gz) {
+    SplitColumns c;
+    const void **out = c.p;
     out[0] = (m & HOMS_HO0) ? h[0] : nullptr;
     for (int k = 1; k <= 3; ++k) out[k] = (m & HOMS_HO1) ? h[k] : (k == 1 ? gx : k == 2 ? gy : gz);
     for (int k = 4; k <= 8; ++k) out[k] = (m & HOMS_HO2) ? h[k] : nullptr;
     for (int k = 9; k <= 15; ++k) out[k] = (m & HOMS_HO3) ? h[k] : nullptr;
     out[16] = (m & HOMS_DW_PRECESSION) ? reinterpret_cast<const void *>(1) : nullptr;
+    return c;
 }
 
 cudaError_t split_reset_error(SplitResident &r, cudaStream_t stream) {
@@ -1779,17 +1781,16 @@ cudaError_t split_run_segment(SplitResident &r, const SplitRunArgs &a, int64_t n
     return split_segment_end(r, a, seg, stream);
 }
 
-cudaError_t split_check(SplitResident &r, cudaStream_t stream, std::string *err) {
-    unsigned int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, r.err, sizeof(h), cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
-    if (h & 64u)
-        *err = "split mode: a field term's phase range within one precession segment exceeds 4096 turns "
+cudaError_t split_read_error(const SplitResident &r, unsigned int *word, cudaStream_t stream) {
+    return cudaMemcpyAsync(word, r.err, sizeof(*word), cudaMemcpyDeviceToHost, stream);
+}
+
+std::string split_error_text(unsigned int word) {
+    if (word & 64u)
+        return "split mode: a field term's phase range within one precession segment exceeds 4096 turns "
                "(max |basis value| x max |field integral|); run it in plain mode";
-    else if (h != 0)
-        *err = "split kernel: a bounded device wait timed out (code " + std::to_string(h) + ")";
-    return cudaSuccess;
+    if (word != 0) return "split kernel: a bounded device wait timed out (code " + std::to_string(word) + ")";
+    return "";
 }
 
 }  // namespace homs

@@ -60,6 +60,12 @@ struct SplitResident {
     }
 };
 
+// The 17 column sources of the prefix table (split_column_sources), passed to
+// the kernels by value.
+struct SplitColumns {
+    const void *p[17];
+};
+
 struct SplitRunArgs {
     size_t sizeof_T;
     int64_t ns, nt, nadc;
@@ -70,11 +76,10 @@ struct SplitRunArgs {
     const uint8_t *exc;
     int32_t nblocks;
     const uint8_t *adc_host;
-    // device tables built once per sequence and method: the global ADC
-    // sample index of every node (0-based, ownership as in the block plan)
-    // and the 17 field-column pointers of the prefix table
+    // the global ADC sample index of every node (0-based, ownership as in the
+    // block plan) and the field columns of the prefix table
     const int32_t *grank = nullptr;
-    const void *const *src_dev = nullptr;
+    SplitColumns cols{};
     bool capture = false;  // the stream is being captured into a CUDA graph
     // resident device arrays (type T = double or float per sizeof_T)
     const void *t, *dt, *gx, *gy, *gz, *b1, *df, *psi, *adc, *bnd, *h[16];
@@ -103,7 +108,7 @@ cudaError_t split_attach(SplitResident &r, const SplitResident &src);
 // node.  `prefix` holds split_prefix_rows(nsamples) rows.
 constexpr int SPLIT_PREFIX_STRIDE = 24, SPLIT_PREFIX_T = 20;
 size_t split_prefix_rows(int64_t nsamples);
-cudaError_t split_prefix_launch(const double *dt, const void *const *src_dev, const uint8_t *adc, const int32_t *grank,
+cudaError_t split_prefix_launch(const double *dt, const SplitColumns &cols, const uint8_t *adc, const int32_t *grank,
                                 int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
                                 double *prefix, cudaStream_t stream);
 
@@ -113,8 +118,8 @@ cudaError_t split_reset_error(SplitResident &r, cudaStream_t stream);
 // The 17 prefix-table column sources for a method mask: h_k when its order
 // is on, the nominal gradient for k = 1..3 when the first order is off,
 // NULL (zero) otherwise, and the constant-one marker for the dw column.
-void split_column_sources(uint32_t method, const void *const h[16], const void *gx, const void *gy, const void *gz,
-                          const void *out[17]);
+SplitColumns split_column_sources(uint32_t method, const void *const h[16], const void *gx, const void *gy,
+                                  const void *gz);
 
 // One precession segment (a run of consecutive precession blocks, nodes
 // [n_lo, n_hi]) on the split tcgen05 kernel; its samples go to sig rows
@@ -153,9 +158,11 @@ cudaError_t split_segment_end(SplitResident &r, const SplitRunArgs &a, const Spl
 // after `budget_cycles` and sets code 256 in *err (device word, cleared first).
 cudaError_t wait_selftest(unsigned int *err, long long budget_cycles, cudaStream_t stream);
 
-// Read the device error word (synchronises the stream).  Sets *err if a
-// bounded wait timed out or a segment's phase range is out of bounds.
-cudaError_t split_check(SplitResident &r, cudaStream_t stream, std::string *err);
+// Copy the device error word to *word (host memory; asynchronous when that is
+// page-locked), and its message: empty for 0, else a bounded wait that timed out
+// or a segment's phase range that is out of bounds.
+cudaError_t split_read_error(const SplitResident &r, unsigned int *word, cudaStream_t stream);
+std::string split_error_text(unsigned int word);
 
 // Device bytes of the split path's operands per spin (phantom operands of one
 // simulation with `ncoils` coils), for admission estimates.

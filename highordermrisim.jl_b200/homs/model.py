@@ -345,12 +345,11 @@ def get_sim_ranges(seqd: HO_DiscreteSequence, max_block_length=math.inf, max_rf_
     n = exc.shape[0]
     parts: List[Tuple[int, int]] = []
     flags: List[bool] = []
-    i = 0
-    while i < n:
+    if n == 0:
+        return parts, flags
+    edges = [0, *(np.flatnonzero(exc[1:] != exc[:-1]) + 1).tolist(), n]
+    for i, j in zip(edges[:-1], edges[1:]):
         flag = bool(exc[i])
-        j = i
-        while j < n and bool(exc[j]) == flag:
-            j += 1
         lim = max_rf_block_length if flag else max_block_length
         k = i
         while k < j:
@@ -358,14 +357,14 @@ def get_sim_ranges(seqd: HO_DiscreteSequence, max_block_length=math.inf, max_rf_
             parts.append((k, e))
             flags.append(flag)
             k = e
-        i = j
     return parts, flags
 
 
 def count_block_adc(adc, parts: Sequence[Tuple[int, int]]) -> List[int]:
     """ADC samples per block: ADC[first+1 .. last] (SimulatorCore.jl:115-116)."""
-    adc = np.asarray(adc, dtype=bool)
-    return [int(adc[f + 1:l + 1].sum()) for f, l in parts]
+    before = np.concatenate([[0], np.cumsum(np.asarray(adc, dtype=bool))])  # samples before each node
+    at = lambda n: int(before[min(max(n, 0), before.shape[0] - 1)])  # noqa: E731
+    return [max(at(l + 1) - at(f + 1), 0) for f, l in parts]
 
 
 @dataclass
