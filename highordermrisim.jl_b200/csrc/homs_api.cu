@@ -841,8 +841,8 @@ inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t met
     HOMS_CUDA(r.prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nsamples)));
     HOMS_CUDA(split_prefix_launch(r.dt.as<double>(), prefix_columns(r, method), r.adc.as<uint8_t>(),
                                   r.grank.as<int32_t>(), n_lo, n_hi, sample0, nsamples, r.gamma,
-                                  r.prefix.as<double>(), ctx->stream));
-    r.launches += 2;
+                                  r.prefix.as<double>(), nullptr, ctx->stream));
+    r.launches += 1;
     const CoilCut pp = precess64_cut(r.ns, r.nc, nsamples);
     HOMS_CUDA(r.partial.ensure(pp.partial_bytes));
     Precess64Args a;
@@ -1652,7 +1652,7 @@ void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDe
     // the prefix kernel looks ranks up by node
     HOMS_CUDA(split_prefix_launch(q.dt, split_column_sources(method, h, q.gx, q.gy, q.gz), q.adc,
                                   ctx->block_rank.as<int32_t>() - (first + 1), first, last, 0, nadc, gamma,
-                                  ctx->block_prefix.as<double>(), ctx->stream));
+                                  ctx->block_prefix.as<double>(), nullptr, ctx->stream));
     const CoilCut pp = precess64_cut(p.ns, p.nc, nadc);
     HOMS_CUDA(ctx->scratch_partial.ensure(pp.partial_bytes));
     // The kernels read and write the state as 16-byte pairs: a caller's array off

@@ -79,7 +79,10 @@
 #include <string>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "homs_common.cuh"
+#include "homs_fp64math.cuh"
 #include "homs_split.cuh"
 
 namespace homs {
@@ -93,6 +96,7 @@ constexpr int PHASE_DIGITS = 5;  // base-256 digits of the phase integers
 constexpr int PREFIX_STRIDE = SPLIT_PREFIX_STRIDE;  // doubles per prefix row: kappa_0..kappa_16, t at PREFIX_T
 constexpr int PREFIX_T = SPLIT_PREFIX_T;
 constexpr int GROUP_COILS = 32;  // coils per kernel pass (N <= 64 output columns)
+constexpr int SPLIT_FIN_ROWS = 16;  // rows per finalize block (TR loop below: 8, 16, 32 rows 17.87, 17.84, 17.93 ms)
 constexpr int NMAG_WARPS = 16;
 constexpr int MMA_WARP = 16;    // coil MMA issuer (allocates TMEM)
 constexpr int LOAD_WARP = 17;
@@ -832,24 +836,22 @@ __global__ void __launch_bounds__(THREADS, 1) split_precession_kernel(const __gr
 // magnetisation digit (64 * 2^24 times the column's sensitivity integers:
 // colsum * 2^14 in the accumulator's units of 2^16), exact in int64 for one
 // slot and rounded once to FP64 (several slots: each rounded, summed in slot
-// order); then the rotation by -angle_offset_error() (the constant offset of
-// the kernel's angles), the power-of-two scales of the operands undone, and
-// complex samples written: column n < ncg is Re S(j, coil0 + n), ncg <= n <
-// 2 ncg is Im.  The accumulator is left zero for the next launch.
+// order); then the rotation (rc, rs) by -angle_offset_error() (the constant
+// offset of the kernel's angles), the power-of-two scales of the operands
+// undone, and complex samples written: column n < ncg is Re S(j, coil0 + n),
+// ncg <= n < 2 ncg is Im.  The accumulator is left zero for the next launch.
+// Bound by latency (a few MB through L2).
 template <typename T>
 __global__ void __launch_bounds__(256) split_finalize_kernel(unsigned long long *acc, int64_t nsamples, int32_t ncg,
                                                              int n_cols, int nacc, const long long *colsum,
-                                                             const int *coil_exp,
-                                                             const unsigned long long *amp_max, cplx<T> *sig,
-                                                             int64_t ldsig) {
+                                                             const int *coil_exp, const unsigned long long *amp_max,
+                                                             double rc, double rs, cplx<T> *sig, int64_t ldsig) {
     // A block takes FIN_ROWS rows x n_cols columns of one time tile (the
-    // accumulator's rows are contiguous per column: coalesced), then writes
-    // every coil's samples of those rows from shared memory.
-    constexpr int FIN_ROWS = 32, PER = FIN_ROWS * 64 / 256;
+    // accumulator's rows are contiguous per column), then writes every coil's
+    // samples of those rows from shared memory.
+    constexpr int FIN_ROWS = SPLIT_FIN_ROWS, PER = FIN_ROWS * 64 / 256;
     __shared__ double sacc[FIN_ROWS * 64];
     const int ea = amp_exp(*amp_max);
-    double rs, rc;
-    sincos(-angle_offset_error(), &rs, &rc);
     const int64_t tiles = (nsamples + TM - 1) / TM;
     const int64_t units = tiles * (TM / FIN_ROWS);
     const int elems = FIN_ROWS * n_cols;  // n_cols <= 64
@@ -1125,7 +1127,7 @@ __global__ void colsum_kernel(const cplx<double> *csm_rows, int64_t ns, int32_t 
 
 // Per-segment spin parameters of every chunk, [turn of arg(m0) x 32 | r2 x 32
 // | l2 x 32]: the initial phase as a 32-bit turn fraction, -log2(e)/T2 and
-// log2|m0| (float; l2_shift_kernel then subtracts the segment's amplitude
+// log2|m0| (float; segment_operands_kernel then subtracts the segment's amplitude
 // exponent); also the largest |m0| (amplitude scale of the segment).
 __global__ void spin_params_kernel(const double *T2, const cplx<double> *xy, int64_t ns, int64_t nchunks,
                                    unsigned long long *amp_max, uint32_t *params) {
@@ -1160,18 +1162,6 @@ __global__ void spin_params_kernel(const double *T2, const cplx<double> *xy, int
     }
 }
 
-// log2|m0| - eA of every spin of the segment (eA = amp_exp of the largest
-// |m0|), so that the magnetisation warps' ex2 argument t r2 + l2 stays small.
-__global__ void l2_shift_kernel(uint32_t *params, int64_t nchunks, const unsigned long long *amp_max) {
-    const float ea = (float)amp_exp(*amp_max);
-    const int64_t total = nchunks * KC;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < total;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t *p = params + (s / KC) * (PARAM_BYTES / 4) + 2 * KC + (s % KC);
-        *p = __float_as_uint(__uint_as_float(*p) - ea);
-    }
-}
-
 // Prefix table of one segment, over blocks (column, part): columns 0..16 are
 // kappa_k, the scaled running trapezoid sums (f(n)+f(n+1)) dt(n), written at
 // every ADC node (row = sample index) and at the end node (row nsamples), with
@@ -1180,9 +1170,13 @@ __global__ void l2_shift_kernel(uint32_t *params, int64_t nchunks, const unsigne
 // A column's intervals are cut into PREFIX_PARTS contiguous parts, and a
 // part into one contiguous run per thread.  Every sum is taken in a fixed
 // order (within a run, runs in thread order, parts in part order), so the
-// table does not depend on timing.  Two launches: the part totals
-// (prefix_part_kernel, into rows nsamples+2 ..), then the scan itself
-// (prefix_kernel), each part starting from the sum of the parts before it.
+// table does not depend on timing.  The parts of a column are one cluster and
+// pass their totals and maxima through distributed shared memory: one launch,
+// 9.5 us for 2,220 intervals, where two (totals, then the scan) took 17; bound by
+// the 256-step chain of the run totals.  With the spin parameters, operands,
+// accumulators and final state in one launch each, a segment's small kernels
+// take 20 us less: a TR loop of 35 segments (80,000 spins x 2,000 samples x 32
+// coils) 18.5 -> 17.8 ms, a served request (3,721 x 5,000 x 8) 345 -> 329 us.
 constexpr int PREFIX_PARTS = 8;
 constexpr int PREFIX_COLS = 18;
 struct PrefixColumn {
@@ -1210,55 +1204,49 @@ __device__ __forceinline__ void prefix_run(int64_t nint, int part, int64_t &i0, 
     i0 = min(p1, p0 + per * threadIdx.x);
     i1 = min(p1, i0 + per);
 }
+constexpr int PREFIX_THREADS = 256;
 // Sum of the runs' values in thread order (thread 0), and each run's exclusive
 // prefix in part[].
-__device__ double block_exclusive(double *part, double local) {
+__device__ void block_exclusive(double *part, double local, double *total) {
     part[threadIdx.x] = local;
     __syncthreads();
-    __shared__ double total;
     if (threadIdx.x == 0) {
         double run = 0.0;
-        for (int i = 0; i < (int)blockDim.x; ++i) {
-            const double v = part[i];
-            part[i] = run;
-            run += v;
+        for (int i = 0; i < PREFIX_THREADS; i += 16) {
+            double v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = part[i + k];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                part[i + k] = run;
+                run += v[k];
+            }
         }
-        total = run;
+        *total = run;
     }
     __syncthreads();
-    return total;
 }
 
-__global__ void prefix_part_kernel(const double *dt, const __grid_constant__ SplitColumns src, int64_t n_lo, int64_t n_hi,
-                                   int64_t nsamples, double gamma, double *prefix) {
-    __shared__ double part[256];
+// zero_word (may be NULL) is set to 0: the segment's amplitude maximum.
+__global__ void __cluster_dims__(1, PREFIX_PARTS, 1) __launch_bounds__(PREFIX_THREADS)
+    prefix_kernel(const double *dt, const __grid_constant__ SplitColumns src, const uint8_t *adc, const int32_t *rank,
+                  int64_t rank_base, int64_t n_lo, int64_t n_hi, int64_t nsamples, double gamma, double *prefix,
+                  unsigned long long *zero_word) {
+    __shared__ double part[PREFIX_THREADS], total, largest;
+    __shared__ double warp_peak[PREFIX_THREADS / 32];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int col = blockIdx.x, pt = blockIdx.y;
-    const PrefixColumn c = prefix_column(src, col, gamma);
-    int64_t i0, i1;
-    prefix_run(n_hi - n_lo, pt, i0, i1);
-    double local = 0.0;
-    for (int64_t i = i0; i < i1; ++i) local += prefix_term(c, dt, n_lo + i);
-    const double total = block_exclusive(part, local);
-    if (threadIdx.x == 0) {
-        prefix[(size_t)(nsamples + 2 + pt) * PREFIX_STRIDE + col] = total;
-        if (pt == 0 && col < 17) prefix[(size_t)(nsamples + 1) * PREFIX_STRIDE + col] = 0.0;  // the maximum, below
-    }
-}
-
-__global__ void prefix_kernel(const double *dt, const __grid_constant__ SplitColumns src, const uint8_t *adc, const int32_t *rank,
-                              int64_t rank_base, int64_t n_lo, int64_t n_hi, int64_t nsamples, double gamma,
-                              double *prefix) {
-    __shared__ double part[256];
-    const int col = blockIdx.x, pt = blockIdx.y;
+    if (zero_word && col == 0 && pt == 0 && threadIdx.x == 0) *zero_word = 0ull;
     const PrefixColumn c = prefix_column(src, col, gamma);
     const int64_t nint = n_hi - n_lo;
     int64_t i0, i1;
     prefix_run(nint, pt, i0, i1);
-    double carry = 0.0;
-    for (int q = 0; q < pt; ++q) carry += prefix[(size_t)(nsamples + 2 + q) * PREFIX_STRIDE + col];
     double local = 0.0;
     for (int64_t i = i0; i < i1; ++i) local += prefix_term(c, dt, n_lo + i);
-    block_exclusive(part, local);
+    block_exclusive(part, local, &total);
+    cluster.sync();
+    double carry = 0.0;
+    for (int q = 0; q < pt; ++q) carry += *cluster.map_shared_rank(&total, q);
     double cum = carry + part[threadIdx.x];
     double peak = 0.0;
     for (int64_t i = i0; i < i1; ++i) {
@@ -1293,18 +1281,23 @@ __global__ void prefix_kernel(const double *dt, const __grid_constant__ SplitCol
             pr[19] = 0.0;
         }
     }
-    // Largest |kappa| of the column (row nsamples+1) for the phase-range check:
-    // the block's maximum, then the parts' by an integer maximum of the bits
-    // (the values are non-negative, so their bits order as they do).
+    // Largest |kappa| of the column (row nsamples+1) for the phase-range check.
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) peak = fmax(peak, __shfl_xor_sync(0xffffffffu, peak, o));
+    if ((threadIdx.x & 31) == 0) warp_peak[threadIdx.x >> 5] = peak;
     __syncthreads();
-    part[threadIdx.x] = peak;
-    __syncthreads();
-    if (threadIdx.x == 0 && col < 17) {
+    if (threadIdx.x == 0) {
         double mx = 0.0;
-        for (int i = 0; i < (int)blockDim.x; ++i) mx = fmax(mx, part[i]);
-        atomicMax(reinterpret_cast<unsigned long long *>(prefix + (size_t)(nsamples + 1) * PREFIX_STRIDE + col),
-                  (unsigned long long)__double_as_longlong(mx));
+        for (int i = 0; i < PREFIX_THREADS / 32; ++i) mx = fmax(mx, warp_peak[i]);
+        largest = mx;
     }
+    cluster.sync();
+    if (pt == 0 && threadIdx.x == 0 && col < 17) {
+        double mx = 0.0;
+        for (int q = 0; q < PREFIX_PARTS; ++q) mx = fmax(mx, *cluster.map_shared_rank(&largest, q));
+        prefix[(size_t)(nsamples + 1) * PREFIX_STRIDE + col] = mx;
+    }
+    cluster.sync();  // no block leaves while another reads its shared memory
 }
 
 // Phase A operand of every tile of a segment and the per-sample rows: for
@@ -1314,16 +1307,30 @@ __global__ void prefix_kernel(const double *dt, const __grid_constant__ SplitCol
 // 2^30 + 128 (quarter-turn offset and the rounding of the 23-bit angle) and
 // the elapsed time.  Rows past nsamples are zero.  Sets error bit 64 when a
 // term's range bmax_k max|kappa_k| exceeds PHASE_RANGE_LIMIT turns.
-__global__ void phase_a_kernel(const double *prefix, int64_t nsamples, int64_t nrows,
-                               const unsigned long long *term_max, unsigned int *err, uint8_t *phase_a,
-                               uint32_t *rows) {
+// In the same launch, what else the split kernel needs by then: log2|m0| - eA of
+// every spin (eA = amp_exp of the largest |m0|, so that the magnetisation
+// warps' ex2 argument t r2 + l2 stays small), and the coil accumulators at zero
+// (each finalize leaves them so, a failed run does not).
+__global__ void segment_operands_kernel(const double *prefix, int64_t nsamples, int64_t nrows,
+                                        const unsigned long long *term_max, unsigned int *err, uint8_t *phase_a,
+                                        uint32_t *rows, uint32_t *params, int64_t nchunks,
+                                        const unsigned long long *amp_max, ulonglong2 *acc, int64_t acc_pairs) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    {
+        const float ea = (float)amp_exp(*amp_max);
+        for (int64_t s = tid; s < nchunks * KC; s += stride) {
+            uint32_t *p = params + (s / KC) * (PARAM_BYTES / 4) + 2 * KC + (s % KC);
+            *p = __float_as_uint(__uint_as_float(*p) - ea);
+        }
+        for (int64_t i = tid; i < acc_pairs; i += stride) acc[i] = make_ulonglong2(0ull, 0ull);
+    }
     const double *kmax = prefix + (size_t)(nsamples + 1) * PREFIX_STRIDE;
     if (blockIdx.x == 0 && threadIdx.x < NSLOT) {
         const double bmax = __longlong_as_double((long long)term_max[threadIdx.x]);
         if (!(bmax * kmax[threadIdx.x + 1] <= PHASE_RANGE_LIMIT)) atomicOr(err, 64u);
     }
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nrows;
-         j += (int64_t)gridDim.x * blockDim.x) {
+    // rows from the last block down: the first ones have the most of the above
+    for (int64_t j = (gridDim.x - 1 - blockIdx.x) * (int64_t)blockDim.x + threadIdx.x; j < nrows; j += stride) {
         uint32_t dig[PHASE_DIGITS][4];
 #pragma unroll
         for (int d = 0; d < PHASE_DIGITS; ++d)
@@ -1372,23 +1379,27 @@ __global__ void phase_a_kernel(const double *prefix, int64_t nsamples, int64_t n
     }
 }
 
-// Final state of a segment in FP64: Mxy = |m0| e^{-T/T2} cis(2 pi theta_end),
-// Mz = Mz e^{-T/T1} + rho (1 - e^{-T/T1}).
+// Final state of a segment in FP64: Mxy = m0 e^{-T/T2} cis(2 pi theta_end), Mz =
+// Mz e^{-T/T1} + rho (1 - e^{-T/T1}).
 __global__ void state_update_kernel(const double *basis, const double *dw, const double *endrow, const double *T1,
                                     const double *T2, const double *rho, int64_t ns, cplx<double> *xy, double *mz) {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < ns; s += (int64_t)gridDim.x * blockDim.x) {
-        const cplx<double> m0 = xy[s];
-        double th = fma(dw[s] * (1.0 / (2.0 * 3.141592653589793)), endrow[16],
-                        atan2(m0.im, m0.re) * (1.0 / (2.0 * 3.141592653589793)));
-        for (int k = 0; k < 16; ++k) th = fma(basis[s * 16 + k], endrow[k], th);
+        const double2 *b = reinterpret_cast<const double2 *>(basis + s * 16);
+        double th = dw[s] * (1.0 / (2.0 * 3.141592653589793)) * endrow[16];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const double2 v = b[k];
+            th = fma(v.x, endrow[2 * k], th);
+            th = fma(v.y, endrow[2 * k + 1], th);
+        }
         const double T = endrow[PREFIX_T];
-        const double mag = hypot(m0.re, m0.im);
-        const double f = th - rint(th);
         double sn, cs;
-        sincospi(2.0 * f, &sn, &cs);
-        const double e2 = exp(-T / T2[s]);
-        xy[s] = cplx<double>{mag * e2 * cs, mag * e2 * sn};
-        const double e1 = exp(-T / T1[s]);
+        cis_turns(th, cs, sn);
+        const double e2 = pow2(-1.4426950408889634 * (T / T2[s]));
+        const cplx<double> m0 = xy[s];
+        const double ec = e2 * cs, es = e2 * sn;
+        xy[s] = cplx<double>{m0.re * ec - m0.im * es, m0.re * es + m0.im * ec};
+        const double e1 = pow2(-1.4426950408889634 * (T / T1[s]));
         mz[s] = mz[s] * e1 + rho[s] * (1.0 - e1);
     }
 }
@@ -1609,14 +1620,13 @@ cudaError_t split_launch(const SplitJobDesc *jobs, int n_jobs, cudaStream_t stre
     return launch_precession(n_mma, ka, (unsigned)G, kernel_smem(n_mma), stream);
 }
 
-size_t split_prefix_rows(int64_t nsamples) { return (size_t)nsamples + 2 + PREFIX_PARTS; }
+size_t split_prefix_rows(int64_t nsamples) { return (size_t)nsamples + 2; }
 
 cudaError_t split_prefix_launch(const double *dt, const SplitColumns &cols, const uint8_t *adc, const int32_t *grank,
                                 int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
-                                double *prefix, cudaStream_t stream) {
-    const dim3 pgrid(PREFIX_COLS, PREFIX_PARTS);
-    prefix_part_kernel<<<pgrid, 256, 0, stream>>>(dt, cols, n_lo, n_hi, nsamples, gamma, prefix);
-    prefix_kernel<<<pgrid, 256, 0, stream>>>(dt, cols, adc, grank, sample0, n_lo, n_hi, nsamples, gamma, prefix);
+                                double *prefix, unsigned long long *zero_word, cudaStream_t stream) {
+    prefix_kernel<<<dim3(PREFIX_COLS, PREFIX_PARTS), PREFIX_THREADS, 0, stream>>>(
+        dt, cols, adc, grank, sample0, n_lo, n_hi, nsamples, gamma, prefix, zero_word);
     return cudaGetLastError();
 }
 
@@ -1637,28 +1647,16 @@ cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t
     seg->slabs = 0;
     const size_t prefix_rows = std::max<size_t>((size_t)(tiles * TM), split_prefix_rows(nsamples));
     if ((e = grow(r.prefix, r.prefix_bytes, prefix_rows * PREFIX_STRIDE * sizeof(double))) != cudaSuccess) return e;
-    if ((e = grow(r.params, r.params_bytes, (size_t)nchunks * PARAM_BYTES)) != cudaSuccess) return e;
     // The segment's samples are the global ADC indices sample0 .. sample0 + nsamples - 1.
     if ((e = split_prefix_launch((const double *)a.dt, a.cols, (const uint8_t *)a.adc, a.grank, n_lo, n_hi, sample0,
-                                 nsamples, a.gamma, (double *)r.prefix, stream)) != cudaSuccess)
+                                 nsamples, a.gamma, (double *)r.prefix, (unsigned long long *)r.amp, stream)) !=
+        cudaSuccess)
         return e;
-    if ((e = cudaMemsetAsync(r.amp, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
-    spin_params_kernel<<<grid_for(r.ns_pad), 256, 0, stream>>>((const double *)a.T2, (const cplx<double> *)a.xy,
-                                                               r.ns, nchunks, (unsigned long long *)r.amp,
-                                                               (uint32_t *)r.params);
-    l2_shift_kernel<<<grid_for(r.ns_pad), 256, 0, stream>>>((uint32_t *)r.params, nchunks,
-                                                            (const unsigned long long *)r.amp);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (a.launches) *a.launches += 4;
+    if (a.launches) *a.launches += 1;
     if (nsamples == 0) return cudaSuccess;
+    if ((e = grow(r.params, r.params_bytes, (size_t)nchunks * PARAM_BYTES)) != cudaSuccess) return e;
     if ((e = grow(r.phase_a, r.phase_a_bytes, (size_t)tiles * PHASE_A_BYTES)) != cudaSuccess) return e;
     if ((e = grow(r.rows, r.rows_bytes, (size_t)tiles * TM * 2 * sizeof(uint32_t))) != cudaSuccess) return e;
-    phase_a_kernel<<<grid_for(tiles * TM), 256, 0, stream>>>((const double *)r.prefix, nsamples, tiles * TM,
-                                                             (const unsigned long long *)r.term_max,
-                                                             (unsigned int *)r.err, (uint8_t *)r.phase_a,
-                                                             (uint32_t *)r.rows);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (a.launches) *a.launches += 1;
     const int slabs = choose_slabs(tiles, nchunks, sm_count());
     if (tiles > INT32_MAX / slabs || nchunks > INT32_MAX || slabs > nchunks) {
         *err = "split mode: segment too large for one launch";
@@ -1666,10 +1664,19 @@ cudaError_t split_segment_begin(SplitResident &r, const SplitRunArgs &a, int64_t
     }
     seg->slabs = slabs;
     seg->nacc = acc_slots(nchunks);
-    // the coil accumulators start at zero (each group's finalize leaves them so)
     const size_t abytes = sizeof(unsigned long long) * (size_t)tiles * seg->nacc * TM * r.n_mma;
     if ((e = grow(r.accum, r.accum_bytes, abytes)) != cudaSuccess) return e;
-    return cudaMemsetAsync(r.accum, 0, abytes, stream);
+    spin_params_kernel<<<grid_for(r.ns_pad), 256, 0, stream>>>((const double *)a.T2, (const cplx<double> *)a.xy,
+                                                               r.ns, nchunks, (unsigned long long *)r.amp,
+                                                               (uint32_t *)r.params);
+    const int64_t pairs = (int64_t)(abytes / sizeof(ulonglong2));
+    const int64_t work = std::max(std::max<int64_t>(r.ns_pad, tiles * TM), pairs / 2);
+    segment_operands_kernel<<<grid_for(work), 256, 0, stream>>>(
+        (const double *)r.prefix, nsamples, tiles * TM, (const unsigned long long *)r.term_max, (unsigned int *)r.err,
+        (uint8_t *)r.phase_a, (uint32_t *)r.rows, (uint32_t *)r.params, nchunks, (const unsigned long long *)r.amp,
+        (ulonglong2 *)r.accum, pairs);
+    if (a.launches) *a.launches += 2;
+    return cudaGetLastError();
 }
 
 SplitJobDesc split_segment_job(const SplitResident &r, const SplitSegment &seg, int grp) {
@@ -1693,12 +1700,13 @@ cudaError_t split_segment_finalize(SplitResident &r, const SplitRunArgs &a, cons
     const int coil0 = grp * GROUP_COILS;
     const int ncg = std::min<int>(GROUP_COILS, r.nc - coil0);
     const int *cexp = reinterpret_cast<const int *>(reinterpret_cast<const unsigned long long *>(r.coil_exp) + r.nc);
-    const int fin_blocks = (int)std::min<int64_t>(seg.tiles * (TM / 32), 148 * 8);
+    const int fin_blocks = (int)std::min<int64_t>(seg.tiles * (TM / SPLIT_FIN_ROWS), 148 * 16);
+    const double rc = std::cos(-angle_offset_error()), rs = std::sin(-angle_offset_error());
     if (a.sizeof_T == 8)
         split_finalize_kernel<double><<<fin_blocks, 256, 0, stream>>>(
             (unsigned long long *)r.accum, seg.nsamples, ncg, r.n_mma, seg.nacc,
-            (const long long *)r.colsum + (size_t)grp * r.n_mma, cexp + coil0, (const unsigned long long *)r.amp,
-            (cplx<double> *)a.sig + sample0 + (int64_t)coil0 * a.nadc, a.nadc);
+            (const long long *)r.colsum + (size_t)grp * r.n_mma, cexp + coil0, (const unsigned long long *)r.amp, rc,
+            rs, (cplx<double> *)a.sig + sample0 + (int64_t)coil0 * a.nadc, a.nadc);
     return cudaGetLastError();
 }
 

@@ -105,12 +105,13 @@ cudaError_t split_attach(SplitResident &r, const SplitResident &src);
 // Prefix table of a segment (nodes n_lo .. n_hi, `nsamples` ADC samples of
 // global index sample0 ..): FP64 rows of kappa_0 .. kappa_16 and, at
 // SPLIT_PREFIX_T, the elapsed time, one row per sample, then the row of the end
-// node.  `prefix` holds split_prefix_rows(nsamples) rows.
+// node.  `prefix` holds split_prefix_rows(nsamples) rows; zero_word (may be NULL)
+// is set to 0.
 constexpr int SPLIT_PREFIX_STRIDE = 24, SPLIT_PREFIX_T = 20;
 size_t split_prefix_rows(int64_t nsamples);
 cudaError_t split_prefix_launch(const double *dt, const SplitColumns &cols, const uint8_t *adc, const int32_t *grank,
                                 int64_t n_lo, int64_t n_hi, int64_t sample0, int64_t nsamples, double gamma,
-                                double *prefix, cudaStream_t stream);
+                                double *prefix, unsigned long long *zero_word, cudaStream_t stream);
 
 // Clear the device error word before a run.
 cudaError_t split_reset_error(SplitResident &r, cudaStream_t stream);
