@@ -567,6 +567,9 @@ struct Resident : ResidentBase {
     double gamma = 0;
     SplitResident split;  // split-precision operands (built on demand)
     bool split_ready = false;
+    // Workspace of plain runs, one allocation; spin_table (unless it is a resident
+    // phantom's), prefix, nodes, walk and partial are views of it then.
+    DevBuf work;
     // Plain FP64 precession: the phantom's spin table and the prefix table of a segment.
     DevBuf spin_table, prefix;
     bool spin_table_ready = false;
@@ -602,7 +605,7 @@ struct Resident : ResidentBase {
         size_t b = split.device_bytes();
         for (const DevBuf *d : {&phantom_block, &sequence_block, &x, &y, &z, &rho, &T1, &T2, &dw, &csm_rows, &t, &dt, &gx,
                                 &gy, &gz, &b1, &df, &psi, &adc, &bnd, &xy, &mz, &acc, &rho_init, &partial, &sig,
-                                &spin_table, &prefix, &block_time, &nodes, &walk, &grank})
+                                &work, &spin_table, &prefix, &block_time, &nodes, &walk, &grank})
             b += d->owned_bytes();
         for (int k = 0; k < 16; ++k) b += h[k].owned_bytes();
         return b;
@@ -826,10 +829,8 @@ SplitColumns prefix_columns(const Resident<T> &r, uint32_t method) {
     return split_column_sources(method, h, r.gx.p, r.gy.p, r.gz.p);
 }
 
-// The plain FP64 path's spin table, unless `r` has it, its own or a resident phantom's.
-inline void ensure_spin_table(homs_context *ctx, Resident<double> &r) {
-    if (r.spin_table_ready) return;
-    HOMS_CUDA(r.spin_table.ensure(precess64_table_bytes(r.ns)));
+// The plain FP64 path's spin table, built in `r.spin_table`.
+inline void build_spin_table(homs_context *ctx, Resident<double> &r) {
     HOMS_CUDA(precess64_table(r.x.as<double>(), r.y.as<double>(), r.z.as<double>(), r.dw.as<double>(),
                               r.T2.as<double>(), r.ns, r.spin_table.p, ctx->stream));
     r.spin_table_ready = true;
@@ -838,13 +839,11 @@ inline void ensure_spin_table(homs_context *ctx, Resident<double> &r) {
 // One plain FP64 precession segment (intervals [n_lo, n_hi), `nsamples` samples from sample0 on).
 inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t method, bool capture, int64_t n_lo,
                             int64_t n_hi, int64_t sample0, int64_t nsamples) {
-    HOMS_CUDA(r.prefix.ensure(sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nsamples)));
     HOMS_CUDA(split_prefix_launch(r.dt.as<double>(), prefix_columns(r, method), r.adc.as<uint8_t>(),
                                   r.grank.as<int32_t>(), n_lo, n_hi, sample0, nsamples, r.gamma,
                                   r.prefix.as<double>(), nullptr, ctx->stream));
     r.launches += 1;
     const CoilCut pp = precess64_cut(r.ns, r.nc, nsamples);
-    HOMS_CUDA(r.partial.ensure(pp.partial_bytes));
     Precess64Args a;
     a.ns = r.ns;
     a.nsamples = nsamples;
@@ -867,20 +866,9 @@ inline void plain_segment64(homs_context *ctx, Resident<double> &r, uint32_t met
                             &r.launches, ctx->stream));
 }
 
-// The plain FP32 path's node table of the sequence and method.
-inline void ensure_nodes32(homs_context *ctx, Resident<float> &r, uint32_t method) {
-    if (r.nodes_method != method) {
-        HOMS_CUDA(r.nodes.ensure(precess32_node_bytes(r.nt)));
-        HOMS_CUDA(precess32_nodes(r.seq(), method, r.block_time.as<float>(), r.nodes.p, ctx->stream));
-        r.nodes_method = method;
-    }
-}
-
 // One launch round of a plain FP32 precession run.
 inline void plain_round32(homs_context *ctx, Resident<float> &r, uint32_t method, bool capture, const Launch &L) {
     const CoilCut cut = precess32_cut(r.ns, r.nc, L.nsamples);
-    HOMS_CUDA(r.walk.ensure(precess32_work_bytes(r.ns, L.nsamples, L.nblocks)));
-    HOMS_CUDA(r.partial.ensure(cut.partial_bytes));
     Precess32Args a;
     a.phantom = r.phantom();
     a.state = StateDev<float>{r.xy.as<cplx<float>>(), r.mz.as<float>(), r.acc.as<float>()};
@@ -902,12 +890,17 @@ inline void plain_round32(homs_context *ctx, Resident<float> &r, uint32_t method
                             &r.launches, ctx->stream));
 }
 
+// Partial sums of an excitation launch.
+template <typename T>
+size_t excitation_partial_bytes(const Resident<T> &r, const Launch &L) {
+    return sizeof(cplx<T>) * (size_t)r.nc * (size_t)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS) * (size_t)L.nsamples;
+}
+
 // One launch of an excitation run (at most excitation_samples samples).
 template <typename T>
 void excitation_launch(Resident<T> &r, uint32_t method, const Launch &L, cudaStream_t stream) {
     const int grid = (int)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-    HOMS_CUDA(r.partial.ensure(sizeof(cplx<T>) * (size_t)r.nc * (size_t)grid *
-                               (size_t)std::max<int64_t>(L.nsamples, 1)));
+    if (r.partial.bytes < excitation_partial_bytes(r, L)) HOMS_CUDA(r.partial.ensure(excitation_partial_bytes(r, L)));
     SegmentArgs<T> a;
     a.n_lo = L.n_lo;
     a.n_hi = L.n_hi;
@@ -936,26 +929,65 @@ int64_t excitation_samples(const Resident<T> &r) {
     return std::max<int64_t>(PLAIN_STAGE, (int64_t)((size_t(512) << 20) / (sizeof(cplx<T>) * (size_t)r.nc * grid)));
 }
 
+// Size the workspace of a plain run's launches and build the tables in it: the
+// phantom's spin table (FP64) or the node table of the sequence and method
+// (FP32).  A later run of the same plan finds all of it in place.
+template <typename T>
+void prepare_plain(homs_context *ctx, Resident<T> &r, uint32_t method, const std::vector<Launch> &plan) {
+    auto align = [](size_t n) { return (n + 255) & ~size_t(255); };
+    size_t table = 0, per_run = 0, partial = 0;
+    for (const Launch &L : plan) {
+        if (L.rf) {
+            partial = std::max(partial, excitation_partial_bytes(r, L));
+        } else if constexpr (sizeof(T) == 8) {
+            per_run = std::max(per_run, sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(L.nsamples));
+            partial = std::max(partial, precess64_cut(r.ns, r.nc, L.nsamples).partial_bytes);
+        } else {
+            per_run = std::max(per_run, precess32_work_bytes(r.ns, L.nsamples, L.nblocks));
+            partial = std::max(partial, precess32_cut(r.ns, r.nc, L.nsamples).partial_bytes);
+        }
+    }
+    bool own_table = true;  // not a resident phantom's
+    if constexpr (sizeof(T) == 8) {
+        const char *t = r.spin_table.template as<char>(), *w = r.work.template as<char>();
+        own_table = !r.spin_table_ready || (t >= w && t < w + r.work.bytes);
+        if (own_table) table = precess64_table_bytes(r.ns);
+    } else {
+        table = precess32_node_bytes(r.nt);
+    }
+    const void *before = r.work.p;
+    HOMS_CUDA(r.work.ensure(align(table) + align(per_run) + align(partial)));
+    char *at = r.work.template as<char>();
+    if constexpr (sizeof(T) == 8) {
+        if (own_table) {
+            const bool stays = r.work.p == before && r.spin_table_ready;
+            r.spin_table.view(at, table);
+            if (!stays) build_spin_table(ctx, r);
+        }
+        r.prefix.view(at + align(table), per_run);
+    } else {
+        const bool stays = r.work.p == before && r.nodes_method == method;
+        r.nodes.view(at, table);
+        if (!stays) {
+            HOMS_CUDA(precess32_nodes(r.seq(), method, r.block_time.template as<float>(), r.nodes.p, ctx->stream));
+            r.nodes_method = method;
+        }
+        r.walk.view(at + align(table), per_run);
+    }
+    r.partial.view(at + align(table) + align(per_run), partial);
+}
+
 template <typename T>
 void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture) {
     const unsigned ev_flags = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
     LaunchLimits lim{excitation_samples(r), INT64_MAX, INT64_MAX};
-    if constexpr (sizeof(T) == 8) {
-        if (capture) {
-            HOMS_REQUIRE(r.spin_table_ready, "internal: spin table missing under capture");
-        } else {
-            ensure_spin_table(ctx, r);
-        }
-    } else {
+    if constexpr (sizeof(T) == 4) {
         lim.precession_samples = precess32_max_samples(r.ns);
         lim.precession_blocks = precess32_max_blocks(r.ns);
-        if (capture) {
-            HOMS_REQUIRE(r.nodes_method == method, "internal: precession tables missing under capture");
-        } else {
-            ensure_nodes32(ctx, r, method);
-        }
     }
-    for (const Launch &L : plan_launches<T>(r, lim)) {
+    const std::vector<Launch> plan = plan_launches<T>(r, lim);
+    if (!capture) prepare_plain(ctx, r, method, plan);
+    for (const Launch &L : plan) {
         if (L.rf) {
             const auto ev = r.next_events();
             HOMS_CUDA(cudaEventRecordWithFlags(ev.first, ctx->stream, ev_flags));
@@ -1915,7 +1947,10 @@ homs_status homs_resident_create(homs_context *ctx, const homs_phantom *phantom,
             auto r = std::make_unique<Resident<double>>();
             fill_phantom<double>(ctx, r.get(), phantom);
             if (mode == HOMS_SPLIT) ensure_split<double>(ctx, *r);
-            else ensure_spin_table(ctx, *r);
+            else {
+                HOMS_CUDA(r->spin_table.ensure(precess64_table_bytes(r->ns)));
+                build_spin_table(ctx, *r);
+            }
             h->res = std::move(r);
         } else {
             auto r = std::make_unique<Resident<float>>();
