@@ -13,7 +13,7 @@
 //
 // What bounds it: the FP64 pipe (64 multiply-adds per SM and clock, the same
 // for DFMA and for the FP64 matrix instruction; the pipe is about 72% busy).
-// Per spin and sample 16 multiply-adds of phase, 41 FP64 operations of sine,
+// Per spin and sample 16 multiply-adds of phase, 34 FP64 operations of sine,
 // cosine, decay and the complex product, 3 per coil of contraction.
 //
 // Organisation: CTA = 8 warps, a tile of samples x a range of 32-spin chunks
@@ -28,10 +28,14 @@
 // k3 = Im M (Re c + Im c); Re = k1 - k3, Im = k1 + k2 (10.87 -> 10.31 ms at 8
 // coils, 6.15 -> 5.86 ms at 32).  wj < 8 (segments of few samples): the other
 // warps take other spin groups of the chunk and write partial sums of their own.
+// The decay is 2^(t_ref r2), once per spin, chunk and tile, times a degree-8
+// series of 2^((t - t_ref) r2) where that argument stays within 1/16 for the
+// whole warp (10.28 -> 9.35 ms, 5.84 -> 5.76 ms); two spin groups per iteration
+// let the two chains overlap (9.09 and 5.63 ms).
 //
 // Measured (B200, prepared runs, against the sequential per-spin kernel that it
 // replaces): 40,000 spins x 4 segments of 10,000 samples x 8 coils 44.6 ->
-// 10.3 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.9 ms.  Three
+// 9.1 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.6 ms.  Three
 // CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
 #include <algorithm>
 
@@ -53,6 +57,7 @@ constexpr double TWO_PI = 2.0 * 3.141592653589793;
 
 __host__ __device__ constexpr int csm_row(int nt) { return nt * 128 + 16; }  // bytes of a staged sensitivity row
 __host__ __device__ constexpr int stage_bytes(int nt) { return CHUNK * (BROW + 16 + 8 + csm_row(nt)); }
+__host__ __device__ constexpr int smem_bytes(int nt) { return NSTAGE * stage_bytes(nt) + 2 * CHUNK * 8; }  // + decays
 
 __host__ __device__ inline int64_t pad_spins(int64_t ns) { return (ns + CHUNK - 1) / CHUNK * CHUNK; }
 
@@ -158,7 +163,11 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
     // This warp's samples: rows 8 mt + r of its 16.  Phase slot of lane q in
     // step i: 4 q + i (the term order of a sum is free, and this one makes a
     // spin's fragment contiguous).
-    double kap[MT][4], k0[MT], tj[MT];
+    double kap[MT][4], k0[MT], tj[MT], dmax = 0.0;
+    const double t_ref =
+        a.prefix[(a.sample0 + imin64((int64_t)blockIdx.x * (8 * MT * WJ) + 4 * MT * WJ, a.round_samples - 1)) *
+                     SPLIT_PREFIX_STRIDE +
+                 SPLIT_PREFIX_T];
     const int64_t jw = (int64_t)blockIdx.x * (8 * MT * WJ) + wj * (8 * MT);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -166,10 +175,17 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
         const bool ok = j < a.round_samples;
         const double *row = a.prefix + (a.sample0 + (ok ? j : 0)) * SPLIT_PREFIX_STRIDE;
         k0[mt] = ok ? row[0] : 0.0;
-        tj[mt] = ok ? row[SPLIT_PREFIX_T] : 0.0;
+        tj[mt] = ok ? row[SPLIT_PREFIX_T] : t_ref;
+        dmax = fmax(dmax, fabs(tj[mt] - t_ref));
 #pragma unroll
         for (int i = 0; i < 4; ++i) kap[mt][i] = ok ? row[1 + 4 * q + i] : 0.0;
     }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+    // Decay of the tile: E = 2^(t_ref r2) once per spin and chunk, by one warp a
+    // chunk ahead, and a short series for the rest.
+    double *decay = reinterpret_cast<double *>(smem + NSTAGE * STAGE);
+    auto load_r2 = [&](int64_t ch) { return a.r2[ch * CHUNK + lane]; };
     const uint32_t on = (a.slots >> (4 * q)) & 15u;
     double k1[MT][NT][2], k2[MT][NT][2], k3[MT][NT][2];
 #pragma unroll
@@ -184,6 +200,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
         if (ch0 + s < ch1) issue(ch0 + s, s);
         cp_commit();
     }
+    if (warp == 0 && ch0 < ch1) decay[(ch0 & 1) * CHUNK + lane] = pow2(t_ref * load_r2(ch0));
     int stage = 0;
     for (int64_t ch = ch0; ch < ch1; ++ch) {
         cp_wait<NSTAGE - 2>();
@@ -191,9 +208,13 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
         const int fill = stage == 0 ? NSTAGE - 1 : stage - 1;  // the stage consumed last
         if (ch + NSTAGE - 1 < ch1) issue(ch + NSTAGE - 1, fill);
         cp_commit();
+        const bool next_decay = ch + 1 < ch1 && warp == (int)(ch & 7);
+        double next_r2 = 0.0;
+        if (next_decay) next_r2 = load_r2(ch + 1);
+        const double *dec = decay + (ch & 1) * CHUNK;
         const uint8_t *st = smem + stage * STAGE;
         if (++stage == NSTAGE) stage = 0;
-#pragma unroll 1
+#pragma unroll 2
         for (int g = kw; g < CHUNK / 8; g += KSPLIT) {
             const double2 *brow = reinterpret_cast<const double2 *>(st + (g * 8 + r) * BROW + q * 32);
             const double2 b01 = brow[0], b23 = brow[1];
@@ -210,16 +231,35 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt) dmma(th[mt], kap[mt][i], b[i]);
             double mr[MT][2], mi[MT][2], ms[MT][2];
+            // m0 and the decay of each element: m0 E and the series of 2^(dt r2), of
+            // degree 8 (error below 1e-17 for |dt r2| <= 1/16), where that holds for
+            // the whole warp; else m0 and 2^(t r2).
+            const bool near = __all_sync(0xffffffffu, dmax * fmax(fabs(rr.x), fabs(rr.y)) <= 0.0625);
+            double2 m[2] = {m0[0], m0[1]};
+            double ex[MT][2];
+            if (near) {
+                const double2 E = *reinterpret_cast<const double2 *>(dec + g * 8 + 2 * q);
+                m[0] = make_double2(m0[0].x * E.x, m0[0].y * E.x);
+                m[1] = make_double2(m0[1].x * E.y, m0[1].y * E.y);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) ex[mt][e] = pow2_small((tj[mt] - t_ref) * (e ? rr.y : rr.x));
+            } else {
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) ex[mt][e] = pow2(tj[mt] * (e ? rr.y : rr.x));
+            }
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     double sn, cs;
                     cis_turns(th[mt][e], cs, sn);
-                    const double ex = pow2(tj[mt] * (e ? rr.y : rr.x));
-                    const double ec = ex * cs, es = ex * sn;
-                    mr[mt][e] = m0[e].x * ec - m0[e].y * es;
-                    mi[mt][e] = m0[e].x * es + m0[e].y * ec;
+                    const double ec = ex[mt][e] * cs, es = ex[mt][e] * sn;
+                    mr[mt][e] = m[e].x * ec - m[e].y * es;
+                    mi[mt][e] = m[e].x * es + m[e].y * ec;
                     ms[mt][e] = mr[mt][e] + mi[mt][e];
                 }
 #pragma unroll
@@ -237,6 +277,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
                     }
                 }
         }
+        if (next_decay) decay[((ch + 1) & 1) * CHUNK + lane] = pow2(t_ref * next_r2);
     }
     cp_wait<0>();
     cplx<double> *out = a.partial + (size_t)(blockIdx.y * KSPLIT + kw) * a.round_samples * a.nc + c0;
@@ -286,7 +327,7 @@ cudaError_t launch(const KernelArgs &ka, int64_t tiles, int groups, cudaStream_t
     cudaError_t e = allow_max_dynamic_smem((const void *)main_kernel<NT, WJ>);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)tiles, (unsigned)ka.parts, (unsigned)groups);
-    main_kernel<NT, WJ><<<grid, THREADS, NSTAGE * stage_bytes(NT), stream>>>(ka);
+    main_kernel<NT, WJ><<<grid, THREADS, smem_bytes(NT), stream>>>(ka);
     return cudaGetLastError();
 }
 template <int NT>

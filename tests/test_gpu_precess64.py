@@ -64,6 +64,18 @@ def test_unused_terms_and_special_values(oracle, gpu_context):
     assert np.all(sig == 0)
 
 
+@pytest.mark.parametrize("low,high", [(0.05, 0.5), (0.5, 2.0), (2.0, 50.0), (0.01, 1e4)])
+def test_decay_series(oracle, gpu_context, low, high):
+    """T2 about and on both sides of the line between the short decay series and
+    2^(t r2) (a tile's half span over T2 ln 2 equal to 1/16), also within one warp."""
+    obj, seq, st = W.high_order_workload(nspins=90, nsteps=300, ncoils=6)
+    seq.adc[:] = np.arange(301) % 2 == 0
+    line = 16.0 * float(seq.t[128] - seq.t[0]) / math.log(2.0)
+    obj.T2[:] = np.random.default_rng(5).permutation(np.geomspace(low, high, 90)) * line
+    got, ref = _both(oracle, obj, seq, [(0, 300)], [False], BlochHighOrder("1111"), st)
+    assert all(nrmse(g, r) <= BAR for g, r in zip(got, ref))
+
+
 def test_block_call_with_state_off_16_bytes(oracle, gpu_context):
     """homs_precession_block accepts a state that is aligned to 8 bytes only."""
     import torch
