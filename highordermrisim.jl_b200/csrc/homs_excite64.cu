@@ -7,18 +7,22 @@
 // src/simulation/Bloch/BlochHighOrderSimulatitonMethod.jl:100-134).  As a
 // rotation of (Mx, My, Mz): with half-angle cosine w and sine v about the unit
 // field n, t = q x M and M' = M + w' t + q x t for q = sqrt(2) v n, w' = sqrt(2) w:
-// 15 operations where the spinor's complex products take about 60.
+// 15 operations where the spinor's complex products take about 60.  w and v / |B|
+// are even in |B|, so a small angle needs no root: two series in z = (half-angle)^2
+// (no root, reciprocal and quarter-turn reduction: 17.87 -> 15.65 ms for the TR loop
+// below).
 //
-// What bounds it: the FP64 pipe and its latency, about 45 operations per spin and
-// node (field 4, |B| and 1/|B| 7, half-angle cosine and sine 17, rotation 21,
-// relaxation 3).  The rotations of UNROLL nodes are formed before they are
+// What bounds it: the FP64 pipe and its latency, about 34 operations per spin and
+// node (field 4, z 1, series 8, rotation vector 3, rotation 15, relaxation 3).
+// The rotations of UNROLL nodes are formed before they are
 // applied, so that only rotation and relaxation are in the spin's dependent
 // chain.  CTAs of 64 threads spread an uneven number of warps over the SMs.
 //
 // Measured (B200, against the spinor kernel of homs_plain.cu): 80,000 spins x 400
-// nodes 449 -> 168 us; a TR loop of 35 such pulses with its split-mode readouts
-// 28.2 -> 18.7 ms.
+// nodes 449 -> 105 us; a TR loop of 35 such pulses with its split-mode readouts
+// 28.2 -> 15.7 ms.
 #include <algorithm>
+#include <type_traits>
 
 #include "homs_common.cuh"
 #include "homs_fp64math.cuh"
@@ -29,7 +33,7 @@ namespace excite64 {
 
 constexpr int THREADS = 64;
 constexpr int NODES = 64;  // nodes per stage
-constexpr int UNROLL = 4;  // rotations formed together (2: 18.89, 3: 18.79, 4: 18.70 ms for the TR loop below)
+constexpr int UNROLL = 4;  // rotations formed together (2, 3, 4, 6: 15.78, 15.76, 15.65, 15.87 ms for the TR loop)
 
 // 1/sqrt(x) from the hardware's approximation (2^-20 or better) by one step of
 // third order; 0 for x below 1e-300 (no field), NaN for NaN.
@@ -41,15 +45,59 @@ __device__ __forceinline__ double rsq(double x) {
     return x < 1e-300 ? 0.0 : y;
 }
 
+// sqrt(2) cos(h) and sqrt(2) sin(h) / h from z = h^2: interpolants at the
+// Chebyshev nodes of [0, 1/32] (degree 4) and [0, 5/8] (degree 7), within 1.3e-16
+// with their rounded coefficients.
+constexpr uint32_t NEAR_HI = 0x3FA00000, MID_HI = 0x3FE40000;  // high words of 1/32 and 5/8
+__device__ __forceinline__ void half_near(double z, double &c, double &s) {
+    c = 3.504430601676957e-05;
+    s = 3.894426466665344e-06;
+    c = fma(c, z, -0.0019641846711878626);
+    s = fma(s, z, -0.0002805978533901853);
+    c = fma(c, z, 0.05892556508959255);
+    s = fma(s, z, 0.0117851130189315);
+    c = fma(c, z, -0.7071067811865113);
+    s = fma(s, z, -0.23570226039551254);
+    c = fma(c, z, 1.4142135623730951);
+    s = fma(s, z, 1.4142135623730951);
+}
+__device__ __forceinline__ void half_mid(double z, double &c, double &s) {
+    c = -1.6053921180070224e-11;
+    s = -1.0715752882141984e-12;
+    c = fma(c, z, 2.9522487684836804e-09);
+    s = fma(s, z, 2.2709913861981155e-10);
+    c = fma(c, z, -3.897192557835503e-07);
+    s = fma(s, z, -3.542902614020508e-08);
+    c = fma(c, z, 3.507474110389768e-05);
+    s = fma(s, z, 3.897193457367114e-06);
+    c = fma(c, z, -0.0019641855032917683);
+    s = fma(s, z, -0.0002805979290420337);
+    c = fma(c, z, 0.058925565098878634);
+    s = fma(s, z, 0.011785113019775773);
+    c = fma(c, z, -0.7071067811865475);
+    s = fma(s, z, -0.23570226039551584);
+    c = fma(c, z, 1.4142135623730951);
+    s = fma(s, z, 1.4142135623730951);
+}
+// Any z (infinities and NaN included).
+__device__ __forceinline__ void half_far(double z, double &c, double &s) {
+    constexpr double SQRT2 = 1.4142135623730951;
+    const double r = rsq(z), h = z * r;
+    cis_turns(h * (0.5 / 3.141592653589793), c, s);
+    c *= SQRT2;
+    s *= SQRT2 * r;
+}
+
 // Spin-independent part of a node's step (the interval that starts there).
 // Its relaxation relative to the stage's first interval dt0: SAME for an equal
 // dt; NEAR for one within 1e-9 dt0 (the differences of rounded node times), dt -
 // dt0 to first order; OTHER anew.
 enum : int { SAME, NEAR, OTHER };
-struct alignas(16) Node {
-    double gx, gy, gz, dfg;  // gradient, df / gamma
-    double b1r, b1i, b2, c;  // B1, |B1|^2, -gamma dt / 2 (half-angle in turns per tesla)
-    double dt;               // dt, or dt - dt0 (NEAR)
+struct alignas(16) Node {  // fields times k = -pi gamma dt (half-angle in radians per tesla)
+    double gx, gy, gz, df;  // gradient, -df / gamma
+    double b1r, b1i, b2;    // B1, |B1|^2
+    double k;
+    double dt;  // dt, or dt - dt0 (NEAR)
     int relax;
 };
 struct Rotation {
@@ -78,17 +126,30 @@ __global__ void __launch_bounds__(THREADS, 9)
 
     // Relaxation over the stage's first interval: factors, rho (1 - e1).
     double e1 = 0.0, e2 = 0.0, c1 = 0.0;
-    auto rotation = [&](const Node &n) {
-        const double bz = fma(n.gx, px, fma(n.gy, py, fma(n.gz, pz, off - n.dfg)));
-        const double B2 = fma(bz, bz, n.b2);
-        const double rB = rsq(B2);
-        const double th = n.c * (B2 * rB);
-        double ch, sh;
-        if (__all_sync(0xffffffffu, (__double2hiint(th) & 0x7FFFFFFF) < 0x3FC00000)) cis_eighth(th, ch, sh);
-        else cis_turns(th, ch, sh);
-        constexpr double SQRT2 = 1.4142135623730951;
-        const double f = (SQRT2 * sh) * rB;
-        return Rotation{SQRT2 * ch, n.b1r * f, n.b1i * f, bz * f};
+    // Rotations of U nodes: one choice of the half-angle's range for all of them.
+    auto rotations = [&](const Node *n, Rotation *r, auto count) {
+        constexpr int U = decltype(count)::value;
+        double z[U];
+        uint32_t top = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            r[u].z = fma(n[u].gx, px, fma(n[u].gy, py, fma(n[u].gz, pz, fma(n[u].k, off, n[u].df))));
+            z[u] = fma(r[u].z, r[u].z, n[u].b2);
+            top = max(top, (uint32_t)__double2hiint(z[u]));
+        }
+        double c[U], f[U];
+        if (__all_sync(0xffffffffu, top < NEAR_HI)) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) half_near(z[u], c[u], f[u]);
+        } else if (__all_sync(0xffffffffu, top < MID_HI)) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) half_mid(z[u], c[u], f[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u) half_far(z[u], c[u], f[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) r[u] = Rotation{c[u], n[u].b1r * f[u], n[u].b1i * f[u], r[u].z * f[u]};
     };
     auto step = [&](const Rotation &r, const Node &n) {
         const double tx = fma(r.y, mz, -(r.z * my)), ty = fma(r.z, mx, -(r.x * mz)), tz = fma(r.x, my, -(r.y * mx));
@@ -112,8 +173,9 @@ __global__ void __launch_bounds__(THREADS, 9)
             const cplx<double> b1 = q.b1[g];
             const double dt = q.dt[g], d = dt - dt0;
             const int relax = d == 0.0 ? SAME : fabs(d) <= 1e-9 * dt0 ? NEAR : OTHER;
-            nodes[i] = Node{q.gx[g], q.gy[g], q.gz[g], q.df[g] / a.gamma_d, b1.re, b1.im,
-                            b1.re * b1.re + b1.im * b1.im, -0.5 * a.gamma_d * dt, relax == NEAR ? d : dt, relax};
+            const double k = -3.141592653589793 * a.gamma_d * dt, br = k * b1.re, bi = k * b1.im;
+            nodes[i] = Node{k * q.gx[g], k * q.gy[g], k * q.gz[g], 3.141592653589793 * q.df[g] * dt, br, bi,
+                            br * br + bi * bi, k, relax == NEAR ? d : dt, relax};
         }
         if (n0 == a.n_lo || dt0 != q.dt[n0 - NODES]) {
             e2 = exp(-dt0 / T2);
@@ -125,12 +187,15 @@ __global__ void __launch_bounds__(THREADS, 9)
         int i = 0;
         for (; i + U <= cnt; i += U) {
             Rotation r[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) r[u] = rotation(nodes[i + u]);
+            rotations(nodes + i, r, std::integral_constant<int, U>());
 #pragma unroll
             for (int u = 0; u < U; ++u) step(r[u], nodes[i + u]);
         }
-        for (; i < cnt; ++i) step(rotation(nodes[i]), nodes[i]);
+        for (; i < cnt; ++i) {
+            Rotation r[1];
+            rotations(nodes + i, r, std::integral_constant<int, 1>());
+            step(r[0], nodes[i]);
+        }
     }
     if (q.boundary[a.n_hi]) turn(q.psi[a.n_hi]);
     if (active) {

@@ -8,7 +8,7 @@ import pytest
 import homs
 from conftest import nrmse
 from homs import workloads as W
-from homs.model import BlochHighOrder
+from homs.model import GAMMA, BlochHighOrder
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,15 @@ def test_varying_steps_blocks_and_large_angles(oracle, gpu_context, precision):
     parts, _ = homs.get_sim_ranges(seq, 7, 7)
     for method in (BlochHighOrder("1111", True, True), BlochHighOrder("0000", False, True)):
         _check(oracle, obj, seq, st, parts, method, precision)
+
+
+@pytest.mark.parametrize("turns", [0.0, 0.004, 0.028, 0.03, 0.1, 0.125, 0.13, 0.4, 3.0])
+def test_half_angle_ranges(oracle, gpu_context, turns):
+    """Half-angles on both sides of the lines between the two series and the general
+    form (0.0281 and 0.1258 turns), within a warp and within the nodes of a step."""
+    obj, seq, st = _case(70, 70)
+    scale = turns / (GAMMA * float(seq.dt[0]) / 2)
+    ramp = np.linspace(0.9, 1.1, 71)
+    seq.b1[:] = scale * ramp * np.exp(1j * np.arange(71))
+    seq.b1[33] = 0
+    _check(oracle, obj, seq, st, [(0, 70)], BlochHighOrder("1111"), "f64")
