@@ -38,7 +38,7 @@ __host__ __device__ constexpr int sample_tiles(int coil_tiles) { return coil_til
 
 // Cut of a launch of `nsamples` samples x `chunks` 32-spin chunks into sample
 // tiles of 8 * sample_tiles * wj rows and `parts` ranges of chunks, for CTAs
-// of 8 warps, two per SM.
+// of 8 warps (`places` at a time; two per SM by default).
 struct CoilCut {
     int wj = 8;           // warps along the samples; the 8 / wj groups of warps split the spins
     int parts = 1;
@@ -46,7 +46,7 @@ struct CoilCut {
     size_t partial_bytes = 0; // FP64 partial sums of a launch
     int tile(int32_t nc) const { return 8 * sample_tiles(coil_tiles(nc)) * wj; }
 };
-inline CoilCut coil_cut(int64_t chunks, int32_t nc, int64_t nsamples, size_t budget) {
+inline CoilCut coil_cut(int64_t chunks, int32_t nc, int64_t nsamples, size_t budget, int64_t places = 148 * 2) {
     CoilCut p;
     if (nsamples <= 0) return p;
     // 8 warps along the samples, or fewer where that tile would be mostly padding
@@ -59,14 +59,14 @@ inline CoilCut coil_cut(int64_t chunks, int32_t nc, int64_t nsamples, size_t bud
     // rounds whose partial sums fit the budget in one part
     const size_t tile_bytes = 16 * (size_t)ksplit * tile * nc;
     p.round_tiles = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)(budget / tile_bytes)));
-    // parts: least waves of 2 CTAs per SM x (chunks of a CTA + 2 for its start and its sums)
-    const int64_t slots = 148 * 2, per_wave = p.round_tiles * groups;
+    // parts: least waves of `places` CTAs x (chunks of a CTA + 2 for its start and its sums)
+    const int64_t per_wave = p.round_tiles * groups;
     const int64_t most = std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>(chunks, 1024), (int64_t)(budget / (tile_bytes * p.round_tiles))));
     int64_t best = INT64_MAX;
     for (int64_t waves = 1; waves <= 8; ++waves) {
-        const int64_t n = std::max<int64_t>(1, std::min<int64_t>(most, waves * slots / per_wave));
-        const int64_t cost = ((per_wave * n + slots - 1) / slots) * ((chunks + n - 1) / n + 2);
+        const int64_t n = std::max<int64_t>(1, std::min<int64_t>(most, waves * places / per_wave));
+        const int64_t cost = ((per_wave * n + places - 1) / places) * ((chunks + n - 1) / n + 2);
         if (cost < best) {
             best = cost;
             p.parts = (int)n;

@@ -19,18 +19,22 @@
 // for 40,000 spins x 2,516 nodes).  Up to SMALL_NS spins a spin takes 8 lanes,
 // each evaluating two of 16 nodes, and only the sum itself runs through the
 // lanes in order (4,096 spins x 2,058 nodes: 147 -> 67 us).
-// coil_kernel is bound by instruction issue for few coils (68 per spin and
-// sample, 96 with sincosf, expf and a division per element: 457 -> 337 us for
-// 40,000 spins x 2,516 samples x 8 coils) and by the FP64 pipe for many: the coil
-// sums are FP64 matrix instructions (homs_precess64.cu has the fragment layouts
-// and the three-product complex form), which leaves the FP32 pipe to the
-// magnetisation and sums the FP32 products without rounding them.  Phases cross
+// coil_kernel waits on latency for few coils (no pipe above 45%, issue 58% with
+// two CTAs per SM; per spin and sample 68 instructions with scalar sine, cosine
+// and decay, 96 with sincosf, expf and a division per element: 457 -> 337 us for
+// 40,000 spins x 2,516 samples x 8 coils), so up to 8 coils take packed FP32
+// operations on two spins at a time and 74 registers for three CTAs per SM (a
+// one-shot run of 4 x 10,000 such samples 10.45 -> 9.93 ms; packed alone 10.35).
+// For many coils it is bound by the FP64 pipe: the coil sums are FP64 matrix
+// instructions (homs_precess64.cu has the fragment layouts and the three-product
+// complex form), which leaves the FP32 pipe to the magnetisation and sums the
+// FP32 products without rounding them.  Phases cross
 // through memory, 4 bytes per spin and sample each way.
 //
 // Measured (B200, against the single kernel): one-shot calls, 4,096 spins x
-// 2,048 samples x 1 coil 1,754 -> 414 us, 40,000 spins x 4 x 10,000 samples x 8
-// coils 33.3 -> 11.8 ms; a prepared run of 48 repetitions of 64 pulse nodes and
-// 128 samples, 29,929 spins x 8 coils, 6.9 -> 4.2 ms.
+// 2,048 samples x 1 coil 1,754 -> 285 us, 40,000 spins x 4 x 10,000 samples x 8
+// coils 33.3 -> 9.9 ms (0.1 and 1.4 ms of it by leaner calls); a prepared run of 48
+// repetitions of 64 pulse nodes and 128 samples, 29,929 spins x 8 coils, 6.9 -> 3.9 ms.
 #include <algorithm>
 
 #include "homs_fp32math.cuh"
@@ -403,7 +407,7 @@ struct CoilArgs {
 };
 
 template <int NT, int WJ>
-__global__ void __launch_bounds__(THREADS, 2) coil_kernel(const CoilArgs a) {
+__global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const CoilArgs a) {
     constexpr int KSPLIT = 8 / WJ, MT = sample_tiles(NT), TILE = 8 * MT * WJ;
     constexpr int CS = csm_row(NT), STAGE = stage_bytes(NT, TILE);
     constexpr int O_CSM = TILE * PROW, O_XY = O_CSM + CHUNK * CS, O_DECAY = NSTAGE * STAGE;
@@ -527,20 +531,24 @@ __global__ void __launch_bounds__(THREADS, 2) coil_kernel(const CoilArgs a) {
                 __all_sync(0xffffffffu,
                            dmax * fmaxf(fabsf(r2.x), fabsf(r2.y)) <= SMALL_DECAY && pmax < CIS32_RANGE)) {
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float x = dtp[mt] * (e ? r2.y : r2.x), E0 = e ? E.y : E.x;
-                        float p = __fmaf_rn(x, 1.0f / 120.0f, 1.0f / 24.0f);
-                        p = __fmaf_rn(p, x, 1.0f / 6.0f);
-                        p = __fmaf_rn(p, x, 0.5f);
-                        p = __fmaf_rn(p, x, 1.0f);
-                        const float ec = __fmaf_rn(E0, x * p, E0);
-                        float sn, cs;
-                        cis32(e ? ph[mt].y : ph[mt].x, cs, sn);
-                        v[mt][e] = cmul(e ? cplx<float>{x4.z, x4.w} : cplx<float>{x4.x, x4.y},
-                                        cplx<float>{ec * cs, ec * sn});
-                    }
+                for (int mt = 0; mt < MT; ++mt) {
+                    // both spins at a time
+                    const f32x2 x = pmul(pack2(dtp[mt], dtp[mt]), pack2(r2.x, r2.y)), E0 = pack2(E.x, E.y);
+                    f32x2 p = pfma(x, pair(1.0f / 120.0f), pair(1.0f / 24.0f));
+                    p = pfma(p, x, pair(1.0f / 6.0f));
+                    p = pfma(p, x, pair(0.5f));
+                    p = pfma(p, x, pair(1.0f));
+                    const f32x2 ec = pfma(E0, pmul(x, p), E0);
+                    f32x2 cs, sn;
+                    cis32_pair(pack2(ph[mt].x, ph[mt].y), cs, sn);
+                    cs = pmul(ec, cs);
+                    sn = pmul(ec, sn);
+                    const f32x2 xr = pack2(x4.x, x4.z), xi = pack2(x4.y, x4.w);
+                    const float2 re = unpack2(pfma(xr, cs, pmul(pneg(xi), sn)));
+                    const float2 im = unpack2(pfma(xr, sn, pmul(xi, cs)));
+                    v[mt][0] = cplx<float>{re.x, im.x};
+                    v[mt][1] = cplx<float>{re.y, im.y};
+                }
             } else {
                 const float2 t2 = *reinterpret_cast<const float2 *>(dec + 2 * CHUNK + sl);
 #pragma unroll
@@ -656,7 +664,11 @@ size_t precess32_work_bytes(int64_t ns, int64_t nsamples, int32_t nblocks) {
            align256(sizeof(RowInfo) * (size_t)nsamples);
 }
 CoilCut precess32_cut(int64_t ns, int32_t nc, int64_t nsamples) {
-    return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, PARTIAL_BUDGET);
+    // Three CTAs per SM for up to 8 coils, unless these only add partial sums to read:
+    // with one tile a part is a few chunks already (48 repetitions of 128 samples:
+    // 3.87 ms with two per SM, 3.98 with three).
+    const int64_t places = coil_tiles(nc) == 1 && nsamples > 6 * 128 ? 148 * 3 : 148 * 2;
+    return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, PARTIAL_BUDGET, places);
 }
 
 cudaError_t precess32_run(const Precess32Args &a, const CoilCut &cut, cudaEvent_t ev_start, cudaEvent_t ev_stop,
