@@ -72,12 +72,25 @@ __device__ __forceinline__ double pow2(double y) {
     return __hiloint2double(__double2hiint(p) + (k << 20), __double2loint(p));
 }
 
-// 2^y for |y| <= 1/16: the exponential series to degree 8 (remainder 1.4e-18).
+// 2^y for |y| <= 1/16: the exponential series to degree 8 (remainder 1.5e-18).
+constexpr double POW2_SMALL = 0.0625;
 __device__ __forceinline__ double pow2_small(double y) {
     double p = 1.3215486790144305e-06;
     p = fma(p, y, 1.5252733804059838e-05);
     p = fma(p, y, 0.00015403530393381606);
     p = fma(p, y, 0.0013333558146428441);
+    p = fma(p, y, 0.009618129107628477);
+    p = fma(p, y, 0.055504108664821576);
+    p = fma(p, y, 0.2402265069591007);
+    p = fma(p, y, 0.6931471805599453);
+    p = fma(p, y, 1.0);
+    return p;
+}
+
+// 2^y for |y| <= 1/128: to degree 5 (remainder 3.5e-17).
+constexpr double POW2_TINY = 0.0078125;
+__device__ __forceinline__ double pow2_tiny(double y) {
+    double p = 0.0013333558146428441;
     p = fma(p, y, 0.009618129107628477);
     p = fma(p, y, 0.055504108664821576);
     p = fma(p, y, 0.2402265069591007);

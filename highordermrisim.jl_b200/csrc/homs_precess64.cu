@@ -12,9 +12,11 @@
 // blocks of a run only restart the same exponentials, so a run is one segment.
 //
 // What bounds it: the FP64 pipe (64 multiply-adds per SM and clock, the same
-// for DFMA and for the FP64 matrix instruction; the pipe is about 72% busy).
-// Per spin and sample 16 multiply-adds of phase, 34 FP64 operations of sine,
-// cosine, decay and the complex product, 3 per coil of contraction.
+// for DFMA and for the FP64 matrix instruction; about 72% busy) and the latency
+// of its chains: leaving out the matrix step of an unused third order gains
+// nothing (9.20 against 9.22 ms at 8 coils), a shorter decay series does.
+// Per spin and sample 16 multiply-adds of phase, 31 to 34 FP64 operations of
+// sine, cosine, decay and the complex product, 3 per coil of contraction.
 //
 // Organisation: CTA = 8 warps, a tile of samples x a range of 32-spin chunks
 // (cp.async, NSTAGE stages).  A warp owns 16 samples (8 for more than 16
@@ -26,16 +28,18 @@
 // fragment of the coil product (samples x spins) (spins x coils), so M never
 // leaves its registers.  The complex product takes three real ones: k1 = (Re M + Im M) Re c, k2 = Re M (Im c - Re c),
 // k3 = Im M (Re c + Im c); Re = k1 - k3, Im = k1 + k2 (10.87 -> 10.31 ms at 8
-// coils, 6.15 -> 5.86 ms at 32).  wj < 8 (segments of few samples): the other
+// coils, 6.15 -> 5.86 ms at 32); above 16 coils, where a warp's 8 samples share a
+// coefficient less, the form with one sum of c and two of M (5.63 -> 5.53 ms).  wj < 8 (segments of few samples): the other
 // warps take other spin groups of the chunk and write partial sums of their own.
-// The decay is 2^(t_ref r2), once per spin, chunk and tile, times a degree-8
-// series of 2^((t - t_ref) r2) where that argument stays within 1/16 for the
-// whole warp (10.28 -> 9.35 ms, 5.84 -> 5.76 ms); two spin groups per iteration
-// let the two chains overlap (9.09 and 5.63 ms).
+// The decay is 2^(t_ref r2), once per spin, chunk and tile, times a series of
+// 2^((t - t_ref) r2) of degree 8 where that argument stays within 1/16 for the
+// whole warp (10.28 -> 9.35 ms, 5.84 -> 5.76 ms) and of degree 5 within 1/128;
+// four spin groups per iteration let their chains overlap (1, 2, 4 groups: 9.09,
+// 8.90, 8.82 ms at 8 coils, 5.57, 5.49, 5.48 ms at 32).
 //
 // Measured (B200, prepared runs, against the sequential per-spin kernel that it
 // replaces): 40,000 spins x 4 segments of 10,000 samples x 8 coils 44.6 ->
-// 9.1 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.6 ms.  Three
+// 8.8 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.5 ms.  Three
 // CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
 #include <algorithm>
 
@@ -118,6 +122,9 @@ struct KernelArgs {
 template <int NT, int WJ>
 __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
     constexpr int CS = csm_row(NT), STAGE = stage_bytes(NT), KSPLIT = 8 / WJ, MT = sample_tiles(NT);
+    // Three-product form: two sums of M and one of c, or one and two; NT of the
+    // latter per element and MT of the former per 8 coils.
+    constexpr bool SUMS_OF_M = NT > MT;
     extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, r = lane >> 2;
     const int wj = warp % WJ, kw = warp / WJ;
@@ -214,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
         const double *dec = decay + (ch & 1) * CHUNK;
         const uint8_t *st = smem + stage * STAGE;
         if (++stage == NSTAGE) stage = 0;
-#pragma unroll 2
+#pragma unroll 4
         for (int g = kw; g < CHUNK / 8; g += KSPLIT) {
             const double2 *brow = reinterpret_cast<const double2 *>(st + (g * 8 + r) * BROW + q * 32);
             const double2 b01 = brow[0], b23 = brow[1];
@@ -230,21 +237,27 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt) dmma(th[mt], kap[mt][i], b[i]);
-            double mr[MT][2], mi[MT][2], ms[MT][2];
-            // m0 and the decay of each element: m0 E and the series of 2^(dt r2), of
-            // degree 8 (error below 1e-17 for |dt r2| <= 1/16), where that holds for
-            // the whole warp; else m0 and 2^(t r2).
-            const bool near = __all_sync(0xffffffffu, dmax * fmax(fabs(rr.x), fabs(rr.y)) <= 0.0625);
+            double mr[MT][2], mi[MT][2], ms[MT][2], md[MT][2];
+            // m0 and the decay of each element: m0 E and a series of 2^(dt r2), of degree
+            // 5 or 8 by the range of dt r2 in the warp; else m0 and 2^(t r2).
+            const double most = dmax * fmax(fabs(rr.x), fabs(rr.y));
             double2 m[2] = {m0[0], m0[1]};
             double ex[MT][2];
-            if (near) {
+            if (__all_sync(0xffffffffu, most <= POW2_SMALL)) {
                 const double2 E = *reinterpret_cast<const double2 *>(dec + g * 8 + 2 * q);
                 m[0] = make_double2(m0[0].x * E.x, m0[0].y * E.x);
                 m[1] = make_double2(m0[1].x * E.y, m0[1].y * E.y);
+                if (__all_sync(0xffffffffu, most <= POW2_TINY)) {
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
+                    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) ex[mt][e] = pow2_small((tj[mt] - t_ref) * (e ? rr.y : rr.x));
+                        for (int e = 0; e < 2; ++e) ex[mt][e] = pow2_tiny((tj[mt] - t_ref) * (e ? rr.y : rr.x));
+                } else {
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) ex[mt][e] = pow2_small((tj[mt] - t_ref) * (e ? rr.y : rr.x));
+                }
             } else {
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt)
@@ -261,6 +274,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
                     mr[mt][e] = m[e].x * ec - m[e].y * es;
                     mi[mt][e] = m[e].x * es + m[e].y * ec;
                     ms[mt][e] = mr[mt][e] + mi[mt][e];
+                    if (SUMS_OF_M) md[mt][e] = mi[mt][e] - mr[mt][e];
                 }
 #pragma unroll
             for (int e = 0; e < 2; ++e)
@@ -268,12 +282,18 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
                 for (int nt = 0; nt < NT; ++nt) {
                     const double2 w = *reinterpret_cast<const double2 *>(st + CHUNK * (BROW + 24) +
                                                                          (g * 8 + 2 * q + e) * CS + (nt * 8 + r) * 16);
-                    const double wd = w.y - w.x, ws = w.x + w.y;
+                    const double ws = w.x + w.y, wd = SUMS_OF_M ? 0.0 : w.y - w.x;
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt) {
-                        dmma(k1[mt][nt], ms[mt][e], w.x);
-                        dmma(k2[mt][nt], mr[mt][e], wd);
-                        dmma(k3[mt][nt], mi[mt][e], ws);
+                        if (SUMS_OF_M) {
+                            dmma(k1[mt][nt], mr[mt][e], ws);
+                            dmma(k2[mt][nt], md[mt][e], w.x);
+                            dmma(k3[mt][nt], ms[mt][e], w.y);
+                        } else {
+                            dmma(k1[mt][nt], ms[mt][e], w.x);
+                            dmma(k2[mt][nt], mr[mt][e], wd);
+                            dmma(k3[mt][nt], mi[mt][e], ws);
+                        }
                     }
                 }
         }

@@ -64,11 +64,13 @@ def test_unused_terms_and_special_values(oracle, gpu_context):
     assert np.all(sig == 0)
 
 
-@pytest.mark.parametrize("low,high", [(0.05, 0.5), (0.5, 2.0), (2.0, 50.0), (0.01, 1e4)])
-def test_decay_series(oracle, gpu_context, low, high):
-    """T2 about and on both sides of the line between the short decay series and
-    2^(t r2) (a tile's half span over T2 ln 2 equal to 1/16), also within one warp."""
-    obj, seq, st = W.high_order_workload(nspins=90, nsteps=300, ncoils=6)
+@pytest.mark.parametrize("ncoils", [6, 20])
+@pytest.mark.parametrize("low,high", [(0.05, 0.5), (0.5, 2.0), (2.0, 6.0), (5.0, 12.0), (12.0, 50.0), (0.01, 1e4)])
+def test_decay_series(oracle, gpu_context, low, high, ncoils):
+    """T2 about and on both sides of the lines between the decay series and 2^(t r2) (a
+    tile's half span over T2 ln 2 equal to 1/16, and an eighth of that), also within
+    one warp; both forms of the complex product."""
+    obj, seq, st = W.high_order_workload(nspins=90, nsteps=300, ncoils=ncoils)
     seq.adc[:] = np.arange(301) % 2 == 0
     line = 16.0 * float(seq.t[128] - seq.t[0]) / math.log(2.0)
     obj.T2[:] = np.random.default_rng(5).permutation(np.geomspace(low, high, 90)) * line
