@@ -35,59 +35,65 @@ using namespace homs;
 namespace {
 
 // Device buffer that grows on demand.  It owns its memory, or is a
-// read-only view of another buffer (a device-resident phantom's arrays):
-// ensure() never writes through a view, it replaces it with owned memory.
+// read-only view of another buffer (a device-resident phantom's arrays, a block
+// of packed inputs): ensure() never writes through a view, it replaces it with
+// owned memory.
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
-    bool owned = true;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), owned(o.owned) { o.p = nullptr; o.bytes = 0; o.owned = true; }
+    DevBuf(DevBuf &&o) noexcept { swap(o); }
     DevBuf &operator=(DevBuf &&o) noexcept {
         if (this != &o) {
             release();
-            p = o.p;
-            bytes = o.bytes;
-            owned = o.owned;
-            o.p = nullptr;
-            o.bytes = 0;
-            o.owned = true;
+            swap(o);
         }
         return *this;
     }
     ~DevBuf() { release(); }
     void release() {
-        if (p && owned) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-        owned = true;
+        if (own_) cudaFree(own_);
+        p = own_ = nullptr;
+        bytes = own_bytes_ = 0;
     }
-    void view(const DevBuf &src) {
-        release();
-        p = src.p;
-        bytes = src.bytes;
-        owned = false;
-    }
+    void view(const DevBuf &src) { view(src.p, src.bytes); }
     void view(void *at, size_t n) {
         release();
+        alias(at, n);
+    }
+    // A view that keeps the buffer's own allocation for a later ensure().
+    void alias(void *at, size_t n) {
         p = at;
         bytes = n;
-        owned = false;
     }
-    size_t owned_bytes() const { return owned ? bytes : 0; }
+    size_t owned_bytes() const { return own_bytes_; }
     cudaError_t ensure(size_t n) {
-        if (n <= bytes && p && owned) return cudaSuccess;
+        if (own_ && n <= own_bytes_) {
+            alias(own_, own_bytes_);
+            return cudaSuccess;
+        }
         release();
         if (n == 0) n = 16;
-        cudaError_t e = cudaMalloc(&p, n);
-        if (e == cudaSuccess) bytes = n;
-        else p = nullptr;
+        cudaError_t e = cudaMalloc(&own_, n);
+        if (e == cudaSuccess) own_bytes_ = n;
+        else own_ = nullptr;
+        alias(own_, own_bytes_);
         return e;
     }
     template <typename U>
     U *as() const { return reinterpret_cast<U *>(p); }
+
+private:
+    void swap(DevBuf &o) {
+        std::swap(p, o.p);
+        std::swap(bytes, o.bytes);
+        std::swap(own_, o.own_);
+        std::swap(own_bytes_, o.own_bytes_);
+    }
+    void *own_ = nullptr;
+    size_t own_bytes_ = 0;
 };
 
 struct Failure {
@@ -136,7 +142,11 @@ inline int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64
 // Host copies between a caller's pageable arrays and a context's page-locked
 // chunks, shared by the calling thread and up to three helper threads (started
 // on the first large copy, joined with the context).  One thread copies about
-// 10 GB/s here and, into fresh pages, waits for the kernel to clear them.
+// 10 GB/s here and, into fresh pages, waits for the kernel to clear them.  A
+// copy that finds another context's under way takes no helpers, and a server's
+// contexts never do: their threads share the cores already (four workers with
+// three helpers each on 16 cores served a stream at 0.3 of its rate, waiting for
+// one another's helpers to be scheduled).
 class CopyPool {
 public:
     struct Piece {
@@ -152,11 +162,13 @@ public:
         cv_.notify_all();
         for (auto &t : threads_) t.join();
     }
+    void no_helpers() { alone_ = true; }
     // Returns when every piece is copied.
     void run(const std::vector<Piece> &pieces) {
         size_t total = 0;
         for (const Piece &p : pieces) total += p.bytes;
-        if (total < PARALLEL_MIN || !start()) {
+        Copying copying;
+        if (total < PARALLEL_MIN || alone_ || copying.others || !start()) {
             for (const Piece &p : pieces) std::memcpy(p.dst, p.src, p.bytes);
             return;
         }
@@ -169,18 +181,27 @@ public:
             std::lock_guard<std::mutex> l(mu_);
             work_ = &work;
             next_.store(0);
-            busy_ = threads_.size();
             ++round_;
         }
         cv_.notify_all();
         drain(work);
+        // A helper that has not woken by now finds no work; the others finish their slice.
         std::unique_lock<std::mutex> l(mu_);
-        done_.wait(l, [&] { return busy_ == 0; });
         work_ = nullptr;
+        done_.wait(l, [&] { return busy_ == 0; });
     }
 
 private:
     static constexpr size_t PARALLEL_MIN = size_t(2) << 20, SLICE = size_t(1) << 20;
+    // Counts the process's copies under way.
+    struct Copying {
+        static std::atomic<int> &count() {
+            static std::atomic<int> n{0};
+            return n;
+        }
+        const bool others = count().fetch_add(1) > 0;
+        ~Copying() { count().fetch_sub(1); }
+    };
     bool start() {
         if (!threads_.empty()) return true;
         const unsigned n = std::min(3u, std::thread::hardware_concurrency() / 4);
@@ -203,6 +224,7 @@ private:
                 if (stop_) return;
                 seen = round_;
                 work = work_;
+                ++busy_;
             }
             drain(*work);
             std::lock_guard<std::mutex> l(mu_);
@@ -214,9 +236,9 @@ private:
     std::condition_variable cv_, done_;
     const std::vector<Piece> *work_ = nullptr;
     std::atomic<size_t> next_{0};
-    size_t busy_ = 0;
+    size_t busy_ = 0;  // helpers in the current copy
     uint64_t round_ = 0;
-    bool stop_ = false;
+    bool stop_ = false, alone_ = false;
 };
 
 }  // namespace
@@ -396,7 +418,9 @@ void upload(homs_context *ctx, DevBuf &dst, const void *src, homs_dtype src_dt, 
 
 // Several small host arrays of one upload: gathered in a page-locked chunk,
 // copied to one device block and, when their type differs from T, widened or
-// narrowed there by one kernel; each destination becomes a view of the block.
+// narrowed there by one kernel; each destination becomes a view of the block and
+// keeps what it had allocated (inputs that alternate about a chunk's size would
+// otherwise free and allocate every array at every call).
 // (Copied one by one, each array costs a driver call and, from pageable
 // memory, its own staging.)  `reals` hold n values of `src_dt`, `raw` n bytes.
 // False, and nothing done, when an array is not ordinary pageable memory, they
@@ -427,13 +451,13 @@ bool upload_packed(homs_context *ctx, DevBuf &block, homs_dtype src_dt, const st
     size_t at = 0;
     for (const UploadItem &u : reals) {
         pieces.push_back({host + at * es, u.src, u.n * es});
-        u.dst->view(dev + at * sizeof(T), u.n * sizeof(T));
+        u.dst->alias(dev + at * sizeof(T), u.n * sizeof(T));
         at += (u.n + ALIGN - 1) / ALIGN * ALIGN;
     }
     size_t off = 0;
     for (const UploadItem &u : raw) {
         pieces.push_back({host + count * es + off, u.src, u.n});
-        u.dst->view(dev + count * sizeof(T) + off, u.n);
+        u.dst->alias(dev + count * sizeof(T) + off, u.n);
         off += (u.n + 255) / 256 * 256;
     }
     ctx->copies.run(pieces);
@@ -2464,6 +2488,8 @@ homs_status server_run_finish(ServerRun *run, void *sig, homs_memory sig_memory,
         return fail(ctx, f);
     }
 }
+
+void context_copies_alone(homs_context *ctx) { ctx->copies.no_helpers(); }
 
 void server_run_free(ServerRun *run) {
     if (!run) return;

@@ -47,5 +47,7 @@ void server_run_done(ServerRun *run, cudaStream_t stream);
 cudaStream_t server_run_stream(const ServerRun *run);  // the run's context's stream
 homs_status server_run_finish(ServerRun *run, void *sig, homs_memory sig_memory, homs_state *state);
 void server_run_free(ServerRun *run);
+// The context's host copies take no helper threads (a server's workers share the cores).
+void context_copies_alone(homs_context *ctx);
 
 }  // namespace homs

@@ -335,6 +335,7 @@ homs_status homs_server_create(const homs_server_options *opts, homs_server **ou
             for (homs_context *c : srv->contexts) homs_context_destroy(c);
             return s;
         }
+        homs::context_copies_alone(ctx);
         srv->contexts.push_back(ctx);
     }
     homs_server *raw = srv.get();
