@@ -791,7 +791,7 @@ def run_homs(args):
             "frac": (achieved_tflops / bf16_peak) if achieved_tflops else None, "traffic": traffic,
             "peak_source": f"{peak_kind} dense bf16 (MEASURED_PEAKS.json)" if peak_kind == "measured" else
             "fallback 1.59 PFLOP/s", "kernel": "split_precession_kernel" if args.mode == "split" else
-            "segment_kernel", "kernel_ms_per_launch": avg_launch_ms,
+            "plain precession kernels and RF pulses", "kernel_ms_per_launch": avg_launch_ms,
             "units_per_launch": seg_units, "flops_per_unit": FLOPS_PER_UNIT}
     if traffic is not None:
         roof["traffic_source"] = "quoted from profiles/split_precession_kernel_cfg2.md (one ncu capture)"
@@ -834,9 +834,8 @@ def run_homs(args):
                      coil_fp64_frac=FLOPS_PER_UNIT * pl["units_per_s"] / fp64_peak,
                      fp64_peak_source=f"{FP64_FMA_PER_SM_CLK:.0f} FMA per SM and clock x {N_SM} SMs x {mhz:.0f} MHz "
                                       "(sampled; FP64 is not among the measured peaks); counts only the coil "
-                                      "contraction's 8 flops per unit, not the field, phase and sincos/exp",
-                     note="the plain kernel (the reference's per-spin sequential trapezoid, FP64) on the same "
-                          "workload, device-timed plan runs")
+                                      "contraction's 8 flops per unit, not the phase, sine, cosine and decay",
+                     note="the plain FP64 path on the same workload, device-timed plan runs")
         d = float(torch.linalg.vector_norm(sig_plain).item())
         nr = float(torch.linalg.vector_norm(sig_dev - sig_plain).item()) / d
         if accuracy is None:

@@ -47,8 +47,10 @@ typedef enum homs_dtype { HOMS_F32 = 0, HOMS_F64 = 1 } homs_dtype;
 typedef enum homs_memory { HOMS_HOST = 0, HOMS_DEVICE = 1 } homs_memory;
 
 /* Arithmetic of a run.
- *   HOMS_PLAIN  -- the reference's per-spin sequential trapezoid and fused coil
- *                  sum in the phantom's dtype (CUDA cores only);
+ *   HOMS_PLAIN  -- the reference's trapezoid and coil sum in the phantom's dtype.
+ *                  FP64: phases from the prefix-integrated field table, FP64
+ *                  throughout; FP32: the phase summed node by node in the
+ *                  reference's order, coil sums in FP64;
  *   HOMS_SPLIT  -- exact integer arithmetic on the tcgen05 tensor cores: the
  *                  phase as a fixed-point turn fraction from int8 digit
  *                  products of the prefix-integrated field table and the
@@ -317,10 +319,10 @@ homs_status homs_plan_run(homs_plan *plan, void *sig, homs_memory sig_memory, ho
 homs_status homs_plan_device_bytes(const homs_plan *plan, size_t *bytes);
 
 /* Device timing of the plan's last run: summed CUDA-event time of the
- * dominant fused kernel (the split tcgen05 kernel in HOMS_SPLIT, the segment
- * kernel in HOMS_PLAIN), its launch count, and all kernels launched.  Plays
- * the role of the reference's per-run `sim_time_sec` (src/simulation/Simulate.jl:210)
- * at kernel granularity. */
+ * dominant kernel (the split tcgen05 kernel in HOMS_SPLIT; in HOMS_PLAIN the
+ * precession kernels of a segment and the RF pulses), its launch count, and all
+ * kernels launched.  Plays the role of the reference's per-run `sim_time_sec`
+ * (src/simulation/Simulate.jl:210) at kernel granularity. */
 typedef struct homs_timing {
     double fused_kernel_ms;
     int64_t fused_launches;
