@@ -15,7 +15,7 @@
 // for DFMA and for the FP64 matrix instruction; about 72% busy) and the latency
 // of its chains: leaving out the matrix step of an unused third order gains
 // nothing (9.20 against 9.22 ms at 8 coils), a shorter decay series does.
-// Per spin and sample 16 multiply-adds of phase, 31 to 34 FP64 operations of
+// Per spin and sample 16 multiply-adds of phase, 27 to 30 FP64 operations of
 // sine, cosine, decay and the complex product, 3 per coil of contraction.
 //
 // Organisation: CTA = 8 warps, a tile of samples x a range of 32-spin chunks
@@ -35,11 +35,14 @@
 // 2^((t - t_ref) r2) of degree 8 where that argument stays within 1/16 for the
 // whole warp (10.28 -> 9.35 ms, 5.84 -> 5.76 ms) and of degree 5 within 1/128;
 // four spin groups per iteration let their chains overlap (1, 2, 4 groups: 9.09,
-// 8.90, 8.82 ms at 8 coils, 5.57, 5.49, 5.48 ms at 32).
+// 8.90, 8.82 ms at 8 coils, 5.57, 5.49, 5.48 ms at 32).  Sine and cosine take the
+// nearest of 256 points of the circle in shared memory and three terms of either
+// series, a shorter chain than two polynomials over a quarter turn (8.83 -> 8.20
+// ms, 5.48 -> 5.30 ms).
 //
 // Measured (B200, prepared runs, against the sequential per-spin kernel that it
 // replaces): 40,000 spins x 4 segments of 10,000 samples x 8 coils 44.6 ->
-// 8.8 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.5 ms.  Three
+// 8.2 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.3 ms.  Three
 // CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
 #include <algorithm>
 
@@ -61,7 +64,7 @@ constexpr double TWO_PI = 2.0 * 3.141592653589793;
 
 __host__ __device__ constexpr int csm_row(int nt) { return nt * 128 + 16; }  // bytes of a staged sensitivity row
 __host__ __device__ constexpr int stage_bytes(int nt) { return CHUNK * (BROW + 16 + 8 + csm_row(nt)); }
-__host__ __device__ constexpr int smem_bytes(int nt) { return NSTAGE * stage_bytes(nt) + 2 * CHUNK * 8; }  // + decays
+__host__ __device__ constexpr int smem_bytes(int nt) { return NSTAGE * stage_bytes(nt) + 2 * CHUNK * 8 + CIS_POINTS * 16; }  // + decays, circle
 
 __host__ __device__ inline int64_t pad_spins(int64_t ns) { return (ns + CHUNK - 1) / CHUNK * CHUNK; }
 
@@ -192,6 +195,8 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
     // Decay of the tile: E = 2^(t_ref r2) once per spin and chunk, by one warp a
     // chunk ahead, and a short series for the rest.
     double *decay = reinterpret_cast<double *>(smem + NSTAGE * STAGE);
+    double2 *circle = reinterpret_cast<double2 *>(decay + 2 * CHUNK);
+    if (tid < CIS_POINTS) cis_turns(tid * (1.0 / CIS_POINTS), circle[tid].x, circle[tid].y);
     auto load_r2 = [&](int64_t ch) { return a.r2[ch * CHUNK + lane]; };
     const uint32_t on = (a.slots >> (4 * q)) & 15u;
     double k1[MT][NT][2], k2[MT][NT][2], k3[MT][NT][2];
@@ -269,7 +274,7 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     double sn, cs;
-                    cis_turns(th[mt][e], cs, sn);
+                    cis_table(circle, th[mt][e], cs, sn);
                     const double ec = ex[mt][e] * cs, es = ex[mt][e] * sn;
                     mr[mt][e] = m[e].x * ec - m[e].y * es;
                     mi[mt][e] = m[e].x * es + m[e].y * ec;

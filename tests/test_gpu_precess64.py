@@ -78,6 +78,16 @@ def test_decay_series(oracle, gpu_context, low, high, ncoils):
     assert all(nrmse(g, r) <= BAR for g, r in zip(got, ref))
 
 
+@pytest.mark.parametrize("sign", [1, -1])
+def test_every_point_of_the_circle(oracle, gpu_context, sign):
+    """Phases over all of the circle and up to 4e4 rad either way.  Bound: 300 roundings
+    of the oracle's running sum at 4e4 rad, 300 * 4e4 * 2^-53 = 1.4e-9."""
+    obj, seq, st = W.high_order_workload(nspins=200, nsteps=300, ncoils=3)
+    obj.dw[:] = sign * np.linspace(0.0, 2e7, 200)
+    got, ref = _both(oracle, obj, seq, [(0, 300)], [False], BlochHighOrder("1111"), st)
+    assert all(nrmse(g, r) <= 1.4e-9 for g, r in zip(got, ref))
+
+
 def test_block_call_with_state_off_16_bytes(oracle, gpu_context):
     """homs_precession_block accepts a state that is aligned to 8 bytes only."""
     import torch
