@@ -408,9 +408,9 @@ def serving_benchmark(n_pool=16, passes=20, load=0.95, slots=4, resident=False, 
 
 
 def plain_per_request(n_pool=16):
-    """The plain per-request kernel: every distinct request of the serving
-    pool once, one at a time, on the reference-order plain kernel in its own
-    precision (phantom uploaded per request)."""
+    """The plain arithmetic per request: every distinct request of the serving
+    pool once, one at a time, in its own precision (phantom uploaded per
+    request; a first pass, allocations included)."""
     import homs
     from homs import workloads as W
     pool = W.serving_pool(n_pool)
