@@ -35,8 +35,8 @@ constexpr int THREADS = 64;
 constexpr int NODES = 64;  // nodes per stage
 constexpr int UNROLL = 4;  // rotations formed together (2, 3, 4, 6: 15.78, 15.76, 15.65, 15.87 ms for the TR loop)
 
-// 1/sqrt(x) from the hardware's approximation (2^-20 or better) by one step of
-// third order; 0 for x below 1e-300 (no field), NaN for NaN.
+// 1/sqrt(x) from the hardware's approximation (2^-20 or better) by one Householder
+// step of third order; 0 for x below 1e-300 (no field), NaN for NaN.
 __device__ __forceinline__ double rsq(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -104,6 +104,15 @@ struct Rotation {
     double w, x, y, z;
 };
 
+// Relaxation factor over dt0 + d for |d| <= 1e-9 dt0, from e = exp(-dt0 / T) to
+// first order in d.  A factor of 0 (T = 0, or far below dt0) or infinity stays:
+// its correction is 0 times or minus infinity, and nothing is lost, since exp
+// leaves the range of FP64 at |dt0 / T| = 745, where the correction is below 1e-6.
+__device__ __forceinline__ double near_factor(double e, double d, double T) {
+    const double f = fma(e, -d / T, e);
+    return isnan(f) ? e : f;
+}
+
 __global__ void __launch_bounds__(THREADS, 9)
     excite_kernel(PhantomDev<double> p, SeqDev<double> q, StateDev<double> st, SegmentArgs<double> a) {
     __shared__ Node nodes[NODES];
@@ -156,8 +165,8 @@ __global__ void __launch_bounds__(THREADS, 9)
         const double nx = fma(r.w, tx, mx), ny = fma(r.w, ty, my), nz = fma(r.w, tz, mz);
         double f2 = e2, f1 = e1, g1 = c1;
         if (n.relax != SAME) {
-            f2 = n.relax == NEAR ? fma(e2, -n.dt / T2, e2) : exp(-n.dt / T2);
-            f1 = n.relax == NEAR ? fma(e1, -n.dt / T1, e1) : exp(-n.dt / T1);
+            f2 = n.relax == NEAR ? near_factor(e2, n.dt, T2) : exp(-n.dt / T2);
+            f1 = n.relax == NEAR ? near_factor(e1, n.dt, T1) : exp(-n.dt / T1);
             g1 = rho * (1.0 - f1);
         }
         mx = fma(r.y, tz, fma(-r.z, ty, nx)) * f2;

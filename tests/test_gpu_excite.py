@@ -64,3 +64,19 @@ def test_half_angle_ranges(oracle, gpu_context, turns):
     seq.b1[:] = scale * ramp * np.exp(1j * np.arange(71))
     seq.b1[33] = 0
     _check(oracle, obj, seq, st, [(0, 70)], BlochHighOrder("1111"), "f64")
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_zero_relaxation_times_and_nearly_equal_steps(oracle, gpu_context, precision):
+    """Spins with T1 or T2 of zero (voxels outside the object) or far below the step
+    relax at once, whatever the last bits of the steps: the factor is exp(-inf) = 0."""
+    obj, seq, st = _case(90, 70)
+    seq.dt[:] = seq.dt[0] * (1 + 1e-12 * np.random.default_rng(4).standard_normal(70))
+    obj.T1[3:6] = obj.T2[5:9] = obj.T1[70:] = obj.T2[70:] = 0.0
+    obj.T1[12] = obj.T2[13] = float(seq.dt[0]) / 800.0
+    _check(oracle, obj, seq, st, [(0, 70)], BlochHighOrder("1111"), precision)
+    parts, exc = [(0, 35), (35, 70)], [True, False]  # the samples that follow the pulse
+    seq.adc[40:70:3] = True
+    ref = oracle.simulate_c(obj, seq, parts, exc, BlochHighOrder("1111").flags, st.xy, st.z)
+    got = homs.run_blocks(obj, seq, parts, exc, BlochHighOrder("1111"), precision, "plain", st)
+    assert all(nrmse(g, r) <= BAR[precision] for g, r in zip(got, ref))
