@@ -21,6 +21,10 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+// The first n (0 .. 16) bytes, then zeros.
+__device__ __forceinline__ void cp16_part(uint32_t dst, const void *src, int n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
 __device__ __forceinline__ void cp8(uint32_t dst, const void *src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }

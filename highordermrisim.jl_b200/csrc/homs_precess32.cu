@@ -461,13 +461,16 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const Co
     auto issue = [&](int64_t ch, int stage) {
         const uint32_t st = sbase + (uint32_t)(stage * STAGE);
         const int64_t s0 = ch * CHUNK;
+        // Bytes of this thread's pieces that hold a spin's phase: the walk writes none for
+        // padding spins, whose phases are zero here (they vote on the path below).
+        const int held = (int)imax64(0, imin64(16, (a.ns - s0 - (tid & 7) * 4) * 4));
 #pragma unroll
         for (int i = 0; i < (TILE * 8 + THREADS - 1) / THREADS; ++i) {
             const int p = tid + i * THREADS, row = p >> 3, piece = p & 7;
             if (TILE * 8 < THREADS && p >= TILE * 8) break;
             const bool ok = row < rows_left;
-            cp16(st + row * PROW + piece * 16, a.w.phi + (a.sample0 + jt + (ok ? row : 0)) * a.ns_pad + s0 + piece * 4,
-                 ok);
+            cp16_part(st + row * PROW + piece * 16,
+                      a.w.phi + (a.sample0 + jt + (ok ? row : 0)) * a.ns_pad + s0 + piece * 4, ok ? held : 0);
         }
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
@@ -506,7 +509,6 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const Co
         float next_T2 = 1.0f;
         if (next_decay) next_T2 = load_T2(ch + 1);
         const float *dec = decay + (int)(ch & 1) * (3 * CHUNK);
-        const bool tail = ch * CHUNK + CHUNK > a.ns;
         const uint8_t *st = smem + stage * STAGE;
         if (++stage == NSTAGE) stage = 0;
 #pragma unroll 1
@@ -559,13 +561,6 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const Co
                         if (!one_block && s + e < a.ns) xy = a.w.xyb[(int64_t)blk[mt] * a.ns_pad + s + e];
                         v[mt][e] = magnetisation(xy, e ? ph[mt].y : ph[mt].x, tp[mt], e ? t2.y : t2.x);
                     }
-            }
-            if (tail) {  // padding spins hold no phase
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e)
-                        if (s + e >= a.ns) v[mt][e] = cplx<float>{0.0f, 0.0f};
             }
             double mr[MT][2], mi[MT][2], ms[MT][2];
 #pragma unroll

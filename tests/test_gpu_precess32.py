@@ -95,3 +95,22 @@ def test_phase_sum_order(gpu_context, nspins):
     phi = (f(-2 * np.pi * GAMMA) * (f(0.5) * acc)).astype(np.float64)
     want = (1 - 0.5j) * np.exp(-float(t) / obj.T2[:n].astype(np.float64)) * np.exp(1j * phi)
     assert np.max(np.abs(got - want) / np.abs(want)) <= 2e-6
+
+
+def test_signal_does_not_depend_on_earlier_calls(homs_lib):
+    """Five spins, the same call on one context after calls that leave small and large
+    values where its padding spins' phases lie (partial sums of 256 coils): the same bits."""
+    obj, seq, st = W.high_order_workload(nspins=5, nsteps=200, ncoils=8)
+    other, oseq, ost = W.high_order_workload(nspins=5, nsteps=16, ncoils=256)
+    method = BlochHighOrder("1111")
+    with homs.Context(0) as ctx:
+        def signal():
+            return homs.run_blocks(obj, seq, [(0, 200)], [False], method, "f32", "plain", st, ctx)[0]
+
+        signal()  # the workspace has its size
+        found = []
+        for scale in (0.0, 1.0, 1e5, 1e20):
+            other.csm[:] = scale * np.exp(1j * np.arange(256))
+            homs.run_blocks(other, oseq, [(0, 16)], [False], method, "f32", "plain", ost, ctx)
+            found.append(signal())
+    assert all(np.array_equal(f, found[0]) for f in found)
