@@ -8,6 +8,8 @@
 
 #include <algorithm>
 
+#include "homs_common.cuh"
+
 namespace homs {
 
 // d (8 x 8) += a (8 x 4) b (4 x 8): lane l holds a[l / 4][l % 4], b[l % 4][l / 4]
@@ -16,6 +18,23 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
+}
+// Re and Im of a complex sum from its three products k1, k2, k3, in k1 and k2;
+// `top` collects the largest high word: from NOT_FINITE on, an infinity or a NaN
+// is among them.  Infinite operands make inf - inf of the three products where the
+// four of the plain form keep the infinity; the kernels then take their sums anew.
+constexpr int NOT_FINITE = 0x7FF00000;
+__device__ __forceinline__ void from_three(double &k1, double &k2, double k3, int &top) {
+    k2 += k1;
+    k1 -= k3;
+    top = max(top, max(__double2hiint(k1) & 0x7FFFFFFF, __double2hiint(k2) & 0x7FFFFFFF));
+}
+// re += x w, im likewise, by four real products.
+__device__ __forceinline__ void dmma4(double (&re)[2], double (&im)[2], double xr, double xi, double wr, double wi) {
+    dmma(re, xr, wr);
+    dmma(re, -xi, wi);
+    dmma(im, xr, wi);
+    dmma(im, xi, wr);
 }
 // Asynchronous copies into shared memory; zeros where !valid (src stays a valid address).
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
@@ -39,6 +58,30 @@ constexpr int COIL_GROUP = 32;  // coils per launch slice
 // sums of 32 coils would not fit the registers beside those of 16 samples.
 inline int coil_tiles(int32_t nc) { return nc <= 8 ? 1 : nc <= 16 ? 2 : 4; }
 __host__ __device__ constexpr int sample_tiles(int coil_tiles) { return coil_tiles == 4 ? 1 : 2; }
+
+// A warp's coil sums into its block of the partial sums, in a kernel of 8 warps, WJ
+// of them along the samples (blockIdx: sample tile, spin part, coil slice).
+template <int NT, int WJ>
+__device__ __forceinline__ void store_sums(cplx<double> *partial, int64_t round_samples, int32_t nc,
+                                           const double (&re)[sample_tiles(NT)][NT][2],
+                                           const double (&im)[sample_tiles(NT)][NT][2]) {
+    constexpr int MT = sample_tiles(NT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+    const int c0 = (int)blockIdx.z * COIL_GROUP, ncg = min(COIL_GROUP, nc - c0);
+    cplx<double> *out = partial + (size_t)(blockIdx.y * (8 / WJ) + warp / WJ) * round_samples * nc + c0;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        const int64_t j = (int64_t)blockIdx.x * (8 * MT * WJ) + warp % WJ * (8 * MT) + mt * 8 + r;
+        if (j >= round_samples) continue;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = nt * 8 + 2 * q + e;
+                if (c < ncg) out[j * nc + c] = cplx<double>{re[mt][nt][e], im[mt][nt][e]};
+            }
+    }
+}
 
 // Cut of a launch of `nsamples` samples x `chunks` 32-spin chunks into sample
 // tiles of 8 * sample_tiles * wj rows and `parts` ranges of chunks, for CTAs

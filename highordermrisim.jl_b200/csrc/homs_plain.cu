@@ -481,14 +481,33 @@ __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
         }
     }
     cp_wait<0>();
-    if (sizeof(T) == 4)
+    if (sizeof(T) == 4) {
+        int top = 0;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                im[nt][e] += re[nt][e];
-                re[nt][e] -= k3[nt][e];
+            for (int e = 0; e < 2; ++e) from_three(re[nt][e], im[nt][e], k3[nt][e], top);
+        // Infinite operands: this warp's sums by four products, straight from memory.
+        if (__any_sync(0xffffffffu, top >= NOT_FINITE)) {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) re[nt][e] = im[nt][e] = 0.0;
+            const bool row = 8 * wj + r < jn;
+#pragma unroll 1
+            for (int64_t k = (CR_SK / 4) * ch0 + kw; k < (CR_SK / 4) * ch1; k += KS) {
+                const int64_t s = 4 * k + q;
+                const bool ok = s < ns;
+                const cplx<T> x = row && ok ? states[(j0 + 8 * wj + r) * ldstates + s] : cplx<T>{T(0), T(0)};
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int c = 8 * nt + r;
+                    const cplx<T> w = c < cn && ok ? csm[(c0 + c) * ldcsm + s] : cplx<T>{T(0), T(0)};
+                    dmma4(re[nt], im[nt], x.re, x.im, w.re, w.im);
+                }
             }
+        }
+    }
     if (KS > 1) {  // add the warps that share the samples, in warp order
         double *sums = reinterpret_cast<double *>(cr_smem);
         __syncthreads();

@@ -406,6 +406,43 @@ struct CoilArgs {
     cplx<double> *partial;
 };
 
+// A warp's sums by four real products, straight from memory (infinite states or
+// sensitivities, see from_three).
+template <int NT, int WJ>
+__device__ __forceinline__ void sums_of_four(const CoilArgs &a) {
+    constexpr int KSPLIT = 8 / WJ, MT = sample_tiles(NT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+    const int c0 = (int)blockIdx.z * COIL_GROUP, ncg = min(COIL_GROUP, a.nc - c0);
+    const int64_t ch0 = a.nchunks * blockIdx.y / a.parts, ch1 = a.nchunks * (blockIdx.y + 1) / a.parts;
+    const int64_t jw = (int64_t)blockIdx.x * (8 * MT * WJ) + warp % WJ * (8 * MT);
+    double re[MT][NT][2] = {}, im[MT][NT][2] = {};
+#pragma unroll 1
+    for (int64_t g = (CHUNK / 8) * ch0 + warp / WJ; g < (CHUNK / 8) * ch1; g += KSPLIT)
+#pragma unroll 1
+        for (int e = 0; e < 2; ++e) {
+            const int64_t s = g * 8 + 2 * q + e;
+            const bool ok = s < a.ns;
+            cplx<float> v[MT];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                v[mt] = cplx<float>{0.0f, 0.0f};
+                if (!ok) continue;
+                const int64_t j = a.sample0 + imin64(jw + mt * 8 + r, a.round_samples - 1);
+                const RowInfo row = a.w.rows[j];
+                v[mt] = magnetisation(a.w.xyb[(int64_t)row.blk * a.ns_pad + s], a.w.phi[j * a.ns_pad + s], row.tp, a.T2[s]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const int c = nt * 8 + r;
+                const cplx<float> w = ok && c < ncg ? a.csm_rows[s * a.nc + c0 + c] : cplx<float>{0.0f, 0.0f};
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) dmma4(re[mt][nt], im[mt][nt], v[mt].re, v[mt].im, w.re, w.im);
+            }
+        }
+    store_sums<NT, WJ>(a.partial, a.round_samples, a.nc, re, im);
+}
+
 template <int NT, int WJ>
 __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const CoilArgs a) {
     constexpr int KSPLIT = 8 / WJ, MT = sample_tiles(NT), TILE = 8 * MT * WJ;
@@ -589,21 +626,15 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const Co
         if (next_decay) fill_decay(ch + 1, next_T2);
     }
     cp_wait<0>();
-    cplx<double> *out = a.partial + (size_t)(blockIdx.y * KSPLIT + kw) * a.round_samples * a.nc + c0;
+    int top = 0;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        const int64_t j = jt + wj * (8 * MT) + mt * 8 + r;
-        if (j >= a.round_samples) continue;
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = nt * 8 + 2 * q + e;
-                if (c < ncg)
-                    out[j * a.nc + c] =
-                        cplx<double>{k1[mt][nt][e] - k3[mt][nt][e], k1[mt][nt][e] + k2[mt][nt][e]};
-            }
-    }
+            for (int e = 0; e < 2; ++e) from_three(k1[mt][nt][e], k2[mt][nt][e], k3[mt][nt][e], top);
+    store_sums<NT, WJ>(a.partial, a.round_samples, a.nc, k1, k2);
+    if (__any_sync(0xffffffffu, top >= NOT_FINITE)) sums_of_four<NT, WJ>(a);
 }
 
 template <int ORD>

@@ -121,6 +121,49 @@ struct KernelArgs {
     cplx<double> *partial;
 };
 
+// A warp's sums by four real products, straight from memory (infinite states or
+// sensitivities, see from_three).
+template <int NT, int WJ>
+__device__ __forceinline__ void sums_of_four(const KernelArgs &a, const double2 *circle) {
+    constexpr int KSPLIT = 8 / WJ, MT = sample_tiles(NT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
+    const int c0 = (int)blockIdx.z * COIL_GROUP, ncg = min(COIL_GROUP, a.nc - c0);
+    const int64_t ch0 = a.nchunks * blockIdx.y / a.parts, ch1 = a.nchunks * (blockIdx.y + 1) / a.parts;
+    const int64_t jw = (int64_t)blockIdx.x * (8 * MT * WJ) + warp % WJ * (8 * MT);
+    double re[MT][NT][2] = {}, im[MT][NT][2] = {};
+#pragma unroll 1
+    for (int64_t g = (CHUNK / 8) * ch0 + warp / WJ; g < (CHUNK / 8) * ch1; g += KSPLIT)
+#pragma unroll 1
+        for (int e = 0; e < 2; ++e) {
+            const int64_t s = g * 8 + 2 * q + e;
+            const bool ok = s < a.ns;
+            cplx<double> v[MT];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                v[mt] = cplx<double>{0.0, 0.0};
+                if (!ok) continue;
+                const int64_t j = imin64(jw + mt * 8 + r, a.round_samples - 1);
+                const double *row = a.prefix + (a.sample0 + j) * SPLIT_PREFIX_STRIDE;
+                double th = row[0], sn, cs;
+                for (int k = 0; k < TERMS; ++k)
+                    if ((a.slots >> k) & 1u) th = fma(row[1 + k], a.basis[s * TERMS + k], th);
+                cis_table(circle, th, cs, sn);
+                const double ex = pow2(row[SPLIT_PREFIX_T] * a.r2[s]), ec = ex * cs, es = ex * sn;
+                const cplx<double> m0 = a.xy[s];
+                v[mt] = cplx<double>{m0.re * ec - m0.im * es, m0.re * es + m0.im * ec};
+            }
+            __syncwarp();
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const int c = nt * 8 + r;
+                const cplx<double> w = ok && c < ncg ? a.csm_rows[s * a.nc + c0 + c] : cplx<double>{0.0, 0.0};
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) dmma4(re[mt][nt], im[mt][nt], v[mt].re, v[mt].im, w.re, w.im);
+            }
+        }
+    store_sums<NT, WJ>(a.partial, a.round_samples, a.nc, re, im);
+}
+
 // NT: 8-coil tiles (at most COIL_GROUP coils per z slice); WJ: warps along the samples.
 template <int NT, int WJ>
 __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
@@ -305,19 +348,15 @@ __global__ void __launch_bounds__(THREADS, 2) main_kernel(const KernelArgs a) {
         if (next_decay) decay[((ch + 1) & 1) * CHUNK + lane] = pow2(t_ref * next_r2);
     }
     cp_wait<0>();
-    cplx<double> *out = a.partial + (size_t)(blockIdx.y * KSPLIT + kw) * a.round_samples * a.nc + c0;
+    int top = 0;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        const int64_t j = jw + mt * 8 + r;
-        if (j >= a.round_samples) continue;
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = nt * 8 + 2 * q + e;
-                if (c < ncg) out[j * a.nc + c] = cplx<double>{k1[mt][nt][e] - k3[mt][nt][e], k1[mt][nt][e] + k2[mt][nt][e]};
-            }
-    }
+            for (int e = 0; e < 2; ++e) from_three(k1[mt][nt][e], k2[mt][nt][e], k3[mt][nt][e], top);
+    store_sums<NT, WJ>(a.partial, a.round_samples, a.nc, k1, k2);
+    if (__any_sync(0xffffffffu, top >= NOT_FINITE)) sums_of_four<NT, WJ>(a, circle);
 }
 
 // State at the segment's end: the same formula at the end row of the prefix
