@@ -123,4 +123,16 @@ inline CoilCut coil_cut(int64_t chunks, int32_t nc, int64_t nsamples, size_t bud
     return p;
 }
 
+// No launch of at most `nsamples` samples has larger partial sums (coil_cut): a
+// launch takes a tile at least, and beyond the budget no more; its parts fill at most
+// 8 waves of `places` CTAs.
+inline size_t coil_cut_bound(int64_t chunks, int32_t nc, int64_t nsamples, size_t budget, int64_t places = 148 * 2) {
+    if (nsamples <= 0) return 0;
+    const int64_t per_warp = 8 * sample_tiles(coil_tiles(nc)), groups = (nc + COIL_GROUP - 1) / COIL_GROUP;
+    const double tile = 16.0 * 8 * per_warp * nc;  // of one part, whatever wj
+    const int64_t tiles = (nsamples + 2 * per_warp - 1) / (2 * per_warp);
+    const double most = tile * std::max(tiles, std::min(tiles * chunks, 8 * places / groups));
+    return (size_t)std::max(tile, std::min((double)budget, most));
+}
+
 }  // namespace homs

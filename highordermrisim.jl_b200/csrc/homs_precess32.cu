@@ -52,7 +52,10 @@ constexpr int F_ADC = 1, F_BLOCK = 2;
 constexpr int WCHUNK = 64;  // nodes per shared-memory stage of the walk (aligned to their index)
 constexpr int SMALL_NS = 16384;
 inline int64_t node_stride(int64_t nnodes) { return (nnodes + WCHUNK - 1) / WCHUNK * WCHUNK; }
-constexpr size_t PHASE_BUDGET = size_t(384) << 20, BLOCK_BUDGET = size_t(64) << 20, PARTIAL_BUDGET = size_t(128) << 20;
+// Memory of a round: 384 MB of phases, or up to 4 GB for rounds of 128 samples (from
+// 786,000 spins on; 4,000,000 spins x 300 samples x 8 coils: rounds of 128, 64 and 32
+// samples 6.4, 7.2 and 9.5 ms), and never fewer than 32 samples.
+constexpr size_t PHASE_BUDGET = size_t(384) << 20, PHASE_MOST = size_t(4) << 30, BLOCK_BUDGET = size_t(64) << 20, PARTIAL_BUDGET = size_t(128) << 20;
 
 __host__ __device__ inline int64_t pad_spins(int64_t ns) { return (ns + 31) / 32 * 32; }
 
@@ -679,7 +682,8 @@ cudaError_t precess32_nodes(const SeqDev<float> &q, uint32_t method, const float
 }
 
 int64_t precess32_max_samples(int64_t ns) {
-    return std::max<int64_t>(128, (int64_t)(PHASE_BUDGET / (sizeof(float) * (size_t)pad_spins(ns))));
+    const size_t row = sizeof(float) * (size_t)pad_spins(ns);
+    return std::max({(int64_t)(PHASE_BUDGET / row), std::min<int64_t>(128, (int64_t)(PHASE_MOST / row)), (int64_t)32});
 }
 int64_t precess32_max_blocks(int64_t ns) {
     return std::max<int64_t>(1, (int64_t)(BLOCK_BUDGET / (sizeof(cplx<float>) * (size_t)pad_spins(ns))));
@@ -688,6 +692,12 @@ size_t precess32_work_bytes(int64_t ns, int64_t nsamples, int32_t nblocks) {
     const size_t np = (size_t)pad_spins(ns);
     return align256(sizeof(float) * np * (size_t)nsamples) + align256(sizeof(cplx<float>) * np * (size_t)nblocks) +
            align256(sizeof(RowInfo) * (size_t)nsamples);
+}
+size_t precess32_run_bytes(int64_t ns, int32_t nc, int64_t nnodes, int64_t nadc, int64_t nblocks, int64_t block_adc) {
+    const int64_t blocks = std::min(nblocks, precess32_max_blocks(ns));
+    const int64_t samples = std::min({nadc, precess32_max_samples(ns), blocks * block_adc});
+    return precess32_node_bytes(nnodes) + precess32_work_bytes(ns, samples, (int32_t)blocks) +
+           coil_cut_bound(pad_spins(ns) / CHUNK, nc, samples, PARTIAL_BUDGET, 148 * 3);
 }
 CoilCut precess32_cut(int64_t ns, int32_t nc, int64_t nsamples) {
     // Three CTAs per SM for up to 8 coils, unless these only add partial sums to read:

@@ -39,6 +39,9 @@ struct Precess32Args {
 };
 size_t precess32_work_bytes(int64_t ns, int64_t nsamples, int32_t nblocks);
 CoilCut precess32_cut(int64_t ns, int32_t nc, int64_t nsamples);
+// Upper bound of what the launches of a run take: node table, a round's work area and
+// partial sums.  block_adc: the most samples of a block.
+size_t precess32_run_bytes(int64_t ns, int32_t nc, int64_t nnodes, int64_t nadc, int64_t nblocks, int64_t block_adc);
 cudaError_t precess32_run(const Precess32Args &a, const CoilCut &cut, cudaEvent_t ev_start, cudaEvent_t ev_stop,
                           unsigned ev_flags, int64_t *launches, cudaStream_t stream);
 

@@ -58,6 +58,7 @@ namespace precess64 {
 constexpr int THREADS = 256;
 constexpr int CHUNK = 32;    // spins per stage
 constexpr int NSTAGE = 3;
+constexpr size_t PARTIAL_BUDGET = size_t(256) << 20;
 constexpr int TERMS = 16;    // phase slots: basis terms 1..15, dw/(2 pi)
 constexpr int BROW = 144;    // bytes of a staged basis row (128 + 16: conflict-free fragment loads)
 constexpr double TWO_PI = 2.0 * 3.141592653589793;
@@ -415,7 +416,12 @@ cudaError_t precess64_table(const double *x, const double *y, const double *z, c
 }
 
 CoilCut precess64_cut(int64_t ns, int32_t nc, int64_t nsamples) {
-    return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, size_t(256) << 20);
+    return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, PARTIAL_BUDGET);
+}
+
+size_t precess64_run_bytes(int64_t ns, int32_t nc, int64_t nadc) {
+    return sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(nadc) +
+           coil_cut_bound(pad_spins(ns) / CHUNK, nc, nadc, PARTIAL_BUDGET);
 }
 
 cudaError_t precess64_run(const Precess64Args &a, const CoilCut &cut, cudaEvent_t ev_start,

@@ -19,6 +19,10 @@ cudaError_t precess64_table(const double *x, const double *y, const double *z, c
 // How a segment is cut (homs_fp64mma.cuh); its partial sums take at most 256 MB.
 CoilCut precess64_cut(int64_t ns, int32_t nc, int64_t nsamples);
 
+// Upper bound of what the launches of a run of `nadc` samples take beside the spin
+// table: prefix table and partial sums.
+size_t precess64_run_bytes(int64_t ns, int32_t nc, int64_t nadc);
+
 struct Precess64Args {
     int64_t ns, nsamples;
     int32_t nc;

@@ -39,6 +39,8 @@
 
 #include "../../include/homs.h"
 #include "homs_internal.cuh"
+#include "homs_precess32.cuh"
+#include "homs_precess64.cuh"
 #include "homs_split.cuh"
 
 namespace {
@@ -84,13 +86,29 @@ size_t estimate_bytes(int64_t nspins, int32_t ncoils, homs_dtype dtype, const ho
         const double slots = std::ceil(nchunks / 262144.0);
         b += tiles * slots * 128 * 64 * 8 + (double)nadc * (192.0 + 96.0 + 8.0);
     } else {
-        const double grid = std::ceil(ns / 256.0);
-        b += std::min(512.0 * (1 << 20), grid * nc * 2 * es * (double)nadc);  // partial sums
-        if (es == 8.0)
-            b += (resident ? 0.0 : ns * 136.0) + (double)nadc * 192.0;  // spin table, prefix table
-        else  // phases and initial states of a round, node table
-            b += std::min(384.0 * (1 << 20), ns * 4.0 * (double)nadc) + std::min(64.0 * (1 << 20), ns * 8.0 * q.nblocks) +
-                 nt * 80.0;
+        // Samples of the pulses, and the most of a block (a request is validated when it
+        // runs, not here).
+        int64_t rf_adc = nadc, block_adc = nadc;
+        if (q.memory == HOMS_HOST && q.adc && q.block_first && q.block_last && q.block_excitation) {
+            rf_adc = block_adc = 0;
+            for (int32_t k = 0; k < q.nblocks; ++k) {
+                int64_t c = 0;
+                for (int64_t n = std::max<int64_t>(q.block_first[k], -1) + 1; n <= q.block_last[k] && n < q.nnodes; ++n)
+                    c += q.adc[n] ? 1 : 0;
+                block_adc = std::max(block_adc, c);
+                if (q.block_excitation[k]) rf_adc += c;
+            }
+        }
+        const double row = std::ceil(ns / 256.0) * nc * 2 * es;
+        b += std::min(std::max(512.0 * (1 << 20), row * 8.0), row * (double)rf_adc);
+        const int64_t spins = std::max<int64_t>(nspins, 1), samples = std::max<int64_t>(nadc, 0);
+        const int32_t coils = std::max(ncoils, 1);
+        if (es == 8.0)  // spin table, prefix table and partial sums of the precession
+            b += (resident ? 0.0 : (double)homs::precess64_table_bytes(spins)) +
+                 (double)homs::precess64_run_bytes(spins, coils, samples);
+        else
+            b += (double)homs::precess32_run_bytes(spins, coils, std::max<int64_t>(q.nnodes, 0), samples,
+                                                   std::max(q.nblocks, 0), std::max<int64_t>(block_adc, 0));
     }
     return (size_t)(b + (64 << 20));
 }
