@@ -241,6 +241,34 @@ private:
     bool stop_ = false, alone_ = false;
 };
 
+// Two page-locked chunks of a context and the events that mark the copies that use
+// them; created when first needed.
+struct Stage {
+    size_t bytes;  // of a chunk
+    void *chunk[2] = {nullptr, nullptr};
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    int next = 0;  // the chunk the next staged copy fills
+    explicit Stage(size_t n) : bytes(n) {}
+    bool ready() const { return chunk[0] && chunk[1] && ev[0] && ev[1]; }
+    bool create() {
+        for (int b = 0; b < 2 && !ready(); ++b) {
+            if (!chunk[b] && cudaHostAlloc(&chunk[b], bytes, cudaHostAllocDefault) != cudaSuccess) chunk[b] = nullptr;
+            if (!ev[b] && cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming) != cudaSuccess) ev[b] = nullptr;
+            if (!chunk[b] || !ev[b]) break;
+        }
+        cudaGetLastError();
+        return ready();
+    }
+    void release() {
+        for (int b = 0; b < 2; ++b) {
+            if (chunk[b]) cudaFreeHost(chunk[b]);
+            if (ev[b]) cudaEventDestroy(ev[b]);
+            chunk[b] = nullptr;
+            ev[b] = nullptr;
+        }
+    }
+};
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -266,11 +294,11 @@ struct homs_context {
     DevBuf selftest_err;  // error word of homs_selftest_wait_timeout
     cudaEvent_t kspace_ev[2] = {nullptr, nullptr};
     bool kspace_timed = false;
-    // Page-locked staging of pageable host inputs: two chunks and the events
-    // that mark the copies reading them (created on first use).
-    void *stage[2] = {nullptr, nullptr};
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
-    int stage_next = 0;  // the chunk the next staged copy fills
+    // Page-locked staging of pageable host arrays: large copies, and packed transfers
+    // of small ones (packing_stage below).
+    Stage stage{size_t(8) << 20}, pack{size_t(1) << 20};
+    int small_uploads = 0, medium_uploads = 0;  // packed before there were chunks for them
+    std::vector<char> pack_host;                // their bytes until then
     CopyPool copies;     // moves bytes between the chunks and pageable arrays
     // Device workspace of homs_simulate, kept between calls (per dtype) so that
     // repeated simulations reuse their buffers instead of reallocating them.
@@ -295,23 +323,19 @@ struct DeviceGuard {
     }
 };
 
-constexpr size_t STAGE_CHUNK = size_t(8) << 20;  // bytes per staging chunk
-constexpr size_t STAGE_MIN = size_t(1) << 20;    // smaller pageable copies go to the driver as they are
+constexpr size_t STAGE_MIN = size_t(1) << 20;  // smaller pageable copies go to the driver as they are
 
-bool stage_ready(homs_context *ctx) {
-    if (ctx->stage[1]) return true;
-    for (int b = 0; b < 2; ++b) {
-        if (!ctx->stage[b] && cudaHostAlloc(&ctx->stage[b], STAGE_CHUNK, cudaHostAllocDefault) != cudaSuccess) {
-            ctx->stage[b] = nullptr;
-            break;
-        }
-        if (!ctx->stage_ev[b] && cudaEventCreateWithFlags(&ctx->stage_ev[b], cudaEventDisableTiming) != cudaSuccess) {
-            ctx->stage_ev[b] = nullptr;
-            break;
-        }
-    }
-    cudaGetLastError();
-    return ctx->stage[0] && ctx->stage[1] && ctx->stage_ev[0] && ctx->stage_ev[1];
+// The chunks for a packed transfer of `bytes`, or NULL.  Page-locking takes 1.3 ms a
+// megabyte chunk and 5 ms an 8 MB one, several times a whole small call, so that a
+// context of a few small calls makes no chunks; `upload` counts calls, and those of a
+// program that goes on pay for them (a call saves about 0.2 ms by one packed upload;
+// from page-locked memory, 15 us of it).
+Stage *packing_stage(homs_context *ctx, size_t bytes, bool upload) {
+    if (bytes > ctx->stage.bytes) return nullptr;
+    if (ctx->stage.ready()) return &ctx->stage;
+    if (bytes <= ctx->pack.bytes)
+        return ctx->pack.ready() || (upload && ++ctx->small_uploads >= 32 && ctx->pack.create()) ? &ctx->pack : nullptr;
+    return upload && ++ctx->medium_uploads >= 128 && ctx->stage.create() ? &ctx->stage : nullptr;
 }
 
 // Ordinary pageable host memory: the only kind the staging below copies with
@@ -333,20 +357,21 @@ bool pageable(const void *p) {
 // pageable memory does.
 void h2d(homs_context *ctx, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return;
-    if (!pageable(src) || bytes < STAGE_MIN || !stage_ready(ctx)) {
+    if (!pageable(src) || bytes < STAGE_MIN || !ctx->stage.create()) {
         HOMS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
         return;
     }
+    Stage &st = ctx->stage;
     const char *s = static_cast<const char *>(src);
     char *d = static_cast<char *>(dst);
-    for (size_t off = 0; off < bytes; off += STAGE_CHUNK) {
-        const size_t n = std::min(STAGE_CHUNK, bytes - off);
-        const int b = ctx->stage_next;
-        ctx->stage_next ^= 1;
-        HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));  // the copy that last read this chunk is done
-        ctx->copies.run({{ctx->stage[b], s + off, n}});
-        HOMS_CUDA(cudaMemcpyAsync(d + off, ctx->stage[b], n, cudaMemcpyHostToDevice, ctx->stream));
-        HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
+    for (size_t off = 0; off < bytes; off += st.bytes) {
+        const size_t n = std::min(st.bytes, bytes - off);
+        const int b = st.next;
+        st.next ^= 1;
+        HOMS_CUDA(cudaEventSynchronize(st.ev[b]));  // the copy that last read this chunk is done
+        ctx->copies.run({{st.chunk[b], s + off, n}});
+        HOMS_CUDA(cudaMemcpyAsync(d + off, st.chunk[b], n, cudaMemcpyHostToDevice, ctx->stream));
+        HOMS_CUDA(cudaEventRecord(st.ev[b], ctx->stream));
     }
 }
 
@@ -357,32 +382,33 @@ void h2d(homs_context *ctx, void *dst, const void *src, size_t bytes) {
 // other out) and holds it when the call returns.
 void d2h(homs_context *ctx, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return;
-    if (!pageable(dst) || bytes < STAGE_MIN || !stage_ready(ctx)) {
+    if (!pageable(dst) || bytes < STAGE_MIN || !ctx->stage.create()) {
         HOMS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         return;
     }
+    Stage &st = ctx->stage;
     const char *s = static_cast<const char *>(src);
     char *d = static_cast<char *>(dst);
     int prev = -1;
     size_t prev_off = 0, prev_n = 0;
-    for (size_t off = 0; off < bytes; off += STAGE_CHUNK) {
-        const size_t n = std::min(STAGE_CHUNK, bytes - off);
-        const int b = ctx->stage_next;
-        ctx->stage_next ^= 1;
+    for (size_t off = 0; off < bytes; off += st.bytes) {
+        const size_t n = std::min(st.bytes, bytes - off);
+        const int b = st.next;
+        st.next ^= 1;
         // The chunk's last reader was a transfer earlier on this stream, or this
         // thread's copy-out two chunks back, which has returned.
-        HOMS_CUDA(cudaMemcpyAsync(ctx->stage[b], s + off, n, cudaMemcpyDeviceToHost, ctx->stream));
-        HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
+        HOMS_CUDA(cudaMemcpyAsync(st.chunk[b], s + off, n, cudaMemcpyDeviceToHost, ctx->stream));
+        HOMS_CUDA(cudaEventRecord(st.ev[b], ctx->stream));
         if (prev >= 0) {
-            HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[prev]));
-            ctx->copies.run({{d + prev_off, ctx->stage[prev], prev_n}});
+            HOMS_CUDA(cudaEventSynchronize(st.ev[prev]));
+            ctx->copies.run({{d + prev_off, st.chunk[prev], prev_n}});
         }
         prev = b;
         prev_off = off;
         prev_n = n;
     }
-    HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[prev]));
-    ctx->copies.run({{d + prev_off, ctx->stage[prev], prev_n}});
+    HOMS_CUDA(cudaEventSynchronize(st.ev[prev]));
+    ctx->copies.run({{d + prev_off, st.chunk[prev], prev_n}});
 }
 
 // Copy `n` elements of dtype `src_dt` at `src` (host or device) into a device
@@ -424,7 +450,7 @@ void upload(homs_context *ctx, DevBuf &dst, const void *src, homs_dtype src_dt, 
 // (Copied one by one, each array costs a driver call and, from pageable
 // memory, its own staging.)  `reals` hold n values of `src_dt`, `raw` n bytes.
 // False, and nothing done, when an array is not ordinary pageable memory, they
-// exceed a chunk or there is none: the caller then uploads them one by one.
+// exceed a chunk, or a megabyte without chunks: the caller then uploads them one by one.
 struct UploadItem {
     DevBuf *dst;
     const void *src;
@@ -438,15 +464,23 @@ bool upload_packed(homs_context *ctx, DevBuf &block, homs_dtype src_dt, const st
     size_t count = 0, raw_bytes = 0;
     for (const UploadItem &u : reals) count += (u.n + ALIGN - 1) / ALIGN * ALIGN;
     for (const UploadItem &u : raw) raw_bytes += (u.n + 255) / 256 * 256;
-    if (count * es + raw_bytes > STAGE_CHUNK) return false;
+    const size_t bytes = count * es + raw_bytes;
     for (const UploadItem &u : reals)
         if (!pageable(u.src)) return false;
-    if (!stage_ready(ctx)) return false;
+    Stage *st = packing_stage(ctx, bytes, true);
+    if (!st && bytes > ctx->pack.bytes) return false;
     HOMS_CUDA(block.ensure(count * sizeof(T) + raw_bytes));
-    const int b = ctx->stage_next;
-    ctx->stage_next ^= 1;
-    HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));
-    char *host = static_cast<char *>(ctx->stage[b]), *dev = block.as<char>();
+    const int b = st ? st->next : 0;
+    char *host;
+    if (st) {
+        st->next ^= 1;
+        HOMS_CUDA(cudaEventSynchronize(st->ev[b]));
+        host = static_cast<char *>(st->chunk[b]);
+    } else {  // the driver has copied the bytes when cudaMemcpyAsync returns
+        ctx->pack_host.resize(std::max(bytes, ctx->pack_host.size()));
+        host = ctx->pack_host.data();
+    }
+    char *dev = block.as<char>();
     std::vector<CopyPool::Piece> pieces;
     size_t at = 0;
     for (const UploadItem &u : reals) {
@@ -462,7 +496,7 @@ bool upload_packed(homs_context *ctx, DevBuf &block, homs_dtype src_dt, const st
     }
     ctx->copies.run(pieces);
     if (es == sizeof(T)) {
-        HOMS_CUDA(cudaMemcpyAsync(dev, host, count * es + raw_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        HOMS_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     } else {
         HOMS_CUDA(ctx->scratch_conv.ensure(count * es));
         HOMS_CUDA(cudaMemcpyAsync(ctx->scratch_conv.p, host, count * es, cudaMemcpyHostToDevice, ctx->stream));
@@ -478,7 +512,7 @@ bool upload_packed(homs_context *ctx, DevBuf &block, homs_dtype src_dt, const st
                                                                            ctx->scratch_conv.as<float>(), n);
         HOMS_CUDA(cudaGetLastError());
     }
-    HOMS_CUDA(cudaEventRecord(ctx->stage_ev[b], ctx->stream));
+    if (st) HOMS_CUDA(cudaEventRecord(st->ev[b], ctx->stream));
     return true;
 }
 
@@ -1279,18 +1313,18 @@ void copy_out(homs_context *ctx, Resident<T> &r, void *sig, homs_memory sig_memo
         total += (es * (size_t)o.n + 255) / 256 * 256;
         pack = pack && o.mem == HOMS_HOST;
     }
-    pack = pack && total <= STAGE_CHUNK;
     for (const Out &o : outs) pack = pack && pageable(o.dst);
-    if (!pack || !stage_ready(ctx)) {
+    Stage *st = pack ? packing_stage(ctx, total, false) : nullptr;
+    if (!st) {
         if (split) check_split<T>(ctx, r);
         for (const Out &o : outs) download<T>(ctx, o.dst, o.mem, o.src, o.n, out_dt);
         HOMS_CUDA(cudaStreamSynchronize(ctx->stream));
         return;
     }
-    const int b = ctx->stage_next;
-    ctx->stage_next ^= 1;
-    HOMS_CUDA(cudaEventSynchronize(ctx->stage_ev[b]));  // no upload still reads this chunk
-    char *host = static_cast<char *>(ctx->stage[b]);
+    const int b = st->next;
+    st->next ^= 1;
+    HOMS_CUDA(cudaEventSynchronize(st->ev[b]));  // no upload still reads this chunk
+    char *host = static_cast<char *>(st->chunk[b]);
     const bool narrow = es != sizeof(T);
     HOMS_REQUIRE(!narrow || (sizeof(T) == 8 && out_dt == HOMS_F32), "internal: unsupported output conversion");
     if (narrow) HOMS_CUDA(ctx->scratch_conv.ensure(total));
@@ -1527,12 +1561,8 @@ homs_status homs_context_destroy(homs_context *ctx) {
         ctx->build_work.release();
         ctx->build_out.release();
         ctx->selftest_err.release();
-        for (int b = 0; b < 2; ++b) {
-            if (ctx->stage[b]) cudaFreeHost(ctx->stage[b]);
-            if (ctx->stage_ev[b]) cudaEventDestroy(ctx->stage_ev[b]);
-            ctx->stage[b] = nullptr;
-            ctx->stage_ev[b] = nullptr;
-        }
+        ctx->stage.release();
+        ctx->pack.release();
         for (cudaEvent_t &e : ctx->kspace_ev)
             if (e) cudaEventDestroy(e);
         ctx->cache[0].reset();
