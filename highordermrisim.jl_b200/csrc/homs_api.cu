@@ -836,6 +836,7 @@ struct Launch {
     int block_start;  // n_lo is the first node of a block
     int64_t sample0, nsamples;
     int32_t nblocks;  // blocks with intervals in the launch
+    bool sequential;  // RF, or a short precession segment: one thread per spin and node by node
 };
 
 template <typename T>
@@ -856,7 +857,7 @@ std::vector<Launch> plan_launches(const Resident<T> &r, const LaunchLimits &lim)
         int64_t n = r.first[k];
         const int64_t n_end = r.last[k2 - 1];
         while (n < n_end) {
-            Launch L{rf, n, n, n == r.first[blk] ? 1 : 0, sample, 0, 1};
+            Launch L{rf, n, n, n == r.first[blk] ? 1 : 0, sample, 0, 1, rf};
             int64_t m = n;
             while (m < n_end) {
                 // interval m -> node m+1
@@ -870,6 +871,8 @@ std::vector<Launch> plan_launches(const Resident<T> &r, const LaunchLimits &lim)
                 if (L.nsamples >= max_samples) break;
             }
             L.n_hi = m;
+            if (!rf && L.block_start)
+                L.sequential = precession_is_short(r.ns, r.nc, m - L.n_lo, L.nsamples, sizeof(T) == 8, false);
             sample += L.nsamples;
             out.push_back(L);
             n = m;
@@ -948,17 +951,19 @@ inline void plain_round32(homs_context *ctx, Resident<float> &r, uint32_t method
                             &r.launches, ctx->stream));
 }
 
-// Partial sums of an excitation launch.
+// Partial sums of a sequential launch.
 template <typename T>
-size_t excitation_partial_bytes(const Resident<T> &r, const Launch &L) {
-    return sizeof(cplx<T>) * (size_t)r.nc * (size_t)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS) * (size_t)L.nsamples;
+size_t sequential_partial_bytes(const Resident<T> &r, const Launch &L) {
+    return (L.rf ? sizeof(cplx<T>) : sizeof(cplx<double>)) * (size_t)r.nc *
+           (size_t)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS) * (size_t)L.nsamples;
 }
 
-// One launch of an excitation run (at most excitation_samples samples).
+// One launch of an excitation run (at most excitation_samples samples), or a short
+// precession segment.
 template <typename T>
-void excitation_launch(Resident<T> &r, uint32_t method, const Launch &L, cudaStream_t stream) {
+void sequential_launch(Resident<T> &r, uint32_t method, const Launch &L, cudaStream_t stream) {
     const int grid = (int)((r.ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-    if (r.partial.bytes < excitation_partial_bytes(r, L)) HOMS_CUDA(r.partial.ensure(excitation_partial_bytes(r, L)));
+    if (r.partial.bytes < sequential_partial_bytes(r, L)) HOMS_CUDA(r.partial.ensure(sequential_partial_bytes(r, L)));
     SegmentArgs<T> a;
     a.n_lo = L.n_lo;
     a.n_hi = L.n_hi;
@@ -971,13 +976,15 @@ void excitation_launch(Resident<T> &r, uint32_t method, const Launch &L, cudaStr
     PhantomDev<T> p = r.phantom();
     SeqDev<T> q = r.seq();
     StateDev<T> st{r.xy.template as<cplx<T>>(), r.mz.template as<T>(), r.acc.template as<T>()};
-    HOMS_CUDA(launch_excitation<T>(p, q, st, a, grid, stream));
+    cplx<T> *sig = r.sig.template as<cplx<T>>() + L.sample0;
+    cplx<double> *sums = r.partial.template as<cplx<double>>();  // of a precession segment
+    if (L.rf) HOMS_CUDA(launch_excitation<T>(p, q, st, a, grid, stream));
+    else HOMS_CUDA(launch_short<T>(p, q, st, a, sums, grid, stream));
     r.launches += 1;
-    if (L.nsamples > 0) {
-        HOMS_CUDA(launch_partial_finalize(a.partial, grid, L.nsamples, r.nc,
-                                          r.sig.template as<cplx<T>>() + L.sample0, r.nadc, stream));
-        r.launches += 1;
-    }
+    if (L.nsamples == 0) return;
+    if (L.rf) HOMS_CUDA(launch_partial_finalize(a.partial, grid, L.nsamples, r.nc, sig, r.nadc, stream));
+    else HOMS_CUDA(launch_partial_finalize(sums, grid, L.nsamples, r.nc, sig, r.nadc, stream));
+    r.launches += 1;
 }
 
 // Samples of an excitation launch whose partial sums take at most 512 MB.
@@ -994,9 +1001,11 @@ template <typename T>
 void prepare_plain(homs_context *ctx, Resident<T> &r, uint32_t method, const std::vector<Launch> &plan) {
     auto align = [](size_t n) { return (n + 255) & ~size_t(255); };
     size_t table = 0, per_run = 0, partial = 0;
+    bool parallel = false;  // launches that need the tables
     for (const Launch &L : plan) {
-        if (L.rf) {
-            partial = std::max(partial, excitation_partial_bytes(r, L));
+        parallel = parallel || !L.sequential;
+        if (L.sequential) {
+            partial = std::max(partial, sequential_partial_bytes(r, L));
         } else if constexpr (sizeof(T) == 8) {
             per_run = std::max(per_run, sizeof(double) * SPLIT_PREFIX_STRIDE * split_prefix_rows(L.nsamples));
             partial = std::max(partial, precess64_cut(r.ns, r.nc, L.nsamples).partial_bytes);
@@ -1009,8 +1018,9 @@ void prepare_plain(homs_context *ctx, Resident<T> &r, uint32_t method, const std
     if constexpr (sizeof(T) == 8) {
         const char *t = r.spin_table.template as<char>(), *w = r.work.template as<char>();
         own_table = !r.spin_table_ready || (t >= w && t < w + r.work.bytes);
+        own_table = own_table && parallel;
         if (own_table) table = precess64_table_bytes(r.ns);
-    } else {
+    } else if (parallel) {
         table = precess32_node_bytes(r.nt);
     }
     const void *before = r.work.p;
@@ -1023,7 +1033,7 @@ void prepare_plain(homs_context *ctx, Resident<T> &r, uint32_t method, const std
             if (!stays) build_spin_table(ctx, r);
         }
         r.prefix.view(at + align(table), per_run);
-    } else {
+    } else if (parallel) {
         const bool stays = r.work.p == before && r.nodes_method == method;
         r.nodes.view(at, table);
         if (!stays) {
@@ -1046,10 +1056,10 @@ void run_plain(homs_context *ctx, Resident<T> &r, uint32_t method, bool capture)
     const std::vector<Launch> plan = plan_launches<T>(r, lim);
     if (!capture) prepare_plain(ctx, r, method, plan);
     for (const Launch &L : plan) {
-        if (L.rf) {
+        if (L.sequential) {
             const auto ev = r.next_events();
             HOMS_CUDA(cudaEventRecordWithFlags(ev.first, ctx->stream, ev_flags));
-            excitation_launch<T>(r, method, L, ctx->stream);
+            sequential_launch<T>(r, method, L, ctx->stream);
             HOMS_CUDA(cudaEventRecordWithFlags(ev.second, ctx->stream, ev_flags));
             continue;
         }
@@ -1180,7 +1190,7 @@ struct SplitRunner {
         while (i < plan.size()) {
             const Launch &L = plan[i];
             if (L.rf) {
-                excitation_launch<T>(*r, sa.method, L, stream);
+                sequential_launch<T>(*r, sa.method, L, stream);
                 ++i;
                 continue;
             }
@@ -1774,8 +1784,8 @@ void block_precess64(homs_context *ctx, const PhantomDev<double> &p, const SeqDe
 // The same in FP32: the block's nodes get a table of their own, then the block
 // runs in launch rounds.
 void block_precess32(homs_context *ctx, const PhantomDev<float> &p, const SeqDev<float> &q, const homs_state &state,
-                     int64_t first, int64_t last, uint32_t method, double gamma, int64_t nadc, void *sig,
-                     int64_t ldsig) {
+                     int64_t first, int64_t last, uint32_t method, double gamma, const std::vector<uint8_t> &adc,
+                     int64_t nadc, void *sig, int64_t ldsig) {
     Resident<float> r;  // the block as a sequence of its own (host side only)
     r.ns = p.ns;
     r.nc = p.nc;
@@ -1784,9 +1794,9 @@ void block_precess32(homs_context *ctx, const PhantomDev<float> &p, const SeqDev
     r.first = {0};
     r.last = {r.nt - 1};
     r.exc = {0};
-    r.adc_host.resize((size_t)r.nt);
-    HOMS_CUDA(cudaMemcpyAsync(r.adc_host.data(), q.adc + first, (size_t)r.nt, cudaMemcpyDeviceToHost, ctx->stream));
-    const std::vector<float> dt = host_array<float>(ctx, q.dt + first, HOMS_F32, HOMS_DEVICE, r.nt - 1);  // waits for both
+    r.adc_host.assign(1, 0);
+    r.adc_host.insert(r.adc_host.end(), adc.begin(), adc.end());
+    const std::vector<float> dt = host_array<float>(ctx, q.dt + first, HOMS_F32, HOMS_DEVICE, r.nt - 1);
     std::vector<float> tp((size_t)r.nt, 0.0f);
     for (int64_t n = 1; n < r.nt; ++n) tp[(size_t)n] = tp[(size_t)(n - 1)] + dt[(size_t)(n - 1)];
     HOMS_CUDA(ctx->block_rank.ensure(sizeof(float) * (size_t)r.nt));
@@ -1869,17 +1879,17 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     qd.adc = q->adc;
     qd.boundary = reinterpret_cast<uint8_t *>(ctx->scratch_bnd.p);
     for (int k = 0; k < 16; ++k) qd.h[k] = (const T *)q->h[k];
-    if (!rf) {
+    if (!rf && !precession_is_short(ns, nc, last - first, nadc, sizeof(T) == 8, true)) {
         if constexpr (sizeof(T) == 8)
             block_precess64(ctx, pd, qd, *state, first, last, method, q->gamma, adc, nadc, sig, ldsig);
         else
-            block_precess32(ctx, pd, qd, *state, first, last, method, q->gamma, nadc, sig, ldsig);
+            block_precess32(ctx, pd, qd, *state, first, last, method, q->gamma, adc, nadc, sig, ldsig);
         return HOMS_OK;
     }
     HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
     const int grid = (int)((ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
-    HOMS_CUDA(ctx->scratch_partial.ensure(sizeof(cplx<T>) * (size_t)grid * (size_t)std::max<int64_t>(nadc, 1) * nc));
-    HOMS_CUDA(ctx->scratch_sig.ensure(sizeof(cplx<T>) * (size_t)std::max<int64_t>(nadc, 1) * nc));
+    const size_t samples = (size_t)std::max<int64_t>(nadc, 1) * nc;
+    HOMS_CUDA(ctx->scratch_partial.ensure((rf ? sizeof(cplx<T>) : sizeof(cplx<double>)) * (size_t)grid * samples));
     StateDev<T> st{(cplx<T> *)state->xy, (T *)state->z, reinterpret_cast<T *>(ctx->scratch_acc.p)};
     SegmentArgs<T> a;
     a.n_lo = first;
@@ -1890,6 +1900,13 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
     a.gamma = T(q->gamma);
     a.gamma_d = q->gamma;
     a.partial = reinterpret_cast<cplx<T> *>(ctx->scratch_partial.p);
+    if (!rf) {
+        cplx<double> *sums = ctx->scratch_partial.as<cplx<double>>();
+        HOMS_CUDA(launch_short<T>(pd, qd, st, a, sums, grid, ctx->stream));
+        if (nadc > 0) HOMS_CUDA(launch_partial_finalize(sums, grid, nadc, nc, (cplx<T> *)sig, ldsig, ctx->stream));
+        return HOMS_OK;
+    }
+    HOMS_CUDA(ctx->scratch_sig.ensure(sizeof(cplx<T>) * samples));
     HOMS_CUDA(launch_excitation<T>(pd, qd, st, a, grid, ctx->stream));
     if (nadc > 0) {
         HOMS_CUDA(launch_partial_finalize(a.partial, grid, nadc, nc, reinterpret_cast<cplx<T> *>(ctx->scratch_sig.p), nadc, ctx->stream));

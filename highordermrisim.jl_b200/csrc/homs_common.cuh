@@ -48,8 +48,8 @@ struct StateDev {
     T *acc;  // running trapezoid sum of the current precession block
 };
 
-// One launch of the excitation kernel: intervals [n_lo, n_hi) of a run of
-// excitation blocks.
+// One launch of the excitation kernel, or of the kernel of short precession
+// segments: intervals [n_lo, n_hi) of a run of blocks.
 template <typename T>
 struct SegmentArgs {
     int64_t n_lo, n_hi;
@@ -72,6 +72,13 @@ namespace homs {
 template <typename T>
 cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st,
                            const SegmentArgs<T> &a, int grid, cudaStream_t stream);
+
+// A short precession segment: intervals [a.n_lo, a.n_hi), from the first node of a
+// block on; FP64 partial sums [grid][nsamples][nc] in place of a.partial.
+bool precession_is_short(int64_t ns, int32_t nc, int64_t nodes, int64_t nsamples, bool f64, bool block_call);
+template <typename T>
+cudaError_t launch_short(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st, const SegmentArgs<T> &a,
+                         cplx<double> *partial, int grid, cudaStream_t stream);
 
 // An FP64 excitation launch without ADC samples (homs_excite64.cu).
 cudaError_t launch_excite64(const PhantomDev<double> &p, const SeqDev<double> &q, StateDev<double> &st,

@@ -84,11 +84,11 @@ __device__ void load_nodes(NodeCache<T> &nc, const SeqDev<T> &q, int64_t c0, int
 
 // Contract `na` staged ADC states X[a][s] (s < PLAIN_THREADS) with the
 // sensitivities of this CTA's spins and write one partial row per sample:
-// out[a * nc + c] = sum_s X[a][s] * csm[s][c], summed over spins in a fixed
-// order (a per-lane sweep, then splits in index order).
-template <typename T>
-__device__ void reduce_stage(const cplx<T> *X, cplx<T> *P, int na, const cplx<T> *csm_rows, int csm_ld,
-                             int nvalid, int32_t nc, cplx<T> *out) {
+// out[a * nc + c] = sum_s X[a][s] * csm[s][c], summed in type A over spins in a
+// fixed order (a per-lane sweep, then splits in index order).
+template <typename T, typename A>
+__device__ void reduce_stage(const cplx<T> *X, cplx<A> *P, int na, const cplx<T> *csm_rows, int csm_ld,
+                             int nvalid, int32_t nc, cplx<A> *out) {
     const int t = threadIdx.x;
     for (int cg = 0; cg < nc; cg += 32) {
         const int left = min(32, nc - cg);
@@ -96,20 +96,22 @@ __device__ void reduce_stage(const cplx<T> *X, cplx<T> *P, int na, const cplx<T>
         while (cw < left) cw <<= 1;
         const int cl = t % cw, split = t / cw;
         const int c = cg + cl;
-        cplx<T> acc[PLAIN_STAGE];
+        cplx<A> acc[PLAIN_STAGE];
 #pragma unroll
-        for (int a = 0; a < PLAIN_STAGE; ++a) acc[a] = cplx<T>{T(0), T(0)};
+        for (int a = 0; a < PLAIN_STAGE; ++a) acc[a] = cplx<A>{A(0), A(0)};
         if (cl < left) {
             for (int i = 0; i < cw; ++i) {
                 const int s = split * cw + i;
                 if (s >= nvalid) break;
-                const cplx<T> w = csm_rows[(int64_t)s * csm_ld + c];
+                const cplx<T> wt = csm_rows[(int64_t)s * csm_ld + c];
+                const cplx<A> w{A(wt.re), A(wt.im)};
                 // Complex multiply-accumulate as four fused multiply-adds: the
                 // reference's coil sum is a BLAS product, which fuses them too.
 #pragma unroll
                 for (int a = 0; a < PLAIN_STAGE; ++a) {
                     if (a < na) {
-                        const cplx<T> x = X[a * PLAIN_THREADS + s];
+                        const cplx<T> xt = X[a * PLAIN_THREADS + s];
+                        const cplx<A> x{A(xt.re), A(xt.im)};
                         acc[a].re = fma(x.re, w.re, fma(-x.im, w.im, acc[a].re));
                         acc[a].im = fma(x.re, w.im, fma(x.im, w.re, acc[a].im));
                     }
@@ -123,9 +125,9 @@ __device__ void reduce_stage(const cplx<T> *X, cplx<T> *P, int na, const cplx<T>
         const int nsplit = PLAIN_THREADS / cw;
         if (t < na * cw) {
             const int a = t / cw, c2 = t % cw;
-            cplx<T> s{T(0), T(0)};
+            cplx<A> s{A(0), A(0)};
             for (int j = 0; j < nsplit; ++j) {
-                cplx<T> v = P[(j * PLAIN_STAGE + a) * cw + c2];
+                cplx<A> v = P[(j * PLAIN_STAGE + a) * cw + c2];
                 s.re = s.re + v.re;
                 s.im = s.im + v.im;
             }
@@ -315,6 +317,121 @@ __global__ void __launch_bounds__(ADC ? PLAIN_THREADS : 64, ADC ? 3 : 8)
     if (active) {
         st.xy[s] = xy;
         st.z[s] = mz;
+    }
+}
+
+// Short precession segments: one thread per spin walks the nodes, field, phase sum,
+// sine, cosine and decay as they come (BlochHighOrderSimulatitonMethod.jl:54-92, in
+// the CPU order), samples staged and contracted as in the excitation kernel, but
+// summed in FP64 for either type (as the parallel kernels sum).
+// Against the kernels that are parallel over samples (homs_precess64.cu,
+// homs_precess32.cu) it needs no tables and pads no sample tile, and its time grows
+// by every node: precession_is_short has the line between them.
+template <typename T>
+struct FieldCache {
+    T dt[NODE_CHUNK + 1];
+    T f[16][NODE_CHUNK + 1];  // field coefficients; 1..3: the nominal gradients where the first order is off
+    uint8_t adc[NODE_CHUNK + 1];
+    uint8_t bnd[NODE_CHUNK + 1];
+};
+
+// Bz at cached node i (BlochHighOrderSimulatitonMethod.jl:70-75).
+template <typename T>
+__device__ __forceinline__ T field_cached(const FieldCache<T> &nc, int i, const T *b, T dwterm, uint32_t m) {
+    const T bz1 = (b[1] * nc.f[1][i] + b[2] * nc.f[2][i]) + b[3] * nc.f[3][i];
+    T bz = ((m & HOMS_HO0) ? nc.f[0][i] : T(0)) + bz1;
+    if (m & HOMS_HO2) {
+        T t = b[4] * nc.f[4][i];
+#pragma unroll
+        for (int k = 5; k <= 8; ++k) t = t + b[k] * nc.f[k][i];
+        bz = bz + t;
+    }
+    if (m & HOMS_HO3) {
+        T t = b[9] * nc.f[9][i];
+#pragma unroll
+        for (int k = 10; k <= 15; ++k) t = t + b[k] * nc.f[k][i];
+        bz = bz + t;
+    }
+    return (m & HOMS_DW_PRECESSION) ? bz + dwterm : bz;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(PLAIN_THREADS, sizeof(T) == 4 ? 3 : 2)
+    short_kernel(PhantomDev<T> p, SeqDev<T> q, StateDev<T> st, SegmentArgs<T> a, cplx<double> *partial) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FieldCache<T> &nc = *reinterpret_cast<FieldCache<T> *>(smem_raw);
+    cplx<T> *X = reinterpret_cast<cplx<T> *>(smem_raw + ((sizeof(FieldCache<T>) + 15) & ~size_t(15)));
+    cplx<double> *P = reinterpret_cast<cplx<double> *>(X + PLAIN_STAGE * PLAIN_THREADS);
+    const int64_t spin0 = (int64_t)blockIdx.x * PLAIN_THREADS, s = spin0 + threadIdx.x;
+    const bool active = s < p.ns;
+    const int64_t si = active ? s : 0;
+    const int nvalid = (int)imin64(PLAIN_THREADS, p.ns - spin0);
+    const uint32_t m = a.method;
+    const double twopig_d = 2.0 * 3.141592653589793 * a.gamma_d;
+    const T c_neg = T(-twopig_d), dwterm = p.dw[si] / T(twopig_d);
+    const T x = p.x[si], y = p.y[si], z = p.z[si], T1 = p.T1[si], T2 = p.T2[si], rho = p.rho[si];
+    const T x2 = x * x, y2 = y * y, z2 = z * z, r2 = (x2 + y2) + z2;
+    const T b[16] = {T(1), x, y, z, x * y, z * y, T(3) * z2 - r2, x * z, x2 - y2, (T(3) * y) * x2 - (y2 * y), (x * z) * y,
+                     (T(5) * z2 - r2) * y, T(5) * (z2 * z) - (T(3) * z) * r2, (T(5) * z2 - r2) * x, x2 * z - y2 * z,
+                     (x2 * x) - (T(3) * x) * y2};
+    cplx<T> xy = active ? st.xy[si] : cplx<T>{T(0), T(0)};
+    T mz = active ? st.z[si] : T(0);
+    T acc = T(0), tp = T(0), prev = T(0);
+    int staged = 0;
+    int64_t sample = 0;
+    cplx<double> *out_base = partial + (int64_t)blockIdx.x * a.nsamples * p.nc;
+    auto reduce = [&] {
+        __syncthreads();
+        reduce_stage(X, P, staged, p.csm + spin0 * p.nc, p.nc, nvalid, p.nc, out_base + sample * p.nc);
+        sample += staged;
+        staged = 0;
+    };
+    for (int64_t c0 = a.n_lo; c0 < a.n_hi; c0 += NODE_CHUNK) {
+        const int nint = (int)imin64(NODE_CHUNK, a.n_hi - c0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < 16 * (NODE_CHUNK + 1); i += PLAIN_THREADS) {
+            const int k = i / (NODE_CHUNK + 1), n = i % (NODE_CHUNK + 1);
+            const int64_t g = c0 + n;
+            if (n > nint) continue;
+            const T *f = q.h[k];
+            if (k >= 1 && k <= 3 && !(m & HOMS_HO1)) f = k == 1 ? q.gx : k == 2 ? q.gy : q.gz;
+            nc.f[k][n] = f[g];
+            if (k == 0) {
+                nc.dt[n] = n < nint ? q.dt[g] : T(0);
+                nc.adc[n] = q.adc[g];
+                nc.bnd[n] = q.boundary[g];
+            }
+        }
+        __syncthreads();
+        if (c0 == a.n_lo) prev = field_cached(nc, 0, b, dwterm, m);
+        for (int i = 0; i < nint; ++i) {
+            const T next = field_cached(nc, i + 1, b, dwterm, m);
+            acc = acc + (next + prev) * nc.dt[i];
+            tp = tp + nc.dt[i];
+            prev = next;
+            if (!nc.adc[i + 1] && !nc.bnd[i + 1]) continue;
+            T sn, cs;
+            Math<T>::sc(c_neg * (T(0.5) * acc), &sn, &cs);
+            const T e = Math<T>::ex(T(0) - tp / T2);
+            const cplx<T> xs = cmul(xy, cplx<T>{e * cs, e * sn});
+            if (nc.adc[i + 1]) {
+                X[staged * PLAIN_THREADS + threadIdx.x] = active ? xs : cplx<T>{T(0), T(0)};
+                if (++staged == PLAIN_STAGE) reduce();
+            }
+            if (nc.bnd[i + 1]) {  // Mxy of the block's last node, Mz relaxed over it, the phase sum restarts
+                xy = xs;
+                const T e1 = Math<T>::ex(-tp / T1);
+                mz = mz * e1 + rho * (T(1) - e1);
+                acc = T(0);
+                tp = T(0);
+            }
+        }
+    }
+    if (staged > 0) reduce();
+    if (active) {
+        st.xy[s] = xy;
+        st.z[s] = mz;
+        if (sizeof(T) == 4) st.acc[s] = acc;  // a later round of the run starts from it
     }
 }
 
@@ -562,6 +679,37 @@ cudaError_t launch_excitation(const PhantomDev<T> &p, const SeqDev<T> &q, StateD
     return cudaGetLastError();
 }
 
+// Nodes, and more so samples and coils, cost the sequential kernel time; the
+// parallel kernels pay per segment: three or four launches, a sample tile of which
+// few rows are used, and in a block call the tables.  The lines come from sweeps of
+// 300 to 1,000,000 spins, 1 to 48 (128) nodes and 1, 3, 8 and 32 coils.  Segments of
+// prepared runs with a pulse of one node each, parallel and sequential: FP32, 3,000
+// spins x 8 coils, 8 nodes with 4 samples 34 and 28 us, 32 with 32 38 and 43; 200,000
+// x 8, 8 with 4 75 and 45, 48 with 24 90 and 104; FP64 the same 40 and 30, 41 and 50,
+// 104 and 59, 104 and 140.  Block calls, every node a sample: FP32, 3,000 x 8, 16
+// nodes 66 and 48, 48 nodes 68 and 71; 200,000 x 8, 16 nodes 117 and 93, 32 nodes 124
+// and 136; FP64 59 and 49, 59 and 77, 136 and 111, 140 and 167.  Where the rule takes
+// the sequential kernel, it is the faster one; on the other side it would have been by
+// up to 0.2 of the time (FP64 x 1,000,000 spins: 0.34).
+bool precession_is_short(int64_t ns, int32_t nc, int64_t nodes, int64_t nsamples, bool f64, bool block_call) {
+    if (nsamples == 0) return nodes <= (block_call ? 16 : 4);
+    static constexpr int limit[2][2][3] = {{{84, 168, 108}, {256, 264, 152}},    // FP32: prepared, block call
+                                           {{140, 212, 104}, {176, 248, 128}}};  // FP64
+    return 2 * nodes + 5 * nsamples + 3 * (int64_t)nc <= limit[f64][block_call][ns <= 16384 ? 0 : ns <= 100000 ? 1 : 2];
+}
+
+template <typename T>
+cudaError_t launch_short(const PhantomDev<T> &p, const SeqDev<T> &q, StateDev<T> &st, const SegmentArgs<T> &a,
+                         cplx<double> *partial, int grid, cudaStream_t stream) {
+    // Node cache, staged samples and the reduction's sums: 52 KB in FP32, 71 KB in FP64.
+    size_t smem = (sizeof(FieldCache<T>) + 15) & ~size_t(15);
+    if (a.nsamples > 0) smem += (sizeof(cplx<T>) + sizeof(cplx<double>)) * PLAIN_STAGE * PLAIN_THREADS;
+    const cudaError_t e = allow_max_dynamic_smem((const void *)short_kernel<T>);
+    if (e != cudaSuccess) return e;
+    short_kernel<T><<<grid, PLAIN_THREADS, smem, stream>>>(p, q, st, a, partial);
+    return cudaGetLastError();
+}
+
 template <typename T, typename S>
 cudaError_t launch_partial_finalize(const cplx<T> *partial, int64_t nparts, int64_t nsamples, int32_t nc,
                                     cplx<S> *sig, int64_t ldsig, cudaStream_t stream) {
@@ -630,6 +778,10 @@ template cudaError_t launch_excitation<double>(const PhantomDev<double> &, const
                                                const SegmentArgs<double> &, int, cudaStream_t);
 template cudaError_t launch_excitation<float>(const PhantomDev<float> &, const SeqDev<float> &, StateDev<float> &,
                                               const SegmentArgs<float> &, int, cudaStream_t);
+template cudaError_t launch_short<double>(const PhantomDev<double> &, const SeqDev<double> &, StateDev<double> &,
+                                          const SegmentArgs<double> &, cplx<double> *, int, cudaStream_t);
+template cudaError_t launch_short<float>(const PhantomDev<float> &, const SeqDev<float> &, StateDev<float> &,
+                                         const SegmentArgs<float> &, cplx<double> *, int, cudaStream_t);
 template cudaError_t launch_partial_finalize<double, double>(const cplx<double> *, int64_t, int64_t, int32_t,
                                                              cplx<double> *, int64_t, cudaStream_t);
 template cudaError_t launch_partial_finalize<float, float>(const cplx<float> *, int64_t, int64_t, int32_t,

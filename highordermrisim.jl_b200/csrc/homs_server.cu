@@ -100,7 +100,8 @@ size_t estimate_bytes(int64_t nspins, int32_t ncoils, homs_dtype dtype, const ho
             }
         }
         const double row = std::ceil(ns / 256.0) * nc * 2 * es;
-        b += std::min(std::max(512.0 * (1 << 20), row * 8.0), row * (double)rf_adc);
+        b += std::max(std::min(std::max(512.0 * (1 << 20), row * 8.0), row * (double)rf_adc),
+                      row * 8.0 / es * std::min<double>((double)nadc, 42.0));  // or of a short segment
         const int64_t spins = std::max<int64_t>(nspins, 1), samples = std::max<int64_t>(nadc, 0);
         const int32_t coils = std::max(ncoils, 1);
         if (es == 8.0)  // spin table, prefix table and partial sums of the precession
