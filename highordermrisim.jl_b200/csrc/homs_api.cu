@@ -69,8 +69,9 @@ struct DevBuf {
         bytes = n;
     }
     size_t owned_bytes() const { return own_bytes_; }
+    bool fits(size_t n) const { return own_ && n <= own_bytes_; }  // ensure(n) would not allocate
     cudaError_t ensure(size_t n) {
-        if (own_ && n <= own_bytes_) {
+        if (fits(n)) {
             alias(own_, own_bytes_);
             return cudaSuccess;
         }
@@ -630,7 +631,7 @@ struct Resident : ResidentBase {
     DevBuf work;
     // Plain FP64 precession: the phantom's spin table and the prefix table of a segment.
     DevBuf spin_table, prefix;
-    bool spin_table_ready = false;
+    bool spin_table_ready = false, spin_table_lent = false;  // lent: a resident phantom's, outside `work`
     // Plain FP32 precession: the block time of every node, the node table of
     // `nodes_method`, a launch round's phases and initial states.
     DevBuf block_time, nodes, walk;
@@ -710,7 +711,7 @@ namespace {
 template <typename T>
 void fill_phantom(homs_context *ctx, Resident<T> *r, const homs_phantom *p) {
     r->split_ready = false;
-    r->spin_table_ready = false;
+    r->spin_table_ready = r->spin_table_lent = false;
     r->dtype = sizeof(T) == 8 ? HOMS_F64 : HOMS_F32;
     r->ns = p->nspins;
     r->nc = p->ncoils;
@@ -744,7 +745,7 @@ void attach_phantom(Resident<T> *r, const Resident<T> &src) {
         HOMS_CUDA(split_attach(r->split, src.split));
         r->split_ready = true;
     }
-    r->spin_table_ready = src.spin_table_ready;
+    r->spin_table_ready = r->spin_table_lent = src.spin_table_ready;
     if (src.spin_table_ready) r->spin_table.view(src.spin_table);
 }
 
@@ -1014,29 +1015,29 @@ void prepare_plain(homs_context *ctx, Resident<T> &r, uint32_t method, const std
             partial = std::max(partial, precess32_cut(r.ns, r.nc, L.nsamples).partial_bytes);
         }
     }
-    bool own_table = true;  // not a resident phantom's
-    if constexpr (sizeof(T) == 8) {
-        const char *t = r.spin_table.template as<char>(), *w = r.work.template as<char>();
-        own_table = !r.spin_table_ready || (t >= w && t < w + r.work.bytes);
-        own_table = own_table && parallel;
-        if (own_table) table = precess64_table_bytes(r.ns);
-    } else if (parallel) {
-        table = precess32_node_bytes(r.nt);
+    const bool own_table = parallel && !(sizeof(T) == 8 && r.spin_table_lent);
+    if (own_table) table = sizeof(T) == 8 ? precess64_table_bytes(r.ns) : precess32_node_bytes(r.nt);
+    const size_t bytes = align(table) + align(per_run) + align(partial);
+    if (!r.work.fits(bytes)) {
+        // Nothing keeps a view of the area that is freed, also when there is none in its place.
+        for (DevBuf *v : {&r.prefix, &r.walk, &r.nodes, &r.partial}) v->release();
+        if (!r.spin_table_lent) {
+            r.spin_table.release();
+            r.spin_table_ready = false;
+        }
+        r.nodes_method = ~0u;
     }
-    const void *before = r.work.p;
-    HOMS_CUDA(r.work.ensure(align(table) + align(per_run) + align(partial)));
+    HOMS_CUDA(r.work.ensure(bytes));
     char *at = r.work.template as<char>();
     if constexpr (sizeof(T) == 8) {
         if (own_table) {
-            const bool stays = r.work.p == before && r.spin_table_ready;
             r.spin_table.view(at, table);
-            if (!stays) build_spin_table(ctx, r);
+            if (!r.spin_table_ready) build_spin_table(ctx, r);
         }
         r.prefix.view(at + align(table), per_run);
-    } else if (parallel) {
-        const bool stays = r.work.p == before && r.nodes_method == method;
+    } else if (own_table) {
         r.nodes.view(at, table);
-        if (!stays) {
+        if (r.nodes_method != method) {
             HOMS_CUDA(precess32_nodes(r.seq(), method, r.block_time.template as<float>(), r.nodes.p, ctx->stream));
             r.nodes_method = method;
         }
