@@ -1169,11 +1169,13 @@ __global__ void spin_params_kernel(const double *T2, const cplx<double> *xy, int
 // time t (entry PREFIX_T) and the constant columns 17 (= 1) and 18, 19 (= 0).
 // A column's intervals are cut into PREFIX_PARTS contiguous parts, and a
 // part into one contiguous run per thread.  Every sum is taken in a fixed
-// order (within a run, runs in thread order, parts in part order), so the
-// table does not depend on timing.  The parts of a column are one cluster and
+// order (within a run, over the runs by a scan, parts in part order), so the
+// table does not depend on timing, and carries its rounding errors along
+// (Sum2): a run cut into many blocks is integrated over all of them, and the
+// plain sum, which restarts at no block, would lose digits against a sum per
+// block.  The parts of a column are one cluster and
 // pass their totals and maxima through distributed shared memory: one launch,
-// 9.5 us for 2,220 intervals, where two (totals, then the scan) took 17; bound by
-// the 256-step chain of the run totals.  With the spin parameters, operands,
+// 9.5 us for 2,220 intervals, where two (totals, then the scan) took 17.  With the spin parameters, operands,
 // accumulators and final state in one launch each, a segment's small kernels
 // take 20 us less: a TR loop of 35 segments (80,000 spins x 2,000 samples x 32
 // coils) 18.5 -> 17.8 ms, a served request (3,721 x 5,000 x 8) 345 -> 329 us.
@@ -1205,26 +1207,49 @@ __device__ __forceinline__ void prefix_run(int64_t nint, int part, int64_t &i0, 
     i1 = min(p1, i0 + per);
 }
 constexpr int PREFIX_THREADS = 256;
-// Sum of the runs' values in thread order (thread 0), and each run's exclusive
-// prefix in part[].
-__device__ void block_exclusive(double *part, double local, double *total) {
-    part[threadIdx.x] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double run = 0.0;
-        for (int i = 0; i < PREFIX_THREADS; i += 16) {
-            double v[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = part[i + k];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                part[i + k] = run;
-                run += v[k];
-            }
-        }
-        *total = run;
+// A sum and the rounding errors of its additions (Knuth's two-sum).  An infinite sum
+// has no error term: value() is the sum itself then.
+struct Sum2 {
+    double s = 0.0, e = 0.0;
+    __device__ __forceinline__ void add(double v, double ve) {
+        const double t = s + v, w = t - s;
+        e += ve + ((s - (t - w)) + (v - w));
+        s = t;
     }
+    __device__ __forceinline__ double value() const {
+        const double v = s + e;
+        return isnan(v) ? s : v;
+    }
+};
+// Each run's exclusive prefix in the block (returned) and the block's total: a scan in
+// the warps, then of their totals, in an order that is fixed.
+__device__ Sum2 block_exclusive(const Sum2 &local, Sum2 *warp_sums, Sum2 *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Sum2 incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        Sum2 before;
+        before.s = __shfl_up_sync(0xffffffffu, incl.s, o);
+        before.e = __shfl_up_sync(0xffffffffu, incl.e, o);
+        if (lane >= o) {
+            before.add(incl.s, incl.e);
+            incl = before;
+        }
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    Sum2 excl;
+    excl.s = __shfl_up_sync(0xffffffffu, incl.s, 1);
+    excl.e = __shfl_up_sync(0xffffffffu, incl.e, 1);
+    if (lane == 0) excl = Sum2{};
     __syncthreads();
+    Sum2 run;
+    for (int i = 0; i < warp; ++i) run.add(warp_sums[i].s, warp_sums[i].e);
+    if (threadIdx.x == PREFIX_THREADS - 1) {
+        *total = run;
+        total->add(incl.s, incl.e);
+    }
+    run.add(excl.s, excl.e);
+    return run;
 }
 
 // zero_word (may be NULL) is set to 0: the segment's amplitude maximum.
@@ -1232,8 +1257,8 @@ __global__ void __cluster_dims__(1, PREFIX_PARTS, 1) __launch_bounds__(PREFIX_TH
     prefix_kernel(const double *dt, const __grid_constant__ SplitColumns src, const uint8_t *adc, const int32_t *rank,
                   int64_t rank_base, int64_t n_lo, int64_t n_hi, int64_t nsamples, double gamma, double *prefix,
                   unsigned long long *zero_word) {
-    __shared__ double part[PREFIX_THREADS], total, largest;
-    __shared__ double warp_peak[PREFIX_THREADS / 32];
+    __shared__ Sum2 warp_sums[PREFIX_THREADS / 32], total;
+    __shared__ double warp_peak[PREFIX_THREADS / 32], largest;
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int col = blockIdx.x, pt = blockIdx.y;
     if (zero_word && col == 0 && pt == 0 && threadIdx.x == 0) *zero_word = 0ull;
@@ -1241,21 +1266,25 @@ __global__ void __cluster_dims__(1, PREFIX_PARTS, 1) __launch_bounds__(PREFIX_TH
     const int64_t nint = n_hi - n_lo;
     int64_t i0, i1;
     prefix_run(nint, pt, i0, i1);
-    double local = 0.0;
-    for (int64_t i = i0; i < i1; ++i) local += prefix_term(c, dt, n_lo + i);
-    block_exclusive(part, local, &total);
+    Sum2 local;
+    for (int64_t i = i0; i < i1; ++i) local.add(prefix_term(c, dt, n_lo + i), 0.0);
+    const Sum2 before = block_exclusive(local, warp_sums, &total);
     cluster.sync();
-    double carry = 0.0;
-    for (int q = 0; q < pt; ++q) carry += *cluster.map_shared_rank(&total, q);
-    double cum = carry + part[threadIdx.x];
+    Sum2 cum;
+    for (int q = 0; q < pt; ++q) {
+        const Sum2 *t = cluster.map_shared_rank(&total, q);
+        cum.add(t->s, t->e);
+    }
+    cum.add(before.s, before.e);
     double peak = 0.0;
     for (int64_t i = i0; i < i1; ++i) {
         const int64_t n = n_lo + i;
-        cum += prefix_term(c, dt, n);
-        peak = fmax(peak, fabs(c.scale * cum));
+        cum.add(prefix_term(c, dt, n), 0.0);
+        const double kappa = c.scale * cum.value();
+        peak = fmax(peak, fabs(kappa));
         if (adc[n + 1]) {
             double *pr = prefix + (size_t)(rank[n + 1] - rank_base) * PREFIX_STRIDE;
-            pr[c.out_col] = c.scale * cum;
+            pr[c.out_col] = kappa;
             if (col == 17) {
                 pr[17] = 1.0;
                 pr[18] = 0.0;
@@ -1264,7 +1293,7 @@ __global__ void __cluster_dims__(1, PREFIX_PARTS, 1) __launch_bounds__(PREFIX_TH
         }
         if (n + 1 == n_hi) {
             double *pr = prefix + (size_t)nsamples * PREFIX_STRIDE;
-            pr[c.out_col] = c.scale * cum;
+            pr[c.out_col] = kappa;
             if (col == 17) {
                 pr[17] = 1.0;
                 pr[18] = 0.0;

@@ -116,3 +116,39 @@ def test_block_call_with_state_off_16_bytes(oracle, gpu_context):
     assert nrmse(raw[1:].cpu().numpy().view(np.complex128), ref[1]) <= BAR
     assert nrmse(z.cpu().numpy(), ref[2]) <= BAR
     assert float(raw[0]) == 0.0 and torch.all(sig[:, 20:] == 0)
+
+
+@pytest.mark.parametrize("block", [10**9, 100, 1])
+def test_phase_of_long_runs_in_blocks(gpu_context, block):
+    """10,000 nodes of a 30 mT/m readout, whole or cut into blocks, against extended
+    precision.  The phase is a sum of 16 terms of at most 256 turns: some 22 roundings
+    (products, kappas) of half an ulp of 2^-45 turns each, adding as their root sum of
+    squares, 2 pi sqrt(22) 2^-46 = 4.2e-13 rad; a rounding running sum of kappa adds 5e-13."""
+    ld, rng, ns, n = np.longdouble, np.random.default_rng(0), 60, 10000
+    pos = rng.uniform(-0.1, 0.1, (3, ns))
+    T2, dw = rng.uniform(0.03, 0.2, ns), rng.uniform(-2000.0, 2000.0, ns)
+    csm = rng.standard_normal((ns, 3)) + 1j * rng.standard_normal((ns, 3))
+    obj = homs.HO_Phantom(x=pos[0], y=pos[1], z=pos[2], rho=np.ones(ns), T1=10 * T2, T2=T2, dw=dw, csm=csm)
+    dt = np.full(n, 1e-6)
+    t = np.concatenate([[0.0], np.cumsum(dt)])
+    h = np.zeros((16, n + 1))
+    for k in (1, 2, 3):
+        h[k] = 30e-3 * np.sin(2 * np.pi * (300 + 100 * k) * t + k)
+    adc = np.arange(n + 1) > 0
+    seq = homs.HO_DiscreteSequence(t, dt=dt, gx=h[1], gy=h[2], gz=h[3], b1=np.zeros(n + 1, complex), adc=adc,
+                                   excitation=np.zeros(n, bool), h=h)
+    parts, exc = homs.get_sim_ranges(seq, block)
+    st = homs.Mag(np.full(ns, 0.6 + 0.3j), np.full(ns, 0.7))
+    sig, xy, _ = homs.run_blocks(obj, seq, parts, exc, BlochHighOrder("1111"), "f64", "plain", st)
+    two_pi = ld(2) * ld("3.14159265358979323846264338327950288")
+    g = h[1:4].astype(ld)
+    moment = np.cumsum(ld(0.5) * (g[:, :-1] + g[:, 1:]) * dt.astype(ld), axis=1)
+    elapsed = np.cumsum(dt.astype(ld))[:, None]
+    turns = -ld(GAMMA) * (moment.T @ pos.astype(ld)) - elapsed * (dw.astype(ld) / two_pi)
+    phase, e = two_pi * (turns - np.rint(turns)), np.exp(-elapsed / T2.astype(ld))
+    re = e * (ld(0.6) * np.cos(phase) - ld(0.3) * np.sin(phase))
+    im = e * (ld(0.6) * np.sin(phase) + ld(0.3) * np.cos(phase))
+    cr, ci = csm.real.astype(ld), csm.imag.astype(ld)
+    for got, want in ((sig, ((re @ cr - im @ ci), (re @ ci + im @ cr))), (xy, (re[-1], im[-1]))):
+        d = (got.real - want[0]) ** 2 + (got.imag - want[1]) ** 2
+        assert float(np.sqrt(d.sum() / (want[0] ** 2 + want[1] ** 2).sum())) <= 4.2e-13
