@@ -114,3 +114,15 @@ def test_signal_does_not_depend_on_earlier_calls(homs_lib):
             homs.run_blocks(other, oseq, [(0, 16)], [False], method, "f32", "plain", ost, ctx)
             found.append(signal())
     assert all(np.array_equal(f, found[0]) for f in found)
+
+
+@pytest.mark.parametrize("nsteps,block", [(281, 1), (290, 2), (1100, 419), (1100, 400)])
+def test_rounds_cut_at_blocks(gpu_context, nsteps, block):
+    """120,000 spins: rounds of at most 69 blocks (the last of few nodes), a round whose
+    samples (838) end with a block, and one that ends inside a later block."""
+    obj, seq, st = W.high_order_workload(nspins=120000, nsteps=nsteps, ncoils=2)
+    parts, exc = homs.get_sim_ranges(seq, block)
+    method = BlochHighOrder("1111")
+    want = _run(obj, seq, parts, exc, method, st, "f64")
+    got = _run(obj, seq, parts, exc, method, st)
+    assert all(nrmse(g, r) <= BAR for g, r in zip(got, want))
