@@ -798,7 +798,7 @@ void fill_sequence(homs_context *ctx, Resident<T> *r, const homs_sequence *q) {
     }
     HOMS_CUDA(r->xy.ensure(sizeof(cplx<T>) * (size_t)ns));
     HOMS_CUDA(r->mz.ensure(sizeof(T) * (size_t)ns));
-    HOMS_CUDA(r->acc.ensure(sizeof(T) * (size_t)ns));
+    if (sizeof(T) == 4) HOMS_CUDA(r->acc.ensure(sizeof(T) * (size_t)ns));  // FP32 precession's running phase sums
     HOMS_CUDA(r->sig.ensure(sizeof(cplx<T>) * (size_t)std::max<int64_t>(nadc * r->nc, 1)));
 }
 
@@ -1081,7 +1081,7 @@ void init_state(homs_context *ctx, Resident<T> &r, const homs_state *state, homs
         HOMS_CUDA(cudaMemsetAsync(r.xy.p, 0, sizeof(cplx<T>) * (size_t)r.ns, ctx->stream));
         HOMS_CUDA(cudaMemcpyAsync(r.mz.p, r.rho.p, sizeof(T) * (size_t)r.ns, cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    HOMS_CUDA(cudaMemsetAsync(r.acc.p, 0, sizeof(T) * (size_t)r.ns, ctx->stream));
+    if (sizeof(T) == 4) HOMS_CUDA(cudaMemsetAsync(r.acc.p, 0, sizeof(T) * (size_t)r.ns, ctx->stream));
 }
 
 // Build the split path's phantom operands (basis table, pre-split
@@ -1173,7 +1173,6 @@ struct SplitRunner {
         sa.csm_rows = res.csm_rows.p;
         sa.xy = res.xy.p;
         sa.mz = res.mz.p;
-        sa.acc = res.acc.p;
         sa.sig = res.sig.p;
         sa.launches = &res.launches;
         // RF runs use the plain FP64 excitation kernel; precession runs are
@@ -1887,7 +1886,7 @@ homs_status block_impl(homs_context *ctx, bool rf, const homs_phantom *p, const 
             block_precess32(ctx, pd, qd, *state, first, last, method, q->gamma, adc, nadc, sig, ldsig);
         return HOMS_OK;
     }
-    HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
+    if (!rf) HOMS_CUDA(ctx->scratch_acc.ensure(sizeof(T) * (size_t)ns));
     const int grid = (int)((ns + PLAIN_THREADS - 1) / PLAIN_THREADS);
     const size_t samples = (size_t)std::max<int64_t>(nadc, 1) * nc;
     HOMS_CUDA(ctx->scratch_partial.ensure((rf ? sizeof(cplx<T>) : sizeof(cplx<double>)) * (size_t)grid * samples));

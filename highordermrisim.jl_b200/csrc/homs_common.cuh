@@ -45,7 +45,7 @@ template <typename T>
 struct StateDev {
     cplx<T> *xy;
     T *z;
-    T *acc;  // running trapezoid sum of the current precession block
+    T *acc;  // FP32 precession: running trapezoid sum of the current block (else unused)
 };
 
 // One launch of the excitation kernel, or of the kernel of short precession

@@ -401,7 +401,7 @@ __host__ __device__ constexpr int coil_smem(int nt, int tile) {
 constexpr float SMALL_DECAY = 0.0625f;  // |dt / T2| up to which the decay series below is used
 
 struct CoilArgs {
-    int64_t ns, ns_pad, nsamples, sample0, round_samples, nchunks;
+    int64_t ns, ns_pad, sample0, round_samples, nchunks;
     int32_t nc, parts;
     const float *T2;
     const cplx<float> *csm_rows;
@@ -738,7 +738,6 @@ cudaError_t precess32_run(const Precess32Args &a, const CoilCut &cut, cudaEvent_
             CoilArgs ca;
             ca.ns = ns;
             ca.ns_pad = w.ns_pad;
-            ca.nsamples = a.nsamples;
             ca.sample0 = t0 * tile;
             ca.round_samples = std::min<int64_t>(nt * tile, a.nsamples - ca.sample0);
             ca.nchunks = w.ns_pad / CHUNK;

@@ -113,7 +113,7 @@ __global__ void table_kernel(const double *x, const double *y, const double *z, 
 }
 
 struct KernelArgs {
-    int64_t ns, nsamples, sample0, nchunks;  // samples sample0 + [0, tiles of the round)
+    int64_t ns, sample0, nchunks;  // samples sample0 + [0, tiles of the round)
     int64_t round_samples;                   // samples of the round (rows of a partial block)
     int32_t nc, parts;
     uint32_t slots;
@@ -438,7 +438,6 @@ cudaError_t precess64_run(const Precess64Args &a, const CoilCut &cut, cudaEvent_
             const int64_t nt = std::min(cut.round_tiles, tiles - t0);
             KernelArgs ka;
             ka.ns = a.ns;
-            ka.nsamples = a.nsamples;
             ka.sample0 = t0 * tile;
             ka.round_samples = std::min<int64_t>(nt * tile, a.nsamples - ka.sample0);
             ka.nchunks = np / CHUNK;

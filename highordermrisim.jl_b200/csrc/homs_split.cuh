@@ -84,7 +84,7 @@ struct SplitRunArgs {
     // resident device arrays (type T = double or float per sizeof_T)
     const void *t, *dt, *gx, *gy, *gz, *b1, *df, *psi, *adc, *bnd, *h[16];
     const void *x, *y, *z, *rho, *T1, *T2, *dw, *csm_rows;
-    void *xy, *mz, *acc, *sig;
+    void *xy, *mz, *sig;
     // instrumentation (optional): events bracketing the fused kernel launch and
     // a counter of kernels launched
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
