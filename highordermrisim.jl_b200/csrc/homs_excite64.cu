@@ -35,16 +35,6 @@ constexpr int THREADS = 64;
 constexpr int NODES = 64;  // nodes per stage
 constexpr int UNROLL = 4;  // rotations formed together (2, 3, 4, 6: 15.78, 15.76, 15.65, 15.87 ms for the TR loop)
 
-// 1/sqrt(x) from the hardware's approximation (2^-20 or better) by one Householder
-// step of third order; 0 for x below 1e-300 (no field), NaN for NaN.
-__device__ __forceinline__ double rsq(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    y = fma(y * e, fma(0.375, e, 0.5), y);
-    return x < 1e-300 ? 0.0 : y;
-}
-
 // sqrt(2) cos(h) and sqrt(2) sin(h) / h from z = h^2: interpolants at the
 // Chebyshev nodes of [0, 1/32] (degree 4) and [0, 5/8] (degree 7), within 1.3e-16
 // with their rounded coefficients.
@@ -82,7 +72,7 @@ __device__ __forceinline__ void half_mid(double z, double &c, double &s) {
 // Any z (infinities and NaN included).
 __device__ __forceinline__ void half_far(double z, double &c, double &s) {
     constexpr double SQRT2 = 1.4142135623730951;
-    const double r = rsq(z), h = z * r;
+    const double r = z < 1e-300 ? 0.0 : rsqrt(z), h = z * r;  // no field: no rotation
     cis_turns(h * (0.5 / 3.141592653589793), c, s);
     c *= SQRT2;
     s *= SQRT2 * r;
