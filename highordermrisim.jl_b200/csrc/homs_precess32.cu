@@ -642,13 +642,14 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 3 : 2) coil_kernel(const Co
 
 template <int ORD>
 cudaError_t launch_walk(const WalkArgs &a, cudaStream_t stream) {
-    // Small phantoms: 8 lanes per spin; else one, in CTAs of one warp until
-    // these give every scheduler several (an even spread over the SMs).
+    // Small phantoms: 8 lanes per spin; else one.  Prepared runs of 4 segments of 512
+    // (2,048) samples x 8 coils, one lane and eight: 12,000 spins 0.41 and 0.41 ms (1.16
+    // and 1.04), 16,000 0.42 and 0.45 (1.23 and 1.20), 20,000 0.48 and 0.54 (1.43 and
+    // 1.51).  One lane in CTAs of 32, 64 and 128 threads, 75,000 x 2,048: 3.31, 3.27, 3.25.
     if (a.p.ns <= SMALL_NS) {
         walk_kernel<ORD, 8><<<(unsigned)((a.p.ns * 8 + 127) / 128), 128, 0, stream>>>(a);
     } else {
-        const int threads = a.p.ns <= 148 * 4 * 4 * 32 ? 32 : 128;
-        walk_kernel<ORD, 1><<<(unsigned)((a.p.ns + threads - 1) / threads), threads, 0, stream>>>(a);
+        walk_kernel<ORD, 1><<<(unsigned)((a.p.ns + 127) / 128), 128, 0, stream>>>(a);
     }
     return cudaGetLastError();
 }
@@ -701,8 +702,11 @@ size_t precess32_run_bytes(int64_t ns, int32_t nc, int64_t nnodes, int64_t nadc,
 }
 CoilCut precess32_cut(int64_t ns, int32_t nc, int64_t nsamples) {
     // Three CTAs per SM for up to 8 coils, unless these only add partial sums to read:
-    // with one tile a part is a few chunks already (48 repetitions of 128 samples:
-    // 3.87 ms with two per SM, 3.98 with three).
+    // with few tiles a part is a few chunks already.  Two per SM and three, 4 segments
+    // x 8 coils: 30,000 spins x 256 samples 0.358 and 0.361 ms, x 512 0.544 and 0.545,
+    // x 768 0.757 and 0.744, x 2,048 1.73 and 1.68; 75,000 x 128 0.353 and 0.356, x 2,048
+    // 3.42 and 3.26; below 12,000 spins within 2% of one another (48 repetitions of 128
+    // samples: 3.87 and 3.98 ms).
     const int64_t places = coil_tiles(nc) == 1 && nsamples > 6 * 128 ? 148 * 3 : 148 * 2;
     return coil_cut(pad_spins(ns) / CHUNK, nc, nsamples, PARTIAL_BUDGET, places);
 }
