@@ -114,3 +114,40 @@ def test_block_calls(oracle, gpu_context, precision, nspins, ncoils, first, last
     assert nrmse(got[:, :n].T, ref[0]) <= BAR[precision] and np.all(got[:, n:] == 0)
     assert nrmse(raw[1:].cpu().numpy().view(c), ref[1]) <= BAR[precision] and float(raw[0]) == 0
     assert nrmse(z.cpu().numpy(), ref[2]) <= BAR[precision]
+
+
+def test_full_size_readout_in_short_blocks(gpu_context):
+    """350,000 spins x 2,000 samples x 32 coils: the parallel FP64 kernel and the split
+    kernel, which both read the prefix table, against the sequential kernel, which does
+    not: 500 block calls of 4 nodes, each from the state that the one before left."""
+    import torch
+    w = W.config(2)
+    obj, seq, method = w.obj, w.seq, BlochHighOrder(w.mask)
+    first = next(f for (f, l), rf in zip(w.parts, w.excitation) if not rf and seq.adc[f + 1:l + 1].sum() > 2000)
+    first += int(np.flatnonzero(seq.adc[first + 1:])[0])
+    last = first + 2000
+    assert seq.adc[first + 1:last + 1].all()
+    rng = np.random.default_rng(6)
+    st = homs.Mag(obj.rho * np.exp(2j * np.pi * rng.uniform(size=len(obj))), 0.5 * obj.rho)
+    D = lambda a, t=np.float64: torch.as_tensor(np.ascontiguousarray(np.asarray(a).astype(t)), device="cuda")  # noqa: E731
+    keep = [D(v) for v in (obj.x, obj.y, obj.z, obj.rho, obj.T1, obj.T2, obj.dw)] + [D(obj.csm.T, np.complex128)]
+    ph = _lib.Phantom(len(obj), obj.ncoils, _lib.HOMS_F64, _lib.HOMS_DEVICE, *[k.data_ptr() for k in keep])
+    node = [D(v) for v in (seq.t, seq.dt, seq.gx, seq.gy, seq.gz)] + [
+        D(seq.b1, np.complex128), D(seq.df), D(seq.psi), D(seq.adc, np.uint8)]
+    h = D(seq.h)
+    hp = (ctypes.c_void_p * 16)(*[h[k].data_ptr() for k in range(16)])
+    sq = _lib.Sequence(len(seq.t), _lib.HOMS_F64, _lib.HOMS_DEVICE, *[v.data_ptr() for v in node], hp, 0, None, None, None,
+                       GAMMA)
+    xy, z = D(st.xy, np.complex128), D(st.z)
+    state = _lib.State(xy.data_ptr(), z.data_ptr(), _lib.HOMS_DEVICE)
+    sig = torch.zeros(obj.ncoils, 2000, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    for k in range(0, 2000, 4):
+        _lib.check(_lib.load().homs_precession_block(
+            gpu_context.handle, ctypes.byref(ph), ctypes.byref(sq), first + k, first + k + 4, method.flags,
+            ctypes.byref(state), sig[:, k:].data_ptr(), 2000), gpu_context.handle)
+    torch.cuda.synchronize()
+    want = sig.cpu().numpy().T, xy.cpu().numpy(), z.cpu().numpy()
+    for mode, bars in (("plain", (1e-12, 1e-12, 1e-12)), ("split", (1e-6, 1e-12, 1e-12))):
+        got = homs.run_blocks(obj, seq, [(first, last)], [False], method, "f64", mode, st)
+        assert all(nrmse(g, r) <= bar for g, r, bar in zip(got, want, bars)), mode
