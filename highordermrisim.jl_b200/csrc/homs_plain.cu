@@ -1,8 +1,8 @@
-// RF excitation in the phantom's own precision (FP64 or FP32) on CUDA cores,
-// fused with a deterministic multi-coil reduction of the samples acquired during
-// the pulse, and the standalone coil reduction.  No per-spin ADC history is
-// written to HBM: ADC states are staged in shared memory and contracted with
-// the receive sensitivities on chip, one CTA partial per (CTA, sample, coil),
+// RF excitation and short precession segments in the phantom's own precision (FP64
+// or FP32) on CUDA cores, fused with a deterministic multi-coil reduction of the
+// samples acquired meanwhile, and the standalone coil reduction.  No per-spin ADC
+// history is written to HBM: ADC states are staged in shared memory and contracted
+// with the receive sensitivities on chip, one CTA partial per (CTA, sample, coil),
 // then summed over CTAs in a fixed order.
 //
 // This translation unit is compiled with -fmad=false so that every product

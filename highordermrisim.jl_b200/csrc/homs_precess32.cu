@@ -29,7 +29,11 @@
 // instructions (homs_precess64.cu has the fragment layouts and the three-product
 // complex form), which leaves the FP32 pipe to the magnetisation and sums the
 // FP32 products without rounding them.  Phases cross
-// through memory, 4 bytes per spin and sample each way.
+// through memory, 4 bytes per spin and sample each way.  A tile of one block takes
+// the packed functions; tiles across blocks (a small max_block_length) take expf,
+// sincosf and the initial state of each sample's own block: 40,000 spins x 4,000
+// samples x 8 coils whole 1.24 ms, in blocks of 16, 4 and 1 nodes 1.36, 1.80 and 3.19
+// (the sequential kernel 3.37 to 3.65).
 //
 // Measured (B200, against the single kernel): one-shot calls, 4,096 spins x
 // 2,048 samples x 1 coil 1,754 -> 285 us, 40,000 spins x 4 x 10,000 samples x 8

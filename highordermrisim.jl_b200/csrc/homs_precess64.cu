@@ -42,7 +42,7 @@
 //
 // Measured (B200, prepared runs, against the sequential per-spin kernel that it
 // replaces): 40,000 spins x 4 segments of 10,000 samples x 8 coils 44.6 ->
-// 8.2 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.3 ms.  Three
+// 8.2 ms, 11,979 spins x 4 x 9,500 samples x 32 coils 48.9 -> 5.2 ms.  Three
 // CTAs per SM (80 registers) run the 8-coil case no faster (10.5 ms).
 #include <algorithm>
 
