@@ -1992,21 +1992,17 @@ homs_status homs_coil_reduce(homs_context *ctx, homs_dtype dtype, int64_t nspins
         }
         HOMS_REQUIRE((nadc + PLAIN_STAGE - 1) / PLAIN_STAGE <= 65535,
                      "nadc above 524280 samples per call (the reduction's grid)");
-        const int64_t parts = coil_reduce_parts(nspins, nadc, ncoils);
-        HOMS_CUDA(ctx->scratch_partial.ensure(es * (size_t)parts * (size_t)nadc * (size_t)ncoils));
-        if (dtype == HOMS_F64) {
-            HOMS_CUDA(launch_coil_reduce<double>(nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
-                                                 (const cplx<double> *)csm, ldcsm, reinterpret_cast<cplx<double> *>(ctx->scratch_partial.p),
+        const CoilReduceCut cut = coil_reduce_cut(nspins, nadc, ncoils, dtype == HOMS_F64);
+        HOMS_CUDA(ctx->scratch_partial.ensure(cut.partial_bytes(nadc, ncoils)));
+        void *sums = ctx->scratch_partial.p;
+        if (dtype == HOMS_F64)
+            HOMS_CUDA(launch_coil_reduce<double>(cut, nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
+                                                 (const cplx<double> *)csm, ldcsm, sums, (cplx<double> *)sig, ldsig,
                                                  ctx->stream));
-            HOMS_CUDA(launch_partial_finalize(reinterpret_cast<cplx<double> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
-                                                      (cplx<double> *)sig, ldsig, ctx->stream));
-        } else {
-            HOMS_CUDA(launch_coil_reduce<float>(nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
-                                                (const cplx<float> *)csm, ldcsm, reinterpret_cast<cplx<float> *>(ctx->scratch_partial.p),
+        else
+            HOMS_CUDA(launch_coil_reduce<float>(cut, nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
+                                                (const cplx<float> *)csm, ldcsm, sums, (cplx<float> *)sig, ldsig,
                                                 ctx->stream));
-            HOMS_CUDA(launch_partial_finalize(reinterpret_cast<cplx<float> *>(ctx->scratch_partial.p), parts, nadc, ncoils,
-                                                     (cplx<float> *)sig, ldsig, ctx->stream));
-        }
         return HOMS_OK;
     } catch (const Failure &f) {
         return fail(ctx, f);

@@ -90,14 +90,25 @@ template <typename P, typename S>
 cudaError_t launch_partial_finalize(const cplx<P> *partial, int64_t nparts, int64_t nsamples, int32_t nc,
                                     cplx<S> *sig, int64_t ldsig, cudaStream_t stream);
 
-// Standalone coil reduction, split-K over spin ranges: coil_reduce_parts()
-// partial (nadc x nc) blocks, at most ceil(ns / PLAIN_THREADS) of them, which
-// launch_partial_finalize sums in part order.
-int64_t coil_reduce_parts(int64_t ns, int64_t nadc, int32_t nc);
+// Standalone coil reduction, split-K over spin ranges: `parts` partial (nadc x nc)
+// blocks, at most ceil(ns / PLAIN_THREADS) of the operands' type, or more of them in
+// FP64 (`wide`; also always for FP64 operands) within CR_PARTIAL_BYTES, then summed in
+// part order into sig.
+constexpr int64_t CR_PARTIAL_BYTES = int64_t(16) << 20;
+struct CoilReduceCut {
+    int64_t parts;
+    bool wide;
+    size_t partial_bytes(int64_t nadc, int32_t nc) const { return (wide ? 16 : 8) * (size_t)parts * (size_t)nadc * nc; }
+};
+CoilReduceCut coil_reduce_cut(int64_t ns, int64_t nadc, int32_t nc, bool f64);
 
 template <typename T>
-cudaError_t launch_coil_reduce(int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
-                               const cplx<T> *csm, int64_t ldcsm, cplx<T> *partial, cudaStream_t stream);
+cudaError_t launch_coil_reduce(const CoilReduceCut &cut, int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states,
+                               int64_t ldstates, const cplx<T> *csm, int64_t ldcsm, void *partial, cplx<T> *sig,
+                               int64_t ldsig, cudaStream_t stream);
+
+// Load the reduction's kernels on the current device: its later launches allocate nothing.
+cudaError_t load_coil_reduce();
 
 template <typename T>
 size_t segment_smem_bytes(int32_t nc);

@@ -24,10 +24,11 @@ void *g_scratch_ptr[kMaxDevices];  // device address of g_reduce_scratch, per de
 
 // Device address of the scratch array on the current device.  Host code only
 // sees a host-side stand-in for the array's name, so the address is resolved
-// with cudaGetSymbolAddress once per device, with that device current.  That
-// first resolution may make the CUDA driver load this library's device code
-// and back the array (an allocation of the driver's own, which can
-// synchronise the device); later calls only read the cached address.  The
+// with cudaGetSymbolAddress once per device, with that device current, and the
+// reduction's kernels are loaded.  That first resolution may make the CUDA driver
+// load this library's device code and back the array (an allocation of the
+// driver's own, which can synchronise the device); later calls only read the
+// cached address, and launch kernels that are there.  The
 // cache is per device ordinal: after a cudaDeviceReset the address would be
 // stale, so a device reset is not supported while the library is in use.
 homs_status scratch_for_current_device(void **out) {
@@ -36,7 +37,7 @@ homs_status scratch_for_current_device(void **out) {
     std::lock_guard<std::mutex> lock(g_scratch_mu);
     if (!g_scratch_ptr[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_reduce_scratch) != cudaSuccess || !p) {
+        if (cudaGetSymbolAddress(&p, g_reduce_scratch) != cudaSuccess || !p || homs::load_coil_reduce() != cudaSuccess) {
             cudaGetLastError();
             return HOMS_ECUDA;
         }
@@ -76,21 +77,16 @@ extern "C" homs_status homs_coil_reduce_noalloc(void *stream, homs_dtype dtype, 
     const double need = (double)es * (double)tiles * (double)nadc * (double)ncoils;
     if (need > (double)kScratchBytes) return HOMS_EINVAL;
     if ((nadc + homs::PLAIN_STAGE - 1) / homs::PLAIN_STAGE > 65535) return HOMS_EINVAL;  // grid.y of the reduce step
-    // The reduce step writes coil_reduce_parts() <= tiles partial blocks, so they fit.
-    const int64_t parts = homs::coil_reduce_parts(nspins, nadc, ncoils);
+    // The reduce step writes at most `tiles` blocks of the operands' type, or more of
+    // them in FP64 within the array: they fit.
+    static_assert(homs::CR_PARTIAL_BYTES <= (int64_t)kScratchBytes);
+    const homs::CoilReduceCut cut = homs::coil_reduce_cut(nspins, nadc, ncoils, dtype == HOMS_F64);
     cudaError_t e;
-    if (dtype == HOMS_F64) {
-        e = homs::launch_coil_reduce<double>(nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
-                                             (const cplx<double> *)csm, ldcsm, (cplx<double> *)scratch, st);
-        if (e == cudaSuccess)
-            e = homs::launch_partial_finalize((const cplx<double> *)scratch, parts, nadc, ncoils,
-                                                      (cplx<double> *)sig, ldsig, st);
-    } else {
-        e = homs::launch_coil_reduce<float>(nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
-                                            (const cplx<float> *)csm, ldcsm, (cplx<float> *)scratch, st);
-        if (e == cudaSuccess)
-            e = homs::launch_partial_finalize((const cplx<float> *)scratch, parts, nadc, ncoils,
-                                                     (cplx<float> *)sig, ldsig, st);
-    }
+    if (dtype == HOMS_F64)
+        e = homs::launch_coil_reduce<double>(cut, nspins, nadc, ncoils, (const cplx<double> *)states, ldstates,
+                                             (const cplx<double> *)csm, ldcsm, scratch, (cplx<double> *)sig, ldsig, st);
+    else
+        e = homs::launch_coil_reduce<float>(cut, nspins, nadc, ncoils, (const cplx<float> *)states, ldstates,
+                                            (const cplx<float> *)csm, ldcsm, scratch, (cplx<float> *)sig, ldsig, st);
     return e == cudaSuccess ? HOMS_OK : HOMS_ECUDA;
 }

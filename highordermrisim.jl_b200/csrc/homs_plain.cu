@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(FIN_OUT *FIN_SLICES)
 // against register-blocked multiply-adds from shared memory, which spent their
 // issue slots on loads): 200,000 x 64 x 32 FP64 200 -> 138 us, FP32 121 -> 111;
 // 200,000 x 64 x 8 FP64 188 -> 59; 200,000 x 96 x 1 FP32 205 -> 80; 30,011 x 33 x 31
-// FP64 47 -> 35; 5,000 x 17 x 3 FP64 41 -> 13.  Chunks of 16 spins in 3 stages: 142 us
+// FP64 47 -> 35; 5,000 x 17 x 3 FP64 41 -> 10.  Chunks of 16 spins in 3 stages: 142 us
 // for the first; 32 in 3, which leaves one CTA per SM: 171.
 constexpr int CR_SK = 32, CR_THREADS = 256, CR_CTAS_PER_SM = 2, CR_STAGES = 2;
 // Bytes of a staged row (CR_SK spins and a pad that keeps fragment loads conflict-free).
@@ -505,10 +505,11 @@ template <typename T>
 constexpr int cr_stage(int nt, int wj) {
     return 8 * (nt + wj) * cr_row<T>();
 }
-template <typename T, int NT, int WJ>
+// P: type of the partial sums.
+template <typename T, typename P, int NT, int WJ>
 __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
     coil_reduce_kernel(int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
-                       const cplx<T> *csm, int64_t ldcsm, int64_t parts, int width, cplx<T> *partial) {
+                       const cplx<T> *csm, int64_t ldcsm, int64_t parts, int width, cplx<P> *partial) {
     using Pair = std::conditional_t<sizeof(T) == 8, double2, float2>;
     constexpr int ROW = cr_row<T>(), STAGE = cr_stage<T>(NT, WJ), KS = 8 / WJ, JB = 8 * WJ, CB = 8 * NT;
     extern __shared__ __align__(16) uint8_t cr_smem[];
@@ -651,13 +652,13 @@ __global__ void __launch_bounds__(CR_THREADS, CR_CTAS_PER_SM)
     }
     const int j = 8 * wj + r;
     if (j < jn) {
-        cplx<T> *out = partial + (p * nadc + j0 + j) * nc + c0;
+        cplx<P> *out = partial + (p * nadc + j0 + j) * nc + c0;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int c = 8 * nt + 2 * q + e;
-                if (c < cn) out[c] = cplx<T>{(T)re[nt][e], (T)im[nt][e]};
+                if (c < cn) out[c] = cplx<P>{(P)re[nt][e], (P)im[nt][e]};
             }
     }
 }
@@ -730,33 +731,37 @@ cudaError_t launch_partial_finalize(const cplx<T> *partial, int64_t nparts, int6
 static int cr_coil_tiles(int32_t nc) { return nc <= 8 ? 1 : nc <= 16 ? 2 : 4; }
 static int cr_sample_warps(int64_t nadc) { return nadc <= 16 ? 2 : nadc <= 32 ? 4 : 8; }
 
-// Parts of the split-K: one wave of CR_CTAS_PER_SM CTAs per SM over all
-// (sample, coil) tiles, at least 256 spins per part (so at most
-// ceil(ns / PLAIN_THREADS) parts).
-int64_t coil_reduce_parts(int64_t ns, int64_t nadc, int32_t nc) {
+// Parts of the split-K: one wave of CR_CTAS_PER_SM CTAs per SM over all (sample, coil)
+// tiles, 256 spins per part at least; more parts, of two chunks at least and with
+// FP64 partial sums within CR_PARTIAL_BYTES, where that leaves SMs idle: up to the wave
+// for the larger tiles, else one CTA per SM (more only add partial sums to read).
+// Before, and so (per call, back to back): 8,001 spins x 64 x 32, an odd leading
+// dimension, FP32 37 and 19 us, FP64 38 and 19; 4,000 x 48 x 8 FP64 20 and 11.
+CoilReduceCut coil_reduce_cut(int64_t ns, int64_t nadc, int32_t nc, bool f64) {
     const int jb = 8 * cr_sample_warps(nadc), cb = 8 * cr_coil_tiles(nc);
-    const int64_t tiles = ((nadc + jb - 1) / jb) * ((nc + cb - 1) / cb);
-    const int64_t want = std::max<int64_t>(1, (148 * CR_CTAS_PER_SM) / tiles);
-    return std::max<int64_t>(1, std::min<int64_t>(want, (ns + PLAIN_THREADS - 1) / PLAIN_THREADS));
+    const int64_t tiles = ((nadc + jb - 1) / jb) * ((nc + cb - 1) / cb), wave = 148 * CR_CTAS_PER_SM / tiles;
+    const int64_t few = std::max<int64_t>(1, std::min(wave, (ns + PLAIN_THREADS - 1) / PLAIN_THREADS));
+    const int64_t more = std::min({jb * cb >= 1024 ? wave : 148 / tiles, CR_PARTIAL_BYTES / (16 * nadc * nc),
+                                   (ns + 2 * CR_SK - 1) / (2 * CR_SK)});
+    return more > few ? CoilReduceCut{more, true} : CoilReduceCut{few, f64};
 }
 
-template <typename T, int NT, int WJ>
+template <typename T, typename P, int NT, int WJ>
 static cudaError_t cr_launch(dim3 grid, int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
-                             const cplx<T> *csm, int64_t ldcsm, int width, cplx<T> *partial, cudaStream_t stream) {
+                             const cplx<T> *csm, int64_t ldcsm, int width, cplx<P> *partial, cudaStream_t stream) {
     const size_t smem = std::max<size_t>(CR_STAGES * cr_stage<T>(NT, WJ), sizeof(double) * 128 * NT * (8 - WJ));
-    cudaError_t e = allow_max_dynamic_smem((const void *)coil_reduce_kernel<T, NT, WJ>);
+    cudaError_t e = allow_max_dynamic_smem((const void *)coil_reduce_kernel<T, P, NT, WJ>);
     if (e != cudaSuccess) return e;
-    coil_reduce_kernel<T, NT, WJ><<<grid, CR_THREADS, smem, stream>>>(ns, nadc, nc, states, ldstates, csm, ldcsm,
-                                                                      (int64_t)grid.x, width, partial);
+    coil_reduce_kernel<T, P, NT, WJ><<<grid, CR_THREADS, smem, stream>>>(ns, nadc, nc, states, ldstates, csm, ldcsm,
+                                                                         (int64_t)grid.x, width, partial);
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_coil_reduce(int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
-                               const cplx<T> *csm, int64_t ldcsm, cplx<T> *partial, cudaStream_t stream) {
-    if (ns == 0 || nadc == 0 || nc == 0) return cudaSuccess;
+template <typename T, typename P>
+static cudaError_t cr_run(int64_t parts, int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states, int64_t ldstates,
+                          const cplx<T> *csm, int64_t ldcsm, cplx<P> *partial, cplx<T> *sig, int64_t ldsig,
+                          cudaStream_t stream) {
     const int nt = cr_coil_tiles(nc), wj = cr_sample_warps(nadc);
-    const int64_t parts = coil_reduce_parts(ns, nadc, nc);
     const int64_t jt = (nadc + 8 * wj - 1) / (8 * wj), ct = (nc + 8 * nt - 1) / (8 * nt);
     if (jt > 65535 || ct > 65535) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)parts, (unsigned)jt, (unsigned)ct);
@@ -764,14 +769,53 @@ cudaError_t launch_coil_reduce(int64_t ns, int64_t nadc, int32_t nc, const cplx<
     const uint64_t bits = reinterpret_cast<uintptr_t>(states) | reinterpret_cast<uintptr_t>(csm) |
                           (uint64_t)ldstates * sizeof(cplx<T>) | (uint64_t)ldcsm * sizeof(cplx<T>);
     const int width = (bits & 15) == 0 ? 16 : (bits & 7) == 0 ? 8 : 4;
+    cudaError_t e = cudaErrorInvalidValue;
 #define CR_CASE(NT_, WJ_) \
     if (nt == NT_ && wj == WJ_) \
-        return cr_launch<T, NT_, WJ_>(grid, ns, nadc, nc, states, ldstates, csm, ldcsm, width, partial, stream);
+        e = cr_launch<T, P, NT_, WJ_>(grid, ns, nadc, nc, states, ldstates, csm, ldcsm, width, partial, stream);
     CR_CASE(1, 2) CR_CASE(1, 4) CR_CASE(1, 8)
     CR_CASE(2, 2) CR_CASE(2, 4) CR_CASE(2, 8)
     CR_CASE(4, 2) CR_CASE(4, 4) CR_CASE(4, 8)
 #undef CR_CASE
+    return e != cudaSuccess ? e : launch_partial_finalize(partial, parts, nadc, nc, sig, ldsig, stream);
+}
+
+template <typename T>
+cudaError_t launch_coil_reduce(const CoilReduceCut &cut, int64_t ns, int64_t nadc, int32_t nc, const cplx<T> *states,
+                               int64_t ldstates, const cplx<T> *csm, int64_t ldcsm, void *partial, cplx<T> *sig,
+                               int64_t ldsig, cudaStream_t stream) {
+    if (ns == 0 || nadc == 0 || nc == 0) return cudaSuccess;
+    if (cut.wide)
+        return cr_run<T, double>(cut.parts, ns, nadc, nc, states, ldstates, csm, ldcsm,
+                                 static_cast<cplx<double> *>(partial), sig, ldsig, stream);
+    if constexpr (sizeof(T) == 4)
+        return cr_run<T, float>(cut.parts, ns, nadc, nc, states, ldstates, csm, ldcsm,
+                                static_cast<cplx<float> *>(partial), sig, ldsig, stream);
     return cudaErrorInvalidValue;
+}
+
+// Load every kernel of the reduction and of its partial sums on the current device
+// (the driver loads a kernel, and may allocate for it, at its first use).
+template <typename T, typename P>
+static cudaError_t load_reduce_kernels() {
+    const void *const kernels[] = {
+        (const void *)coil_reduce_kernel<T, P, 1, 2>, (const void *)coil_reduce_kernel<T, P, 1, 4>,
+        (const void *)coil_reduce_kernel<T, P, 1, 8>, (const void *)coil_reduce_kernel<T, P, 2, 2>,
+        (const void *)coil_reduce_kernel<T, P, 2, 4>, (const void *)coil_reduce_kernel<T, P, 2, 8>,
+        (const void *)coil_reduce_kernel<T, P, 4, 2>, (const void *)coil_reduce_kernel<T, P, 4, 4>,
+        (const void *)coil_reduce_kernel<T, P, 4, 8>, (const void *)partial_finalize_kernel<P, T, 8>,
+        (const void *)partial_finalize_kernel<P, T, 32>};
+    for (const void *k : kernels) {
+        cudaFuncAttributes a;
+        const cudaError_t e = cudaFuncGetAttributes(&a, k);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+cudaError_t load_coil_reduce() {
+    cudaError_t e = load_reduce_kernels<double, double>();
+    if (e == cudaSuccess) e = load_reduce_kernels<float, float>();
+    return e != cudaSuccess ? e : load_reduce_kernels<float, double>();
 }
 
 template cudaError_t launch_excitation<double>(const PhantomDev<double> &, const SeqDev<double> &, StateDev<double> &,
@@ -788,10 +832,12 @@ template cudaError_t launch_partial_finalize<float, float>(const cplx<float> *, 
                                                            cplx<float> *, int64_t, cudaStream_t);
 template cudaError_t launch_partial_finalize<double, float>(const cplx<double> *, int64_t, int64_t, int32_t,
                                                             cplx<float> *, int64_t, cudaStream_t);
-template cudaError_t launch_coil_reduce<double>(int64_t, int64_t, int32_t, const cplx<double> *, int64_t,
-                                                const cplx<double> *, int64_t, cplx<double> *, cudaStream_t);
-template cudaError_t launch_coil_reduce<float>(int64_t, int64_t, int32_t, const cplx<float> *, int64_t,
-                                               const cplx<float> *, int64_t, cplx<float> *, cudaStream_t);
+template cudaError_t launch_coil_reduce<double>(const CoilReduceCut &, int64_t, int64_t, int32_t, const cplx<double> *,
+                                                int64_t, const cplx<double> *, int64_t, void *, cplx<double> *, int64_t,
+                                                cudaStream_t);
+template cudaError_t launch_coil_reduce<float>(const CoilReduceCut &, int64_t, int64_t, int32_t, const cplx<float> *,
+                                               int64_t, const cplx<float> *, int64_t, void *, cplx<float> *, int64_t,
+                                               cudaStream_t);
 template size_t segment_smem_bytes<double>(int32_t);
 template size_t segment_smem_bytes<float>(int32_t);
 

@@ -49,3 +49,32 @@ def test_tiles_and_alignment(gpu_context, precision, offset, pad, nspins, nadc, 
     bound = 5e-13 if precision == "f64" else 5e-6
     assert np.linalg.norm(got[:, :nadc].T - ref) <= bound * math.sqrt(nspins * nadc * nc)
     assert np.all(got[:, nadc:] == 7 - 3j)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("nspins,nadc,nc", [(63, 33, 9), (65, 33, 9), (8001, 64, 32), (37_888, 7, 3), (37_889, 7, 3),
+                                            (75_776, 33, 17), (75_777, 33, 17), (60_000, 100, 3)])
+def test_parts(gpu_context, precision, nspins, nadc, nc):
+    """Both sides of the lines between parts of 256 spins (FP32 partial sums for FP32
+    operands) and more parts with FP64 partial sums; the entry without allocation
+    computes the same bits."""
+    import torch
+    rng = np.random.default_rng(12)
+    ct = np.complex128 if precision == "f64" else np.complex64
+    code = _lib.HOMS_F64 if precision == "f64" else _lib.HOMS_F32
+    states, csm = ((rng.standard_normal((nspins, n)) + 1j * rng.standard_normal((nspins, n))).astype(ct)
+                   for n in (nadc, nc))
+    (ks, ps), (kc, pc) = _column_major(states, 0, nspins), _column_major(csm, 0, nspins)
+    sig = [torch.zeros(nc, nadc, dtype=torch.complex128 if precision == "f64" else torch.complex64, device="cuda")
+           for _ in range(2)]
+    torch.cuda.synchronize()
+    args = [(code, nspins, nadc, nc, ctypes.c_void_p(ps), nspins, ctypes.c_void_p(pc), nspins,
+             ctypes.c_void_p(s.data_ptr()), nadc) for s in sig]
+    _lib.check(_lib.load().homs_coil_reduce(gpu_context.handle, *args[0]), gpu_context.handle)
+    _lib.check(_lib.load().homs_coil_reduce_noalloc(None, *args[1]), gpu_context.handle)
+    torch.cuda.synchronize()
+    got = sig[0].cpu().numpy()
+    ref = states.astype(np.complex128).T @ csm.astype(np.complex128)
+    bound = 5e-13 if precision == "f64" else 5e-6
+    assert np.linalg.norm(got.T - ref) <= bound * math.sqrt(nspins * nadc * nc)
+    assert np.array_equal(got, sig[1].cpu().numpy())
